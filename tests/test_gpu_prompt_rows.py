@@ -1,0 +1,41 @@
+"""Row kernels of prompt chunks against the single-token path they restate."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _bf(pkg, a):
+    return pkg.f32_to_bf16(np.ascontiguousarray(a, dtype=np.float32))
+
+
+@pytest.mark.parametrize("kernel", [1, 2, 3, 8])
+@pytest.mark.parametrize("dim", [64, 62, 320])
+def test_conv_over_a_chunk_is_the_repeated_single_step(pkg, kernel, dim):
+    """Portions around the run length and the kernel size, carried from one to the next: the state is the same bits as token by
+    token (bit-exact against the reference's known answers elsewhere), and so is the last token's output up to the order of the
+    sums in the head's product. 62 channels do not divide into the vector form."""
+    P, vocab, width, bcx = pkg.plan, 512, (dim + 63) // 64 * 64, (3 * dim + 7) // 8 * 8
+    rng = np.random.default_rng(7 * kernel + dim)
+    desc = pkg.BuffersDesc(hidden=width, slot_dim=3 * width, vocab=vocab, max_seq=256, max_batch=1, conv_layers=1, conv_dim=dim, conv_kernel=kernel)
+    store = pkg.WeightStore(0)
+    store.add_dense("rows", _bf(pkg, rng.normal(size=(vocab, width))))
+    store.add_dense("bcx", _bf(pkg, rng.normal(size=(vocab, bcx))))
+    store.add_dense("taps", _bf(pkg, rng.normal(size=(dim, kernel))))
+    store.add_dense("norm", _bf(pkg, np.ones(width)))
+    store.add_q4_mlx("head", *pkg.synth_q4(vocab, width, seed=5, centered=True))
+    steps = [P._step(P.STEP_EMBED, out_buf=P.BUF_HIDDEN, n=width, weight="rows"), P._step(P.STEP_EMBED, out_buf=P.BUF_S1, n=bcx, weight="bcx"),
+             P._step(P.STEP_CONV_STATE_UPDATE, layer=0, in_buf=P.BUF_S1, out_buf=P.BUF_HIDDEN, n=dim, conv_kernel=kernel, weight="taps"),
+             P._step(P.STEP_COPY_RMSNORM, in_buf=P.BUF_HIDDEN, out_buf=P.BUF_S0, n=width, eps=1e-5, weight="norm"),
+             P._step(P.STEP_QGEMV, in_buf=P.BUF_S0, out_buf=P.BUF_LOGITS, n=vocab, k=width, weight="head"),
+             P._step(P.STEP_ARGMAX, in_buf=P.BUF_LOGITS, n=vocab)]
+    chunked, single = pkg.InferenceModel(store, steps, desc), pkg.InferenceModel(store, steps, desc)
+    single.set_prefill_chunk(0)
+    for n in (1, 3, 16, 33, 2, 47):
+        tokens = rng.integers(0, vocab, size=n)
+        chunked.prefill_sequence(0, tokens)
+        single.prefill(tokens[None])
+        assert np.array_equal(chunked.read_conv(0, 0), single.read_conv(0, 0))
+        got, ref = pkg.bf16_to_f32(chunked.logits()), pkg.bf16_to_f32(single.logits())
+        assert np.abs(got - ref).max() <= 1e-2 * np.abs(ref).max()   # one bf16 rounding (2^-9 of the largest) on either side
+    chunked.close(), single.close(), store.close()
