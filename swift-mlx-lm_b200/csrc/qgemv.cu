@@ -1159,6 +1159,9 @@ int qgemv_counter_count(const Q4Tiled& w) { return w.row_tiles; }
 static int build_params(const QGemvLaunch& a, QGemvParams& p, QGemvConfig& c);
 
 int launch_qgemv(const QGemvLaunch& a, cudaStream_t s) {
+    // few rows: the kernel with the activations in registers; the one below is left with what carries a fused norm or an exchange
+    // between ranks (tensor parallelism) and with rows longer than 32768
+    if (!a.norm.mode && !a.push && !a.in_tp && qgemv_rows_takes(*a.w, a.m)) return launch_qgemv_rows(a, s);
     QGemvParams p{};
     QGemvConfig c{};
     int rc = build_params(a, p, c);

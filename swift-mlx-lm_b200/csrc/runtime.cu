@@ -404,6 +404,9 @@ int compile_plan(swlm_plan* plan) {
         Launch& B = plan->launches[i + 1];
         if (A.kind != L_RMSNORM || B.kind != L_QGEMV) continue;
         if (B.st.in_buf != A.st.out_buf || B.w->k != A.st.n || A.st.n > 4096 || (A.st.n & 15)) continue;
+        // several rows: a norm of its own (a few us on one CTA per row) is cheaper than every CTA of the product reading and
+        // norming all rows (16 rows of 4096: 74 us for the gate/up product with the norm in it, about 31 us for the two launches)
+        if (ctx->tp_size == 1 && m > 1 && qgemv_rows_takes(*B.w, m)) continue;
         bool ok = true;
         for (int q = 0; q < B.n_seg; ++q) ok &= B.seg_buf[q] != A.st.in_buf && B.seg_buf[q] != SWLM_BUF_RESIDUAL;
         for (size_t j = i + 2; j < plan->launches.size() && ok; ++j) {
@@ -1289,6 +1292,7 @@ int swlm_ctx_create(int device_id, int tp_rank, int tp_size, swlm_ctx** out) {
     cudaError_t e = cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking);
     if (e != cudaSuccess) { delete ctx; return cuda_fail(e, "cudaStreamCreate"); }
     int rc = qgemv_init();
+    if (!rc) rc = qgemv_rows_init();
     if (!rc) rc = attn_init();
     if (!rc) rc = qgemm_tc_init();
     if (!rc) rc = bgemm_init();

@@ -205,6 +205,10 @@ struct QGemvLaunch {
 size_t qgemv_scratch_floats(const Q4Tiled& w, int m);
 int qgemv_counter_count(const Q4Tiled& w);
 int launch_qgemv(const QGemvLaunch& a, cudaStream_t s);
+// 2..16 rows without a fused norm or an exchange (qgemv_rows.cu); launch_qgemv goes there by itself
+int qgemv_rows_init();
+bool qgemv_rows_takes(const Q4Tiled& w, int m);
+int launch_qgemv_rows(const QGemvLaunch& a, cudaStream_t s);
 // SWLM_TRACE=1: slot for the phase timestamps of one launch (nullptr when tracing is off or the slots are used up)
 unsigned long long* qgemv_trace_slot(int ctas, int row_tiles, int kt4, int epi, int norm);
 int qgemv_init();  // sets shared-memory attributes once per process
