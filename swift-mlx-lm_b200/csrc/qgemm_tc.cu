@@ -1,355 +1,587 @@
-// Q4 group-64 prefill GEMM for sm_100a on the 5th-generation tensor cores (tcgen05 / TMEM).
+// Q4 group-64 products of 17 and more activation rows for sm_100a on the 5th-generation tensor cores (tcgen05 / TMEM).
 //
-// Replaces the reference's `gemm_q4_g64` for M >= 64 (Generator/MetalSourceGenerator+Quantized.swift:88-156,
-// which repeats the per-row dot product for every sequence position and so re-reads the weights M times)
-// with a real contraction whose result equals the fp32-weight product up to the order of the fp32 sums. The weight
-// is split as scale*q + zero = scale*(q - 8) + (zero + 8*scale): |q - 8| <= 8 has at most three significant bits (or
-// is a power of two) and a bf16 or fp16 scale at most eleven, so scale*(q - 8) is EXACT in fp16 and is the A operand;
-// the second term is constant over a group of 64 and multiplies the group's sum of activations, which becomes three
-// extra K-columns per group appended after the real ones (c_hi x sum_hi, c_lo x sum_hi, c_hi x sum_lo, fp16 pairs
-// that carry 22 bits). tcgen05.mma kind::f16 wants both operands in one format (fp16 weights against bf16 activations
-// is an illegal instruction on this part), so a small kernel first copies the activations to fp16, every token row
-// times a power of two that puts its largest magnitude at 2^14 (exact for every element within 2^-28 of the row's
-// largest, immune to fp16's range, undone per token in the epilogue), and appends the per-group sums. (A dequantised
-// weight rounded to 16 bits, the reference's dequantise-then-matmul route of +Quantized.swift:361-416, does not hold
-// 1e-2 per output against `gemm_q4_g64`: bf16 weights leave outputs a tenth of the typical magnitude 1-5 % off,
-// fp16 weights 1 %.)
+// Replaces the reference's `gemm_q4_g64` (Generator/MetalSourceGenerator+Quantized.swift:88-156, which repeats the per-row dot
+// product for every sequence position and so re-reads the weights M times) with a real contraction whose result equals the
+// fp32-weight product up to the order of the fp32 sums. The weight is split as scale*q + zero = scale*(q - 8) + (zero + 8*scale):
+// |q - 8| <= 8 has at most three significant bits (or is a power of two) and a bf16 scale at most eight (an fp16 one eleven), so
+// scale*(q - 8) is EXACT in fp16 for bf16 scales and is the A operand; the second term is constant over a group of 64 and
+// multiplies the group's sum of activations, which becomes three extra K-columns per group appended after the real ones
+// (c_hi x sum_hi, c_lo x sum_hi, c_hi x sum_lo, fp16 pairs that carry 22 bits). Both operands of tcgen05.mma kind::f16 have the
+// same type, so a small kernel first copies the activations to fp16, every row times a power of two that puts its largest
+// magnitude at 2^14 (exact for every element within 2^-28 of the row's largest, immune to fp16's range, undone in the epilogue),
+// and appends the per-group sums. (A dequantised weight rounded to 16 bits, the reference's dequantise-then-matmul route of
+// +Quantized.swift:361-416, does not hold 1e-2 per output against `gemm_q4_g64`.)
 //
-// One CTA (18 warps) computes a 128 (weight rows) x BN (tokens) tile of Y^T:
-//   * a TMA warp (one thread) keeps a ring of stages full, two cp.async.bulk.tensor.2d per 64-column group
-//     (every CTA fetches its own copy): the packed weights of the group (128 rows x 32 bytes) and the activation tile (BN tokens
-//     x 64 columns of fp16, 128-byte swizzle, rows past the last token filled with zeros); an mbarrier per
-//     stage counts the bytes;
-//   * 16 warps dequantise: four threads own one weight row, per group each reads 8 packed bytes from shared
-//     memory, takes the row's (scale, zero) from registers (fetched eight groups at a time), turns nibble
-//     pairs into fp16 with LOP3 (1024+q), subtracts 1032 and multiplies by the scale with one f16x2 instruction
-//     each — scale*(q - 8), exact — and stores its 16 values into the row's lane of tensor memory
-//     (tcgen05.st): the A operand of the MMA is read from TMEM, so the dequantised weights never cross shared
-//     memory and four such tiles (32 columns each) fit beside the accumulator;
-//   * an MMA warp (one thread) issues four tcgen05.mma (M=128, N=BN, K=16, kind::f16, A from TMEM, B through
-//     a shared-memory descriptor, fp32 accumulator in TMEM) per group as soon as the group's weights and
-//     activations are in place; tcgen05.commit signals an mbarrier when the stage and the weight tile may
-//     be overwritten;
-//   * the epilogue reads the accumulator with tcgen05.ld, rounds to bf16 and stores Y[token][row].
-// Every mbarrier wait is bounded: on expiry an error word is set, the CTA stops issuing, waits (bounded) for
-// the copies it has in flight, frees its TMEM and returns.
+// A step of the pipeline is 128 columns of K (two groups). Roles:
+//   * a TMA thread keeps a ring of stages full of activations (128 fp16 per row, two 128-byte-swizzled halves);
+//   * 16 warps dequantise, each one 16 x 64 tile of the streaming layout per step, through a cp.async ring of its own; nibble pairs to fp16 with LOP3 (1024 + q or 1024 + 16 q), one subtraction and one multiplication of
+//     fp16 pairs; what falls out is the A fragment of mma.m16n8k16, which tcgen05.st.16x256b puts into tensor memory as it is:
+//     the copy of the activations has its columns in the same order. The A operand is read from TMEM;
+//   * one thread issues eight tcgen05.mma (K = 16) per step; tcgen05.commit frees stage and weight tile;
+//   * epilogue: tcgen05.ld, undo the row's power of two, round once to bf16, Y[token][row]; or gate and up rows of the interleaved
+//     layout together, activated.
+// The long form (many rows) pairs two SMs: 256 weight rows x 256 activation rows per tile, each CTA dequantises its 128 weight
+// rows and fetches half of the activations.
+//
+// What bounded the kernel this one replaced (one group per step, weights by TMA as 128 rows of 32 bytes, one tile per CTA): the L2
+// traffic of 256 activation rows per 128 weight rows (with seven of eight MMAs left out 2048 x 28672 x 4096 still took 411 of
+// 509 us, 10.7 TB/s), 512 arrivals per group, eight MMAs issued by a lone lane (470 to 850 clocks), and two waves of CTAs, the second
+// half empty. What bounds it now: the MMAs of the long form (about 0.65 of their rate under the power cap), dequantising in the short one.
+// Measured: 14336 x 4096 at 512 rows 88 -> 63 us (950 TFLOP/s); 28672 x 4096 at 2048 rows 705 us under ncu -> 442 us (1090 TFLOP/s);
+// 28672 x 4096 at 41 rows 68 us under ncu -> 38 us; 14336 -> 4096 at 41 rows 50.7 + 8.8 (a second launch) -> 30 us.
+//
+// Every mbarrier wait is bounded: on expiry an error word is set, the CTA stops issuing, waits (bounded) for the copies and MMAs
+// it has in flight, frees its TMEM and returns.
+#include <algorithm>
 #include <cstdlib>
+
+#include <cooperative_groups.h>
 #include <cuda.h>
+
 #include "swlm_internal.h"
 #include "tc_device.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace swlm {
 namespace {
 
-constexpr int kTcThreads = 512;          // dequantising threads
-constexpr int kTcAllThreads = kTcThreads + 64;  // + the MMA warp and the activation (TMA) warp
-constexpr int kTcRows = 128;            // weight rows per CTA = UMMA M
-constexpr int kTcBK = 64;               // one quantisation group per pipeline stage
+constexpr int kTcRows = 128;             // weight rows per CTA = lanes of tensor memory
+constexpr int kTcStep = 128;             // columns of K per pipeline step
+constexpr int kTcDeqWarps = 16;
+constexpr int kTcMaxA = 4;               // dequantised weight tiles in flight at most, 64 columns of TMEM each
+constexpr int kTcSet = kTcDeqWarps / 2;  // they take turns: half of them dequantise the even steps, the others the odd ones
+constexpr int kTcAhead = 3;              // ring of a dequantising warp: steps of its own whose weights it has requested
+constexpr int kTcSlotBytes = 1024 + 128; // two 16 x 64 tiles and their 16 times two scale / zero pairs
+constexpr int kTcRingBytes = kTcDeqWarps * kTcAhead * kTcSlotBytes;
+constexpr int kTcEpiWarps = 8;           // long form: warps that only store results
 
 struct QGemmTcParams {
-    const uint32_t* w;        // [n][k/8] MLX words
-    const uint16_t* scales;   // [n][k/64] bf16
-    const uint16_t* biases;
-    int n, k;
-    const __half* x;          // [m][x_stride]: the activations as fp16, every token row scaled by a power of two
-    const float* rscale;      // [m]: the inverse of each row's scale
-    int x_stride, m;
-    int ext_steps;            // 64-column steps of appended group-sum columns (three planes of ceil(k/64/64) steps)
+    const uint4* tiles;       // [row tile][k-tile][32 lanes], see Q4Tiled
+    const unsigned* sb;       // [row tile][k-tile / 4][16 rows][4] pairs
+    int row_tiles, kt;        // row tiles, k-tiles (groups of 64, a multiple of four)
+    int g_pad;                // columns of one plane of appended group sums
+    const float* rscale;      // [m]: the inverse of each row's power of two
+    int m;
+    int real_steps, steps;    // steps over the weights; those over the appended columns follow
+    int tok_tiles, n_tiles;   // long form: tiles of 256 rows, all tiles
+    int splits;               // short form: CTAs of a cluster along K
+    int gated, gated_act;     // rows 0-7 of a row tile are gate rows, rows 8-15 the up rows that belong to them
     TcSegments out;           // weight rows [end[q-1], end[q]) go to out.y[q][token][row - end[q-1]]
     int* status;              // set non-zero when a bounded wait expired
-    // launches of at most 64 token rows over few weight rows: K is cut into gridDim.z ranges of `split_steps` groups
-    // (a multiple of 8) so that more SMs take part; every range writes its fp32 sums to part[z][m][n] and a second
-    // launch adds the ranges in order. The last range also takes the appended group-sum steps.
-    float* part;
-    int split_steps;
 };
 
-// Instruction descriptor for kind::f16: D = fp32, A = B = fp16 (format 0), both K-major, M = 128, N = BN.
-__host__ __device__ constexpr unsigned umma_idesc(int bn) {
-    return (1u << 4) | (0u << 7) | (0u << 10) | ((unsigned)(bn >> 3) << 17) | ((unsigned)(kTcRows >> 4) << 24);
+// Instruction descriptor for kind::f16: D = fp32, A = B = fp16 (format 0), both K-major, M rows, N = BN.
+__host__ __device__ constexpr unsigned umma_idesc(int m, int bn) {
+    return (1u << 4) | (0u << 7) | (0u << 10) | ((unsigned)(bn >> 3) << 17) | ((unsigned)(m >> 4) << 24);
 }
-
-// D[tmem] (+)= A[tmem] x B[shared memory]: the A operand (128 rows x 16 bf16 = 8 columns of 32 bits) is read from
-// tensor memory, where the dequantising threads put it, so it never crosses shared memory
-__device__ __forceinline__ void umma_f16_ta(unsigned d_tmem, unsigned a_tmem, unsigned long long b_desc, unsigned idesc, unsigned accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-        ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
+// D[tmem] (+)= A[tmem] x B[shared memory]; CG = 2: the rows of A and D and those of B lie half in either CTA of the pair
+template <int CG>
+__device__ __forceinline__ void umma_f16_ta(unsigned d_tmem, unsigned a_tmem, unsigned b_desc_lo, unsigned idesc, unsigned accumulate) {
+    if (CG == 1)
+        asm volatile("{\n\t.reg .pred p;\n\t.reg .b64 d;\n\tsetp.ne.b32 p, %5, 0;\n\tmov.b64 d, {%2, %3};\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], [%1], d, %4, p;\n\t}"
+                     ::"r"(d_tmem), "r"(a_tmem), "r"(b_desc_lo), "r"(kUmmaDescHi), "r"(idesc), "r"(accumulate) : "memory");
+    else
+        asm volatile("{\n\t.reg .pred p;\n\t.reg .b64 d;\n\tsetp.ne.b32 p, %5, 0;\n\tmov.b64 d, {%2, %3};\n\ttcgen05.mma.cta_group::2.kind::f16 [%0], [%1], d, %4, p;\n\t}"
+                     ::"r"(d_tmem), "r"(a_tmem), "r"(b_desc_lo), "r"(kUmmaDescHi), "r"(idesc), "r"(accumulate) : "memory");
+}
+// arrival at the same barrier of both CTAs of a pair when the MMAs issued so far are done
+__device__ __forceinline__ void umma_commit_pair(unsigned long long* bar) {
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
+                 ::"r"(smem_u32(bar)), "h"((unsigned short)3) : "memory");
 }
 // One result, rounded once to bf16, to the output its weight row belongs to.
 __device__ __forceinline__ void tc_store(const TcSegments& o, int token, int row, float val) {
-    const int q = row < o.end[0] ? 0 : row < o.end[1] ? 1 : 2;
-    const int first = q == 0 ? 0 : o.end[q - 1];
-    o.y[q][(size_t)token * o.stride[q] + (row - first)] = __float2bfloat16_rn(val);
+    const __nv_bfloat16 v = __float2bfloat16_rn(val);
+    if (row < o.end[0]) o.y[0][(size_t)token * o.stride[0] + row] = v;
+    else if (row < o.end[1]) o.y[1][(size_t)token * o.stride[1] + (row - o.end[0])] = v;
+    else if (row < o.end[2]) o.y[2][(size_t)token * o.stride[2] + (row - o.end[1])] = v;
+}
+// A gate row's and its up row's result: both are rounded to bf16 first because the reference stores them to bf16 scratch before
+// `swiglu` reads them (Primitives/ElementwiseFragment.swift:49-54).
+__device__ __forceinline__ void tc_store_gated(const QGemmTcParams& p, int token, int row, float gate, float up) {
+    if (row < p.out.end[0])
+        p.out.y[0][(size_t)token * p.out.stride[0] + row] = __float2bfloat16_rn(gated_activation(
+            __bfloat162float(__float2bfloat16_rn(gate)), __bfloat162float(__float2bfloat16_rn(up)), p.gated_act));
+}
+__device__ __forceinline__ void tmem_ld16(unsigned addr, unsigned (&v)[16]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
+                   "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+                 : "r"(addr) : "memory");
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+// 16 lanes x 32 columns in the order of four m16n8 accumulator fragments: lane (g, t), register 4 i + r: row g + 8 (r >> 1),
+// column 8 i + 2 t + (r & 1)
+__device__ __forceinline__ void tmem_st_frag(unsigned addr, const unsigned (&v)[16]) {
+    asm volatile("tcgen05.st.sync.aligned.16x256b.x4.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
+                 ::"r"(addr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]), "r"(v[10]),
+                   "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]) : "memory");
+}
+__device__ __forceinline__ unsigned pair_leader(unsigned addr) {   // the same shared-memory place in the cluster's first CTA
+    unsigned r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(r) : "r"(addr));
+    return r;
+}
+template <int CG>
+__device__ __forceinline__ void tc_arrive(unsigned bar) {   // CG = 2: `bar` is a cluster address
+    if (CG == 1) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+    else asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");   // (with a release of cluster scope an arrival takes 1200 clocks)
 }
 
-// F16SB: scale and zero are fp16 (tensors uploaded as STAF blocks) instead of bf16 (MLX tensors).
-//
-// Dequantising thread (warp w, lane l): weight row 32 (w & 3) + l (= its TMEM lane), columns 16 (w >> 2) ..
-// + 15 of every group. ready_bar[kt % SA] collects the 512 arrivals of group kt; full_bar[kt % SB] completes
-// when the group's stage has landed; empty_bar[kt % SB] when its MMAs are done. With SA = 2 the dequantisation
-// of group kt had to wait for the MMAs of group kt - 2 (measured: 200 clocks per group); SA = 4 removes that.
-template <int BN, int STAGES, bool F16SB>
-__global__ void __launch_bounds__(kTcAllThreads) qgemm_tc_kernel(const QGemmTcParams p, const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap wmap) {
-    constexpr int SA = BN == 64 ? 2 : 4, SB = STAGES;   // dequantised weight tiles in flight
-    constexpr unsigned kTmemCols = BN == 256 ? 512 : BN == 128 ? 256 : 128;   // accumulator (BN) + SA weight tiles of 32, power of two
-    constexpr unsigned kACol0 = BN;                                            // first column of the weight tiles
-    static_assert(SB >= 3, "the activation ring must be deeper than the weight ring");
-    extern __shared__ __align__(1024) unsigned char smem_raw[];
-    // 1024-byte alignment for the swizzle atoms
-    unsigned char* smem = smem_raw + ((1024 - (smem_u32(smem_raw) & 1023)) & 1023);
-    constexpr int B_BYTES = BN * 128;
-    constexpr int W_BYTES = kTcRows * 32;        // packed weights of one group
-    constexpr int STAGE_BYTES = B_BYTES + W_BYTES;
-    __shared__ __align__(8) unsigned long long empty_bar[STAGES];
-    __shared__ __align__(8) unsigned long long full_bar[STAGES];    // the activation tile of a stage has landed
-    __shared__ __align__(8) unsigned long long ready_bar[4];   // a weight tile and its activation tile are in place
-    __shared__ __align__(8) unsigned long long done_bar;
-    __shared__ unsigned tmem_base_smem;
-    __shared__ int failed;
+// A ring position and the parity of its phase.
+template <int N>
+struct RingPos {
+    int s = 0; unsigned par = 0;
+    __device__ __forceinline__ void next() { if (++s == N) { s = 0; par ^= 1u; } }
+    __device__ __forceinline__ void skip2() { s += 2; if (s >= N) { s -= N; par ^= 1u; } }
+};
 
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int r = (warp & 3) * 32 + lane, part = (warp >> 2) & 3;   // TMEM lane = weight row; part: which 16 of the group's 64 columns
-    const int row0 = blockIdx.x * kTcRows, tok0 = blockIdx.y * BN;
-    const int kt_total = p.k / kTcBK;
-    // this CTA's range of groups [kt_lo, kt_lo + real_steps) and, for the last range, the appended group-sum columns
-    const int kt_lo = gridDim.z > 1 ? (int)blockIdx.z * p.split_steps : 0;
-    const int real_steps = gridDim.z > 1 ? min(p.split_steps, kt_total - kt_lo) : kt_total;
-    const int ext_steps = blockIdx.z == gridDim.z - 1 ? p.ext_steps : 0;
-    const int steps_total = real_steps + ext_steps;
-    unsigned char* const b_ring = smem;
+template <int STAGES>
+struct TcBars {
+    unsigned long long full[STAGES], empty[STAGES];   // a stage has landed; its MMAs are done
+    unsigned long long ready[kTcMaxA];                 // a weight tile is in tensor memory (one arrival per dequantising warp)
+    unsigned long long acc_full, acc_empty;           // accumulator complete; read (long kernel)
+    unsigned tmem;
+    int failed;
+};
 
-    if (tid == 0) {
+// Common start: barriers and tensor memory. Ends with all threads (of the pair) synchronised.
+template <int STAGES, unsigned COLS, int CG>
+__device__ __forceinline__ unsigned tc_setup(TcBars<STAGES>& b) {
+    if (threadIdx.x == 0) {
 #pragma unroll
-        for (int s = 0; s < STAGES; ++s) { mbar_init(&empty_bar[s], 1); mbar_init(&full_bar[s], 1); }
-        for (int i = 0; i < 4; ++i) mbar_init(&ready_bar[i], kTcThreads);
-        mbar_init(&done_bar, 1);
-        failed = 0;
+        for (int s = 0; s < STAGES; ++s) { mbar_init(&b.empty[s], 1); mbar_init(&b.full[s], 1); }
+#pragma unroll
+        for (int i = 0; i < kTcMaxA; ++i) mbar_init(&b.ready[i], kTcSet * CG);
+        mbar_init(&b.acc_full, 1);
+        mbar_init(&b.acc_empty, kTcEpiWarps * CG);
+        b.failed = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == 0) {
+    if (threadIdx.x < 32) {
         __syncwarp();  // the allocation is a warp-wide instruction: re-converge after the single-thread block
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_smem)), "r"(kTmemCols) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        if (CG == 1) {
+            asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&b.tmem)), "r"(COLS) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        } else {
+            asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&b.tmem)), "r"(COLS) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+        }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
+    if (CG == 2) cg::this_cluster().sync();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const unsigned tmem_d = tmem_base_smem;
+    return b.tmem;
+}
+__device__ __forceinline__ void tc_fail(int* status, int* failed, int code) { atomicExch(status, code); *reinterpret_cast<volatile int*>(failed) = 1; }
 
-    const int row = row0 + r;
-    const bool row_ok = row < p.n;
-    const uint16_t* srow = p.scales + (size_t)(row_ok ? row : 0) * kt_total;
-    const uint16_t* zrow = p.biases + (size_t)(row_ok ? row : 0) * kt_total;
-    constexpr unsigned idesc = umma_idesc(BN);
+// ---- producer: a step's activations (`rows` rows of shared memory) into a stage ---------------------------------------------
+template <int ROWS>
+__device__ __forceinline__ void tc_issue(const CUtensorMap* xmap, unsigned stage, unsigned bar, int kt, int tok0) {
+    mbar_expect(bar, (unsigned)ROWS * 256u);
+    tma_load_2d(stage, xmap, kt * kTcStep, tok0, bar);
+    tma_load_2d(stage + ROWS * 128, xmap, kt * kTcStep + 64, tok0, bar);
+}
+// ---- the eight MMAs of a step; ROWS: activation rows in this CTA's shared memory ----------------------------------------------
+template <int CG, int ROWS>
+__device__ __forceinline__ void tc_mma_step(unsigned d_tmem, unsigned a_tmem, unsigned stage, bool first) {
+    const unsigned lo = umma_desc_lo(stage);
+#pragma unroll
+    for (int j = 0; j < kTcStep / 16; ++j)   // 16 fp16 = 8 columns of A, 32 bytes along K inside B's 128-byte row
+        umma_f16_ta<CG>(d_tmem, a_tmem + 8u * j, lo + (j >> 2) * (ROWS * 8) + 2 * (j & 3), umma_idesc(kTcRows * CG, ROWS * CG), j > 0 ? 1u : first ? 0u : 1u);
+}
 
-    // scales and zeros of groups kt0..kt0+7 of this thread's row (16-bit each), one 16-byte load each when the
-    // rows are 16-byte aligned; they do not depend on the preceding kernel
-    const bool sz_vec = (kt_total & 7) == 0;
-    auto load8 = [&](const uint16_t* rowp, int kt0) {
-        uint4 v = make_uint4(0, 0, 0, 0);
-        if (!row_ok || kt0 >= kt_total) return v;
-        if (sz_vec) return __ldg(reinterpret_cast<const uint4*>(rowp + kt0));
-        unsigned h[8];
+// ---- dequantising warps: warp w takes row tile 2 (w & 3) + ((w >> 2) & 1) of the eight of the CTA's rows (its lanes of tensor
+// memory) in every other step ---------------------------------------------------------------------------------
+template <bool F16SB>
+__device__ __forceinline__ float tc_scale(unsigned pair) { return F16SB ? __half2float(__ushort_as_half((unsigned short)(pair & 0xFFFFu))) : __uint_as_float(pair << 16); }
+template <bool F16SB>
+__device__ __forceinline__ float tc_zero(unsigned pair) { return F16SB ? __half2float(__ushort_as_half((unsigned short)(pair >> 16))) : __uint_as_float(pair & 0xFFFF0000u); }
+// the scale as an fp16 pair: a bf16 (MLX) scale converts exactly (8 mantissa bits into 11) unless it lies below fp16's normal range,
+// where the weights it scales are nil anyway
+template <bool F16SB>
+__device__ __forceinline__ __half2 tc_scale2(unsigned pair) {
+    if (F16SB) { const unsigned v = __byte_perm(pair, 0, 0x1010); return *reinterpret_cast<const __half2*>(&v); }
+    return __float2half2_rn(__uint_as_float(pair << 16));
+}
+// 16 x 64 nibbles -> scale * (q - 8) in fragment order; the low nibble of each byte is row g, the high one row g + 8
+__device__ __forceinline__ void tc_unpack(const uint4& wq, __half2 lo, __half2 hi, unsigned (&a)[16]) {
+    const unsigned w[4] = {wq.x, wq.y, wq.z, wq.w};
+    const unsigned c1032 = 0x64086408u, c16th = 0x2C002C00u, c72 = 0xD480D480u;   // 1024 + 8; 1 / 16; -(64 + 8)
+    const __half2 off = *reinterpret_cast<const __half2*>(&c1032), sixteenth = *reinterpret_cast<const __half2*>(&c16th), off16 = *reinterpret_cast<const __half2*>(&c72);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) h[j] = kt0 + j < kt_total ? (unsigned)__ldg(rowp + kt0 + j) : 0u;
-        return make_uint4(h[0] | (h[1] << 16), h[2] | (h[3] << 16), h[4] | (h[5] << 16), h[6] | (h[7] << 16));
-    };
-    auto pick16 = [](const uint4& v, int j) {  // 16-bit element j (0..7)
-        const unsigned lo = (j & 2) ? v.y : v.x, hi = (j & 2) ? v.w : v.z;
-        const unsigned w = (j & 4) ? hi : lo;
-        return (j & 1) ? w >> 16 : w & 0xFFFFu;
-    };
-    if (warp == kTcThreads / 32) {
-        // ---- MMA warp: one thread issues the four MMAs of a group as soon as its tiles are in place; the
-        // dequantising warps are already busy with the next group by then -----------------------------------
-        if (lane == 0) {
-            for (int kt = 0; kt < steps_total; ++kt) {
-                if (!mbar_wait(&ready_bar[kt % SA], (unsigned)((kt / SA) & 1)) || !mbar_wait(&full_bar[kt % SB], (unsigned)((kt / SB) & 1))) {
-                    // giving up: let done_bar complete behind the MMAs already issued, so that tensor memory is not
-                    // freed under them
-                    atomicExch(p.status, 2); failed = 1; umma_commit(&done_bar); break;
-                }
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const unsigned a_addr = tmem_d + kACol0 + (unsigned)(kt % SA) * 32u, b_addr = smem_u32(b_ring + (kt % SB) * STAGE_BYTES);
+    for (int j = 0; j < 4; ++j)
 #pragma unroll
-                for (int j = 0; j < kTcBK / 16; ++j)  // 16 bf16 = 8 columns of A, 32 bytes along K inside B's 128-byte row
-                    umma_f16_ta(tmem_d, a_addr + 8u * j, umma_desc(b_addr + 32 * j), idesc, (kt > 0 || j > 0) ? 1u : 0u);
-                umma_commit(&empty_bar[kt % SB]);
-                if (kt == steps_total - 1) umma_commit(&done_bar);
-            }
+        for (int r = 0; r < 4; ++r) {
+            const unsigned v = (r & 1) ? w[j] >> 8 : w[j];
+            const unsigned pr = ((r >> 1) ? v & 0x00F000F0u : v & 0x000F000Fu) | 0x64006400u;
+            const __half2 m = *reinterpret_cast<const __half2*>(&pr);
+            const __half2 h = __hmul2((r >> 1) ? __hfma2(m, sixteenth, off16) : __hsub2(m, off), (r >> 1) ? hi : lo);
+            a[4 * j + r] = *reinterpret_cast<const unsigned*>(&h);
         }
-        __syncwarp();
-    } else if (warp == kTcThreads / 32 + 1) {
-        // ---- activation warp: one thread keeps the ring of activation tiles full ----------------------------
-        if (lane == 0) {
-            pdl_wait();                         // the activations may come from the kernel just before this one
-            int issued = 0;
-            for (int kt = 0; kt < steps_total; ++kt) {
-                const int s = kt % SB;
-                // the MMAs that read this stage SB groups ago are done
-                if (kt >= SB && !mbar_wait(&empty_bar[s], (unsigned)((kt / SB - 1) & 1))) { atomicExch(p.status, 3); failed = 1; break; }
-                if (failed) break;
-                const unsigned bar = smem_u32(&full_bar[s]);
-                const bool real = kt < real_steps;   // an appended step has activations (the group sums) but no packed weights
-                const int kg = real ? kt_lo + kt : kt_total + (kt - real_steps);   // 64-column step within the activation rows
-                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"((unsigned)(real ? STAGE_BYTES : B_BYTES)) : "memory");
-                if (real)
-                    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-                                 ::"r"(smem_u32(b_ring + s * STAGE_BYTES + B_BYTES)), "l"(reinterpret_cast<unsigned long long>(&wmap)), "r"(kg * 32), "r"(row0), "r"(bar) : "memory");
-                asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-                             ::"r"(smem_u32(b_ring + s * STAGE_BYTES)), "l"(reinterpret_cast<unsigned long long>(&xmap)), "r"(kg * kTcBK), "r"(tok0), "r"(bar) : "memory");
-                issued = kt + 1;
-            }
-            if (failed) {
-                // stopping early: the copies already requested still write shared memory; wait for them (bounded)
-                for (int kt = issued > SB ? issued - SB : 0; kt < issued; ++kt) mbar_wait(&full_bar[kt % SB], (unsigned)((kt / SB) & 1));
-            }
-        }
-        __syncwarp();
-    } else {
-    uint4 s_cur = load8(srow, kt_lo), z_cur = load8(zrow, kt_lo), s_nxt = load8(srow, kt_lo + 8), z_nxt = load8(zrow, kt_lo + 8);
-
-    // ring bookkeeping without divisions: stage and parity of this group's activations/packed weights, and of
-    // the group SA back whose MMAs free this group's weight tile
-    int fs = 0, es = 0, as = 0;
-    unsigned fpar = 0, epar = 0;
-    const unsigned char* const w_src = b_ring + B_BYTES + r * 32 + part * 8;
-    const unsigned a_dst = tmem_d + ((unsigned)((warp & 3) * 32) << 16) + kACol0 + (unsigned)part * 8u;
-    const unsigned full0 = smem_u32(&full_bar[0]), empty0 = smem_u32(&empty_bar[0]), ready0 = smem_u32(&ready_bar[0]);
-    // one group; j = kt & 7 is a compile-time constant in the unrolled loop below, so picking the group's scale and
-    // zero out of the 16-byte vectors costs one instruction each
-    auto group = [&](int kt, int j) {
-        // ---- the MMAs of group kt - SA are done: its weight tile (this group's) may be overwritten -----------
-        if (kt >= SA) {
-            if (!mbar_wait_addr(empty0 + 8u * es, epar)) { atomicExch(p.status, 1); failed = 1; }
-            if (++es == SB) { es = 0; epar ^= 1u; }
-        }
-        // ---- this group's packed weights have landed (with its activations) ---------------------------------
-        if (!mbar_wait_addr(full0 + 8u * fs, fpar)) { atomicExch(p.status, 1); failed = 1; }
-        // ---- weights: 16 nibbles of this thread's row -> 16 bf16 = bf16(scale * q + zero) -----------------
-        const uint2 wq = *reinterpret_cast<const uint2*>(w_src + fs * STAGE_BYTES);
-        if (++fs == SB) { fs = 0; fpar ^= 1u; }
-        const unsigned vs = pick16(s_cur, j), vz = pick16(z_cur, j);
-        // the scale as an fp16 pair: STAF tensors carry fp16 already; a bf16 (MLX) scale converts exactly (8 mantissa
-        // bits into 11) unless it lies below fp16's normal range, where the weights it scales are nil anyway
-        const __half s16 = F16SB ? __ushort_as_half((unsigned short)vs) : __float2half_rn(__uint_as_float(vs << 16));
-        const __half2 sc = __half2half2(s16);
-        (void)vz;
-        const unsigned c1032 = 0x64086408u;   // fp16 1032 = 1024 + 8
-        const __half2 off = *reinterpret_cast<const __half2*>(&c1032);
-        const unsigned words[2] = {wq.x, wq.y};
-        unsigned a_regs[8];
+}
+// The A operand of 64 appended columns from col0 on (counted from the first of them): c = 64 (zero + 8 scale) as an fp16 pair
+// (hi, lo); plane 0 carries c_hi (against sum_hi), plane 1 c_lo (against sum_hi), plane 2 c_hi (against sum_lo). The activation
+// side holds sum / 64 so that neither factor leaves fp16's range.
+template <bool F16SB>
+__device__ __forceinline__ void tc_appended(const QGemmTcParams& p, int rt, int col0, unsigned (&a)[16]) {
+    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    const int plane = col0 / p.g_pad, st0 = (col0 - plane * p.g_pad) >> 2;   // four groups per 16-byte entry
 #pragma unroll
-        for (int c = 0; c < 2; ++c) {
-            // a word holds 8 consecutive columns, nibble i = column i; pairs (i, i+4) come out of one LOP3
-            const unsigned wv = words[c];
-            unsigned o[4];
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int st = st0 + 4 * j + t;
+            uint4 v = make_uint4(0, 0, 0, 0);
+            if (rt < p.row_tiles && plane < 3 && st < p.kt / 4) v = __ldg(reinterpret_cast<const uint4*>(p.sb) + ((size_t)rt * (p.kt / 4) + st) * 16 + g + 8 * h);
+            const unsigned u[4] = {v.x, v.y, v.z, v.w};
+            float c[4];
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
-                const unsigned pr = ((wv >> (4 * i)) & 0x000F000Fu) | 0x64006400u;         // fp16 (1024+q_i, 1024+q_{i+4})
-                __half2 q2 = __hsub2(*reinterpret_cast<const __half2*>(&pr), off);        // (q_i - 8, q_{i+4} - 8), exact
-                q2 = __hmul2(q2, sc);                                                      // scale * (q - 8): exact in fp16
-                o[i] = *reinterpret_cast<const unsigned*>(&q2);                            // lo = column i, hi = column i+4
-            }
-            // reorder the pairs (i, i+4) into consecutive columns 0..7
-            a_regs[4 * c + 0] = __byte_perm(o[0], o[1], 0x5410); a_regs[4 * c + 1] = __byte_perm(o[2], o[3], 0x5410);
-            a_regs[4 * c + 2] = __byte_perm(o[0], o[1], 0x7632); a_regs[4 * c + 3] = __byte_perm(o[2], o[3], 0x7632);
-        }
-        // 16 bf16 of this row -> 8 columns of the row's TMEM lane (a warp owns the 32 lanes of its quarter)
-        asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
-                     ::"r"(a_dst + (unsigned)as * 32u), "r"(a_regs[0]), "r"(a_regs[1]), "r"(a_regs[2]), "r"(a_regs[3]), "r"(a_regs[4]), "r"(a_regs[5]), "r"(a_regs[6]), "r"(a_regs[7]) : "memory");
-        // the stores to tensor memory are complete and ordered before the MMA warp's reads, then tell the MMA warp
-        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(ready0 + 8u * as) : "memory");
-        if (++as == SA) as = 0;
-    };
-    // (group indices are local to this CTA's range: they only drive the rings; the scales come from kt_lo on)
-    for (int kt0 = 0; kt0 < real_steps && !failed; kt0 += 8) {
-        if (kt0 > 0) { s_cur = s_nxt; z_cur = z_nxt; s_nxt = load8(srow, kt_lo + kt0 + 8); z_nxt = load8(zrow, kt_lo + kt0 + 8); }
-#pragma unroll
-        for (int j = 0; j < 8; ++j)
-            if (kt0 + j < real_steps) group(kt0 + j, j);
-    }
-    // ---- appended steps: the A operand is the groups' constant term c = 64 (zero + 8 scale) as an fp16 pair (hi, lo);
-    // plane 0 carries c_hi (against sum_hi), plane 1 c_lo (against sum_hi), plane 2 c_hi (against sum_lo); the
-    // activation side holds sum / 64 so that neither factor leaves fp16's range -----------------------------------
-    const int plane_steps = p.ext_steps / 3;
-    for (int e = 0; e < ext_steps && !failed; ++e) {
-        const int kt = real_steps + e;
-        if (kt >= SA) {
-            if (!mbar_wait_addr(empty0 + 8u * es, epar)) { atomicExch(p.status, 1); failed = 1; }
-            if (++es == SB) { es = 0; epar ^= 1u; }
-        }
-        if (!mbar_wait_addr(full0 + 8u * fs, fpar)) { atomicExch(p.status, 1); failed = 1; }
-        if (++fs == SB) { fs = 0; fpar ^= 1u; }
-        const int plane = e / plane_steps, g0 = (e - plane * plane_steps) * 64 + part * 16;
-        unsigned a_regs[8];
-#pragma unroll
-        for (int h8 = 0; h8 < 2; ++h8) {
-            const uint4 sv = load8(srow, g0 + 8 * h8), zv = load8(zrow, g0 + 8 * h8);   // zero beyond the last group
-            float c[8];
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                const unsigned bs = pick16(sv, i), bz = pick16(zv, i);
-                const float sf = F16SB ? __half2float(__ushort_as_half((unsigned short)bs)) : __uint_as_float(bs << 16);
-                const float zf = F16SB ? __half2float(__ushort_as_half((unsigned short)bz)) : __uint_as_float(bz << 16);
-                const float cf = 64.0f * fmaf(8.0f, sf, zf);
-                const float hi = __half2float(__float2half_rn(cf));
+                const float cf = 64.0f * fmaf(8.0f, tc_scale<F16SB>(u[i]), tc_zero<F16SB>(u[i])), hi = __half2float(__float2half_rn(cf));
                 c[i] = plane == 1 ? cf - hi : hi;
             }
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
+            for (int i = 0; i < 2; ++i) {
                 const __half2 pr = __floats2half2_rn(c[2 * i], c[2 * i + 1]);
-                a_regs[4 * h8 + i] = *reinterpret_cast<const unsigned*>(&pr);
+                a[4 * j + 2 * h + i] = *reinterpret_cast<const unsigned*>(&pr);
             }
         }
-        asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
-                     ::"r"(a_dst + (unsigned)as * 32u), "r"(a_regs[0]), "r"(a_regs[1]), "r"(a_regs[2]), "r"(a_regs[3]), "r"(a_regs[4]), "r"(a_regs[5]), "r"(a_regs[6]), "r"(a_regs[7]) : "memory");
-        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(ready0 + 8u * as) : "memory");
-        if (++as == SA) as = 0;
-    }
-    }  // dequantising warps
+}
 
-    // ---- epilogue: TMEM -> registers -> bf16 -> Y[token][row] --------------------------------------------
-    // a warp reads the 32 accumulator lanes of its quarter (warp & 3); warps 4i..4i+3 take the i-th quarter of
-    // the token columns
-    bool ok = !failed && warp < kTcThreads / 32;
-    if (ok && !mbar_wait(&done_bar, 0u)) { atomicExch(p.status, 1); ok = false; }
-    if (failed && tid == 0) mbar_wait(&done_bar, 0u);   // (bounded) the MMAs issued before the failure have drained
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    if (ok) {
-        const int erow = row0 + (warp & 3) * 32 + lane;
-        const int cbase = (warp >> 2) * (BN / 4);
-#pragma unroll 1
-        for (int c0 = cbase; c0 < cbase + BN / 4; c0 += 16) {
-            if (tok0 + c0 >= p.m) break;  // uniform across the warp
-            unsigned v[16];
-            const unsigned taddr = tmem_d + ((unsigned)((warp & 3) * 32) << 16) + (unsigned)c0;
-            asm volatile(
-                "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-                : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-                  "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-                : "r"(taddr) : "memory");
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-            if (erow < p.n) {
+// Everything a dequantising warp does: the steps [lo, hi) of tiles `tile`, `tile` + stride, ... below `end`, of all of which it takes
+// every other one (counted over the tiles). rt_of(tile): the first row tile of the CTA's rows; w_ring: the CTA's weight rings.
+// Returns false when a wait expired. (What bounds a step is this warp's chain of waits, shared-memory reads, unpacking and the store to
+// tensor memory, about 1600 clocks with all warps in every step; two sets of warps have twice the time, and the waits and the arrival
+// serve two tiles. Weights kept ahead in registers were waited for as if the latest request were needed.)
+template <int CG, int SA, int STAGES, bool F16SB, typename RowTile>
+__device__ __forceinline__ bool tc_dequant(const QGemmTcParams& p, TcBars<STAGES>& b, unsigned w_ring, unsigned tmem_a, int tile, int stride, int end, int lo, int hi, RowTile rt_of) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, set = warp / kTcSet;
+    const int own_rt = 2 * (warp & 3) + ((warp >> 2) & 1);
+    const unsigned a_dst = tmem_a + ((unsigned)((warp & 3) * 32 + ((warp >> 2) & 1) * 16) << 16);
+    const unsigned full0 = smem_u32(&b.full[0]), empty0 = smem_u32(&b.empty[0]);
+    const unsigned ready0 = CG == 1 ? smem_u32(&b.ready[0]) : pair_leader(smem_u32(&b.ready[0]));
+    const unsigned ring = w_ring + warp * (kTcAhead * kTcSlotBytes);
+    const int real_hi = min(hi, p.real_steps), odd = (hi - lo) & 1;
+
+    // request side: this warp's steps over real weights, in order (rows beyond the last are not stored: what they hold does not matter)
+    int f_tile = tile, f_kt = lo + set, f_set = set;
+    auto fetch = [&](int slot) {
+        while (f_kt >= real_hi && f_tile < end) {   // on to the next tile; with an odd number of steps the sets change places
+            f_tile += stride;
+            f_set ^= odd;
+            f_kt = lo + f_set;
+            if (lo >= real_hi) f_tile = end;        // (a CTA whose share of K is appended columns only)
+        }
+        if (f_tile < end) {
+            const int rt = min(rt_of(f_tile) + own_rt, p.row_tiles - 1), kt = 2 * f_kt;
+            const unsigned dst = ring + slot * kTcSlotBytes;
+            const uint4* w = p.tiles + ((size_t)rt * p.kt + kt) * 32 + lane;
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + lane * 16), "l"(w) : "memory");
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 512 + lane * 16), "l"(w + 32) : "memory");
+            if (lane < 16) asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst + 1024 + lane * 8), "l"(p.sb + ((size_t)rt * (p.kt / 4) + (kt >> 2)) * 64 + lane * 4 + (kt & 3)) : "memory");
+            f_kt += 2;
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+
+    // this warp's place in the sequence of all steps: `at` is a stage's place, `old` that of the step SA back, a_slot its weight tile
+    RingPos<STAGES> at, old;
+    at.s = set;
+    old.s = (SA & 1) ^ set;                       // the first step of this set that waits is SA + that
+    int a_slot = set % SA, fresh = (SA + 1 - set) / 2;   // steps without one SA back
+    auto begin = [&]() {   // the MMAs of the step SA back are done (its weight tile may be overwritten)
+        if (fresh > 0) { --fresh; return true; }
+        const bool ok = mbar_wait_warp(empty0 + 8u * old.s, old.par);
+        old.skip2();
+        return ok;
+    };
+    auto finish = [&]() {
+        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");   // the stores are ordered before the MMAs of the thread that waits
+        // the CTA's activations have landed: one warp's arrival covers them for the MMAs
+        if ((warp & (kTcSet - 1)) == 0 && !mbar_wait_warp(full0 + 8u * at.s, at.par)) return false;
+        __syncwarp();
+        if (lane == 0) tc_arrive<CG>(ready0 + 8u * a_slot);
+        a_slot += 2;
+        if (a_slot >= SA) a_slot -= SA;
+        at.skip2();
+        return true;
+    };
+    static_assert(SA >= 2 && STAGES >= 2, "steps advance by two");
+
 #pragma unroll
-                for (int i = 0; i < 16; ++i) {
-                    const int tkn = tok0 + c0 + i;
-                    // undo the token row's power-of-two scaling (exact), round once to bf16 (or leave this K range's
-                    // sum for the launch that adds the ranges up)
-                    if (tkn < p.m) {
-                        const float val = __uint_as_float(v[i]) * __ldg(p.rscale + tkn);
-                        if (gridDim.z > 1) p.part[((size_t)blockIdx.z * p.m + tkn) * p.n + erow] = val;
-                        else tc_store(p.out, tkn, erow, val);
+    for (int i = 0; i < kTcAhead - 1; ++i) fetch(i);
+    int slot = 0, s_now = set;
+    bool ok = true;
+    for (; tile < end && ok; tile += stride, s_now ^= odd) {
+        int kt = lo + s_now;
+        for (; kt < real_hi; kt += 2) {
+            fetch(slot == 0 ? kTcAhead - 1 : slot - 1);   // (that slot was read a step ago, by all lanes)
+            asm volatile("cp.async.wait_group %0;" ::"n"(kTcAhead - 1) : "memory");
+            __syncwarp();
+            const unsigned src = ring + slot * kTcSlotBytes;
+            if (++slot == kTcAhead) slot = 0;
+            uint4 w0, w1;
+            uint2 s_lo, s_hi;
+            asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(w0.x), "=r"(w0.y), "=r"(w0.z), "=r"(w0.w) : "r"(src + lane * 16));
+            asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(w1.x), "=r"(w1.y), "=r"(w1.z), "=r"(w1.w) : "r"(src + 512 + lane * 16));
+            asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(s_lo.x), "=r"(s_lo.y) : "r"(src + 1024 + (lane >> 2) * 8));
+            asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(s_hi.x), "=r"(s_hi.y) : "r"(src + 1088 + (lane >> 2) * 8));
+            unsigned a[16];
+            tc_unpack(w0, tc_scale2<F16SB>(s_lo.x), tc_scale2<F16SB>(s_hi.x), a);
+            if (!begin()) { ok = false; break; }
+            tmem_st_frag(a_dst + (unsigned)a_slot * 64u, a);
+            tc_unpack(w1, tc_scale2<F16SB>(s_lo.y), tc_scale2<F16SB>(s_hi.y), a);
+            tmem_st_frag(a_dst + (unsigned)a_slot * 64u + 32u, a);
+            if (!finish()) { ok = false; break; }
+        }
+        for (; kt < hi && ok; kt += 2) {
+            if (!begin()) { ok = false; break; }
+#pragma unroll 1
+            for (int half = 0; half < 2; ++half) {
+                unsigned a[16];
+                tc_appended<F16SB>(p, rt_of(tile) + own_rt, (kt - p.real_steps) * kTcStep + half * 64, a);
+                tmem_st_frag(a_dst + (unsigned)a_slot * 64u + half * 32u, a);
+            }
+            if (!finish()) ok = false;
+        }
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    return ok;
+}
+
+// Results of one lane's 16 columns from c0 on: `row0 + lane` is its weight row.
+__device__ __forceinline__ void tc_store16(const QGemmTcParams& p, const unsigned (&v)[16], int row0, int token0) {
+    const int lane = threadIdx.x & 31, row = row0 + lane;
+    if (!p.gated) {
+        if (row >= p.out.end[2]) return;
+        const int q = row < p.out.end[0] ? 0 : row < p.out.end[1] ? 1 : 2;
+        const int stride = q == 0 ? p.out.stride[0] : q == 1 ? p.out.stride[1] : p.out.stride[2];
+        __nv_bfloat16* dst = (q == 0 ? p.out.y[0] : q == 1 ? p.out.y[1] : p.out.y[2]) + (row - (q == 0 ? 0 : q == 1 ? p.out.end[0] : p.out.end[1])) + (size_t)token0 * stride;
+#pragma unroll
+        for (int i = 0; i < 16; ++i)
+            if (token0 + i < p.m) dst[(size_t)i * stride] = __float2bfloat16_rn(__uint_as_float(v[i]) * __ldg(p.rscale + token0 + i));
+        return;
+    }
+    // gate rows sit in the lanes of the first eight of 16, up rows in the others: a gate lane finishes even columns, its up lane odd ones
+    const bool up_lane = lane & 8;
+    const int out_row = (row >> 4) * 8 + (row & 7);
+#pragma unroll
+    for (int i = 0; i < 16; i += 2) {
+        const float other = __uint_as_float(__shfl_xor_sync(0xffffffffu, up_lane ? v[i] : v[i + 1], 8));
+        const int token = token0 + i + (up_lane ? 1 : 0);
+        if (token < p.m) {
+            const float sc = __ldg(p.rscale + token);
+            if (up_lane) tc_store_gated(p, token, out_row, other * sc, __uint_as_float(v[i + 1]) * sc);
+            else tc_store_gated(p, token, out_row, __uint_as_float(v[i]) * sc, other * sc);
+        }
+    }
+}
+
+// ---- long form: many activation rows. Pairs of CTAs walk tiles of 256 weight rows x 256 activation rows; eight warps of their own
+// store a tile's results while the next tile's first stages are fetched and dequantised. ------------------------------------
+constexpr int kTcPairRows = 128;   // activation rows in a CTA's shared memory
+template <int STAGES, bool F16SB>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__((kTcDeqWarps + 2 + kTcEpiWarps) * 32, 1) qgemm_tc_kernel(const QGemmTcParams p, const __grid_constant__ CUtensorMap xmap) {
+    constexpr int SA = 4;
+    constexpr unsigned kTmemCols = 512;                      // accumulator 256, four weight tiles
+    constexpr unsigned STAGE_BYTES = kTcPairRows * 256;
+    extern __shared__ __align__(1024) unsigned char smem_raw[];
+    const unsigned ring = (smem_u32(smem_raw) + 1023u) & ~1023u;   // the swizzle pattern repeats every 1024 bytes
+    __shared__ __align__(8) TcBars<STAGES> bars;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, rank = (int)blockIdx.x & 1;
+    const int first = (int)blockIdx.x >> 1, pairs = (int)gridDim.x >> 1;
+    const unsigned tmem_d = tc_setup<STAGES, kTmemCols, 2>(bars);
+    pdl_launch_dependents();   // (behind the allocation: a CTA of the next kernel cannot take tensor memory that this one still waits for)
+    volatile int* const failed = &bars.failed;
+
+    if (warp == kTcDeqWarps) {
+        if (rank == 0) {   // the first CTA issues for both
+            const bool el = elect_one();
+            RingPos<STAGES> full;
+            int a_slot = 0, done = 0;   // done: tiles whose completion has been requested
+            unsigned a_par = 0;
+            bool ok = true;
+            for (int tile = first; tile < p.n_tiles && ok; tile += pairs) {
+                // the accumulators of the tile before have been read
+                if (done > 0 && !mbar_wait_warp(&bars.acc_empty, (unsigned)((done - 1) & 1))) { ok = false; break; }
+                for (int kt = 0; kt < p.steps; ++kt) {
+                    if (!mbar_wait_warp(&bars.ready[a_slot], a_par)) { ok = false; break; }
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    if (el) {
+                        tc_mma_step<2, kTcPairRows>(tmem_d, tmem_d + 256u + a_slot * 64u, ring + full.s * STAGE_BYTES, kt == 0);
+                        umma_commit_pair(&bars.empty[full.s]);
                     }
+                    __syncwarp();
+                    if (++a_slot == SA) { a_slot = 0; a_par ^= 1u; }
+                    full.next();
+                }
+                if (ok) { if (el) umma_commit_pair(&bars.acc_full); ++done; }
+                __syncwarp();
+            }
+            if (!ok && el) {   // the MMAs issued so far end before tensor memory is freed
+                tc_fail(p.status, &bars.failed, 2);
+                umma_commit_pair(&bars.acc_full);
+                if (done > 0) mbar_wait(&bars.acc_full, (unsigned)((done - 1) & 1));
+                mbar_wait(&bars.acc_full, (unsigned)(done & 1));
+            }
+        }
+        __syncwarp();
+    } else if (warp == kTcDeqWarps + 1) {
+        if (lane == 0) {
+            pdl_wait();                         // the activations come from the kernel just before this one
+            RingPos<STAGES> at;
+            int issued = 0;
+            bool ok = true;
+            for (int tile = first; tile < p.n_tiles && ok; tile += pairs) {
+                const int tok0 = tile % p.tok_tiles * 256 + rank * kTcPairRows;
+                for (int kt = 0; kt < p.steps; ++kt) {
+                    // the MMAs that read this stage a round ago are done
+                    if (*failed || (issued >= STAGES && !mbar_wait(&bars.empty[at.s], at.par ^ 1u))) { ok = false; break; }
+                    tc_issue<kTcPairRows>(&xmap, ring + at.s * STAGE_BYTES, smem_u32(&bars.full[at.s]), kt, tok0);
+                    at.next();
+                    ++issued;
                 }
             }
+            if (!ok) tc_fail(p.status, &bars.failed, 3);
+            // every copy has landed before the CTA leaves (also when it stops early)
+            for (int i = issued > STAGES ? issued - STAGES : 0; i < issued; ++i) mbar_wait(&bars.full[i % STAGES], (unsigned)((i / STAGES) & 1));
+        }
+        __syncwarp();
+    } else if (warp < kTcDeqWarps) {
+        if (!tc_dequant<2, SA, STAGES, F16SB>(p, bars, ring + STAGES * STAGE_BYTES, tmem_d + 256u, first, pairs, p.n_tiles, 0, p.steps,
+                                              [&](int tile) { return tile / p.tok_tiles * 16 + rank * 8; })) tc_fail(p.status, &bars.failed, 1);
+        __syncwarp();
+    } else {
+        // a warp reads the 32 accumulator lanes of its quarter (warp & 3) and half of the columns
+        const int half = (warp - kTcDeqWarps - 2) >> 2;
+        const unsigned acc_empty = pair_leader(smem_u32(&bars.acc_empty));
+        unsigned par = 0;
+        for (int tile = first; tile < p.n_tiles; tile += pairs, par ^= 1u) {
+            if (!mbar_wait_warp(&bars.acc_full, par)) { tc_fail(p.status, &bars.failed, 4); break; }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const int row0 = tile / p.tok_tiles * 256 + rank * kTcRows + (warp & 3) * 32, tok0 = tile % p.tok_tiles * 256;
+#pragma unroll 1
+            for (int c0 = half * 128; c0 < (half + 1) * 128; c0 += 16) {
+                if (tok0 + c0 >= p.m) break;  // uniform across the warp
+                unsigned v[16];
+                tmem_ld16(tmem_d + ((unsigned)((warp & 3) * 32) << 16) + (unsigned)c0, v);
+                tc_store16(p, v, row0, tok0 + c0);
+            }
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) tc_arrive<2>(acc_empty);
+        }
+        __syncwarp();
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    cg::this_cluster().sync();   // nobody arrives at a barrier of a CTA that has left, and no MMA reads its tensor memory
+    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_d), "r"(kTmemCols) : "memory");
+}
+
+// ---- short kernel: few activation rows, or few tiles. K is cut over the CTAs of a cluster; each sends its part of a tile's results
+// to the CTA that finishes a row, through distributed shared memory (the ring's, which is free by then). ---------------------------
+template <int BN, int STAGES, int PER_SM, bool F16SB>
+__global__ void __launch_bounds__((kTcDeqWarps + 2) * 32, PER_SM) qgemm_tc_short_kernel(const QGemmTcParams p, const __grid_constant__ CUtensorMap xmap) {
+    constexpr unsigned kTmemCols = PER_SM == 1 ? 512 : 256;
+    constexpr int SA = (int)(kTmemCols - BN) / 64 > kTcMaxA ? kTcMaxA : (int)(kTmemCols - BN) / 64;   // what two CTAs of an SM have room for
+    constexpr unsigned STAGE_BYTES = BN * 256;
+    static_assert((size_t)STAGES * STAGE_BYTES >= (size_t)BN * kTcRows * 4, "the ring takes what the cluster sends");
+    extern __shared__ __align__(1024) unsigned char smem_raw[];
+    unsigned char* const ring_ptr = smem_raw + ((1024 - (smem_u32(smem_raw) & 1023)) & 1023);
+    const unsigned ring = smem_u32(ring_ptr);
+    __shared__ __align__(8) TcBars<STAGES> bars;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int rank = (int)blockIdx.x % p.splits, row0 = (int)blockIdx.x / p.splits * kTcRows, tok0 = blockIdx.y * BN;
+    const int lo = p.steps * rank / p.splits, hi = p.steps * (rank + 1) / p.splits;
+    const unsigned tmem_d = tc_setup<STAGES, kTmemCols, 1>(bars);
+    pdl_launch_dependents();   // (behind the allocation: a CTA of the next kernel cannot take tensor memory that this one still waits for)
+    volatile int* const failed = &bars.failed;
+
+    if (warp == kTcDeqWarps) {
+        const bool el = elect_one();
+        RingPos<STAGES> full;
+        int a_slot = 0;
+        unsigned a_par = 0;
+        for (int kt = lo; kt < hi; ++kt) {
+            if (!mbar_wait_warp(&bars.ready[a_slot], a_par)) { tc_fail(p.status, &bars.failed, 2); break; }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            if (el) {
+                tc_mma_step<1, BN>(tmem_d, tmem_d + BN + a_slot * 64u, ring + full.s * STAGE_BYTES, kt == lo);
+                umma_commit(&bars.empty[full.s]);
+            }
+            __syncwarp();
+            if (++a_slot == SA) { a_slot = 0; a_par ^= 1u; }
+            full.next();
+        }
+        if (el) umma_commit(&bars.acc_full);   // also behind a failure: tensor memory is not freed under MMAs in flight
+        __syncwarp();
+    } else if (warp == kTcDeqWarps + 1) {
+        if (lane == 0) {
+            pdl_wait();                         // the activations come from the kernel just before this one
+            RingPos<STAGES> at;
+            int issued = 0;
+            for (int kt = lo; kt < hi; ++kt) {
+                if (*failed || (issued >= STAGES && !mbar_wait(&bars.empty[at.s], at.par ^ 1u))) { tc_fail(p.status, &bars.failed, 3); break; }
+                tc_issue<BN>(&xmap, ring + at.s * STAGE_BYTES, smem_u32(&bars.full[at.s]), kt, tok0);
+                at.next();
+                ++issued;
+            }
+            // every copy has landed before the ring is given to the cluster (also behind a failure)
+            for (int i = issued > STAGES ? issued - STAGES : 0; i < issued; ++i) mbar_wait(&bars.full[i % STAGES], (unsigned)((i / STAGES) & 1));
+        }
+        __syncwarp();
+    } else {
+        if (!tc_dequant<1, SA, STAGES, F16SB>(p, bars, ring + STAGES * STAGE_BYTES, tmem_d + BN, 0, 1, 1, lo, hi, [&](int) { return row0 / 16; })) tc_fail(p.status, &bars.failed, 1);
+        __syncwarp();
+    }
+    // ---- results: warp w reads the lanes of quarter w & 3 and a quarter of the columns ---------------------------------------
+    const bool done = mbar_wait_warp(&bars.acc_full, 0u);
+    if (!done && lane == 0) tc_fail(p.status, &bars.failed, 5);
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const int r = (warp & 3) * 32 + lane;
+    constexpr int CW = 16;                          // columns per read; with 32 columns two of a quarter's four warps read
+    const cg::cluster_group cluster = cg::this_cluster();
+    if (p.splits > 1) cluster.sync();               // every ring of the cluster is free
+    const int own = BN / p.splits;                  // columns that a CTA of the cluster finishes
+    if (done && warp < kTcDeqWarps) {
+#pragma unroll 1
+        for (int c0 = (warp >> 2) * CW; c0 < BN; c0 += 4 * CW) {
+            if (tok0 + c0 >= p.m) break;
+            unsigned v[CW];
+            tmem_ld16(tmem_d + ((unsigned)((warp & 3) * 32) << 16) + (unsigned)c0, v);
+            if (p.splits == 1) {
+                tc_store16(p, v, row0 + (warp & 3) * 32, tok0 + c0);
+                continue;
+            }
+#pragma unroll
+            for (int i = 0; i < CW; ++i) {
+                const int c = c0 + i, owner = c / own;
+                if (tok0 + c < p.m) reinterpret_cast<float*>(cluster.map_shared_rank(ring_ptr, owner))[(rank * own + (c - owner * own)) * kTcRows + r] = __uint_as_float(v[i]);
+            }
+        }
+    }
+    if (p.splits > 1) {
+        cluster.sync();
+        const float* got = reinterpret_cast<const float*>(ring_ptr);
+        const int rows = p.gated ? kTcRows / 2 : kTcRows;
+        for (int o = threadIdx.x; o < own * rows; o += blockDim.x) {
+            const int cl = o / rows, i = o % rows, token = tok0 + rank * own + cl;
+            if (token >= p.m) continue;
+            const int ra = p.gated ? (i >> 3) * 16 + (i & 7) : i;   // a gate row, its up row eight further on
+            const float* src = got + cl * kTcRows + ra;
+            float va = 0.f, vb = 0.f;
+            for (int z = 0; z < p.splits; ++z) {   // ranges in order
+                va += src[z * own * kTcRows];
+                if (p.gated) vb += src[z * own * kTcRows + 8];
+            }
+            const float sc = __ldg(p.rscale + token);
+            if (p.gated) tc_store_gated(p, token, row0 / 2 + i, va * sc, vb * sc);
+            else tc_store(p.out, token, row0 + i, va * sc);
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -357,76 +589,172 @@ __global__ void __launch_bounds__(kTcAllThreads) qgemm_tc_kernel(const QGemmTcPa
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_d), "r"(kTmemCols) : "memory");
 }
 
-// Y[t][n] = bf16(sum over the K ranges, in order) for a launch whose K was cut in `splits` ranges.
-__global__ void __launch_bounds__(256) tc_sum_splits_kernel(const float* part, int splits, int m, int n, const TcSegments out) {
-    pdl_launch_dependents();
-    pdl_wait();
-    const size_t total = (size_t)m * n;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
-        float acc = 0.f;
-        for (int z = 0; z < splits; ++z) acc += __ldcg(part + (size_t)z * total + i);
-        const int t = (int)(i / n), r = (int)(i - (size_t)t * n);
-        tc_store(out, t, r, acc);
-    }
+// Activations bf16 -> fp16, one CTA per row: the row's largest magnitude goes to [2^14, 2^15), so that nothing overflows fp16 and
+// every element within 2^-28 of the largest converts exactly (bf16 carries 8 significant bits, fp16 11). rscale[row] = the inverse
+// factor. Within a group of 64 column 16 t + 4 j + i goes to place 16 j + 4 t + i, the order of the weights' fragments. Behind the k
+// values (and zeros up to the weights' padding) the row gets three planes of g_pad columns: sum / 64 of every group of 64 converted values as an fp16
+// pair, laid out (hi, hi, lo) to meet the (c_hi, c_lo, c_hi) planes of the weight side; the rest is zeros.
+// HOLD: a row of up to 16384 values stays in registers between the two passes (reading 4 bytes per lane twice took 24 us for
+// 2048 x 4096 under ncu, this takes 15).
+struct F16Rows { int k, k_pad, g_pad; __half* xh; int stride; float* rscale; };   // columns, padded, of a plane; the copy and its pitch
+// bf16 magnitudes order like their bit patterns: two 16-bit maxima at a time
+__device__ __forceinline__ unsigned f16_top(unsigned mx, const uint4& v) {
+    mx = __vmaxu2(mx, v.x & 0x7FFF7FFFu); mx = __vmaxu2(mx, v.y & 0x7FFF7FFFu);
+    mx = __vmaxu2(mx, v.z & 0x7FFF7FFFu); return __vmaxu2(mx, v.w & 0x7FFF7FFFu);
 }
-
-// Activations bf16 -> fp16, one CTA per token row: the row's largest magnitude goes to [2^14, 2^15), so that nothing
-// overflows fp16 and every element within 2^-28 of the largest converts exactly (bf16 carries 8 significant bits,
-// fp16 11). rscale[row] = the inverse factor, applied to the accumulators in the product's epilogue. Behind the k
-// converted values the row gets three planes of g_pad columns: sum / 64 of every group of 64 converted values as an
-// fp16 pair, laid out (hi, hi, lo) to meet the (c_hi, c_lo, c_hi) planes of the weight side; columns past the last
-// group are zero.
-__global__ void __launch_bounds__(256) x_to_f16_kernel(const __nv_bfloat16* x, int x_stride, int k, int g_pad, __half* xh, int xh_stride, float* rscale) {
-    pdl_launch_dependents();
-    pdl_wait();
-    __shared__ unsigned red[8];
-    const int row = blockIdx.x, tid = threadIdx.x;
-    const unsigned* src = reinterpret_cast<const unsigned*>(x + (size_t)row * x_stride);
-    unsigned mx = 0;
-    for (int i = tid; i < k / 2; i += 256) {
-        const unsigned w = src[i];
-        mx = max(mx, max(w & 0x7FFFu, (w >> 16) & 0x7FFFu));   // bf16 magnitudes order like their bit patterns
-    }
-    for (int o = 16; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    if ((tid & 31) == 0) red[tid >> 5] = mx;
+// the power of two of a row out of its threads' maxima
+__device__ __forceinline__ int f16_shift(unsigned mx, unsigned* red) {
+    mx = __reduce_max_sync(0xffffffffu, max(mx & 0xFFFFu, mx >> 16));
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = mx;
     __syncthreads();
     mx = 0;
+#pragma unroll
     for (int i = 0; i < 8; ++i) mx = max(mx, red[i]);
     const int e = (int)(mx >> 7);                                   // biased exponent of the largest magnitude
-    const int sh = (e == 0 || e == 255) ? 0 : max(-100, min(100, 141 - e));
-    const float mul = __uint_as_float((unsigned)(127 + sh) << 23);  // 2^sh
-    __half* out = xh + (size_t)row * xh_stride;
-    // a warp converts one group of 64 at a time (one 32-bit word of two values per lane) and sums it
-    const int lane = tid & 31, warp = tid >> 5, groups = k / 64;
-    for (int g = warp; g < g_pad; g += 8) {
-        float sum = 0.f;
-        if (g < groups) {
-            const unsigned w = src[g * 32 + lane];
-            const __half2 h = __floats2half2_rn(__uint_as_float(w << 16) * mul, __uint_as_float(w & 0xFFFF0000u) * mul);
-            reinterpret_cast<unsigned*>(out)[g * 32 + lane] = *reinterpret_cast<const unsigned*>(&h);
-            const float2 f = __half22float2(h);
-            sum = f.x + f.y;
-        }
-        for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-        if (lane == 0) {
-            const float sc = sum * 0.015625f;
-            const __half hi = __float2half_rn(sc), lo = __float2half_rn(sc - __half2float(hi));
-            out[k + g] = hi; out[k + g_pad + g] = hi; out[k + 2 * g_pad + g] = lo;
-        }
+    return (e == 0 || e == 255) ? 0 : max(-100, min(100, 141 - e));
+}
+// eight values, the i-th eight of the row; lanes of eight share a group (k is a multiple of 64)
+__device__ __forceinline__ void f16_put(const F16Rows& f, __half* out, int i, const uint4& v, float mul) {
+    const unsigned u[4] = {v.x, v.y, v.z, v.w};
+    float sum = 0.f;
+    unsigned o[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const __half2 h = __floats2half2_rn(__uint_as_float(u[j] << 16) * mul, __uint_as_float(u[j] & 0xFFFF0000u) * mul);
+        o[j] = *reinterpret_cast<const unsigned*>(&h);
+        const float2 g = __half22float2(h);
+        sum += g.x + g.y;
     }
-    if (tid == 0) rscale[row] = __uint_as_float((unsigned)(127 - sh) << 23);
+    // eight columns 8 u .. of a group: t = u / 2, j = 2 (u & 1) and the next one
+    __half* dst = out + (i >> 3) * 64 + 32 * (i & 1) + 4 * ((i & 7) >> 1);
+    *reinterpret_cast<uint2*>(dst) = make_uint2(o[0], o[1]);
+    *reinterpret_cast<uint2*>(dst + 16) = make_uint2(o[2], o[3]);
+    const unsigned lane = threadIdx.x & 31, mask = 0xFFu << (lane & 24);
+    sum += __shfl_xor_sync(mask, sum, 1);
+    sum += __shfl_xor_sync(mask, sum, 2);
+    sum += __shfl_xor_sync(mask, sum, 4);
+    if ((lane & 7) == 0) {
+        const float sc = sum * 0.015625f;
+        const __half hi = __float2half_rn(sc), lo = __float2half_rn(sc - __half2float(hi));
+        __half* ext = out + f.k_pad + (i >> 3);
+        ext[0] = hi; ext[f.g_pad] = hi; ext[2 * f.g_pad] = lo;
+    }
+}
+// what lies behind the values and behind the planes' groups
+__device__ __forceinline__ void f16_pad(const F16Rows& f, __half* out, int row, int sh) {
+    for (int i = f.k + threadIdx.x; i < f.k_pad; i += 256) out[i] = __ushort_as_half(0);
+    const int groups = f.k / 64;
+    for (int i = threadIdx.x; i < f.stride - f.k_pad; i += 256)
+        if (i >= 3 * f.g_pad || i % f.g_pad >= groups) out[f.k_pad + i] = __ushort_as_half(0);
+    if (threadIdx.x == 0) f.rscale[row] = __uint_as_float((unsigned)(127 - sh) << 23);
 }
 
-template <int BN, int STAGES>
-constexpr size_t tc_smem_bytes() { return (size_t)STAGES * (BN * 128 + kTcRows * 32) + 1024; }
+template <bool HOLD>
+__global__ void __launch_bounds__(256) x_to_f16_kernel(const __nv_bfloat16* x, int x_stride, const F16Rows f) {
+    pdl_launch_dependents();
+    pdl_wait();
+    constexpr int CH = HOLD ? 8 : 1;
+    __shared__ unsigned red[8];
+    const int row = blockIdx.x, tid = threadIdx.x, n8 = f.k / 8;
+    const uint4* src = reinterpret_cast<const uint4*>(x + (size_t)row * x_stride);
+    uint4 held[CH];
+    unsigned mx = 0;
+    if (HOLD) {
+#pragma unroll
+        for (int c = 0; c < CH; ++c) {
+            held[c] = make_uint4(0, 0, 0, 0);
+            if (tid + c * 256 < n8) held[c] = src[tid + c * 256];
+        }
+#pragma unroll
+        for (int c = 0; c < CH; ++c) mx = f16_top(mx, held[c]);
+    } else {
+        for (int i = tid; i < n8; i += 256) mx = f16_top(mx, src[i]);
+    }
+    const int sh = f16_shift(mx, red);
+    const float mul = __uint_as_float((unsigned)(127 + sh) << 23);  // 2^sh
+    __half* out = f.xh + (size_t)row * f.stride;
+    if (HOLD) {
+#pragma unroll
+        for (int c = 0; c < CH; ++c)
+            if (tid + c * 256 < n8) f16_put(f, out, tid + c * 256, held[c], mul);
+    } else {
+        for (int i = tid; i < n8; i += 256) f16_put(f, out, i, src[i], mul);
+    }
+    f16_pad(f, out, row, sh);
+}
 
-// fp16 activations X[m][x_stride] as a 2-D tensor (k innermost); box = 64 columns x bn tokens, 128-byte swizzle
-int make_x_map(const __half* x, int x_stride, int m, int k, int bn, CUtensorMap* map) {
+// A norm step (see rmsnorm_kernel) whose result goes to its buffer and, converted, to the product behind it: one pass instead of two
+// launches. MODE: 0 copy, 1 residual add and copy, 2 residual add.
+template <int MODE>
+__global__ void __launch_bounds__(256) norm_to_f16_kernel(const __nv_bfloat16* in, int in_stride, __nv_bfloat16* residual, int res_stride, const __nv_bfloat16* weight,
+                                                          float eps, float weight_bias, __nv_bfloat16* y, int y_stride, const F16Rows f) {
+    pdl_launch_dependents();
+    pdl_wait();
+    extern __shared__ __align__(16) float norm_h[];   // the unrounded row, then the rounded one in its place (a thread's own eights)
+    __shared__ unsigned red[8];
+    __shared__ float sums[8];
+    const int row = blockIdx.x, tid = threadIdx.x, n8 = f.k / 8;
+    const uint4* in4 = reinterpret_cast<const uint4*>(in + (size_t)row * in_stride);
+    uint4* res4 = reinterpret_cast<uint4*>(residual + (size_t)row * res_stride);
+    auto pack = [](float a, float b) { const __nv_bfloat162 v = __floats2bfloat162_rn(a, b); return *reinterpret_cast<const unsigned*>(&v); };
+    float ss = 0.f;
+    for (int i = tid; i < n8; i += 256) {
+        const uint4 v = in4[i];
+        const unsigned u[4] = {v.x, v.y, v.z, v.w};
+        float h[8];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) { h[2 * j] = __uint_as_float(u[j] << 16); h[2 * j + 1] = __uint_as_float(u[j] & 0xFFFF0000u); }
+        if (MODE != 0) {
+            const uint4 r = res4[i];
+            const unsigned q[4] = {r.x, r.y, r.z, r.w};
+#pragma unroll
+            for (int j = 0; j < 4; ++j) { h[2 * j] += __uint_as_float(q[j] << 16); h[2 * j + 1] += __uint_as_float(q[j] & 0xFFFF0000u); }
+        }
+        if (MODE != 2) res4[i] = make_uint4(pack(h[0], h[1]), pack(h[2], h[3]), pack(h[4], h[5]), pack(h[6], h[7]));
+#pragma unroll
+        for (int e = 0; e < 8; ++e) ss = fmaf(h[e], h[e], ss);
+        reinterpret_cast<float4*>(norm_h)[2 * i] = make_float4(h[0], h[1], h[2], h[3]);
+        reinterpret_cast<float4*>(norm_h)[2 * i + 1] = make_float4(h[4], h[5], h[6], h[7]);
+    }
+    for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+    if ((tid & 31) == 0) sums[tid >> 5] = ss;
+    __syncthreads();
+    float total = 0.f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) total += sums[i];
+    const float rs = rsqrtf(total / (float)f.k + eps);
+    unsigned mx = 0;
+    for (int i = tid; i < n8; i += 256) {
+        const uint4 w = reinterpret_cast<const uint4*>(weight)[i];
+        const unsigned u[4] = {w.x, w.y, w.z, w.w};
+        const float4 a = reinterpret_cast<const float4*>(norm_h)[2 * i], b = reinterpret_cast<const float4*>(norm_h)[2 * i + 1];
+        const float h[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+        unsigned o[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            o[j] = pack(h[2 * j] * rs * (__uint_as_float(u[j] << 16) + weight_bias), h[2 * j + 1] * rs * (__uint_as_float(u[j] & 0xFFFF0000u) + weight_bias));
+        const uint4 v = make_uint4(o[0], o[1], o[2], o[3]);
+        reinterpret_cast<uint4*>(y + (size_t)row * y_stride)[i] = v;
+        reinterpret_cast<uint4*>(norm_h)[2 * i] = v;
+        mx = f16_top(mx, v);
+    }
+    const int sh = f16_shift(mx, red);
+    const float mul = __uint_as_float((unsigned)(127 + sh) << 23);
+    __half* out = f.xh + (size_t)row * f.stride;
+    for (int i = tid; i < n8; i += 256) f16_put(f, out, i, reinterpret_cast<const uint4*>(norm_h)[2 * i], mul);
+    f16_pad(f, out, row, sh);
+}
+
+// rows: activation rows in a CTA's shared memory
+constexpr size_t tc_smem_bytes(int rows, int stages) { return (size_t)stages * rows * 256 + kTcRingBytes + 1024; }
+
+// fp16 activations X[m][x_stride] as a 2-D tensor (k innermost); box = 64 columns x bn rows, 128-byte swizzle
+int make_x_map(const __half* x, int x_stride, int m, int bn, CUtensorMap* map) {
     TensorMapEncodeFn fn = tensor_map_encode_fn();
     if (!fn) { set_error("qgemm (tcgen05): cuTensorMapEncodeTiled is not available"); return SWLM_ERR_CUDA; }
-    const cuuint64_t dims[2] = {(cuuint64_t)k, (cuuint64_t)m};
+    const cuuint64_t dims[2] = {(cuuint64_t)x_stride, (cuuint64_t)m};
     const cuuint64_t strides[1] = {(cuuint64_t)x_stride * 2};
-    const cuuint32_t box[2] = {(cuuint32_t)kTcBK, (cuuint32_t)bn};
+    const cuuint32_t box[2] = {64, (cuuint32_t)bn};
     const cuuint32_t estr[2] = {1, 1};
     const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<__half*>(x), dims, strides, box, estr,
                           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
@@ -434,128 +762,150 @@ int make_x_map(const __half* x, int x_stride, int m, int k, int bn, CUtensorMap*
     if (r != CUDA_SUCCESS) { set_error("qgemm (tcgen05): cuTensorMapEncodeTiled failed (%d)", (int)r); return SWLM_ERR_CUDA; }
     return SWLM_OK;
 }
+// forms: short with 32 or 64 activation rows per tile and two CTAs or one per SM, with 128 and one, long with 256; their stages
+constexpr int kTcStages32x2 = 6, kTcStages32 = 8, kTcStages64x2 = 3, kTcStages64 = 6, kTcStages128 = 4, kTcStagesPair = 5;
+constexpr int kTcSMs = 148;
 
-template <int BN, int STAGES>
-int tc_init_one() {
-    SWLM_CUDA(cudaFuncSetAttribute(qgemm_tc_kernel<BN, STAGES, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc_smem_bytes<BN, STAGES>()));
-    SWLM_CUDA(cudaFuncSetAttribute(qgemm_tc_kernel<BN, STAGES, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc_smem_bytes<BN, STAGES>()));
+template <typename K>
+int tc_init_one(K kernel, size_t smem) {
+    SWLM_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     return SWLM_OK;
 }
-// packed weights W[n][k/2 bytes] as a 2-D byte tensor; box = 32 bytes (one group) x 128 rows, no swizzle
-int make_w_map(const uint32_t* w, int n, int k, CUtensorMap* map) {
-    TensorMapEncodeFn fn = tensor_map_encode_fn();
-    if (!fn) { set_error("qgemm (tcgen05): cuTensorMapEncodeTiled is not available"); return SWLM_ERR_CUDA; }
-    const cuuint64_t dims[2] = {(cuuint64_t)k / 2, (cuuint64_t)n};
-    const cuuint64_t strides[1] = {(cuuint64_t)k / 2};
-    const cuuint32_t box[2] = {32, (cuuint32_t)kTcRows};
-    const cuuint32_t estr[2] = {1, 1};
-    const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<uint32_t*>(w), dims, strides, box, estr,
-                          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) { set_error("qgemm (tcgen05): cuTensorMapEncodeTiled failed for the weights (%d)", (int)r); return SWLM_ERR_CUDA; }
-    return SWLM_OK;
-}
-
-template <int BN, int STAGES>
-int tc_launch_one(const QGemmTcParams& p, bool f16, cudaStream_t s) {
-    CUtensorMap xmap, wmap;
-    int rc = make_x_map(p.x, p.x_stride, p.m, p.x_stride, BN, &xmap);   // the appended columns are part of the tensor
+template <int BN, int STAGES, int PER_SM>
+int tc_launch_short(QGemmTcParams& p, bool f16, const __half* xh, int xh_stride, int splits, cudaStream_t s) {
+    CUtensorMap xmap;
+    const int rc = make_x_map(xh, xh_stride, p.m, BN, &xmap);
     if (rc) return rc;
-    if ((rc = make_w_map(p.w, p.n, p.k, &wmap))) return rc;
-    const int splits = p.split_steps > 0 ? (p.k / kTcBK + p.split_steps - 1) / p.split_steps : 1;
-    const dim3 grid((unsigned)((p.n + kTcRows - 1) / kTcRows), (unsigned)((p.m + BN - 1) / BN), (unsigned)splits);
-    const cudaError_t e = f16 ? launch_k(qgemm_tc_kernel<BN, STAGES, true>, grid, dim3(kTcAllThreads), tc_smem_bytes<BN, STAGES>(), s, p, xmap, wmap)
-                              : launch_k(qgemm_tc_kernel<BN, STAGES, false>, grid, dim3(kTcAllThreads), tc_smem_bytes<BN, STAGES>(), s, p, xmap, wmap);
-    if (e != cudaSuccess) return cuda_fail(e, "qgemm_tc launch");
-    if (splits > 1) {
-        const size_t total = (size_t)p.m * p.n;
-        const cudaError_t e2 = launch_k(tc_sum_splits_kernel, dim3((unsigned)std::min<size_t>(296, (total + 1023) / 1024)), dim3(256), 0, s,
-                                        (const float*)p.part, splits, p.m, p.n, p.out);
-        if (e2 != cudaSuccess) return cuda_fail(e2, "qgemm_tc split sum launch");
-    }
-    return SWLM_OK;
+    p.splits = splits;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)((p.row_tiles + 7) / 8 * splits), (unsigned)((p.m + BN - 1) / BN));
+    cfg.blockDim = dim3((kTcDeqWarps + 2) * 32); cfg.dynamicSmemBytes = tc_smem_bytes(BN, STAGES); cfg.stream = s;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)splits; attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr; cfg.numAttrs = pdl_enabled() ? 2 : 1;
+    const cudaError_t e = f16 ? cudaLaunchKernelEx(&cfg, qgemm_tc_short_kernel<BN, STAGES, PER_SM, true>, p, xmap)
+                              : cudaLaunchKernelEx(&cfg, qgemm_tc_short_kernel<BN, STAGES, PER_SM, false>, p, xmap);
+    return e == cudaSuccess ? SWLM_OK : cuda_fail(e, "qgemm_tc short launch");
+}
+int tc_launch_long(QGemmTcParams& p, bool f16, const __half* xh, int xh_stride, cudaStream_t s) {
+    CUtensorMap xmap;
+    const int rc = make_x_map(xh, xh_stride, p.m, kTcPairRows, &xmap);
+    if (rc) return rc;
+    p.splits = 1;
+    p.tok_tiles = (p.m + 255) / 256;
+    p.n_tiles = (p.row_tiles + 15) / 16 * p.tok_tiles;
+    const dim3 grid((unsigned)(2 * std::min(p.n_tiles, kTcSMs / 2))), block((kTcDeqWarps + 2 + kTcEpiWarps) * 32);
+    const size_t smem = tc_smem_bytes(kTcPairRows, kTcStagesPair);
+    const cudaError_t e = f16 ? launch_k(qgemm_tc_kernel<kTcStagesPair, true>, grid, block, smem, s, p, xmap)
+                              : launch_k(qgemm_tc_kernel<kTcStagesPair, false>, grid, block, smem, s, p, xmap);
+    return e == cudaSuccess ? SWLM_OK : cuda_fail(e, "qgemm_tc launch");
 }
 
-// K ranges for a launch of at most 64 token rows: as many as keep all CTAs resident at once (two per SM for the
-// 64-token tile: 576 threads x 42 registers, 74 KB of shared memory, 128 columns of tensor memory each), each a whole
-// number of 8-group blocks (the scale/zero vectors are read 8 groups at a time) and all of equal length. 0 = no split.
-constexpr int kTcSplitMaxRows = 64;
-constexpr int kTcSplitMaxCtas = 296;
-constexpr size_t kTcSplitBytes = (size_t)kTcSplitMaxRows * kTcSplitMaxCtas * kTcRows * 4;   // fp32 partial sums of all CTAs
-int tc_pick_split_steps(int m, int n, int k) {
-    static const bool off = [] { const char* v = getenv("SWLM_TC_KSPLIT"); return v && v[0] == '0'; }();
-    if (off || m > kTcSplitMaxRows) return 0;
-    static const int cap = [] { const char* v = getenv("SWLM_TC_KSPLIT_CTAS"); const int c = v ? atoi(v) : 0; return c >= 1 && c <= kTcSplitMaxCtas ? c : kTcSplitMaxCtas; }();
-    const int n_tiles = (n + kTcRows - 1) / kTcRows, kt_total = k / kTcBK;
-    int best = 0;
-    for (int per = kt_total - 8; per >= 8; per -= 8) {
-        if (kt_total % per) continue;
-        if (n_tiles * (kt_total / per) > cap) break;
-        best = per;
+// columns of one plane of appended group sums (whole 64s) and of all of them in whole steps, for `kt` groups
+int ext_plane_cols(int kt) { return (kt + 63) / 64 * 64; }
+int ext_cols(int kt) { return (3 * ext_plane_cols(kt) + kTcStep - 1) / kTcStep * kTcStep; }
+int kt_padded(int k) { return (k / 64 + 3) / 4 * 4; }
+
+// How a product of m rows over `tiles16` row tiles runs: the form with the least time by what was measured over K = 2048 .. 14336,
+// n = 2048 .. 128256 and m = 20 .. 512 (us; graphs of launches, weights from memory). A CTA alone on its SM takes 0.45 us per step
+// (0.5 with 128 rows), two of them 0.9; a pair of the long form 0.87. A launch starts and ends in about 6. Cutting K over a cluster
+// costs the exchange: 5 over four CTAs, 7 to 9 over two (4096 x 4096 at 41 rows: 20.7 / 19.1 / 14.7 for 1, 2, 4; 14336 -> 4096: 62 / 43 / 30),
+// and over eight more than it saves (2048 x 2048: 11.6 for 4, 18.6 for 8). One CTA per SM with its deeper rings is the better
+// form while all tiles fit the GPU (16384 x 2048 at 41 rows 14.6 against 19.9), two per SM beyond (28672 x 4096: 37.6 against 42.5).
+struct TcChoice { int bn, per_sm, splits; };
+TcChoice tc_choose(int m, int tiles16, int steps) {
+    const int row_tiles = (tiles16 + 7) / 8, bn = m <= 32 ? 32 : m <= 64 ? 64 : 128;
+    const long long tiles = (long long)row_tiles * ((m + bn - 1) / bn);
+    TcChoice best{bn, 1, 1};
+    double least = 1e30;
+    auto offer = [&](double cost, const TcChoice& c) { if (cost < least) { least = cost; best = c; } };
+    for (int z = 1; z <= 4 && z <= steps; z *= 2) {
+        const double exchange = z == 1 ? 0 : z == 4 ? 5 : bn == 128 ? 9 : 7;
+        offer((double)((tiles * z + kTcSMs - 1) / kTcSMs) * ((bn == 128 ? 0.5 : 0.45) * ((steps + z - 1) / z) + 2) + 4 + exchange, {bn, 1, z});
+    }
+    if (bn <= 64 && tiles > kTcSMs) offer((double)((tiles + 2 * kTcSMs - 1) / (2 * kTcSMs)) * (0.9 * steps + 2) + 4, {bn, 2, 1});
+    if (m > 128) {
+        const long long pairs = (long long)((tiles16 + 15) / 16) * ((m + 255) / 256);
+        offer((double)((pairs + kTcSMs / 2 - 1) / (kTcSMs / 2)) * (0.87 * steps + 1.5) + 5, {256, 1, 1});
     }
     return best;
 }
 
 }  // namespace
 
+template <int BN, int STAGES, int PER_SM>
+static int tc_init_short() {
+    const int rc = tc_init_one(qgemm_tc_short_kernel<BN, STAGES, PER_SM, false>, tc_smem_bytes(BN, STAGES));
+    return rc ? rc : tc_init_one(qgemm_tc_short_kernel<BN, STAGES, PER_SM, true>, tc_smem_bytes(BN, STAGES));
+}
 int qgemm_tc_init() {
     int rc;
-    if ((rc = tc_init_one<64, 6>())) return rc;
-    if ((rc = tc_init_one<128, 6>())) return rc;
-    if ((rc = tc_init_one<256, 6>())) return rc;
+    if ((rc = tc_init_short<32, kTcStages32x2, 2>()) || (rc = tc_init_short<32, kTcStages32, 1>()) || (rc = tc_init_short<64, kTcStages64x2, 2>()) ||
+        (rc = tc_init_short<64, kTcStages64, 1>()) || (rc = tc_init_short<128, kTcStages128, 1>()) ||
+        (rc = tc_init_one(qgemm_tc_kernel<kTcStagesPair, false>, tc_smem_bytes(kTcPairRows, kTcStagesPair))) ||
+        (rc = tc_init_one(qgemm_tc_kernel<kTcStagesPair, true>, tc_smem_bytes(kTcPairRows, kTcStagesPair)))) return rc;
     return SWLM_OK;
 }
 
-// Y[m][n] = bf16(X[m][k] . fp16(W)^T) on the tcgen05 path. xh (m * k fp16 values) and rscale (m floats) are scratch
-// for the fp16 copy of the activations. `status` is a device word the kernel sets when a
-// bounded wait expires. Token tile: 256 when there are that many tokens (each dequantised weight then feeds
-// 256 columns of the MMA), else 128 or 64.
-// columns of one plane of appended group sums: the groups of a row, padded to whole 64-column steps
-static int ext_plane_cols(int k) { return (k / 64 + 63) / 64 * 64; }
-// [partial sums of a K-split launch][fp16 activations + group sums][one float per token row]
-size_t qgemm_tc_scratch_bytes(int m, int k) { return kTcSplitBytes + ((size_t)m * (k + 3 * ext_plane_cols(k)) * 2 + 255) / 256 * 256 + (size_t)m * 4; }
+// [fp16 activations + group sums][one float per row]
+static int xh_cols(int k) { return kt_padded(k) * 64 + ext_cols(kt_padded(k)); }
+size_t qgemm_tc_scratch_bytes(int m, int k) { return ((size_t)m * xh_cols(k) * 2 + 255) / 256 * 256 + (size_t)m * 4; }
 
-int qgemm_tc_launch_count(const Q4Raw& w, int m, bool reuse_x) {
-    return (reuse_x ? 0 : 1) + 1 + (tc_pick_split_steps(m, w.n, w.k) > 0 ? 1 : 0);
+int qgemm_tc_launch_count(bool reuse_x) { return (reuse_x ? 0 : 1) + 1; }
+
+static F16Rows f16_rows(int m, int k, void* scratch) {
+    F16Rows f{};
+    f.k = k; f.k_pad = kt_padded(k) * 64; f.g_pad = ext_plane_cols(kt_padded(k)); f.xh = static_cast<__half*>(scratch); f.stride = xh_cols(k);
+    f.rscale = reinterpret_cast<float*>(static_cast<unsigned char*>(scratch) + ((size_t)m * f.stride * 2 + 255) / 256 * 256);
+    return f;
 }
 
-int launch_qgemm_tc(const Q4Raw& w, int m, const __nv_bfloat16* x, int x_stride, __nv_bfloat16* y, int y_stride,
-                    void* scratch, int* status, cudaStream_t s, bool reuse_x, const TcSegments* segments) {
-    float* part = static_cast<float*>(scratch);
-    __half* xh = scratch ? reinterpret_cast<__half*>(static_cast<unsigned char*>(scratch) + kTcSplitBytes) : nullptr;
-    const int g_pad = ext_plane_cols(w.k), xh_stride = w.k + 3 * g_pad;
-    float* rscale = scratch ? reinterpret_cast<float*>(static_cast<unsigned char*>(scratch) + kTcSplitBytes + ((size_t)m * xh_stride * 2 + 255) / 256 * 256) : nullptr;
-    if (w.k % kTcBK || (x_stride & 7) || (reinterpret_cast<uintptr_t>(x) & 15) || (reinterpret_cast<uintptr_t>(xh) & 15) || !xh || !rscale) {
+int launch_norm_to_f16(int mode, int m, int dim, const __nv_bfloat16* in, int in_stride, __nv_bfloat16* residual, int res_stride, const __nv_bfloat16* weight,
+                       float eps, float weight_bias, __nv_bfloat16* out, int out_stride, void* scratch, cudaStream_t s) {
+    if (dim % 64 || in_stride % 8 || res_stride % 8 || out_stride % 8 || dim > 12288) { set_error("rmsnorm: dim=%d", dim); return SWLM_ERR_INVALID; }
+    const F16Rows f = f16_rows(m, dim, scratch);
+    const size_t smem = (size_t)dim * 4;
+    cudaError_t e;
+    if (mode == SWLM_STEP_COPY_RMSNORM) e = launch_k(norm_to_f16_kernel<0>, dim3((unsigned)m), dim3(256), smem, s, in, in_stride, residual, res_stride, weight, eps, weight_bias, out, out_stride, f);
+    else if (mode == SWLM_STEP_RESADD_COPY_RMSNORM) e = launch_k(norm_to_f16_kernel<1>, dim3((unsigned)m), dim3(256), smem, s, in, in_stride, residual, res_stride, weight, eps, weight_bias, out, out_stride, f);
+    else e = launch_k(norm_to_f16_kernel<2>, dim3((unsigned)m), dim3(256), smem, s, in, in_stride, residual, res_stride, weight, eps, weight_bias, out, out_stride, f);
+    return e == cudaSuccess ? SWLM_OK : cuda_fail(e, "norm_to_f16 launch");
+}
+
+// Y[m][n] = bf16(X[m][k] . W^T). `scratch` (qgemm_tc_scratch_bytes) takes the fp16 copy of the activations; `status` is a device
+// word the kernel sets when a bounded wait expires.
+int launch_qgemm_tc(const Q4Tiled& w, int m, const __nv_bfloat16* x, int x_stride, const TcSegments& out, int epilogue, int gated_act,
+                    void* scratch, int* status, cudaStream_t s, bool reuse_x) {
+    const F16Rows f = f16_rows(m, w.k, scratch);
+    __half* const xh = f.xh;
+    const int xh_stride = f.stride;
+    if (w.k % 64 || (x_stride & 7) || (reinterpret_cast<uintptr_t>(x) & 15) || (reinterpret_cast<uintptr_t>(xh) & 15) || !xh) {
         set_error("qgemm (tcgen05): bad shape, alignment or scratch");
         return SWLM_ERR_INVALID;
     }
-    // xh: m rows of w.k fp16 values followed by three planes of g_pad group sums
-    // (reuse_x: the scratch still holds the copy of these very rows, made for the product before this one)
+    QGemmTcParams p{};
+    p.tiles = w.tiles; p.sb = reinterpret_cast<const unsigned*>(w.sb); p.row_tiles = w.row_tiles; p.kt = w.kt_pad; p.g_pad = f.g_pad;
+    p.rscale = f.rscale;
+    p.m = m; p.status = status;
+    p.real_steps = w.kt_pad * 64 / kTcStep; p.steps = xh_stride / kTcStep;
+    p.gated = epilogue == QGEMV_EPI_SWIGLU; p.gated_act = gated_act;
+    p.out = out;
+    if (out.count < 1 || out.count > 3 || (p.gated && (out.count != 1 || !w.interleaved))) { set_error("qgemm (tcgen05): output segments"); return SWLM_ERR_INVALID; }
+    for (int q = out.count; q < 3; ++q) p.out.end[q] = p.out.end[out.count - 1];   // never stored to
+    // (reuse_x: the scratch still holds the copy of these very rows, made for the product before this one or by their norm)
     if (!reuse_x) {
-        cudaError_t e = launch_k(x_to_f16_kernel, dim3((unsigned)m), dim3(256), 0, s, x, x_stride, w.k, g_pad, xh, xh_stride, rscale);
+        const cudaError_t e = w.k <= 16384 ? launch_k(x_to_f16_kernel<true>, dim3((unsigned)m), dim3(256), 0, s, x, x_stride, f)
+                                           : launch_k(x_to_f16_kernel<false>, dim3((unsigned)m), dim3(256), 0, s, x, x_stride, f);
         if (e != cudaSuccess) return cuda_fail(e, "x_to_f16 launch");
     }
-    QGemmTcParams p{};
-    p.w = w.w; p.scales = w.scales; p.biases = w.biases; p.n = w.n; p.k = w.k;
-    p.x = xh; p.rscale = rscale; p.x_stride = xh_stride; p.m = m; p.status = status;
-    if (segments) {
-        p.out = *segments;
-        if (p.out.count < 1 || p.out.count > 3 || p.out.end[p.out.count - 1] != w.n) { set_error("qgemm (tcgen05): output segments do not cover the %d weight rows", w.n); return SWLM_ERR_INVALID; }
-        for (int q = p.out.count; q < 3; ++q) p.out.end[q] = p.out.end[p.out.count - 1];   // never selected
-    } else {
-        p.out.count = 1; p.out.y[0] = y; p.out.stride[0] = y_stride; p.out.end[0] = p.out.end[1] = p.out.end[2] = w.n;
-    }
-    p.ext_steps = 3 * g_pad / 64;
-    p.part = part;
-    p.split_steps = tc_pick_split_steps(m, w.n, w.k);
-    int rc;
-    int bn = m > 128 ? 256 : m > 64 ? 128 : 64;
-    static const int forced_bn = [] { const char* v = getenv("SWLM_TC_BN"); return v ? atoi(v) : 0; }();
-    if (forced_bn == 64 || forced_bn == 128 || forced_bn == 256) bn = forced_bn;
-    if (bn == 256) rc = tc_launch_one<256, 6>(p, w.sb_f16, s);
-    else if (bn == 128) rc = tc_launch_one<128, 6>(p, w.sb_f16, s);
-    else rc = tc_launch_one<64, 6>(p, w.sb_f16, s);
-    return rc;
+    const TcChoice c = tc_choose(m, w.row_tiles, p.steps);
+    if (c.bn == 32) return c.per_sm == 2 ? tc_launch_short<32, kTcStages32x2, 2>(p, w.sb_f16, xh, xh_stride, c.splits, s) : tc_launch_short<32, kTcStages32, 1>(p, w.sb_f16, xh, xh_stride, c.splits, s);
+    if (c.bn == 64) return c.per_sm == 2 ? tc_launch_short<64, kTcStages64x2, 2>(p, w.sb_f16, xh, xh_stride, c.splits, s) : tc_launch_short<64, kTcStages64, 1>(p, w.sb_f16, xh, xh_stride, c.splits, s);
+    if (c.bn == 128) return tc_launch_short<128, kTcStages128, 1>(p, w.sb_f16, xh, xh_stride, c.splits, s);
+    return tc_launch_long(p, w.sb_f16, xh, xh_stride, s);
 }
 
 }  // namespace swlm

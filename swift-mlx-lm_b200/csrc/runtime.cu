@@ -152,19 +152,6 @@ int add_q4_raw(swlm_ctx* ctx, const char* name, int n, int k, const uint32_t* w,
             if (uses) { cudaFree(it->second.tiles); cudaFree(it->second.sb); it = ctx->tiled.erase(it); }
             else ++it;
         }
-        for (auto it = ctx->raw_cat.begin(); it != ctx->raw_cat.end();) {
-            bool uses = false;
-            size_t start = 0;
-            const std::string& key = it->first;
-            while (start <= key.size()) {
-                size_t end = key.find('|', start);
-                if (end == std::string::npos) end = key.size();
-                uses |= key.compare(start, end - start, needle) == 0;
-                start = end + 1;
-            }
-            if (uses) { cudaFree(it->second.w); cudaFree(it->second.scales); cudaFree(it->second.biases); it = ctx->raw_cat.erase(it); }
-            else ++it;
-        }
     }
     Q4Raw r;
     r.n = sl.rows * sl.parts; r.k = sl.cols; r.sb_f16 = f16; r.shard_kind = shard_kind;
@@ -769,34 +756,38 @@ int capture_graph(swlm_state* s, bool body_only, cudaGraphExec_t* out) {
     return SWLM_OK;
 }
 
+// Row-wise execution: does the product behind norm step `si` take its rows in the fp16 form the norm can write?
+bool norm_converts(const swlm_plan* plan, size_t si) {
+    const std::vector<swlm_step>& st = plan->steps;
+    if (!plan->rows_groups_ready || si + 1 >= st.size() || st[si + 1].kind != SWLM_STEP_QGEMV || plan->rows_groups[si + 1].count == 0) return false;
+    const swlm_step& n = st[si];
+    return (n.kind == SWLM_STEP_COPY_RMSNORM || n.kind == SWLM_STEP_RESADD_COPY_RMSNORM || n.kind == SWLM_STEP_RESADD_RMSNORM) &&
+           st[si + 1].in_buf == n.out_buf && plan->rows_groups[si + 1].w->k == n.n && n.n % 64 == 0 && n.n <= 12288;
+}
+
 int launches_per_step(const swlm_plan* plan, bool body_only) {
     int n = 0;
     bool has_argmax = false;
     if (plan->stream()) return stream_launches_per_step(plan);
     if (plan->desc.max_batch > kQGemvMaxRows) {
-        // more than 16 sequences: the unfused steps, as enqueue_rows issues them
+        // more than 16 sequences: the steps as enqueue_rows issues them
         int converted_buf = -1, converted_k = 0;
-        for (const swlm_step& st : plan->steps) {
+        for (size_t si = 0; si < plan->steps.size(); ++si) {
+            const swlm_step& st = plan->steps[si];
+            const swlm_plan::RowsGroup* grp = plan->rows_groups_ready ? &plan->rows_groups[si] : nullptr;
+            if (grp && grp->count == 0) continue;
             const bool head = st.kind == SWLM_STEP_RESADD_RMSNORM || st.kind == SWLM_STEP_ARGMAX ||
                               (st.kind == SWLM_STEP_QGEMV && st.out_buf == SWLM_BUF_LOGITS);
             if (head && body_only) continue;
             if (st.kind == SWLM_STEP_QGEMV) {
-                const size_t si = (size_t)(&st - plan->steps.data());
-                const Q4Raw* raw = nullptr;
-                if (plan->rows_groups_ready) {
-                    if (plan->rows_groups[si].count == 0) continue;
-                    raw = plan->rows_groups[si].raw;
-                } else {
-                    auto it = plan->ctx->raw.find(st.weight);
-                    if (it != plan->ctx->raw.end()) raw = &it->second;
-                }
-                if (!raw) continue;
-                const bool reuse = converted_buf == st.in_buf && converted_k == raw->k;
-                n += qgemm_tc_launch_count(*raw, plan->desc.max_batch, reuse);
-                converted_buf = st.in_buf; converted_k = raw->k;
+                if (!grp) { n += 2; continue; }
+                n += qgemm_tc_launch_count(converted_buf == st.in_buf && converted_k == grp->w->k);
+                converted_buf = st.in_buf; converted_k = grp->w->k;
+                if (grp->gated && plan->steps[si + 2].out_buf == converted_buf) converted_buf = -1;
                 continue;
             }
             converted_buf = -1;
+            if (norm_converts(plan, si)) { converted_buf = st.out_buf; converted_k = st.n; }
             n += st.kind == SWLM_STEP_ARGMAX ? 2 : 1;
             has_argmax |= st.kind == SWLM_STEP_ARGMAX;
         }
@@ -927,34 +918,6 @@ int check_position_room(swlm_state* s, int steps) {
 constexpr int kPrefillMinChunk = 32;
 
 // can the plan's steps run row-wise (enqueue_rows)?
-// The rows of several source-layout tensors one after the other (q | k | v, gate | up), built once per set of names.
-int get_raw_cat(swlm_ctx* ctx, const std::vector<std::string>& names, const Q4Raw** out) {
-    std::string key = names[0];
-    for (size_t i = 1; i < names.size(); ++i) key += "|" + names[i];
-    auto hit = ctx->raw_cat.find(key);
-    if (hit != ctx->raw_cat.end()) { *out = &hit->second; return SWLM_OK; }
-    Q4Raw cat;
-    const Q4Raw& first = ctx->raw.at(names[0]);
-    cat.k = first.k; cat.sb_f16 = first.sb_f16; cat.shard_kind = first.shard_kind;
-    for (const std::string& nm : names) cat.n += ctx->raw.at(nm).n;
-    const size_t wpr = (size_t)cat.k / 8, gpr = (size_t)cat.k / 64;
-    int rc;
-    if ((rc = dev_alloc(&cat.w, (size_t)cat.n * wpr, &ctx->bytes))) return rc;
-    if ((rc = dev_alloc(&cat.scales, (size_t)cat.n * gpr, &ctx->bytes))) return rc;
-    if ((rc = dev_alloc(&cat.biases, (size_t)cat.n * gpr, &ctx->bytes))) return rc;
-    size_t row = 0;
-    for (const std::string& nm : names) {
-        const Q4Raw& r = ctx->raw.at(nm);
-        SWLM_CUDA(cudaMemcpy(cat.w + row * wpr, r.w, (size_t)r.n * wpr * 4, cudaMemcpyDeviceToDevice));
-        SWLM_CUDA(cudaMemcpy(cat.scales + row * gpr, r.scales, (size_t)r.n * gpr * 2, cudaMemcpyDeviceToDevice));
-        SWLM_CUDA(cudaMemcpy(cat.biases + row * gpr, r.biases, (size_t)r.n * gpr * 2, cudaMemcpyDeviceToDevice));
-        row += r.n;
-    }
-    ctx->raw_cat[key] = cat;
-    *out = &ctx->raw_cat[key];
-    return SWLM_OK;
-}
-
 // Decide which products of the unfused step list run together (allocates: never call while a stream is capturing).
 // SWLM_ROWS_FUSE=0 keeps one product per step.
 int ensure_rows_groups(swlm_plan* plan) {
@@ -963,18 +926,42 @@ int ensure_rows_groups(swlm_plan* plan) {
     swlm_ctx* ctx = plan->ctx;
     const std::vector<swlm_step>& st = plan->steps;
     plan->rows_groups.assign(st.size(), swlm_plan::RowsGroup{});
+    // Are the values of `buf` that the gated step `at` reads of no use afterwards? The rows of a prompt are scratch, those of more
+    // than 16 sequences are buffers that the host may read after a step: there something has to overwrite them.
+    auto gone_after = [&](int buf, size_t at) {
+        if (st[at].out_buf == buf) return true;
+        for (size_t j = at + 1; j < st.size(); ++j) {
+            const swlm_step& c = st[j];
+            if (c.in_buf == buf || c.in2_buf == buf || c.in3_buf == buf || (c.kind == SWLM_STEP_SSM_RECURRENCE && c.in4_buf == buf)) return false;
+            if (c.kind != SWLM_STEP_QK_NORM && c.kind != SWLM_STEP_ARGMAX && c.out_buf == buf) return true;
+        }
+        return plan->desc.max_batch <= kQGemvMaxRows;
+    };
     for (size_t i = 0; i < st.size(); ++i) {
-        if (plan->rows_groups[i].count == 0 || st[i].kind != SWLM_STEP_QGEMV) continue;
+        swlm_plan::RowsGroup& grp = plan->rows_groups[i];
+        if (grp.count == 0 || st[i].kind != SWLM_STEP_QGEMV) continue;
         auto it = ctx->raw.find(st[i].weight);
         if (it == ctx->raw.end()) { set_error("tensor '%s' not in the weight store", st[i].weight); return SWLM_ERR_NOT_FOUND; }
         const Q4Raw& r0 = it->second;
-        plan->rows_groups[i].raw = &r0;
         const bool partial = ctx->tp_size > 1 && r0.shard_kind == SWLM_SHARD_ROW;   // its rows go through an exchange
-        if (!fuse || st[i].out_buf == SWLM_BUF_LOGITS || partial) continue;
+        const bool alone = !fuse || st[i].out_buf == SWLM_BUF_LOGITS || partial;
         std::vector<std::string> names{st[i].weight};
-        size_t j = i + 1;
-        while (j < st.size() && names.size() < 3 && st[j].kind == SWLM_STEP_QGEMV && st[j].in_buf == st[i].in_buf &&
-               st[j].out_buf != st[i].in_buf && st[j].out_buf != SWLM_BUF_LOGITS) {
+        grp.n[0] = r0.n;
+        int mode = 0;
+        if (!alone && i + 2 < st.size() && st[i + 1].kind == SWLM_STEP_QGEMV && (st[i + 2].kind == SWLM_STEP_SWIGLU || st[i + 2].kind == SWLM_STEP_GEGLU) &&
+            st[i + 1].in_buf == st[i].in_buf && st[i + 2].in_buf == st[i].out_buf && st[i + 2].in2_buf == st[i + 1].out_buf && r0.n % 8 == 0) {
+            auto jt = ctx->raw.find(st[i + 1].weight);
+            if (jt != ctx->raw.end() && jt->second.k == r0.k && jt->second.n == r0.n && jt->second.sb_f16 == r0.sb_f16 &&
+                gone_after(st[i].out_buf, i + 2) && gone_after(st[i + 1].out_buf, i + 2)) {
+                names.push_back(st[i + 1].weight);
+                mode = 1;
+                grp.gated = true;
+                grp.count = 3;
+                plan->rows_groups[i + 1].count = plan->rows_groups[i + 2].count = 0;
+            }
+        }
+        for (size_t j = i + 1; !alone && !grp.gated && j < st.size() && names.size() < 3 && st[j].kind == SWLM_STEP_QGEMV && st[j].in_buf == st[i].in_buf &&
+                               st[j].out_buf != st[i].in_buf && st[j].out_buf != SWLM_BUF_LOGITS; ++j) {
             auto jt = ctx->raw.find(st[j].weight);
             if (jt == ctx->raw.end()) break;
             const Q4Raw& rj = jt->second;
@@ -982,16 +969,13 @@ int ensure_rows_groups(swlm_plan* plan) {
             bool clash = false;
             for (size_t q = i; q < j; ++q) clash |= st[q].out_buf == st[j].out_buf;
             if (clash) break;
+            grp.n[names.size()] = rj.n;
             names.push_back(st[j].weight);
-            ++j;
+            grp.count = grp.parts = (int)names.size();
+            plan->rows_groups[j].count = 0;
         }
-        if (names.size() < 2) continue;
-        const Q4Raw* cat = nullptr;
-        int rc = get_raw_cat(ctx, names, &cat);
+        const int rc = get_tiled(ctx, names, mode, &grp.w);
         if (rc) return rc;
-        plan->rows_groups[i].count = (int)names.size();
-        plan->rows_groups[i].raw = cat;
-        for (size_t q = i + 1; q < j; ++q) plan->rows_groups[q].count = 0;
     }
     plan->rows_groups_ready = true;
     return SWLM_OK;
@@ -1083,12 +1067,19 @@ int enqueue_rows(swlm_state* s, bool wide, const int32_t* tokens, int c, int pos
     int rc = SWLM_OK;
     const __nv_bfloat16* converted = nullptr;  // rows whose fp16 copy the product scratch still holds
     int converted_k = 0;
-    auto product = [&](const Q4Raw& raw, int rows, const __nv_bfloat16* x, int xs, __nv_bfloat16* y, int ys, const TcSegments* seg = nullptr) {
-        const bool reuse = converted == x && converted_k == raw.k;
-        const int r = launch_qgemm_tc(raw, rows, x, xs, y, ys, wide ? s->wide_xh : s->pf_xh, s->pf_status, stream, reuse, seg);
-        converted = x; converted_k = raw.k;
-        s->launches += qgemm_tc_launch_count(raw, rows, reuse);
+    auto product = [&](const swlm_plan::RowsGroup& g, int rows, const __nv_bfloat16* x, int xs, const TcSegments& out, int act = GATED_ACT_SILU) {
+        const bool reuse = converted == x && converted_k == g.w->k;
+        const int r = launch_qgemm_tc(*g.w, rows, x, xs, out, g.gated ? QGEMV_EPI_SWIGLU : QGEMV_EPI_STORE, act, wide ? s->wide_xh : s->pf_xh, s->pf_status, stream, reuse);
+        converted = x; converted_k = g.w->k;
+        for (int q = 0; q < out.count; ++q)
+            if (out.y[q] == x) converted = nullptr;   // (the gated result may take its input's place)
+        s->launches += qgemm_tc_launch_count(reuse);
         return r;
+    };
+    auto whole = [](int n, __nv_bfloat16* y, int stride) {
+        TcSegments o;
+        o.end[0] = n; o.y[0] = y; o.stride[0] = stride;
+        return o;
     };
     bool advanced = false;
     const int tp = ctx->tp_size;   // > 1 only for prompt chunks: heads, conv channels and the products' rows are this rank's share
@@ -1098,6 +1089,7 @@ int enqueue_rows(swlm_state* s, bool wide, const int32_t* tokens, int c, int pos
         const swlm_plan::RowsGroup& grp = plan->rows_groups[si];
         if (grp.count == 0) continue;   // ran with an earlier product
         const bool is_product = st.kind == SWLM_STEP_QGEMV;
+        bool by_norm = false;
         switch (st.kind) {
         case SWLM_STEP_EMBED:
             if (const DenseTensor* table = find_dense(ctx, st.weight))
@@ -1108,44 +1100,55 @@ int enqueue_rows(swlm_state* s, bool wide, const int32_t* tokens, int c, int pos
             break;
         case SWLM_STEP_COPY_RMSNORM:
         case SWLM_STEP_RESADD_COPY_RMSNORM:
-            rc = launch_rmsnorm(st.kind, c, st.n, pf[st.in_buf], wd[st.in_buf], pf[SWLM_BUF_RESIDUAL], wd[SWLM_BUF_RESIDUAL],
-                                find_dense(ctx, st.weight)->data, st.eps, st.weight_bias, pf[st.out_buf], wd[st.out_buf], stream);
-            s->launches += 1;
-            break;
-        case SWLM_STEP_RESADD_RMSNORM: {  // final norm: part of the output head
-            if (wide ? body_only : head_row < 0) break;
-            const int r0 = wide ? 0 : head_row, rows = wide ? c : 1;
-            rc = launch_rmsnorm(st.kind, rows, st.n, pf[st.in_buf] + (size_t)r0 * wd[st.in_buf], wd[st.in_buf],
-                                pf[SWLM_BUF_RESIDUAL] + (size_t)r0 * wd[SWLM_BUF_RESIDUAL], wd[SWLM_BUF_RESIDUAL],
-                                find_dense(ctx, st.weight)->data, st.eps, st.weight_bias,
-                                pf[st.out_buf] + (size_t)r0 * wd[st.out_buf], wd[st.out_buf], stream);
+        case SWLM_STEP_RESADD_RMSNORM: {
+            const bool last = st.kind == SWLM_STEP_RESADD_RMSNORM;   // final norm: part of the output head
+            if (last && (wide ? body_only : head_row < 0)) break;
+            const int r0 = last && !wide ? head_row : 0, rows = last && !wide ? 1 : c;
+            const __nv_bfloat16* in = pf[st.in_buf] + (size_t)r0 * wd[st.in_buf];
+            __nv_bfloat16 *res = pf[SWLM_BUF_RESIDUAL] + (size_t)r0 * wd[SWLM_BUF_RESIDUAL], *out = pf[st.out_buf] + (size_t)r0 * wd[st.out_buf];
+            const __nv_bfloat16* w = find_dense(ctx, st.weight)->data;
+            if (norm_converts(plan, si)) {
+                rc = launch_norm_to_f16(st.kind, rows, st.n, in, wd[st.in_buf], res, wd[SWLM_BUF_RESIDUAL], w, st.eps, st.weight_bias, out, wd[st.out_buf],
+                                        wide ? s->wide_xh : s->pf_xh, stream);
+                converted = out; converted_k = st.n;
+                by_norm = true;
+            } else {
+                rc = launch_rmsnorm(st.kind, rows, st.n, in, wd[st.in_buf], res, wd[SWLM_BUF_RESIDUAL], w, st.eps, st.weight_bias, out, wd[st.out_buf], stream);
+            }
             s->launches += 1;
             break;
         }
         case SWLM_STEP_QGEMV: {
-            const Q4Raw& raw = *grp.raw;
+            const Q4Raw& raw = ctx->raw.at(st.weight);
+            if (grp.gated) {
+                // gate, up and the activation: one product over the interleaved rows
+                const swlm_step& sa = plan->steps[si + 2];
+                rc = product(grp, c, pf[st.in_buf], wd[st.in_buf], whole(grp.n[0], pf[sa.out_buf], wd[sa.out_buf]),
+                             sa.kind == SWLM_STEP_GEGLU ? GATED_ACT_GELU_TANH : GATED_ACT_SILU);
+                break;
+            }
             if (grp.count > 1) {
-                // q | k | v or gate | up: one product over the concatenated rows, each part to its own buffer
+                // q | k | v: one product over the concatenated rows, each part to its own buffer
                 TcSegments seg;
-                seg.count = grp.count;
+                seg.count = grp.parts;
                 int end = 0;
-                for (int q = 0; q < grp.count; ++q) {
+                for (int q = 0; q < grp.parts; ++q) {
                     const swlm_step& sq = plan->steps[si + q];
-                    end += ctx->raw.at(sq.weight).n;
+                    end += grp.n[q];
                     seg.end[q] = end; seg.y[q] = pf[sq.out_buf]; seg.stride[q] = wd[sq.out_buf];
                 }
-                rc = product(raw, c, pf[st.in_buf], wd[st.in_buf], nullptr, 0, &seg);
+                rc = product(grp, c, pf[st.in_buf], wd[st.in_buf], seg);
                 break;
             }
             if (st.out_buf == SWLM_BUF_LOGITS) {
                 if (wide ? body_only : head_row < 0) break;
                 // the logits buffer belongs to the state (one row per sequence), also for a chunk's last token
-                if (wide) rc = product(raw, c, pf[st.in_buf], wd[st.in_buf], s->buf[SWLM_BUF_LOGITS], wd[SWLM_BUF_LOGITS]);
-                else rc = product(raw, 1, pf[st.in_buf] + (size_t)head_row * wd[st.in_buf], wd[st.in_buf],
-                                  s->buf[SWLM_BUF_LOGITS] + (size_t)seq * wd[SWLM_BUF_LOGITS], wd[SWLM_BUF_LOGITS]);
+                if (wide) rc = product(grp, c, pf[st.in_buf], wd[st.in_buf], whole(raw.n, s->buf[SWLM_BUF_LOGITS], wd[SWLM_BUF_LOGITS]));
+                else rc = product(grp, 1, pf[st.in_buf] + (size_t)head_row * wd[st.in_buf], wd[st.in_buf],
+                                  whole(raw.n, s->buf[SWLM_BUF_LOGITS] + (size_t)seq * wd[SWLM_BUF_LOGITS], wd[SWLM_BUF_LOGITS]));
                 break;
             }
-            rc = product(raw, c, pf[st.in_buf], wd[st.in_buf], pf[st.out_buf], wd[st.out_buf]);
+            rc = product(grp, c, pf[st.in_buf], wd[st.in_buf], whole(raw.n, pf[st.out_buf], wd[st.out_buf]));
             if (!rc && tp > 1 && raw.shard_kind == SWLM_SHARD_ROW) {
                 // row-parallel weight: the rows are partial sums; add them up across the ranks, in place
                 rc = launch_tp_rows_allreduce(s->tp, pf[st.out_buf], wd[st.out_buf], c, raw.n, ++s->tp_rows_epoch,
@@ -1245,7 +1248,7 @@ int enqueue_rows(swlm_state* s, bool wide, const int32_t* tokens, int c, int pos
             return SWLM_ERR_UNSUPPORTED;
         }
         if (rc) return rc;
-        if (!is_product) converted = nullptr;
+        if (!is_product && !by_norm) converted = nullptr;
     }
     if (wide) {
         if (!advanced) { rc = launch_advance(c, s->position, nullptr, stream); s->launches += 1; }
@@ -1312,7 +1315,6 @@ void swlm_ctx_destroy(swlm_ctx* ctx) {
     cudaSetDevice(ctx->device);
     for (auto& kv : ctx->raw) { cudaFree(kv.second.w); cudaFree(kv.second.scales); cudaFree(kv.second.biases); }
     for (auto& kv : ctx->tiled) { cudaFree(kv.second.tiles); cudaFree(kv.second.sb); }
-    for (auto& kv : ctx->raw_cat) { cudaFree(kv.second.w); cudaFree(kv.second.scales); cudaFree(kv.second.biases); }
     for (auto& kv : ctx->dense) cudaFree(kv.second.data);
     for (auto& kv : ctx->densef) cudaFree(kv.second.data);
     for (auto& kv : ctx->matrices) if (!kv.second.view) cudaFree(kv.second.data);
@@ -2399,10 +2401,8 @@ int swlm_op_qgemm_dev(swlm_ctx* ctx, const char* weight, int m, const void* x_de
         SWLM_CUDA(cudaMemsetAsync(ctx->tc_status, 0, sizeof(int), ctx->stream));
         SWLM_CUDA(cudaStreamSynchronize(ctx->stream));
     }
-    // m >= 64: tensor-core contraction straight from the packed source copy
-    auto raw = ctx->raw.find(weight);
-    if (m >= kQGemmTcMinRows && raw != ctx->raw.end() && raw->second.k % 64 == 0) {
-        const size_t need = qgemm_tc_scratch_bytes(m, raw->second.k);
+    if (m >= kQGemmTcMinRows) {   // tensor-core contraction
+        const size_t need = qgemm_tc_scratch_bytes(m, w->k);
         if (need > ctx->op_xh_bytes) {
             SWLM_CUDA(cudaDeviceSynchronize());
             cudaFree(ctx->op_xh);
@@ -2410,23 +2410,19 @@ int swlm_op_qgemm_dev(swlm_ctx* ctx, const char* weight, int m, const void* x_de
             if ((rc = dev_alloc(&ctx->op_xh, need))) return rc;
             ctx->op_xh_bytes = need;
         }
-        return launch_qgemm_tc(raw->second, m, static_cast<const __nv_bfloat16*>(x_dev), raw->second.k,
-                               static_cast<__nv_bfloat16*>(y_dev), raw->second.n, ctx->op_xh, ctx->tc_status, stream);
+        TcSegments out;
+        out.end[0] = w->n; out.y[0] = static_cast<__nv_bfloat16*>(y_dev); out.stride[0] = w->n;
+        return launch_qgemm_tc(*w, m, static_cast<const __nv_bfloat16*>(x_dev), w->k, out, QGEMV_EPI_STORE, GATED_ACT_SILU, ctx->op_xh, ctx->tc_status, stream);
     }
-    // 16 < m < 64 runs as passes of 16 rows: each pass re-streams the weights
-    for (int m0 = 0; m0 < m; m0 += 16) {
-        const int mc = std::min(16, m - m0);
-        rc = op_scratch(ctx, *w, mc);
-        if (rc) return rc;
-        QGemvLaunch a;
-        a.w = w; a.m = mc;
-        a.x = static_cast<const __nv_bfloat16*>(x_dev) + (size_t)m0 * w->k; a.x_stride = w->k;
-        a.y[0] = static_cast<__nv_bfloat16*>(y_dev) + (size_t)m0 * w->n; a.y_stride[0] = w->n; a.seg_end[0] = w->n;
-        a.partial = ctx->op_partial; a.counters = ctx->op_counters;
-        rc = launch_qgemv(a, stream);
-        if (rc) return rc;
-    }
-    return SWLM_OK;
+    if (m <= 0) return SWLM_OK;
+    rc = op_scratch(ctx, *w, m);
+    if (rc) return rc;
+    QGemvLaunch a;
+    a.w = w; a.m = m;
+    a.x = static_cast<const __nv_bfloat16*>(x_dev); a.x_stride = w->k;
+    a.y[0] = static_cast<__nv_bfloat16*>(y_dev); a.y_stride[0] = w->n; a.seg_end[0] = w->n;
+    a.partial = ctx->op_partial; a.counters = ctx->op_counters;
+    return launch_qgemv(a, stream);
 }
 
 int swlm_op_qgemm(swlm_ctx* ctx, const char* weight, int m, const uint16_t* x_bf16, uint16_t* y_bf16) {

@@ -314,23 +314,25 @@ int launch_flash_decode_static(int device, int m, int heads, int kv_heads, int h
                                const __nv_bfloat16* q, const __nv_bfloat16* k, const __nv_bfloat16* v, __nv_bfloat16* out,
                                cudaStream_t s);
 
-// Tensor-core (tcgen05) form of the quantised product for m >= kQGemmTcMinRows, fed from the packed source copy.
-constexpr int kQGemmTcMinRows = 17;   // 17..63 token rows ride in a 64-token tile whose other rows are zero
+// Tensor-core (tcgen05) form of the quantised product for m >= kQGemmTcMinRows.
+constexpr int kQGemmTcMinRows = 17;
 int qgemm_tc_init();
-size_t qgemm_tc_scratch_bytes(int m, int k);   // fp16 copy of the activations + one float per token row
-// kernels one call of launch_qgemm_tc issues: the fp16 copy of the rows (unless reused), the product, and the sum over
-// K ranges when a short launch is split
-int qgemm_tc_launch_count(const Q4Raw& w, int m, bool reuse_x);
+size_t qgemm_tc_scratch_bytes(int m, int k);   // fp16 copy of the activations + one float per row
+// kernels one call of launch_qgemm_tc issues: the fp16 copy of the rows (unless reused) and the product
+int qgemm_tc_launch_count(bool reuse_x);
 // Where the rows of a product over concatenated weights go: rows [end[q-1], end[q]) to y[q] (up to three outputs,
-// e.g. q | k | v); null = all rows to `y`.
+// e.g. q | k | v). With the gated epilogue one output, end[0] its width.
 struct TcSegments {
     int count = 1;
     int end[3] = {0, 0, 0};
     __nv_bfloat16* y[3] = {nullptr, nullptr, nullptr};
     int stride[3] = {0, 0, 0};
 };
-int launch_qgemm_tc(const Q4Raw& w, int m, const __nv_bfloat16* x, int x_stride, __nv_bfloat16* y, int y_stride,
-                    void* scratch, int* status, cudaStream_t s, bool reuse_x = false, const TcSegments* segments = nullptr);
+// launch_rmsnorm whose result also goes, converted, to `scratch` for a product of the same m rows behind it
+int launch_norm_to_f16(int mode, int m, int dim, const __nv_bfloat16* in, int in_stride, __nv_bfloat16* residual, int res_stride, const __nv_bfloat16* weight,
+                       float eps, float weight_bias, __nv_bfloat16* out, int out_stride, void* scratch, cudaStream_t s);
+int launch_qgemm_tc(const Q4Tiled& w, int m, const __nv_bfloat16* x, int x_stride, const TcSegments& out, int epilogue, int gated_act,
+                    void* scratch, int* status, cudaStream_t s, bool reuse_x = false);
 
 // Tensor-parallel sum of `rows` bf16 partial rows (prompt chunks): every rank copies its partials into every rank's
 // exchange buffer and raises a flag carrying `epoch` (the host counts exchanges); then each rank waits (bounded) for

@@ -144,7 +144,6 @@ struct swlm_ctx {
     cudaStream_t stream = nullptr;
     std::map<std::string, Q4Raw> raw;
     std::map<std::string, Q4Tiled> tiled;  // plain and fused tensors, keyed by name ("a|b|c" for fused)
-    std::map<std::string, Q4Raw> raw_cat;  // source-layout tensors with the rows of several raw tensors one after the other ("a|b|c")
     std::map<std::string, DenseTensor> dense;
     std::map<std::string, Matrix> matrices;      // bf16 matrices of the dense products
     std::map<std::string, Matrix> matrix_cat;    // the rows of several of them one after the other ("a|b|c"); the parts become views of it
@@ -171,10 +170,10 @@ struct swlm_plan {
     int attn_splits = 1;
     size_t attn_scratch = 0, qgemv_partial = 0, qgemv_counters = 0;
     int final_res = 0;  // physical residual buffer that holds the residual stream after a step
-    // Row-wise execution (prompt chunks, more than 16 sequences): consecutive products of one input run as one product
-    // over their concatenated rows. Per step: how many steps the product starting there covers (0: covered by an
-    // earlier one) and the tensor it multiplies.
-    struct RowsGroup { int count = 1; const Q4Raw* raw = nullptr; };
+    // Row-wise execution (prompt chunks, more than 16 sequences): consecutive products of one input run as one product over their
+    // concatenated rows, gate, up and activation as one over the interleaved rows. Per step: how many steps the product starting
+    // there covers (0: covered by an earlier one), the tensor it multiplies and the rows of its parts.
+    struct RowsGroup { int count = 1; const Q4Tiled* w = nullptr; int parts = 1; int n[3] = {0, 0, 0}; bool gated = false; };
     std::vector<RowsGroup> rows_groups;
     bool rows_groups_ready = false;
     // fp32-stream plans (desc.stream_dtype != 0)

@@ -39,6 +39,10 @@ __device__ __forceinline__ bool mbar_wait_addr(unsigned addr, unsigned parity) {
 }
 __device__ __forceinline__ bool mbar_wait(unsigned long long* bar, unsigned parity) { return mbar_wait_addr(smem_u32(bar), parity); }
 
+// The same for a converged warp: all its lanes get the same answer, also when some of them saw the limit.
+__device__ __forceinline__ bool mbar_wait_warp(unsigned addr, unsigned parity) { return __all_sync(0xffffffffu, mbar_wait_addr(addr, parity)); }
+__device__ __forceinline__ bool mbar_wait_warp(unsigned long long* bar, unsigned parity) { return mbar_wait_warp(smem_u32(bar), parity); }
+
 // Shared-memory matrix descriptor: K-major operand, 128-byte swizzle, rows of 128 bytes, 8-row groups 1024
 // bytes apart (stride byte offset); leading byte offset unused for this layout; descriptor version 1.
 __device__ __forceinline__ unsigned long long umma_desc(unsigned smem_addr) {
@@ -48,6 +52,19 @@ __device__ __forceinline__ unsigned long long umma_desc(unsigned smem_addr) {
     d |= 1ull << 46;
     d |= 2ull << 61;
     return d;
+}
+
+// The same descriptor as its low word (the rest is constant for this layout): places 32 bytes apart along K differ by 2, a tile
+// `bytes` further on by bytes / 16. Built where it is used, so that a loop over the MMAs of a step adds 32-bit numbers only.
+__device__ __forceinline__ unsigned umma_desc_lo(unsigned smem_addr) { return (smem_addr & 0x3FFFFu) >> 4; }
+constexpr unsigned kUmmaDescHi = (1024u >> 4) | 1u << 14 | 2u << 29;
+
+// One lane of a converged warp, the same one every time: the MMAs of a warp that runs its loop as a whole are issued by it. (A loop
+// inside `if (lane == 0)` spends 60 to 100 clocks per MMA on moving operands to uniform registers.)
+__device__ __forceinline__ bool elect_one() {
+    unsigned p;
+    asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\tselp.u32 %0, 1, 0, q;\n\t}" : "=r"(p));
+    return p != 0;
 }
 
 __device__ __forceinline__ void umma_commit(unsigned long long* bar) {

@@ -47,3 +47,34 @@ def test_rows_of_very_different_size(pkg, oracle):
     for i in (j for j in range(m) if j != 4):
         assert rel_err(got[i], ref[i]).max() <= RTOL
     store.close()
+
+
+@pytest.mark.parametrize("n,k", [(128, 64), (200, 192), (1000, 320), (4096, 4096), (264, 14336), (72, 16448)])
+@pytest.mark.parametrize("m", [17, 32, 33, 64, 65, 129, 300])
+def test_products_on_the_tensor_cores(pkg, oracle, n, k, m):
+    """Tiles of 32, 64, 128 and 256 rows with remainders; half steps of K and of the appended group sums; K over 1, 2, 4 and 8 CTAs;
+    rows longer than what the conversion keeps in registers."""
+    if n * k * m > 2 ** 31:
+        m = min(m, 65)
+    store = pkg.WeightStore(0)
+    w, s, b = pkg.synth_q4(n, k, seed=n + k, centered=True)
+    x = pkg.f32_to_bf16(np.random.default_rng(m).normal(size=(m, k)).astype(np.float32))
+    store.add_q4_mlx("mlx", w, s, b)
+    ref = pkg.bf16_to_f32(oracle.qgemm(x, w, s, b))
+    assert rel_err(pkg.bf16_to_f32(store.qgemm("mlx", x, n)), ref).max() <= RTOL
+    store.add_q4_staf("staf", pkg.formats.repack_mlx_to_staf(w, s, b), n, k)
+    assert rel_err(pkg.bf16_to_f32(store.qgemm("staf", x, n)), ref).max() <= RTOL
+    store.close()
+
+
+def test_more_tiles_than_multiprocessors(pkg, oracle):
+    """The long form walks several tiles per CTA; its results are compared at rows of the first, a middle and the last tile."""
+    n, k, m = 14336, 512, 600
+    store = pkg.WeightStore(0)
+    w, s, b = pkg.synth_q4(n, k, seed=9, centered=True)
+    x = pkg.f32_to_bf16(np.random.default_rng(4).normal(size=(m, k)).astype(np.float32))
+    store.add_q4_mlx("w", w, s, b)
+    got = pkg.bf16_to_f32(store.qgemm("w", x, n))
+    rows = np.r_[0:40, 255:258, 511:514, 590:600]
+    assert rel_err(got[rows], pkg.bf16_to_f32(oracle.qgemm(np.ascontiguousarray(x[rows]), w, s, b))).max() <= RTOL
+    store.close()
