@@ -1189,6 +1189,7 @@ int enqueue_rows(swlm_state* s, bool wide, const int32_t* tokens, int c, int pos
             a.scratch = s->attn_scratch;
             a.counters = wide ? s->attn_counters : s->pf_attn_counters;
             a.splits = wide ? plan->attn_splits : 1;
+            a.status = s->pf_status;
             rc = launch_attn_decode(a, stream);
             s->launches += wide ? 1 : 2;
             break;

@@ -298,8 +298,13 @@ struct AttnLaunch {
     const __half* qjl_matrix = nullptr;
     __half* qjl_res = nullptr;
     int qjl_dim = 0;
+    int* status = nullptr;   // prompt ingestion: device word set when a bounded wait expires
     PrefetchTarget prefetch;
 };
+// prompt ingestion on the tensor cores (attn_prompt.cu); the chunk's rows are in the cache
+int attn_prompt_init();
+bool attn_prompt_takes(const AttnLaunch& a);
+int launch_attn_prompt(const AttnLaunch& a, cudaStream_t s);
 int attn_pick_splits(int m, int kv_heads, int max_ctx);
 size_t attn_scratch_floats(int m, int heads, int head_dim, int splits);
 // decode: q rows are unrotated; RoPE, KV append and the current token's unrounded term are handled inside.

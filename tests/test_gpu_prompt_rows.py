@@ -39,3 +39,40 @@ def test_conv_over_a_chunk_is_the_repeated_single_step(pkg, kernel, dim):
         got, ref = pkg.bf16_to_f32(chunked.logits()), pkg.bf16_to_f32(single.logits())
         assert np.abs(got - ref).max() <= 1e-2 * np.abs(ref).max()   # one bf16 rounding (2^-9 of the largest) on either side
     chunked.close(), single.close(), store.close()
+
+
+@pytest.mark.parametrize("heads,kv_heads,hd", [(8, 2, 128), (4, 4, 64), (8, 1, 64), (4, 2, 128), (6, 2, 64)])
+@pytest.mark.parametrize("window,rope_dim", [(0, 0), (0, 64), (1, 64), (40, 24), (150, 64)])
+def test_prompt_attention_is_the_repeated_single_step(pkg, heads, kv_heads, hd, window, rope_dim):
+    """Portions around the key tile (64) and the query tile (128 rows), carried on, against the decode kernel token by token. The
+    cache is full of NaN before, so that a row nobody wrote shows (in the portion's last tile, and behind a KV head's last row).
+    Three query heads per KV head take the general kernel."""
+    P, vocab, max_seq, width = pkg.plan, 256, 300, heads * hd
+    rng = np.random.default_rng(heads * 100 + hd + window)
+    desc = pkg.BuffersDesc(hidden=width, slot_dim=width, vocab=vocab, max_seq=max_seq, max_batch=1, kv_layers=1, kv_heads=kv_heads, head_dim=hd)
+    store = pkg.WeightStore(0)
+    store.add_dense("q", _bf(pkg, rng.normal(size=(vocab, width)) * 2))
+    store.add_dense("k", _bf(pkg, rng.normal(size=(vocab, kv_heads * hd))))
+    store.add_dense("v", _bf(pkg, rng.normal(size=(vocab, kv_heads * hd))))
+    store.add_q4_mlx("head", *pkg.synth_q4(vocab, width, seed=5, centered=True))
+    steps = [P._step(P.STEP_EMBED, out_buf=P.BUF_S1, n=width, weight="q"), P._step(P.STEP_EMBED, out_buf=P.BUF_S2, n=kv_heads * hd, weight="k"),
+             P._step(P.STEP_EMBED, out_buf=P.BUF_S3, n=kv_heads * hd, weight="v"),
+             P._step(P.STEP_ATTN_DECODE, layer=0, in_buf=P.BUF_S1, in2_buf=P.BUF_S2, in3_buf=P.BUF_S3, out_buf=P.BUF_S0, heads=heads, kv_heads=kv_heads,
+                     head_dim=hd, rope_dim=rope_dim, rope_base=10000.0, scale=hd ** -0.5, window_left=window),
+             P._step(P.STEP_QGEMV, in_buf=P.BUF_S0, out_buf=P.BUF_LOGITS, n=vocab, k=width, weight="head"),
+             P._step(P.STEP_ARGMAX, in_buf=P.BUF_LOGITS, n=vocab)]
+    chunked, single = pkg.InferenceModel(store, steps, desc), pkg.InferenceModel(store, steps, desc)
+    single.set_prefill_chunk(0)
+    nan = np.full((max_seq, hd), 0x7FC0, dtype=np.uint16)
+    for head in range(kv_heads):
+        for which in (0, 1):
+            chunked.write_kv(which, 0, 0, head, nan)
+    for n in (1, 31, 32, 129, 64, 43):
+        tokens = rng.integers(0, vocab, size=n)
+        chunked.prefill_sequence(0, tokens)
+        single.prefill(tokens[None])
+        got, ref = pkg.bf16_to_f32(chunked.logits()), pkg.bf16_to_f32(single.logits())
+        # a token's own rotated key is rounded to bf16 (2^-9) in the cache and not in the single step: its score moves by up to
+        # 2^-9 |q| |k| / sqrt(hd), about 2 % of its weight for the longest of these rows
+        assert np.abs(got - ref).max() <= 3e-2 * np.abs(ref).max(), n
+    chunked.close(), single.close(), store.close()
