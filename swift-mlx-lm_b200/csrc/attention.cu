@@ -640,6 +640,7 @@ __global__ void __launch_bounds__(kQ8Threads, ROTOR && G <= 4 ? 2 : 0) attn_q8_s
     __shared__ float kcur[HD], vcur[HD];
     __shared__ float osm[kQ8Warps][kMaxGroup][HD];   // (sized for the merge scratch below whatever G is)
     __shared__ float msm[kQ8Warps][kMaxGroup], lsm[kQ8Warps][kMaxGroup];
+    __shared__ __align__(16) float weights[kQ8Warps][8 * G];   // of a batch of eight rows
     __shared__ int is_last;
     __shared__ float kres[ROTOR ? HD : 1];          // the new k row minus its dequantised blocks
     __shared__ float qp[ROTOR ? G : 1][64];         // Phi . q of every head of the group
@@ -647,6 +648,18 @@ __global__ void __launch_bounds__(kQ8Threads, ROTOR && G <= 4 ? 2 : 0) attn_q8_s
     const int qjl = ROTOR ? p.qjl_dim : 0;
     pdl_wait();
     const int n_ctx = p.position[b];
+    const size_t head_bytes = (size_t)p.max_seq * ROW_BYTES;
+    unsigned char* kbase = reinterpret_cast<unsigned char*>(p.kcache) + ((size_t)b * p.kv_heads + kvh) * head_bytes;
+    unsigned char* vbase = reinterpret_cast<unsigned char*>(p.vcache) + ((size_t)b * p.kv_heads + kvh) * head_bytes;
+    // the split's share of the cached rows [t_lo, n_ctx): contiguous; a warp takes every eighth row of it. All of it is asked into L2
+    // before q is staged and rotated
+    const int t_lo = p.window > 0 ? max(0, n_ctx + 1 - p.window) : 0;
+    const int per = (n_ctx - t_lo + p.splits - 1) / p.splits;
+    const int t0 = t_lo + split * per, t1 = min(n_ctx, t0 + per);
+    for (int off = tid * 128; off < (t1 - t0) * ROW_BYTES; off += kQ8Threads * 128) {
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(kbase + (size_t)t0 * ROW_BYTES + off));
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(vbase + (size_t)t0 * ROW_BYTES + off));
+    }
     for (int idx = tid; idx < G * HD; idx += kQ8Threads)
         qs[idx / HD][idx % HD] = __bfloat162float(p.q[(size_t)b * p.q_stride + (size_t)kvh * G * HD + idx]);
     for (int d = tid; d < HD; d += kQ8Threads) {
@@ -675,9 +688,6 @@ __global__ void __launch_bounds__(kQ8Threads, ROTOR && G <= 4 ? 2 : 0) attn_q8_s
         }
         __syncthreads();
     }
-    const size_t head_bytes = (size_t)p.max_seq * ROW_BYTES;
-    unsigned char* kbase = reinterpret_cast<unsigned char*>(p.kcache) + ((size_t)b * p.kv_heads + kvh) * head_bytes;
-    unsigned char* vbase = reinterpret_cast<unsigned char*>(p.vcache) + ((size_t)b * p.kv_heads + kvh) * head_bytes;
     const __half* const res_base = ROTOR && qjl > 0 ? p.qjl_res + ((size_t)b * p.kv_heads + kvh) * p.max_seq * qjl : nullptr;
     if (split == 0 && n_ctx < p.max_seq) {
         q8_quantise_row<ROTOR>(kcur, kbase + (size_t)n_ctx * ROW_BYTES, HD, BITS, GROUP, warp, lane, kres);
@@ -746,12 +756,12 @@ __global__ void __launch_bounds__(kQ8Threads, ROTOR && G <= 4 ? 2 : 0) attn_q8_s
             for (int j = 0; j < EPL; ++j) acc[r][j] = fmaf(w, vf[j], acc[r][j] * corr);
         }
     };
-    // the split's share of the cached rows [t_lo, n_ctx): contiguous; a warp takes every fourth row of it
-    const int t_lo = p.window > 0 ? max(0, n_ctx + 1 - p.window) : 0;
-    const int per = (n_ctx - t_lo + p.splits - 1) / p.splits;
-    const int t0 = t_lo + split * per, t1 = min(n_ctx, t0 + per);
     // eight rows per warp are requested before the first is used: one trip to memory per eight rows instead of one per row
     constexpr int UN = 8;
+    constexpr int NV = UN * G, VPL = NV > 32 ? NV / 32 : 1, REP = NV < 32 ? 32 / NV : 1;   // values of a batch, per lane, lanes per value
+    float m_l[VPL], l_l[VPL];   // running maximum and sum (of this lane's rows) of the heads this lane's values belong to
+#pragma unroll
+    for (int e = 0; e < VPL; ++e) { m_l[e] = -INFINITY; l_l[e] = 0.f; }
     for (int tb = t0 + warp; tb < t1; tb += kQ8Warps * UN) {
         unsigned kw[UN], vw[UN], khd[UN], vhd[UN];
         unsigned short rz0[ROTOR ? UN : 1], rz1[ROTOR ? UN : 1];   // the row's projected residual, columns lane and lane + 32
@@ -773,8 +783,8 @@ __global__ void __launch_bounds__(kQ8Threads, ROTOR && G <= 4 ? 2 : 0) attn_q8_s
                 }
             }
         }
-        // the scores of the eight rows for all heads: 8 x G independent dot products and warp reductions, interleaved
-        float sc[UN][G];
+        // the scores of the eight rows for all heads, value u * G + r: partial sums of this lane's elements
+        float sc[NV];
 #pragma unroll
         for (int u = 0; u < UN; ++u) {
             const __half2 kh = *reinterpret_cast<const __half2*>(&khd[u]);
@@ -784,54 +794,79 @@ __global__ void __launch_bounds__(kQ8Threads, ROTOR && G <= 4 ? 2 : 0) attn_q8_s
             for (int j = 0; j < EPL; ++j) kf[j] = fmaf(ks, (float)((kw[u] >> (BITS * j)) & qmask), kz);
 #pragma unroll
             for (int r = 0; r < G; ++r) {
-                sc[u][r] = 0.f;
+                float a = 0.f;
 #pragma unroll
-                for (int j = 0; j < EPL; ++j) sc[u][r] = fmaf(qr[r][j], kf[j], sc[u][r]);
+                for (int j = 0; j < EPL; ++j) a = fmaf(qr[r][j], kf[j], a);
+                sc[u * G + r] = a;
             }
             if (ROTOR) {
                 const float r0 = __half2float(__ushort_as_half(rz0[u])), r1 = __half2float(__ushort_as_half(rz1[u]));
 #pragma unroll
-                for (int r = 0; r < G; ++r) sc[u][r] = fmaf(qpr[r][1], r1, fmaf(qpr[r][0], r0, sc[u][r]));
+                for (int r = 0; r < G; ++r) sc[u * G + r] = fmaf(qpr[r][1], r1, fmaf(qpr[r][0], r0, sc[u * G + r]));
             }
         }
+        // summed over the warp so that every lane ends with values of its own: at each exchange a lane keeps one half of what it has
+        // and gives the other away (31 exchanges for 32 values instead of 160), and one lane works out a value's weight instead of all
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1)
+        for (int st = 0; st < 5; ++st) {
+            const int o = 16 >> st, have = NV >> st;
+            if (have > 1) {
+                const bool up = lane & o;
 #pragma unroll
-            for (int u = 0; u < UN; ++u)
+                for (int i = 0; i < (have > 1 ? have / 2 : 1); ++i) {
+                    const float keep = up ? sc[have / 2 + i] : sc[i], give = up ? sc[i] : sc[have / 2 + i];
+                    sc[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+                }
+            } else {
+                sc[0] += __shfl_xor_sync(0xffffffffu, sc[0], o);
+            }
+        }
+        float corr_l[VPL];
 #pragma unroll
-                for (int r = 0; r < G; ++r) sc[u][r] += __shfl_xor_sync(0xffffffffu, sc[u][r], o);
-        // the eight rows enter the running softmax together: one new maximum and one rescale per head for the lot
-        // (rows past the end carry the score -inf, i.e. weight 0)
-        float vfu[UN][EPL];
+        for (int e = 0; e < VPL; ++e) {
+            const int idx = lane * VPL / REP + e, u = idx / G;   // rows past the end get weight 0
+            const float s = tb + u * kQ8Warps < t1 ? sc[e] * p.scale_log2 : -INFINITY;
+            float top = s;   // over the rows of the same head
+            top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 4));
+            top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 8));
+            top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 16));
+            const float m_new = fmaxf(m_l[e], top);              // finite: the batch's first row is inside the range
+            corr_l[e] = exp2f(m_l[e] - m_new);
+            const float w = exp2f(s - m_new);
+            l_l[e] = l_l[e] * corr_l[e] + w;
+            m_l[e] = m_new;
+            if (lane % REP == 0) weights[warp][idx] = w;
+        }
+        __syncwarp();
+#pragma unroll
+        for (int r = 0; r < G; ++r) {
+            const float corr = __shfl_sync(0xffffffffu, corr_l[r % VPL], r * REP / VPL);
+#pragma unroll
+            for (int j = 0; j < EPL; ++j) acc[r][j] *= corr;
+        }
 #pragma unroll
         for (int u = 0; u < UN; ++u) {
             const __half2 vh = *reinterpret_cast<const __half2*>(&vhd[u]);
             const float vs = __low2float(vh), vz = __high2float(vh);
+            float vf[EPL];
 #pragma unroll
-            for (int j = 0; j < EPL; ++j) vfu[u][j] = fmaf(vs, (float)((vw[u] >> (BITS * j)) & qmask), vz);
-        }
+            for (int j = 0; j < EPL; ++j) vf[j] = fmaf(vs, (float)((vw[u] >> (BITS * j)) & qmask), vz);
 #pragma unroll
-        for (int r = 0; r < G; ++r) {
-            float m_new = m_run[r];
+            for (int r = 0; r < G; ++r) {
+                const float w = weights[warp][u * G + r];
 #pragma unroll
-            for (int u = 0; u < UN; ++u) {
-                sc[u][r] = tb + u * kQ8Warps < t1 ? sc[u][r] * p.scale_log2 : -INFINITY;
-                m_new = fmaxf(m_new, sc[u][r]);
+                for (int j = 0; j < EPL; ++j) acc[r][j] = fmaf(w, vf[j], acc[r][j]);
             }
-            const float corr = exp2f(m_run[r] - m_new);   // m_new is finite: the batch's first row is inside the range
-            float wsum = 0.f;
-#pragma unroll
-            for (int j = 0; j < EPL; ++j) acc[r][j] *= corr;
-#pragma unroll
-            for (int u = 0; u < UN; ++u) {
-                const float w = exp2f(sc[u][r] - m_new);
-                wsum += w;
-#pragma unroll
-                for (int j = 0; j < EPL; ++j) acc[r][j] = fmaf(w, vfu[u][j], acc[r][j]);
-            }
-            l_run[r] = l_run[r] * corr + wsum;
-            m_run[r] = m_new;
         }
+        __syncwarp();
+    }
+#pragma unroll
+    for (int e = 0; e < VPL; ++e)
+        for (int o = 4; o < 32; o <<= 1) l_l[e] += __shfl_xor_sync(0xffffffffu, l_l[e], o);
+#pragma unroll
+    for (int r = 0; r < G; ++r) {
+        m_run[r] = __shfl_sync(0xffffffffu, m_l[r % VPL], r * REP / VPL);
+        l_run[r] = __shfl_sync(0xffffffffu, l_l[r % VPL], r * REP / VPL);
     }
     if (split == 0 && warp == 0) {   // the new token: unrounded rotated k, v as given
         float vf[EPL], sc[G];
