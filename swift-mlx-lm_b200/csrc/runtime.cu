@@ -361,7 +361,7 @@ int compile_plan(swlm_plan* plan) {
         }
         plan->launches.push_back(L);
     }
-    plan->attn_splits = attn_pick_splits(m, std::max(1, d.kv_heads / std::max(1, ctx->tp_size)), d.max_seq);
+    plan->attn_splits = attn_pick_splits(m, std::max(1, d.kv_heads / std::max(1, ctx->tp_size)), d.max_seq, true);
 
     // A gate/up launch with the SwiGLU epilogue writes while other CTAs may still be reading its input:
     // when both are the same buffer, send the result to scratch slot 4 and point the readers there.

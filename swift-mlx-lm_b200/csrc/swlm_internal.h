@@ -305,7 +305,8 @@ struct AttnLaunch {
 int attn_prompt_init();
 bool attn_prompt_takes(const AttnLaunch& a);
 int launch_attn_prompt(const AttnLaunch& a, cudaStream_t s);
-int attn_pick_splits(int m, int kv_heads, int max_ctx);
+// ragged: the sequences may be of unequal length
+int attn_pick_splits(int m, int kv_heads, int max_ctx, bool ragged = false);
 size_t attn_scratch_floats(int m, int heads, int head_dim, int splits);
 // decode: q rows are unrotated; RoPE, KV append and the current token's unrounded term are handled inside.
 int launch_attn_decode(const AttnLaunch& a, cudaStream_t s);
