@@ -64,6 +64,8 @@ struct AttnParams {
     const __half* qjl_matrix;
     __half* qjl_res;
     int qjl_dim;
+    const __nv_bfloat16* q_norm; const __nv_bfloat16* k_norm;   // decode: per-head RMS norm before the rotation (null: none)
+    float qk_eps, qk_bias;
 };
 
 __device__ __forceinline__ unsigned long long attn_timer_ns() {
@@ -97,11 +99,13 @@ __device__ __forceinline__ float rope_elem(const float* v, int d, int rope_dim, 
 // MODE 0: plain flash-decode over an existing cache (q already rotated, context length from the host).
 // MODE 1: decode step: sequence b at the device-resident position; rotates q and the new k, appends k/v to the
 //         cache and adds the new token's own term from the unrounded values.
+// MODE 3: the same behind a per-head RMS norm of q and the new k (a form of its own: plans without that norm keep their code).
 // MODE 2: prompt ingestion: "sequence" b is prompt token b of ONE sequence at position pos_base + b; all of the
 //         chunk's k/v rows are already in the cache (rope_append_kernel), token b attends rows 0..pos_base+b.
 template <int HD, int MODE>
 __global__ void __launch_bounds__(kSplitThreads) attn_split_kernel(const AttnParams p) {
-    constexpr bool DECODE = MODE == 1;
+    constexpr bool DECODE = MODE == 1 || MODE == 3;
+    constexpr bool QK_NORM = MODE == 3;
     constexpr bool PREFILL = MODE == 2;
     const int cta_linear = (blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
     if (p.trace && threadIdx.x == 0) p.trace[cta_linear * 4] = attn_timer_ns();
@@ -229,6 +233,22 @@ __global__ void __launch_bounds__(kSplitThreads) attn_split_kernel(const AttnPar
     const int n_ctas = gridDim.x * gridDim.y * gridDim.z;
     const bool stamp0 = p.trace && cta_linear == 0 && threadIdx.x == 0;  // finer stamps of the first CTA only
     if (stamp0) p.trace[n_ctas * 4 + 1] = attn_timer_ns();
+    if (QK_NORM) {
+        // batched_qk_rms_norm_2 (Generator/MetalSourceGenerator+Batched.swift:681-760) of the G rows of q and of the new k, a warp
+        // per row, with the bf16 rounding that a launch of its own leaves; every split repeats it (0.2 us instead of a launch)
+        for (int r = warp; r <= G; r += kSplitWarps) {
+            const __nv_bfloat16* w = r < G ? p.q_norm : p.k_norm;
+            float ss = 0.f;
+#pragma unroll
+            for (int i = 0; i < HD / 32; ++i) { const float v = qk[r][lane + 32 * i]; ss = fmaf(v, v, ss); }
+            for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+            const float rs = rsqrtf(ss / (float)HD + p.qk_eps);
+#pragma unroll
+            for (int i = 0; i < HD / 32; ++i)
+                qk[r][lane + 32 * i] = __bfloat162float(__float2bfloat16_rn(qk[r][lane + 32 * i] * rs * (__bfloat162float(w[lane + 32 * i]) + p.qk_bias)));
+        }
+        __syncthreads();
+    }
     if (rotate) {
         // rotate-half RoPE (Generator/MetalSourceGenerator+Attention.swift:596-617): pairs (i, i + rope_dim/2)
         if (rot_i < pairs)
@@ -1041,6 +1061,7 @@ int launch_attn_decode(const AttnLaunch& a, cudaStream_t s) {
     p.part_o = a.scratch;
     p.part_ml = a.scratch + (size_t)a.m * a.heads * a.splits * a.head_dim;
     p.counters = a.counters;
+    p.q_norm = a.q_norm; p.k_norm = a.k_norm; p.qk_eps = a.qk_eps; p.qk_bias = a.qk_bias;
     p.prefetch = a.prefetch;
     if (a.pos_base < 0 && a.m * a.kv_heads * a.splits + a.m * a.kv_heads <= 512)
         p.trace = qgemv_trace_slot(a.m * a.kv_heads * a.splits, -a.kv_heads * a.m, a.splits, 9, 0);
@@ -1082,7 +1103,7 @@ int launch_attn_decode(const AttnLaunch& a, cudaStream_t s) {
         if (attn_prompt_takes(a)) return launch_attn_prompt(a, s);
         return launch_both<2>(p, a.m, a.head_dim, s);
     }
-    return launch_both<1>(p, a.m, a.head_dim, s);
+    return a.q_norm ? launch_both<3>(p, a.m, a.head_dim, s) : launch_both<1>(p, a.m, a.head_dim, s);
 }
 
 int launch_flash_decode_plain(int m, int heads, int kv_heads, int hd, int ctx_len, int ctx_stride, float scale,

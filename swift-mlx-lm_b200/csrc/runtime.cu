@@ -412,6 +412,30 @@ int compile_plan(swlm_plan* plan) {
         B.steps_covered += 1;
         plan->launches.erase(plan->launches.begin() + i);
     }
+    // Fold the per-head norm of q and k into the attention launch behind it (bf16 cache), when nothing else reads their buffers before
+    // they are written again (a plan's last values stay as they were: the host may read any buffer after a step).
+    for (size_t i = 0; i + 1 < plan->launches.size(); ++i) {
+        Launch& A = plan->launches[i];
+        Launch& B = plan->launches[i + 1];
+        if (A.kind != L_QK_NORM || B.kind != L_ATTN || swlm_kv_bits(d.kv_scheme) || (B.st.head_dim != 64 && B.st.head_dim != 128)) continue;
+        if (A.st.in_buf != B.st.in_buf || A.st.in2_buf != B.st.in2_buf || A.st.in_buf == A.st.in2_buf || A.st.heads != B.st.heads || A.st.head_dim != B.st.head_dim) continue;
+        bool ok = B.st.in3_buf != A.st.in_buf && B.st.in3_buf != A.st.in2_buf;
+        for (int buf : {A.st.in_buf, A.st.in2_buf}) {
+            bool written = B.st.out_buf == buf;
+            for (size_t j = i + 2; j < plan->launches.size() && ok && !written; ++j) {
+                const Launch& C = plan->launches[j];
+                if ((C.norm.kind ? C.x_buf : C.st.in_buf) == buf || C.st.in2_buf == buf || C.st.in3_buf == buf || (C.kind == L_SSM && C.st.in4_buf == buf)) ok = false;
+                written = C.kind != L_QGEMV && C.kind != L_QK_NORM && C.kind != L_ARGMAX && C.st.out_buf == buf;
+                for (int q = 0; q < C.n_seg && C.kind == L_QGEMV; ++q) written |= C.seg_buf[q] == buf;
+            }
+            ok &= written;
+        }
+        if (!ok) continue;
+        B.qk = A.st; B.d1 = A.d1; B.d2 = A.d2;
+        B.label = "qk_norm+" + B.label;
+        B.steps_covered += 1;
+        plan->launches.erase(plan->launches.begin() + i);
+    }
     // residual ping-pong: a fused norm reads one physical residual buffer and writes the other
     int cur = 0;
     for (Launch& L : plan->launches) {
@@ -684,6 +708,7 @@ int enqueue_step(swlm_state* s, bool body_only, cudaStream_t stream, int only_ki
             a.max_seq = d.max_seq; a.position = s->position;
             a.out = s->buf[st.out_buf]; a.out_stride = s->width[st.out_buf];
             a.scratch = s->attn_scratch; a.counters = s->attn_counters; a.splits = plan->attn_splits;
+            if (L.qk.kind) { a.q_norm = L.d1->data; a.k_norm = L.d2->data; a.qk_eps = L.qk.eps; a.qk_bias = L.qk.weight_bias; }
             if (L.prefetch_launch >= 0) a.prefetch = prefetch_of(plan->launches[L.prefetch_launch]);
             rc = launch_attn_decode(a, stream);
             s->launches += 1;

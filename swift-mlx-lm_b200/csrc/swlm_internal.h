@@ -299,6 +299,10 @@ struct AttnLaunch {
     __half* qjl_res = nullptr;
     int qjl_dim = 0;
     int* status = nullptr;   // prompt ingestion: device word set when a bounded wait expires
+    // decode steps over a bf16 cache: per-head RMS norm of q and the new k before the rotation (null: none, or done before)
+    const __nv_bfloat16* q_norm = nullptr;
+    const __nv_bfloat16* k_norm = nullptr;
+    float qk_eps = 0.f, qk_bias = 0.f;
     PrefetchTarget prefetch;
 };
 // prompt ingestion on the tensor cores (attn_prompt.cu); the chunk's rows are in the cache

@@ -58,6 +58,7 @@ struct Launch {
     // residual add / copy / RMSNorm folded into this product's prologue (norm.kind == 0: none)
     swlm_step norm{};
     const DenseTensor* norm_w = nullptr;
+    swlm_step qk{};            // attention: the per-head norm of q and k folded into it (qk.kind == 0: none); weights d1, d2
     int x_buf = -1;            // buffer the product reads (the norm's input when fused)
     int push = 0, in_tp = 0;   // tensor parallel: partial rows pushed to all ranks / pushed partials consumed
     int res_in = 0, res_out = 0;  // physical residual buffers (0 or 1) this launch reads / writes
