@@ -340,12 +340,14 @@ struct TcParams {
 __host__ __device__ constexpr unsigned tc_idesc(int bn) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(bn >> 3) << 17) | ((unsigned)(kTileRows >> 4) << 24);
 }
-__device__ __forceinline__ void umma_bf16(unsigned d_tmem, unsigned long long a_desc, unsigned long long b_desc, unsigned idesc, unsigned accumulate) {
+// (descriptors by their low words)
+__device__ __forceinline__ void umma_bf16(unsigned d_tmem, unsigned a_lo, unsigned b_lo, unsigned idesc, unsigned accumulate) {
     asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
+        "{\n\t.reg .pred p;\n\t.reg .b64 a, b;\n\t"
+        "setp.ne.b32 p, %5, 0;\n\t"
+        "mov.b64 a, {%1, %3};\n\tmov.b64 b, {%2, %3};\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %4, p;\n\t}"
+        ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(kUmmaDescHi), "r"(idesc), "r"(accumulate) : "memory");
 }
 
 __device__ __forceinline__ void tmem_ld16(unsigned (&v)[16], unsigned at) {
@@ -428,23 +430,29 @@ __global__ void __launch_bounds__(kTcBlock) bgemm_tc_kernel(const TcParams p, co
         }
         __syncwarp();
     } else if (warp == 1) {
-        if (lane == 0) {
-            constexpr unsigned idesc = tc_idesc(BN);
-            for (int kt = 0; kt < steps; ++kt) {
-                const int s = kt % STAGES;
-                if (!mbar_wait(&full_bar[s], (unsigned)((kt / STAGES) & 1))) { atomicExch(p.status, 32); failed = 1; break; }
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const unsigned a = smem_u32(smem + s * STAGE), b = a + 2 * A_BYTES;
+        // the warp runs its loop as a whole, one lane issues (a lone lane's loop took longer over its eight MMAs than a step of 128
+        // activation rows takes to multiply)
+        constexpr unsigned idesc = tc_idesc(BN);
+        const bool el = elect_one();
+        int s = 0;
+        unsigned par = 0;
+        for (int kt = 0; kt < steps; ++kt) {
+            if (!mbar_wait_warp(&full_bar[s], par)) { if (el) { atomicExch(p.status, 32); failed = 1; } break; }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            if (el) {
+                const unsigned a = umma_desc_lo(smem_u32(smem + s * STAGE)), b = a + 2 * A_BYTES / 16;
 #pragma unroll
                 for (int j = 0; j < kTcK / 16; ++j) {
-                    const unsigned acc = (kt > 0 || j > 0) ? 1u : 0u;
-                    umma_bf16(tmem, umma_desc(a + 32 * j), umma_desc(b + 32 * j), idesc, acc);
-                    if (nt == 2) umma_bf16(tmem + BN, umma_desc(a + A_BYTES + 32 * j), umma_desc(b + 32 * j), idesc, acc);
+                    const unsigned acc = j > 0 ? 1u : kt > 0 ? 1u : 0u;
+                    umma_bf16(tmem, a + 2 * j, b + 2 * j, idesc, acc);
+                    if (nt == 2) umma_bf16(tmem + BN, a + A_BYTES / 16 + 2 * j, b + 2 * j, idesc, acc);
                 }
                 umma_commit(&empty_bar[s]);
             }
-            umma_commit(&done_bar);   // also behind whatever was issued before a failure
+            __syncwarp();
+            if (++s == STAGES) { s = 0; par ^= 1u; }
         }
+        if (el) umma_commit(&done_bar);   // also behind whatever was issued before a failure
         __syncwarp();
     } else {
         // ---- epilogue: a warp reads the 32 accumulator lanes of its quarter (warp & 3), lane = weight row; the two warps of a
