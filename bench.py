@@ -938,7 +938,7 @@ def main():
     kv_bytes = args.batch * cfg.kv_layer_count * (cfg.kv_heads // world) * kv_row_bytes * 2 * model.position
     kv_bytes += args.batch * cfg.kv_layer_count * cfg.kv_heads * cfg.kv_qjl_dim * 2 * model.position   # projected K residuals
     n_gemv = sum(1 for l in model.describe().splitlines() if "qgemv" in l)
-    kernel_name = "qgemv1_kernel" if args.batch == 1 else "qgemv_kernel"
+    kernel_name = "qgemv1_kernel" if args.batch == 1 else "qgemv_rows_kernel" if world == 1 else "qgemv_kernel"
     kernel_scope = "all %d launches of one decode step, timed back to back" % n_gemv
     if wide:
         kernel_name, kernel_scope = "qgemm_tc_kernel", "weight bytes over the WHOLE decode step; the products are not timed apart at more than 16 sequences"
