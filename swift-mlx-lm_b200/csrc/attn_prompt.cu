@@ -77,8 +77,16 @@ __device__ __forceinline__ void pa_split(float a, float b, unsigned& hi, unsigne
     lo = pa_pack(a - __uint_as_float(hi << 16), b - __uint_as_float(hi & 0xFFFF0000u));
 }
 
+// A wait by parity cannot tell a phase from the one two before it, so the phase before the awaited one has to be known to be over:
+//   q_ready, o_done  have one phase;
+//   k_full, p_ready  are waited for phase by phase (MMA warp);
+//   v_full           phase by phase by the MMA warp; by a softmax warp for tile j behind pv_done(j - 1), whose product read tile j - 1;
+//   s_full[j & 1]    phase by phase by the softmax warps and the TMA thread;
+//   pv_done          phase by phase by the TMA thread; for tile j - 1 by the MMA warp, which has waited for tile j - 2 in the round before,
+//                    and by a softmax warp behind s_full(j): the scores of tile j are issued behind pv_done(j - 2). Behind the last tile no
+//                    scores follow that would imply the tile before it, so that its products' end has a barrier of its own, o_done.
 struct PaBars {
-    unsigned long long q_ready, k_full, v_full, s_full[2], p_ready[2], pv_done;
+    unsigned long long q_ready, k_full, v_full, s_full[2], p_ready[2], pv_done, o_done;   // o_done: every MMA issued is done
     unsigned tmem;
     int failed;
 };
@@ -107,7 +115,7 @@ __global__ void __launch_bounds__(kPaThreads, 2) attn_prompt_kernel(const Prompt
     auto fail = [&](int code) { atomicExch(p.status, code); *failed = 1; };
 
     if (tid == 0) {
-        mbar_init(&bars.q_ready, 4); mbar_init(&bars.k_full, 1); mbar_init(&bars.v_full, 1); mbar_init(&bars.pv_done, 1);
+        mbar_init(&bars.q_ready, 4); mbar_init(&bars.k_full, 1); mbar_init(&bars.v_full, 1); mbar_init(&bars.pv_done, 1); mbar_init(&bars.o_done, 1);
         for (int i = 0; i < 2; ++i) { mbar_init(&bars.s_full[i], 1); mbar_init(&bars.p_ready[i], 4); }
         bars.failed = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -163,7 +171,6 @@ __global__ void __launch_bounds__(kPaThreads, 2) attn_prompt_kernel(const Prompt
             __syncwarp();
         };
         bool ok = mbar_wait_warp(&bars.q_ready, 0u) && mbar_wait_warp(&bars.k_full, 0u);
-        int pv = 0;   // value products issued
         if (ok) { pa_after(); scores(0); }
         for (int j = 0; j < n_tiles && ok; ++j) {
             if (j + 1 < n_tiles) {
@@ -184,15 +191,13 @@ __global__ void __launch_bounds__(kPaThreads, 2) attn_prompt_kernel(const Prompt
                 umma_commit(&bars.pv_done);
             }
             __syncwarp();
-            ++pv;
         }
-        if (!ok && el) {   // tensor memory is not freed under MMAs in flight
-            fail(7);
-            umma_commit(&bars.pv_done);
-            if (pv > 0) mbar_wait(&bars.pv_done, (unsigned)((pv - 1) & 1));
-            mbar_wait(&bars.pv_done, (unsigned)(pv & 1));
+        if (el) {
+            if (!ok) fail(7);
+            umma_commit(&bars.o_done);   // also behind whatever was issued before a failure
         }
         __syncwarp();
+        if (!mbar_wait_warp(&bars.o_done, 0u) && el) fail(7);   // tensor memory is not freed under MMAs in flight
     } else {
         const int r = tid, tl = r / G, head = r - tl * G;
         const bool row_ok = tl < n_tok;
@@ -330,7 +335,8 @@ __global__ void __launch_bounds__(kPaThreads, 2) attn_prompt_kernel(const Prompt
             pa_st32(region + 32u, lo);
             pa_wait_st();
             if (key0 + kPaKeys - 1 > last_row) {   // value rows that nobody wrote get weight 0: they must not hold NaN or infinity
-                if (!mbar_wait_warp(&bars.v_full, (unsigned)(j & 1))) { ok = false; break; }
+                // (tile j - 1 of the values may still be on its way into the slot: first its product)
+                if ((j > 0 && !mbar_wait_warp(&bars.pv_done, (unsigned)((j - 1) & 1))) || !mbar_wait_warp(&bars.v_full, (unsigned)(j & 1))) { ok = false; break; }
                 const int first = last_row + 1 - key0;
                 for (int idx = tid; idx < (kPaKeys - first) * HALVES * 8; idx += 128) {
                     const int row = first + idx / (HALVES * 8), c = idx % (HALVES * 8);
@@ -342,7 +348,7 @@ __global__ void __launch_bounds__(kPaThreads, 2) attn_prompt_kernel(const Prompt
             __syncwarp();
             if (lane == 0) pa_arrive(&bars.p_ready[j & 1]);
         }
-        if (ok && !mbar_wait_warp(&bars.pv_done, (unsigned)((n_tiles - 1) & 1))) ok = false;
+        if (ok && (!mbar_wait_warp(&bars.o_done, 0u) || *failed)) ok = false;
         if (!ok) fail(8);
         __syncwarp();
         pa_after();
