@@ -190,6 +190,8 @@ __global__ void conv_step_kernel(int dim, int kernel, __nv_bfloat16* state, size
 // channels under ncu; with the runs a prompt through ten such layers went from 24.3 to 10.3 ms, all of it here. Sums are formed in the order of the single step, so results are the same bits.
 // The state is read and replaced by the threads of the first run alone: the last inputs are worked out again instead of
 // being handed over by the last run, which could overwrite the history before the first run has read it.
+// A step whose output takes its input's place (a token's result lies where its B was) is one run: other runs would read inputs that
+// are already overwritten. There a thread reads what it needs of a token, and what the state needs of the last ones, before it writes.
 constexpr int kConvMaxKernel = 8;
 constexpr int kConvRun = 16;
 static_assert(kConvRun >= kConvMaxKernel, "only the first run may look in front of the chunk");
@@ -222,13 +224,13 @@ __device__ __forceinline__ void conv_past(int t, int dim, int c, const __nv_bflo
     for (int i = 0; i < V; ++i) v[i] = __bfloat162float(__float2bfloat16_rn(b[i] * x[i]));
 }
 template <int K, int V>
-__global__ void __launch_bounds__(128) conv_prefill_kernel(int dim, int tokens, __nv_bfloat16* state, const __nv_bfloat16* in, int in_stride,
+__global__ void __launch_bounds__(128) conv_prefill_kernel(int dim, int tokens, int run, __nv_bfloat16* state, const __nv_bfloat16* in, int in_stride,
                                                            const __nv_bfloat16* weight, __nv_bfloat16* out, int out_stride) {
     pdl_launch_dependents();
     pdl_wait();
     const int c = (blockIdx.y * blockDim.x + threadIdx.x) * V;
     if (c >= dim) return;
-    const int t0 = blockIdx.x * kConvRun, t1 = min(tokens, t0 + kConvRun);
+    const int t0 = blockIdx.x * run, t1 = min(tokens, t0 + run);
     float w[K][V], win[K][V];   // win[1 ..]: the inputs in front of the token at hand, oldest first
 #pragma unroll
     for (int k = 0; k < K; ++k)
@@ -267,11 +269,12 @@ __global__ void __launch_bounds__(128) conv_prefill_kernel(int dim, int tokens, 
 template <int K>
 void launch_conv_runs(int tokens, int dim, __nv_bfloat16* state, const __nv_bfloat16* in, int in_stride, const __nv_bfloat16* weight,
                       __nv_bfloat16* out, int out_stride, cudaStream_t s) {
-    const unsigned runs = (unsigned)((tokens + kConvRun - 1) / kConvRun);
+    const int run = out == in ? tokens : kConvRun;
+    const unsigned runs = (unsigned)((tokens + run - 1) / run);
     // four channels per thread where every row of them starts on 8 bytes
     const bool quads = !((dim | in_stride | out_stride) & 3) && !((reinterpret_cast<uintptr_t>(state) | reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) & 7);
-    if (quads) launch_k(conv_prefill_kernel<K, 4>, dim3(runs, (dim / 4 + 127) / 128), 128, 0, s, dim, tokens, state, in, in_stride, weight, out, out_stride);
-    else launch_k(conv_prefill_kernel<K, 1>, dim3(runs, (dim + 127) / 128), 128, 0, s, dim, tokens, state, in, in_stride, weight, out, out_stride);
+    if (quads) launch_k(conv_prefill_kernel<K, 4>, dim3(runs, (dim / 4 + 127) / 128), 128, 0, s, dim, tokens, run, state, in, in_stride, weight, out, out_stride);
+    else launch_k(conv_prefill_kernel<K, 1>, dim3(runs, (dim + 127) / 128), 128, 0, s, dim, tokens, run, state, in, in_stride, weight, out, out_stride);
 }
 
 // ---- argmax -----------------------------------------------------------------------------------------

@@ -41,6 +41,35 @@ def test_conv_over_a_chunk_is_the_repeated_single_step(pkg, kernel, dim):
     chunked.close(), single.close(), store.close()
 
 
+@pytest.mark.parametrize("kernel,dim", [(3, 64), (8, 320), (4, 192)])
+def test_conv_in_place_over_a_chunk(pkg, kernel, dim):
+    """A convolution whose output buffer is its input buffer, over portions of several runs: the state is the same bits as token by token,
+    the last token's output the same up to the order of the sums in the head's product."""
+    P, vocab = pkg.plan, 512
+    rng = np.random.default_rng(kernel + dim)
+    desc = pkg.BuffersDesc(hidden=dim, slot_dim=3 * dim, vocab=vocab, max_seq=512, max_batch=1, conv_layers=1, conv_dim=dim, conv_kernel=kernel)
+    store = pkg.WeightStore(0)
+    store.add_dense("bcx", _bf(pkg, rng.normal(size=(vocab, 3 * dim))))
+    store.add_dense("taps", _bf(pkg, rng.normal(size=(dim, kernel))))
+    store.add_dense("norm", _bf(pkg, np.ones(dim)))
+    store.add_q4_mlx("head", *pkg.synth_q4(vocab, dim, seed=5, centered=True))
+    steps = [P._step(P.STEP_EMBED, out_buf=P.BUF_S1, n=3 * dim, weight="bcx"),
+             P._step(P.STEP_CONV_STATE_UPDATE, layer=0, in_buf=P.BUF_S1, out_buf=P.BUF_S1, n=dim, conv_kernel=kernel, weight="taps"),
+             P._step(P.STEP_COPY_RMSNORM, in_buf=P.BUF_S1, out_buf=P.BUF_S0, n=dim, eps=1e-5, weight="norm"),
+             P._step(P.STEP_QGEMV, in_buf=P.BUF_S0, out_buf=P.BUF_LOGITS, n=vocab, k=dim, weight="head"),
+             P._step(P.STEP_ARGMAX, in_buf=P.BUF_LOGITS, n=vocab)]
+    chunked, single = pkg.InferenceModel(store, steps, desc), pkg.InferenceModel(store, steps, desc)
+    single.set_prefill_chunk(0)
+    for n in (33, 100, 2, 290):
+        tokens = rng.integers(0, vocab, size=n)
+        chunked.prefill_sequence(0, tokens)
+        single.prefill(tokens[None])
+        assert np.array_equal(chunked.read_conv(0, 0), single.read_conv(0, 0))
+        got, ref = pkg.bf16_to_f32(chunked.logits()), pkg.bf16_to_f32(single.logits())
+        assert np.abs(got - ref).max() <= 1e-2 * np.abs(ref).max()   # one bf16 rounding (2^-9 of the largest) on either side
+    chunked.close(), single.close(), store.close()
+
+
 @pytest.mark.parametrize("heads,kv_heads,hd", [(8, 2, 128), (4, 4, 64), (8, 1, 64), (4, 2, 128), (6, 2, 64)])
 @pytest.mark.parametrize("window,rope_dim", [(0, 0), (0, 64), (1, 64), (40, 24), (150, 64)])
 def test_prompt_attention_is_the_repeated_single_step(pkg, heads, kv_heads, hd, window, rope_dim):
