@@ -246,7 +246,7 @@ int compile_plan(swlm_plan* plan) {
             // gate, up, swiglu -> one launch over row-interleaved weights with a SwiGLU epilogue
             if (i + 2 < st.size() && st[i + 1].kind == SWLM_STEP_QGEMV && (st[i + 2].kind == SWLM_STEP_SWIGLU || st[i + 2].kind == SWLM_STEP_GEGLU) &&
                 st[i + 1].in_buf == s.in_buf && st[i + 1].k == s.k && st[i + 1].n == s.n &&
-                st[i + 2].in_buf == s.out_buf && st[i + 2].in2_buf == st[i + 1].out_buf && (s.n % 8) == 0) {
+                st[i + 2].in_buf == s.out_buf && st[i + 2].in2_buf == st[i + 1].out_buf && st[i + 2].n == s.n && (s.n % 8) == 0) {
                 rc = get_tiled(ctx, {s.weight, st[i + 1].weight}, 1, &L.w);
                 if (rc) return rc;
                 L.w_names = {s.weight, st[i + 1].weight}; L.w_mode = 1;
@@ -954,6 +954,7 @@ int ensure_rows_groups(swlm_plan* plan) {
     // Are the values of `buf` that the gated step `at` reads of no use afterwards? The rows of a prompt are scratch, those of more
     // than 16 sequences are buffers that the host may read after a step: there something has to overwrite them.
     auto gone_after = [&](int buf, size_t at) {
+        if (buf == SWLM_BUF_RESIDUAL) return false;   // read by norms that do not name it
         if (st[at].out_buf == buf) return true;
         for (size_t j = at + 1; j < st.size(); ++j) {
             const swlm_step& c = st[j];
@@ -976,8 +977,9 @@ int ensure_rows_groups(swlm_plan* plan) {
         if (!alone && i + 2 < st.size() && st[i + 1].kind == SWLM_STEP_QGEMV && (st[i + 2].kind == SWLM_STEP_SWIGLU || st[i + 2].kind == SWLM_STEP_GEGLU) &&
             st[i + 1].in_buf == st[i].in_buf && st[i + 2].in_buf == st[i].out_buf && st[i + 2].in2_buf == st[i + 1].out_buf && r0.n % 8 == 0) {
             auto jt = ctx->raw.find(st[i + 1].weight);
+            // (an activation of fewer values than there are rows leaves the rest of its output alone)
             if (jt != ctx->raw.end() && jt->second.k == r0.k && jt->second.n == r0.n && jt->second.sb_f16 == r0.sb_f16 &&
-                gone_after(st[i].out_buf, i + 2) && gone_after(st[i + 1].out_buf, i + 2)) {
+                st[i + 2].n / ctx->tp_size == r0.n && gone_after(st[i].out_buf, i + 2) && gone_after(st[i + 1].out_buf, i + 2)) {
                 names.push_back(st[i + 1].weight);
                 mode = 1;
                 grp.gated = true;

@@ -2,6 +2,8 @@
 import numpy as np
 import pytest
 
+from swlm_helpers import rel_err
+
 pytestmark = pytest.mark.gpu
 
 
@@ -153,4 +155,46 @@ def test_prompt_attention_repeats_itself(pkg, heads, kv_heads, hd, tokens):
             assert np.array_equal(attended(), first), i
         else:   # (the last token attends to every row of both layers)
             assert np.array_equal(model.logits(), last), i
+    model.close(), store.close()
+
+
+@pytest.mark.parametrize("batch", [1, 3, 20])
+def test_an_activation_of_fewer_values_than_its_products_have(pkg, oracle, batch):
+    """Gate and up products of 128 rows, an activation of 64 values: the other half of its output buffer keeps what was there, in single
+    steps, in prompt chunks and in steps of more than 16 sequences."""
+    P, vocab, width, half = pkg.plan, 256, 128, 64
+    rng = np.random.default_rng(batch)
+    desc = pkg.BuffersDesc(hidden=width, slot_dim=width, vocab=vocab, max_seq=128, max_batch=batch)
+    store = pkg.WeightStore(0)
+    rows = {n: _bf(pkg, rng.normal(size=(vocab, width))) for n in ("x", "base")}
+    for n, v in rows.items():
+        store.add_dense(n, v)
+    q4 = {n: pkg.synth_q4(width, width, seed=i, centered=True) for i, n in enumerate(("gate", "up"))}
+    for n, v in q4.items():
+        store.add_q4_mlx(n, *v)
+    store.add_q4_mlx("head", *pkg.synth_q4(vocab, width, seed=5, centered=True))
+    steps = [P._step(P.STEP_EMBED, out_buf=P.BUF_S1, n=width, weight="x"), P._step(P.STEP_EMBED, out_buf=P.BUF_S0, n=width, weight="base"),
+             P._step(P.STEP_QGEMV, in_buf=P.BUF_S1, out_buf=P.BUF_S2, n=width, k=width, weight="gate"),
+             P._step(P.STEP_QGEMV, in_buf=P.BUF_S1, out_buf=P.BUF_S3, n=width, k=width, weight="up"),
+             P._step(P.STEP_SWIGLU, in_buf=P.BUF_S2, in2_buf=P.BUF_S3, out_buf=P.BUF_S0, n=half),
+             P._step(P.STEP_QGEMV, in_buf=P.BUF_S0, out_buf=P.BUF_LOGITS, n=vocab, k=width, weight="head"),
+             # (something writes gate and up again: what a step leaves in them is not of use)
+             P._step(P.STEP_EMBED, out_buf=P.BUF_S2, n=width, weight="x"), P._step(P.STEP_EMBED, out_buf=P.BUF_S3, n=width, weight="x"),
+             P._step(P.STEP_ARGMAX, in_buf=P.BUF_LOGITS, n=vocab)]
+    model = pkg.InferenceModel(store, steps, desc)
+    tokens = rng.integers(0, vocab, size=batch)
+    model.decode(tokens)
+    got = model.read_buffer(P.BUF_S0, width)
+    assert np.array_equal(got[:, half:], rows["base"][tokens][:, half:])
+    gate, up = (pkg.bf16_to_f32(oracle.qgemm(np.ascontiguousarray(rows["x"][tokens]), *q4[n]))[:, :half] for n in ("gate", "up"))
+    assert rel_err(pkg.bf16_to_f32(got)[:, :half], gate / (1 + np.exp(-gate)) * up).max() <= 2e-2   # three bf16 roundings, 2^-9 each, and sums in another order
+    if batch == 1:   # a chunk's last row, against the same token in a step of its own
+        model.reset_state()
+        ids = np.append(rng.integers(0, vocab, size=63), tokens)
+        model.prefill_sequence(0, ids)
+        single = model.logits()
+        model.reset_state()
+        model.set_prefill_chunk(0)
+        model.prefill(ids[None])
+        assert np.abs(pkg.bf16_to_f32(model.logits()) - pkg.bf16_to_f32(single)).max() <= 1e-2 * np.abs(pkg.bf16_to_f32(single)).max()
     model.close(), store.close()
