@@ -546,11 +546,18 @@ int check_launch(const char* what) {
 
 }  // namespace
 
+int norm_init() {
+    SWLM_CUDA(cudaFuncSetAttribute(rmsnorm_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, kNormMaxDim * 4));
+    SWLM_CUDA(cudaFuncSetAttribute(rmsnorm_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kNormMaxDim * 4));
+    SWLM_CUDA(cudaFuncSetAttribute(rmsnorm_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kNormMaxDim * 4));
+    return SWLM_OK;
+}
+
 int launch_rmsnorm(int mode, int m, int dim, const __nv_bfloat16* in, int in_stride, __nv_bfloat16* residual,
                    int res_stride, const __nv_bfloat16* weight, float eps, float weight_bias, __nv_bfloat16* out,
                    int out_stride, cudaStream_t s) {
-    if (dim % 8 || in_stride % 8 || res_stride % 8 || out_stride % 8 || dim > 12288) {
-        set_error("rmsnorm: dim=%d must be a multiple of 8 and <= 12288 with 16-byte aligned rows", dim);
+    if (dim % 8 || in_stride % 8 || res_stride % 8 || out_stride % 8 || dim > kNormMaxDim) {
+        set_error("rmsnorm: dim=%d must be a multiple of 8 and <= %d with 16-byte aligned rows", dim, kNormMaxDim);
         return SWLM_ERR_INVALID;
     }
     const size_t smem = (size_t)dim * 4;

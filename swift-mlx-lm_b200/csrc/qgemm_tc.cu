@@ -846,7 +846,9 @@ int qgemm_tc_init() {
     if ((rc = tc_init_short<32, kTcStages32x2, 2>()) || (rc = tc_init_short<32, kTcStages32, 1>()) || (rc = tc_init_short<64, kTcStages64x2, 2>()) ||
         (rc = tc_init_short<64, kTcStages64, 1>()) || (rc = tc_init_short<128, kTcStages128, 1>()) ||
         (rc = tc_init_one(qgemm_tc_kernel<kTcStagesPair, false>, tc_smem_bytes(kTcPairRows, kTcStagesPair))) ||
-        (rc = tc_init_one(qgemm_tc_kernel<kTcStagesPair, true>, tc_smem_bytes(kTcPairRows, kTcStagesPair)))) return rc;
+        (rc = tc_init_one(qgemm_tc_kernel<kTcStagesPair, true>, tc_smem_bytes(kTcPairRows, kTcStagesPair))) ||
+        (rc = tc_init_one(norm_to_f16_kernel<0>, (size_t)kNormMaxDim * 4)) || (rc = tc_init_one(norm_to_f16_kernel<1>, (size_t)kNormMaxDim * 4)) ||
+        (rc = tc_init_one(norm_to_f16_kernel<2>, (size_t)kNormMaxDim * 4))) return rc;
     return SWLM_OK;
 }
 
@@ -865,7 +867,7 @@ static F16Rows f16_rows(int m, int k, void* scratch) {
 
 int launch_norm_to_f16(int mode, int m, int dim, const __nv_bfloat16* in, int in_stride, __nv_bfloat16* residual, int res_stride, const __nv_bfloat16* weight,
                        float eps, float weight_bias, __nv_bfloat16* out, int out_stride, void* scratch, cudaStream_t s) {
-    if (dim % 64 || in_stride % 8 || res_stride % 8 || out_stride % 8 || dim > 12288) { set_error("rmsnorm: dim=%d", dim); return SWLM_ERR_INVALID; }
+    if (dim % 64 || in_stride % 8 || res_stride % 8 || out_stride % 8 || dim > kNormMaxDim) { set_error("rmsnorm: dim=%d", dim); return SWLM_ERR_INVALID; }
     const F16Rows f = f16_rows(m, dim, scratch);
     const size_t smem = (size_t)dim * 4;
     cudaError_t e;

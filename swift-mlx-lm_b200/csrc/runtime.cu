@@ -787,7 +787,7 @@ bool norm_converts(const swlm_plan* plan, size_t si) {
     if (!plan->rows_groups_ready || si + 1 >= st.size() || st[si + 1].kind != SWLM_STEP_QGEMV || plan->rows_groups[si + 1].count == 0) return false;
     const swlm_step& n = st[si];
     return (n.kind == SWLM_STEP_COPY_RMSNORM || n.kind == SWLM_STEP_RESADD_COPY_RMSNORM || n.kind == SWLM_STEP_RESADD_RMSNORM) &&
-           st[si + 1].in_buf == n.out_buf && plan->rows_groups[si + 1].w->k == n.n && n.n % 64 == 0 && n.n <= 12288;
+           st[si + 1].in_buf == n.out_buf && plan->rows_groups[si + 1].w->k == n.n && n.n % 64 == 0 && n.n <= kNormMaxDim;
 }
 
 int launches_per_step(const swlm_plan* plan, bool body_only) {
@@ -1324,6 +1324,7 @@ int swlm_ctx_create(int device_id, int tp_rank, int tp_size, swlm_ctx** out) {
     if (e != cudaSuccess) { delete ctx; return cuda_fail(e, "cudaStreamCreate"); }
     int rc = qgemv_init();
     if (!rc) rc = qgemv_rows_init();
+    if (!rc) rc = norm_init();
     if (!rc) rc = attn_init();
     if (!rc) rc = qgemm_tc_init();
     if (!rc) rc = bgemm_init();

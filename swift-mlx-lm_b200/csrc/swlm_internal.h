@@ -215,6 +215,8 @@ int qgemv_init();  // sets shared-memory attributes once per process
 void qgemv_trace_report();  // SWLM_TRACE=1: phase timeline of the batch-1 launches, to stderr
 
 // rmsnorm family: mode = SWLM_STEP_COPY_RMSNORM / RESADD_COPY_RMSNORM / RESADD_RMSNORM
+constexpr int kNormMaxDim = 12288;   // a row in fp32 takes 48 KB of shared memory, a little above what a kernel gets unasked
+int norm_init();
 int launch_rmsnorm(int mode, int m, int dim, const __nv_bfloat16* in, int in_stride, __nv_bfloat16* residual,
                    int res_stride, const __nv_bfloat16* weight, float eps, float weight_bias,
                    __nv_bfloat16* out, int out_stride, cudaStream_t s);

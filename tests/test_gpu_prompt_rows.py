@@ -198,3 +198,39 @@ def test_an_activation_of_fewer_values_than_its_products_have(pkg, oracle, batch
         model.prefill(ids[None])
         assert np.abs(pkg.bf16_to_f32(model.logits()) - pkg.bf16_to_f32(single)).max() <= 1e-2 * np.abs(pkg.bf16_to_f32(single)).max()
     model.close(), store.close()
+
+
+@pytest.mark.parametrize("width", [12224, 12288])
+def test_norms_of_the_widest_rows(pkg, oracle, width):
+    """A row of 12288 values in fp32 takes all of the 48 KB of shared memory that a kernel gets unasked: norms of single steps and those
+    that also write a product's fp16 rows, with and without a residual, against the oracle's products of normed rows."""
+    P, vocab = pkg.plan, 128
+    rng = np.random.default_rng(width)
+    desc = pkg.BuffersDesc(hidden=width, slot_dim=width, vocab=vocab, max_seq=128, max_batch=1)
+    store = pkg.WeightStore(0)
+    table, weight = _bf(pkg, rng.normal(size=(vocab, width))), _bf(pkg, 1 + 0.1 * rng.normal(size=width))
+    store.add_dense("rows", table), store.add_dense("norm", weight)
+    q4 = {n: pkg.synth_q4(r, width, seed=i, centered=True) for i, (n, r) in enumerate((("mix", width), ("head", vocab)))}
+    for n, v in q4.items():
+        store.add_q4_mlx(n, *v)
+    steps = [P._step(P.STEP_EMBED, out_buf=P.BUF_HIDDEN, n=width, weight="rows"),
+             P._step(P.STEP_COPY_RMSNORM, in_buf=P.BUF_HIDDEN, out_buf=P.BUF_S0, n=width, eps=1e-5, weight="norm"),
+             P._step(P.STEP_QGEMV, in_buf=P.BUF_S0, out_buf=P.BUF_HIDDEN, n=width, k=width, weight="mix"),
+             P._step(P.STEP_RESADD_RMSNORM, in_buf=P.BUF_HIDDEN, out_buf=P.BUF_S0, n=width, eps=1e-5, weight="norm"),
+             P._step(P.STEP_QGEMV, in_buf=P.BUF_S0, out_buf=P.BUF_LOGITS, n=vocab, k=width, weight="head"),
+             P._step(P.STEP_ARGMAX, in_buf=P.BUF_LOGITS, n=vocab)]
+
+    def norm(h):
+        return pkg.f32_to_bf16((h / np.sqrt((h * h).mean(1, keepdims=True) + 1e-5) * pkg.bf16_to_f32(weight)).astype(np.float32))
+
+    ids = rng.integers(0, vocab, size=40)
+    x = pkg.bf16_to_f32(table[ids[-1:]])
+    mixed = pkg.bf16_to_f32(oracle.qgemm(norm(x), *q4["mix"]))
+    ref = pkg.bf16_to_f32(oracle.qgemm(norm(x + mixed), *q4["head"]))
+    model = pkg.InferenceModel(store, steps, desc)
+    model.prefill_sequence(0, ids)   # (a chunk: its last row goes through the head)
+    assert np.abs(pkg.bf16_to_f32(model.logits()) - ref).max() <= 2e-2 * np.abs(ref).max()   # three bf16 roundings of 2^-9 in front of the head's sums
+    model.reset_state()
+    model.decode(ids[-1:])
+    assert np.abs(pkg.bf16_to_f32(model.logits()) - ref).max() <= 2e-2 * np.abs(ref).max()
+    model.close(), store.close()
