@@ -90,6 +90,9 @@ __device__ __forceinline__ void umma_commit_pair(unsigned long long* bar) {
     asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
                  ::"r"(smem_u32(bar)), "h"((unsigned short)3) : "memory");
 }
+// A row's factor. Its writer may still have been running when this kernel started: read from L2, neither through the non-coherent path
+// nor out of a line that an earlier CTA of this SM may have left in L1.
+__device__ __forceinline__ float tc_rscale(const QGemmTcParams& p, int token) { return __ldcg(p.rscale + token); }
 // One result, rounded once to bf16, to the output its weight row belongs to.
 __device__ __forceinline__ void tc_store(const TcSegments& o, int token, int row, float val) {
     const __nv_bfloat16 v = __float2bfloat16_rn(val);
@@ -363,7 +366,7 @@ __device__ __forceinline__ void tc_store16(const QGemmTcParams& p, const unsigne
         __nv_bfloat16* dst = (q == 0 ? p.out.y[0] : q == 1 ? p.out.y[1] : p.out.y[2]) + (row - (q == 0 ? 0 : q == 1 ? p.out.end[0] : p.out.end[1])) + (size_t)token0 * stride;
 #pragma unroll
         for (int i = 0; i < 16; ++i)
-            if (token0 + i < p.m) dst[(size_t)i * stride] = __float2bfloat16_rn(__uint_as_float(v[i]) * __ldg(p.rscale + token0 + i));
+            if (token0 + i < p.m) dst[(size_t)i * stride] = __float2bfloat16_rn(__uint_as_float(v[i]) * tc_rscale(p, token0 + i));
         return;
     }
     // gate rows sit in the lanes of the first eight of 16, up rows in the others: a gate lane finishes even columns, its up lane odd ones
@@ -374,7 +377,7 @@ __device__ __forceinline__ void tc_store16(const QGemmTcParams& p, const unsigne
         const float other = __uint_as_float(__shfl_xor_sync(0xffffffffu, up_lane ? v[i] : v[i + 1], 8));
         const int token = token0 + i + (up_lane ? 1 : 0);
         if (token < p.m) {
-            const float sc = __ldg(p.rscale + token);
+            const float sc = tc_rscale(p, token);
             if (up_lane) tc_store_gated(p, token, out_row, other * sc, __uint_as_float(v[i + 1]) * sc);
             else tc_store_gated(p, token, out_row, __uint_as_float(v[i]) * sc, other * sc);
         }
@@ -579,7 +582,7 @@ __global__ void __launch_bounds__((kTcDeqWarps + 2) * 32, PER_SM) qgemm_tc_short
                 va += src[z * own * kTcRows];
                 if (p.gated) vb += src[z * own * kTcRows + 8];
             }
-            const float sc = __ldg(p.rscale + token);
+            const float sc = tc_rscale(p, token);
             if (p.gated) tc_store_gated(p, token, row0 / 2 + i, va * sc, vb * sc);
             else tc_store(p.out, token, row0 + i, va * sc);
         }
