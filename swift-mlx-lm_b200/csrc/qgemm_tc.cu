@@ -90,9 +90,13 @@ __device__ __forceinline__ void umma_commit_pair(unsigned long long* bar) {
     asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
                  ::"r"(smem_u32(bar)), "h"((unsigned short)3) : "memory");
 }
-// A row's factor. Its writer may still have been running when this kernel started: read from L2, neither through the non-coherent path
-// nor out of a line that an earlier CTA of this SM may have left in L1.
-__device__ __forceinline__ float tc_rscale(const QGemmTcParams& p, int token) { return __ldcg(p.rscale + token); }
+// A row's factor, by a thread that has waited for the kernel in front (pdl_wait), which writes it: what that kernel wrote is visible to
+// plain loads then, not to the non-coherent ones. (From L2 for every lane and column: 2 % to 5 % of a product.)
+__device__ __forceinline__ float tc_rscale(const QGemmTcParams& p, int token) {
+    float v;
+    asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p.rscale + token));
+    return v;
+}
 // One result, rounded once to bf16, to the output its weight row belongs to.
 __device__ __forceinline__ void tc_store(const TcSegments& o, int token, int row, float val) {
     const __nv_bfloat16 v = __float2bfloat16_rn(val);
@@ -463,6 +467,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__((kTcDeqWarps + 2 + k
         const int half = (warp - kTcDeqWarps - 2) >> 2;
         const unsigned acc_empty = pair_leader(smem_u32(&bars.acc_empty));
         unsigned par = 0;
+        pdl_wait();   // (the rows' factors)
         for (int tile = first; tile < p.n_tiles; tile += pairs, par ^= 1u) {
             if (!mbar_wait_warp(&bars.acc_full, par)) { tc_fail(p.status, &bars.failed, 4); break; }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -543,6 +548,7 @@ __global__ void __launch_bounds__((kTcDeqWarps + 2) * 32, PER_SM) qgemm_tc_short
         __syncwarp();
     }
     // ---- results: warp w reads the lanes of quarter w & 3 and a quarter of the columns ---------------------------------------
+    pdl_wait();   // (the rows' factors)
     const bool done = mbar_wait_warp(&bars.acc_full, 0u);
     if (!done && lane == 0) tc_fail(p.status, &bars.failed, 5);
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
