@@ -130,11 +130,13 @@ __device__ __forceinline__ unsigned pair_leader(unsigned addr) {   // the same s
     asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(r) : "r"(addr));
     return r;
 }
-template <int CG>
-__device__ __forceinline__ void tc_arrive(unsigned bar) {   // CG = 2: `bar` is a cluster address
-    if (CG == 1) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-    else asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");   // (with a release of cluster scope an arrival takes 1200 clocks)
-}
+// Arrivals at the barriers that an MMA warp waits at.
+// Within a CTA: hands over whatever the arriving warp has done or waited for.
+__device__ __forceinline__ void tc_arrive(unsigned bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory"); }
+// From either CTA of a pair (`bar`: a cluster address), for what was done to tensor memory: tcgen05 operations are ordered by the waits
+// and fences of their own on either side and by the arrival being seen. A release of cluster scope would order nothing more that the
+// MMAs read, and waits for the weights that the arriving warp has requested ahead (1200 clocks).
+__device__ __forceinline__ void tc_arrive_tmem(unsigned bar) { asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory"); }
 
 // A ring position and the parity of its phase.
 template <int N>
@@ -190,6 +192,13 @@ __device__ __forceinline__ void tc_issue(const CUtensorMap* xmap, unsigned stage
     mbar_expect(bar, (unsigned)ROWS * 256u);
     tma_load_2d(stage, xmap, kt * kTcStep, tok0, bar);
     tma_load_2d(stage + ROWS * 128, xmap, kt * kTcStep + 64, tok0, bar);
+}
+// The same for a pair: both CTAs' copies count on the barrier of the CTA that issues the MMAs (`bar`: a cluster address). The other CTA's
+// may get there before the bytes are announced: the phase ends with the announcement at the earliest.
+template <int ROWS>
+__device__ __forceinline__ void tc_issue_pair(const CUtensorMap* xmap, unsigned stage, unsigned bar, int kt, int tok0) {
+    tma_load_2d_pair(stage, xmap, kt * kTcStep, tok0, bar);
+    tma_load_2d_pair(stage + ROWS * 128, xmap, kt * kTcStep + 64, tok0, bar);
 }
 // ---- the eight MMAs of a step; ROWS: activation rows in this CTA's shared memory ----------------------------------------------
 template <int CG, int ROWS>
@@ -308,16 +317,22 @@ __device__ __forceinline__ bool tc_dequant(const QGemmTcParams& p, TcBars<STAGES
     auto finish = [&]() {
         asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");   // the stores are ordered before the MMAs of the thread that waits
-        // the CTA's activations have landed: one warp's arrival covers them for the MMAs
-        if ((warp & (kTcSet - 1)) == 0 && !mbar_wait_warp(full0 + 8u * at.s, at.par)) return false;
+        // the CTA's activations have landed: one warp's arrival covers them for the MMAs (of a pair the MMA warp waits for both CTAs')
+        if (CG == 1 && (warp & (kTcSet - 1)) == 0 && !mbar_wait_warp(full0 + 8u * at.s, at.par)) return false;
         __syncwarp();
-        if (lane == 0) tc_arrive<CG>(ready0 + 8u * a_slot);
+        if (lane == 0) {
+            if (CG == 1) tc_arrive(ready0 + 8u * a_slot);
+            else tc_arrive_tmem(ready0 + 8u * a_slot);
+        }
         a_slot += 2;
         if (a_slot >= SA) a_slot -= SA;
         at.skip2();
         return true;
     };
     static_assert(SA >= 2 && STAGES >= 2, "steps advance by two");
+    // a wait by parity cannot tell a phase from the one two before: when a step is seen to be SA steps behind the MMAs, the copies and
+    // MMAs of the step STAGES back (the phase before of its stage's barriers) have to be over
+    static_assert(STAGES >= SA, "a stage's phase may not lap a waiting warp");
 
 #pragma unroll
     for (int i = 0; i < kTcAhead - 1; ++i) fetch(i);
@@ -414,9 +429,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__((kTcDeqWarps + 2 + k
             bool ok = true;
             for (int tile = first; tile < p.n_tiles && ok; tile += pairs) {
                 // the accumulators of the tile before have been read
-                if (done > 0 && !mbar_wait_warp(&bars.acc_empty, (unsigned)((done - 1) & 1))) { ok = false; break; }
+                if (done > 0 && !mbar_wait_cluster_warp(&bars.acc_empty, (unsigned)((done - 1) & 1))) { ok = false; break; }
                 for (int kt = 0; kt < p.steps; ++kt) {
-                    if (!mbar_wait_warp(&bars.ready[a_slot], a_par)) { ok = false; break; }
+                    if (!mbar_wait_cluster_warp(&bars.full[full.s], full.par) || !mbar_wait_cluster_warp(&bars.ready[a_slot], a_par)) { ok = false; break; }
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     if (el) {
                         tc_mma_step<2, kTcPairRows>(tmem_d, tmem_d + 256u + a_slot * 64u, ring + full.s * STAGE_BYTES, kt == 0);
@@ -441,6 +456,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__((kTcDeqWarps + 2 + k
         if (lane == 0) {
             pdl_wait();                         // the activations come from the kernel just before this one
             RingPos<STAGES> at;
+            const unsigned full0 = pair_leader(smem_u32(&bars.full[0]));
             int issued = 0;
             bool ok = true;
             for (int tile = first; tile < p.n_tiles && ok; tile += pairs) {
@@ -448,14 +464,19 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__((kTcDeqWarps + 2 + k
                 for (int kt = 0; kt < p.steps; ++kt) {
                     // the MMAs that read this stage a round ago are done
                     if (*failed || (issued >= STAGES && !mbar_wait(&bars.empty[at.s], at.par ^ 1u))) { ok = false; break; }
-                    tc_issue<kTcPairRows>(&xmap, ring + at.s * STAGE_BYTES, smem_u32(&bars.full[at.s]), kt, tok0);
+                    if (rank == 0) mbar_expect(smem_u32(&bars.full[at.s]), 2u * STAGE_BYTES);
+                    tc_issue_pair<kTcPairRows>(&xmap, ring + at.s * STAGE_BYTES, full0 + 8u * at.s, kt, tok0);
                     at.next();
                     ++issued;
                 }
             }
             if (!ok) tc_fail(p.status, &bars.failed, 3);
-            // every copy has landed before the CTA leaves (also when it stops early)
-            for (int i = issued > STAGES ? issued - STAGES : 0; i < issued; ++i) mbar_wait(&bars.full[i % STAGES], (unsigned)((i / STAGES) & 1));
+            // every copy of the pair has landed before either CTA leaves: they meet again behind this. Where one of them stopped early the
+            // last wait is for a phase that does not end: its limit is the time that the other's copies get.
+            if (rank == 0) {
+                for (int i = issued > STAGES ? issued - STAGES : 0; i < issued; ++i) mbar_wait(&bars.full[i % STAGES], (unsigned)((i / STAGES) & 1));
+                if (!ok) mbar_wait(&bars.full[at.s], at.par);
+            }
         }
         __syncwarp();
     } else if (warp < kTcDeqWarps) {
@@ -481,7 +502,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__((kTcDeqWarps + 2 + k
             }
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
-            if (lane == 0) tc_arrive<2>(acc_empty);
+            if (lane == 0) tc_arrive_tmem(acc_empty);
         }
         __syncwarp();
     }

@@ -18,30 +18,40 @@ __device__ __forceinline__ void mbar_init(unsigned long long* bar, unsigned coun
 // Bounded wait on phase parity; returns false when the limit was reached. The loop is two instructions per
 // attempt (try_wait suspends the warp for a while by itself): waiting warps share their scheduler with warps
 // that still dequantise.
+#define SWLM_MBAR_WAIT(SEM)                                                            \
+    asm volatile(                                                                      \
+        "{\n\t"                                                                        \
+        ".reg .pred p, q;\n\t"                                                         \
+        ".reg .u32 n;\n\t"                                                             \
+        "mov.u32 n, 0;\n\t"                                                            \
+        "SWLM_TRY:\n\t"                                                                \
+        "mbarrier.try_wait.parity" SEM ".shared::cta.b64 p, [%1], %2;\n\t"             \
+        "@p bra SWLM_DONE;\n\t"                                                        \
+        "add.u32 n, n, 1;\n\t"                                                         \
+        "setp.lt.u32 q, n, %3;\n\t"                                                    \
+        "@q bra SWLM_TRY;\n\t"                                                         \
+        "SWLM_DONE:\n\t"                                                               \
+        "selp.u32 %0, 1, 0, p;\n\t"                                                    \
+        "}"                                                                            \
+        : "=r"(done) : "r"(addr), "r"(parity), "r"((unsigned)kTcSpinLimit) : "memory")
 __device__ __forceinline__ bool mbar_wait_addr(unsigned addr, unsigned parity) {
     unsigned done;
-    asm volatile(
-        "{\n\t"
-        ".reg .pred p, q;\n\t"
-        ".reg .u32 n;\n\t"
-        "mov.u32 n, 0;\n\t"
-        "SWLM_TRY:\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "@p bra SWLM_DONE;\n\t"
-        "add.u32 n, n, 1;\n\t"
-        "setp.lt.u32 q, n, %3;\n\t"
-        "@q bra SWLM_TRY;\n\t"
-        "SWLM_DONE:\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t"
-        "}"
-        : "=r"(done) : "r"(addr), "r"(parity), "r"((unsigned)kTcSpinLimit) : "memory");
+    SWLM_MBAR_WAIT("");
     return done != 0;
 }
+// The same where threads of another CTA of the cluster arrive.
+__device__ __forceinline__ bool mbar_wait_cluster_addr(unsigned addr, unsigned parity) {
+    unsigned done;
+    SWLM_MBAR_WAIT(".acquire.cluster");
+    return done != 0;
+}
+#undef SWLM_MBAR_WAIT
 __device__ __forceinline__ bool mbar_wait(unsigned long long* bar, unsigned parity) { return mbar_wait_addr(smem_u32(bar), parity); }
 
 // The same for a converged warp: all its lanes get the same answer, also when some of them saw the limit.
 __device__ __forceinline__ bool mbar_wait_warp(unsigned addr, unsigned parity) { return __all_sync(0xffffffffu, mbar_wait_addr(addr, parity)); }
 __device__ __forceinline__ bool mbar_wait_warp(unsigned long long* bar, unsigned parity) { return mbar_wait_warp(smem_u32(bar), parity); }
+__device__ __forceinline__ bool mbar_wait_cluster_warp(unsigned long long* bar, unsigned parity) { return __all_sync(0xffffffffu, mbar_wait_cluster_addr(smem_u32(bar), parity)); }
 
 // Shared-memory matrix descriptor: K-major operand, 128-byte swizzle, rows of 128 bytes, 8-row groups 1024
 // bytes apart (stride byte offset); leading byte offset unused for this layout; descriptor version 1.
@@ -74,6 +84,11 @@ __device__ __forceinline__ void umma_commit(unsigned long long* bar) {
 // One tile of a 2-D tensor map (x = innermost coordinate), completion counted on an mbarrier of this CTA.
 __device__ __forceinline__ void tma_load_2d(unsigned smem_dst, const CUtensorMap* map, int x, int y, unsigned bar) {
     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
+                 ::"r"(smem_dst), "l"(reinterpret_cast<unsigned long long>(map)), "r"(x), "r"(y), "r"(bar) : "memory");
+}
+// The same where the mbarrier (a cluster address) may lie in the other CTA of a pair.
+__device__ __forceinline__ void tma_load_2d_pair(unsigned smem_dst, const CUtensorMap* map, int x, int y, unsigned bar) {
+    asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
                  ::"r"(smem_dst), "l"(reinterpret_cast<unsigned long long>(map)), "r"(x), "r"(y), "r"(bar) : "memory");
 }
 // `bytes` contiguous bytes (16-byte aligned, a multiple of 16) into shared memory.

@@ -78,3 +78,127 @@ def test_more_tiles_than_multiprocessors(pkg, oracle):
     rows = np.r_[0:40, 255:258, 511:514, 590:600]
     assert rel_err(got[rows], pkg.bf16_to_f32(oracle.qgemm(np.ascontiguousarray(x[rows]), w, s, b))).max() <= RTOL
     store.close()
+
+
+def _form(m, rows, k, gated=False):
+    """Which form `tc_choose` takes for m activation rows, by its estimates of the time: (rows per tile, CTAs per SM, CTAs along K) and the
+    number of steps. The tests below name the form they are about; they have to follow when the rule moves."""
+    kt = (k // 64 + 3) // 4 * 4
+    steps = (kt * 64 + -(-3 * (-(-kt // 64) * 64) // 128) * 128) // 128
+    tiles16 = -(-rows // 8) if gated else -(-rows // 16)
+    bn = 32 if m <= 32 else 64 if m <= 64 else 128
+    tiles = -(-tiles16 // 8) * -(-m // bn)
+    offers = []
+    for z in (1, 2, 4):
+        if z <= steps:
+            exchange = 0 if z == 1 else 5 if z == 4 else 9 if bn == 128 else 7
+            offers.append((-(-tiles * z // 148) * ((0.5 if bn == 128 else 0.45) * -(-steps // z) + 2) + 4 + exchange, (bn, 1, z)))
+    if bn <= 64 and tiles > 148:
+        offers.append((-(-tiles // 296) * (0.9 * steps + 2) + 4, (bn, 2, 1)))
+    if m > 128:
+        offers.append((-(--(-tiles16 // 16) * -(-m // 256) // 74) * (0.87 * steps + 1.5) + 5, (256, 1, 1)))
+    return min(offers)[1], steps
+
+
+PAIR, PAIR_TILES = (256, 1, 1), 74
+
+
+@pytest.mark.parametrize("m,n,k,form,steps", [
+    (700, 6648, 512, PAIR, 6), (513, 11368, 4160, PAIR, 37),   # pairs of SMs, several tiles each: even and odd steps (the sets of
+    (700, 9536, 8192, PAIR, 67),                               # dequantising warps change places), ragged rows and columns
+    (20, 19500, 320, (32, 2, 1), 6), (50, 19500, 576, (64, 2, 1), 8),   # two CTAs per SM, three weight tiles in flight
+    (20, 19500, 4160, (32, 2, 1), 37), (64, 21000, 4224, (64, 2, 1), 37),
+    (41, 4096, 14336, (64, 1, 4), 118), (100, 14336, 1024, (128, 1, 1), 10),
+])
+def test_forms_of_the_tensor_core_products(pkg, oracle, m, n, k, form, steps):
+    """Every form with remainders, bf16 and fp16 scales; compared at rows of the first, the middle and the last tiles."""
+    assert _form(m, n, k) == (form, steps)
+    if form == PAIR:
+        assert -(-n // 256) * -(-m // 256) > PAIR_TILES and m % 256 and n % 256
+    store = pkg.WeightStore(0)
+    w, s, b = pkg.synth_q4(n, k, seed=n + k, centered=True)
+    x = pkg.f32_to_bf16(np.random.default_rng(m).normal(size=(m, k)).astype(np.float32))
+    rows = np.unique(np.r_[0:4, 30:34, 62:66, 126:130, 254:258, 510:514, m // 2:m // 2 + 3, m - 4:m] % m)
+    store.add_q4_mlx("mlx", w, s, b)
+    ref = pkg.bf16_to_f32(oracle.qgemm(np.ascontiguousarray(x[rows]), w, s, b))
+    assert rel_err(pkg.bf16_to_f32(store.qgemm("mlx", x, n))[rows], ref).max() <= RTOL
+    store.add_q4_staf("staf", pkg.formats.repack_mlx_to_staf(w, s, b), n, k)
+    assert rel_err(pkg.bf16_to_f32(store.qgemm("staf", x, n))[rows], ref).max() <= RTOL
+    store.close()
+
+
+@pytest.mark.parametrize("staf", [False, True])
+@pytest.mark.parametrize("m,ff,k,form", [(20, 9728, 320, (32, 2, 1)), (41, 9728, 576, (64, 2, 1)), (24, 2048, 4160, (32, 1, 4))])
+def test_gated_products_of_a_batch(pkg, oracle, staf, m, ff, k, form):
+    """Gate, up and activation as one product in a step of more than 16 sequences, against the oracle's two products."""
+    assert _form(m, ff, k, gated=True)[0] == form
+    P, vocab = pkg.plan, 128
+    rng = np.random.default_rng(m + k)
+    store, q4, table = _gated_store(pkg, rng, vocab, k, ff, staf)
+    desc = pkg.BuffersDesc(hidden=k, slot_dim=max(ff, k), vocab=vocab, max_seq=16, max_batch=m)
+    steps = [P._step(P.STEP_EMBED, out_buf=P.BUF_S3, n=k, weight="rows")] + _gated_steps(P, k, ff) + [
+        P._step(P.STEP_QGEMV, in_buf=P.BUF_S0, out_buf=P.BUF_LOGITS, n=vocab, k=ff, weight="down"),
+        # (something writes gate and up again: what a step leaves in them is not of use)
+        P._step(P.STEP_EMBED, out_buf=P.BUF_S1, n=k, weight="rows"), P._step(P.STEP_EMBED, out_buf=P.BUF_S2, n=k, weight="rows"),
+        P._step(P.STEP_ARGMAX, in_buf=P.BUF_LOGITS, n=vocab)]
+    model = pkg.InferenceModel(store, steps, desc)
+    tokens = rng.integers(0, vocab, size=m)
+    model.decode(tokens)
+    got = pkg.bf16_to_f32(model.read_buffer(P.BUF_S0, ff))
+    ref = _gated_ref(pkg, oracle, table[tokens], q4)
+    for i in range(m):
+        assert rel_err(got[i], ref[i]).max() <= 2 * RTOL   # two products' errors
+    model.close(), store.close()
+
+
+@pytest.mark.parametrize("staf", [False, True])
+@pytest.mark.parametrize("m,ff,k,steps", [(600, 9600, 576, 8), (513, 5696, 4160, 37)])
+def test_gated_products_of_a_prompt(pkg, oracle, staf, m, ff, k, steps):
+    """The same over pairs of SMs, several tiles each, in a prompt chunk: a second product of every token's result lands in the value
+    cache, where it can be read."""
+    assert _form(m, ff, k, gated=True) == (PAIR, steps) and -(-ff // 128) * -(-m // 256) > PAIR_TILES
+    P, vocab, hd = pkg.plan, 128, 64
+    rng = np.random.default_rng(m + k)
+    store, q4, table = _gated_store(pkg, rng, vocab, k, ff, staf, down=hd)
+    desc = pkg.BuffersDesc(hidden=k, slot_dim=max(ff, k), vocab=vocab, max_seq=m + 8, max_batch=1, kv_layers=1, kv_heads=1, head_dim=hd)
+    steps = [P._step(P.STEP_EMBED, out_buf=P.BUF_S3, n=k, weight="rows")] + _gated_steps(P, k, ff) + [
+        P._step(P.STEP_QGEMV, in_buf=P.BUF_S0, out_buf=P.BUF_S2, n=hd, k=ff, weight="down"),
+        P._step(P.STEP_ATTN_DECODE, layer=0, in_buf=P.BUF_S3, in2_buf=P.BUF_S3, in3_buf=P.BUF_S2, out_buf=P.BUF_S1, heads=1, kv_heads=1, head_dim=hd, scale=0.125),
+        P._step(P.STEP_QGEMV, in_buf=P.BUF_S1, out_buf=P.BUF_LOGITS, n=vocab, k=hd, weight="head"), P._step(P.STEP_ARGMAX, in_buf=P.BUF_LOGITS, n=vocab)]
+    store.add_q4_mlx("head", *pkg.synth_q4(vocab, hd, seed=5, centered=True))
+    model = pkg.InferenceModel(store, steps, desc)
+    tokens = rng.integers(0, vocab, size=m)
+    model.prefill_sequence(0, tokens)
+    got = pkg.bf16_to_f32(model.read_kv(1, 0, 0, 0, m))
+    act = _gated_ref(pkg, oracle, table, q4)
+    ref = pkg.bf16_to_f32(oracle.qgemm(pkg.f32_to_bf16(act), *q4["down"]))[tokens]
+    for i in range(m):   # every token: a tile that was left out or taken twice shows
+        # ff terms that may differ by three bf16 roundings (gate, up, their product; rms 2^-9 / sqrt(3) of a term each): 2^-9 of the row's
+        # rms as a standard deviation, eight of them, and the result's own rounding of 2^-9 of up to four times the rms. A tile of 128
+        # terms left out would be 15 %.
+        assert np.abs(got[i] - ref[i]).max() <= 2.4e-2 * np.sqrt((ref[i] ** 2).mean()), i
+    model.close(), store.close()
+
+
+def _gated_store(pkg, rng, vocab, k, ff, staf, down=None):
+    table = pkg.f32_to_bf16(rng.normal(size=(vocab, k)).astype(np.float32))
+    q4 = {name: pkg.synth_q4(n, kk, seed=i, centered=True) for i, (name, n, kk) in enumerate((("gate", ff, k), ("up", ff, k), ("down", down or vocab, ff)))}
+    store = pkg.WeightStore(0)
+    store.add_dense("rows", table)
+    for name, (w, s, b) in q4.items():
+        if staf:
+            store.add_q4_staf(name, pkg.formats.repack_mlx_to_staf(w, s, b), w.shape[0], w.shape[1] * 8)
+        else:
+            store.add_q4_mlx(name, w, s, b)
+    return store, q4, table
+
+
+def _gated_steps(P, k, ff):
+    return [P._step(P.STEP_QGEMV, in_buf=P.BUF_S3, out_buf=P.BUF_S1, n=ff, k=k, weight="gate"),
+            P._step(P.STEP_QGEMV, in_buf=P.BUF_S3, out_buf=P.BUF_S2, n=ff, k=k, weight="up"),
+            P._step(P.STEP_SWIGLU, in_buf=P.BUF_S1, in2_buf=P.BUF_S2, out_buf=P.BUF_S0, n=ff)]
+
+
+def _gated_ref(pkg, oracle, x, q4):
+    gate, up = (pkg.bf16_to_f32(oracle.qgemm(np.ascontiguousarray(x), *q4[n])) for n in ("gate", "up"))
+    return (gate / (1 + np.exp(-gate)) * up).astype(np.float32)
