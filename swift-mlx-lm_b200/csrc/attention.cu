@@ -1019,11 +1019,23 @@ int attn_pick_splits(int m, int kv_heads, int max_ctx, bool ragged) {
     static const int forced = [] { const char* v = getenv("SWLM_ATTN_SPLITS"); return v ? atoi(v) : 0; }();
     if (forced >= 1 && forced <= 64) return forced;
     if (m <= 0 || kv_heads <= 0) return 1;
-    // Two CTAs fit an SM. Below 300 (sequence, KV head) pairs the splits fill the GPU once. From 150 pairs on that would leave every
-    // pair to one CTA, and the longest sequence of a ragged batch would hold up the step (41 sequences of 1000 to 4091 tokens: a
-    // model's step takes 1.35 ms with one split, 1.28 with two, 1.30 / 1.32 / 1.37 with three, four, eight): two rounds of CTAs then.
-    int s = 300 / (m * kv_heads);
-    if (ragged && s <= 1) s = (600 + m * kv_heads / 2) / (m * kv_heads);
+    // Two CTAs fit an SM. Below 300 (sequence, KV head) pairs the splits fill the GPU once. From 150 pairs on that leaves every pair to
+    // one CTA, and the longest sequence of a ragged batch, or a second round that is nearly empty, holds up the step. In a long cache at
+    // least 450 CTAs then, one and a half rounds. Steps of a model of four layers, 8 KV heads of 128, against one split; sequences of
+    // equal length / down to a quarter of it:
+    //   pairs  splits   2200 tokens      4000 tokens      two splits at 4000
+    //    152      3     -2.3 / -7.6 %    -3.5 / -12.5 %   +1.9 / -10.6 %
+    //    192      3     -0.5 / -5.0      -0.3 /  -8.5     +4.4 /  -8.7
+    //    240      2                      -4.1 /  -8.3
+    //    296      2     -0.8 / -3.0      -4.0 /  -7.3
+    //    328      2                      -8.5 /  -5.8
+    //    384      2     -4.1 / +0.8      -9.1 /  -4.6
+    //    512      2                      -2.2 /  +0.2
+    // Short caches lose (192 pairs: +1.4 % at 1000 tokens, 240 pairs at 600 ragged: +1.6), the more pairs the longer: hence ten rows per
+    // pair, and from 450 pairs on one split. (A short batch in a long cache pays 1 to 2 % for what it gains when it is long.)
+    const int pairs = m * kv_heads;
+    int s = 300 / pairs;
+    if (ragged && s <= 1 && pairs < 450 && max_ctx >= 10 * pairs) s = (450 + pairs - 1) / pairs;
     const int cap = max_ctx / 128;
     if (s > 32) s = 32;
     if (s > cap) s = cap;

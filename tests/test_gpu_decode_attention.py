@@ -1,4 +1,4 @@
-"""Decode attention of a plan: the per-head norm of q and k inside its launch, and the splits of ragged batches."""
+"""Decode attention of a plan: the per-head norm of q and k inside its launch, and the splits of large batches."""
 import numpy as np
 import pytest
 
@@ -47,11 +47,16 @@ def test_norm_in_the_attention_launch_is_the_norm_of_its_own(pkg, heads, kv_head
     apart.close(), inside.close(), store.close()
 
 
-@pytest.mark.parametrize("batch,kv_heads,hd", [(19, 8, 64), (37, 4, 128), (38, 4, 64), (64, 8, 128)])
-def test_ragged_batches_attend_as_each_sequence_alone(pkg, batch, kv_heads, hd):
-    """Either side of 150 (sequence, KV head) pairs, where the longest sequence would hold up the step and the cache is split further:
-    sequences from empty to full, each against a model of its own, to one bf16 rounding (2^-8) and the order of the sums."""
-    P, vocab, max_seq, width = pkg.plan, 256, 320, 2 * kv_heads * hd
+@pytest.mark.parametrize("batch,kv_heads,hd,max_seq", [
+    (19, 8, 64, 320), (37, 4, 128, 320), (38, 4, 64, 320), (64, 8, 128, 320),   # short caches: one or two splits
+    (19, 8, 64, 1536), (25, 8, 64, 2000),                                       # 152 and 200 pairs in long caches: three splits
+    (38, 8, 64, 3040), (38, 8, 64, 3039),                                       # 304 pairs: two splits from 3040 rows on, one below
+    (57, 8, 64, 4608),                                                          # 456 pairs: one split whatever the length
+])
+def test_ragged_batches_attend_as_each_sequence_alone(pkg, batch, kv_heads, hd, max_seq):
+    """Either side of the rules for the splits of large batches: sequences from empty (so that some splits have no rows) to full, each
+    against a model of its own, to one bf16 rounding (2^-8) and the order of the sums."""
+    P, vocab, width = pkg.plan, 256, 2 * kv_heads * hd
     rng = np.random.default_rng(batch + hd)
     store = pkg.WeightStore(0)
     for name, n in (("q", width), ("k", kv_heads * hd), ("v", kv_heads * hd)):
