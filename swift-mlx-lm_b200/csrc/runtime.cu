@@ -13,6 +13,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <algorithm>
+#include <climits>
 #include <cmath>
 
 #include "swlm_runtime.h"
@@ -204,6 +205,55 @@ int rope_table_for(swlm_plan* plan, int rope_dim, float base, int* index) {
 }
 
 bool buf_ok(int b) { return b >= 0 && b < SWLM_BUF_COUNT; }
+
+// How many values of each row of `buf`, from its front, a step reads, and how many it is sure to write (a rank's share). Steps that are
+// not listed read everything and write nothing.
+int step_reads(const swlm_step& s, int buf, int tp) {
+    int n = 0;
+    auto takes = [&](int b, int width) { if (b == buf) n = std::max(n, width); };
+    switch (s.kind) {
+    case SWLM_STEP_EMBED: break;
+    case SWLM_STEP_COPY_RMSNORM: takes(s.in_buf, s.n); break;
+    case SWLM_STEP_RESADD_COPY_RMSNORM:
+    case SWLM_STEP_RESADD_RMSNORM: takes(s.in_buf, s.n); takes(SWLM_BUF_RESIDUAL, s.n); break;
+    case SWLM_STEP_QGEMV: takes(s.in_buf, s.k); break;
+    case SWLM_STEP_ATTN_DECODE: takes(s.in3_buf, s.kv_heads * s.head_dim / tp); [[fallthrough]];
+    case SWLM_STEP_QK_NORM: takes(s.in_buf, s.heads * s.head_dim / tp); takes(s.in2_buf, s.kv_heads * s.head_dim / tp); break;
+    case SWLM_STEP_SWIGLU:
+    case SWLM_STEP_GEGLU: takes(s.in_buf, s.n / tp); takes(s.in2_buf, s.n / tp); break;
+    case SWLM_STEP_CONV_STATE_UPDATE: takes(s.in_buf, 3 * (s.n / tp)); break;
+    case SWLM_STEP_ARGMAX: takes(s.in_buf, s.n); break;
+    default: takes(s.in_buf, INT_MAX); takes(s.in2_buf, INT_MAX); takes(s.in3_buf, INT_MAX); takes(s.in4_buf, INT_MAX); break;
+    }
+    return n;
+}
+int step_writes(const swlm_step& s, int buf, int tp) {
+    int n = 0;
+    switch (s.kind) {
+    case SWLM_STEP_COPY_RMSNORM:
+    case SWLM_STEP_RESADD_COPY_RMSNORM: if (buf == SWLM_BUF_RESIDUAL) n = s.n; [[fallthrough]];
+    case SWLM_STEP_EMBED:
+    case SWLM_STEP_RESADD_RMSNORM: if (s.out_buf == buf) n = s.n; break;
+    case SWLM_STEP_QGEMV:
+    case SWLM_STEP_SWIGLU:
+    case SWLM_STEP_GEGLU:
+    case SWLM_STEP_CONV_STATE_UPDATE: if (s.out_buf == buf) n = s.n / tp; break;
+    case SWLM_STEP_ATTN_DECODE: if (s.out_buf == buf) n = s.heads * s.head_dim / tp; break;
+    default: break;
+    }
+    return n;
+}
+// Are the first n values of a buffer written anew by what runs at `first` and behind it, before any of them is read? `otherwise`: the
+// answer when nothing reads them and nothing writes them all.
+template <typename Reads, typename Writes>
+bool replaced_unread(size_t first, size_t end, int n, bool otherwise, Reads reads, Writes writes) {
+    int anew = 0;
+    for (size_t j = first; j < end && anew < n; ++j) {
+        if (reads(j) > anew) return false;
+        anew = std::max(anew, writes(j));
+    }
+    return anew >= n || otherwise;
+}
 
 int compile_plan(swlm_plan* plan) {
     swlm_ctx* ctx = plan->ctx;
@@ -953,15 +1003,9 @@ int ensure_rows_groups(swlm_plan* plan) {
     plan->rows_groups.assign(st.size(), swlm_plan::RowsGroup{});
     // Are the values of `buf` that the gated step `at` reads of no use afterwards? The rows of a prompt are scratch, those of more
     // than 16 sequences are buffers that the host may read after a step: there something has to overwrite them.
-    auto gone_after = [&](int buf, size_t at) {
-        if (buf == SWLM_BUF_RESIDUAL) return false;   // read by norms that do not name it
-        if (st[at].out_buf == buf) return true;
-        for (size_t j = at + 1; j < st.size(); ++j) {
-            const swlm_step& c = st[j];
-            if (c.in_buf == buf || c.in2_buf == buf || c.in3_buf == buf || (c.kind == SWLM_STEP_SSM_RECURRENCE && c.in4_buf == buf)) return false;
-            if (c.kind != SWLM_STEP_QK_NORM && c.kind != SWLM_STEP_ARGMAX && c.out_buf == buf) return true;
-        }
-        return plan->desc.max_batch <= kQGemvMaxRows;
+    auto gone_after = [&](int buf, size_t at, int n) {
+        return replaced_unread(at + 1, st.size(), n, plan->desc.max_batch <= kQGemvMaxRows, [&](size_t j) { return step_reads(st[j], buf, ctx->tp_size); },
+                               [&](size_t j) { return step_writes(st[j], buf, ctx->tp_size); });
     };
     for (size_t i = 0; i < st.size(); ++i) {
         swlm_plan::RowsGroup& grp = plan->rows_groups[i];
@@ -979,7 +1023,8 @@ int ensure_rows_groups(swlm_plan* plan) {
             auto jt = ctx->raw.find(st[i + 1].weight);
             // (an activation of fewer values than there are rows leaves the rest of its output alone)
             if (jt != ctx->raw.end() && jt->second.k == r0.k && jt->second.n == r0.n && jt->second.sb_f16 == r0.sb_f16 &&
-                st[i + 2].n / ctx->tp_size == r0.n && gone_after(st[i].out_buf, i + 2) && gone_after(st[i + 1].out_buf, i + 2)) {
+                st[i + 2].n / ctx->tp_size == r0.n && (st[i].out_buf == st[i + 2].out_buf || gone_after(st[i].out_buf, i + 2, r0.n)) &&
+                (st[i + 1].out_buf == st[i + 2].out_buf || gone_after(st[i + 1].out_buf, i + 2, r0.n))) {
                 names.push_back(st[i + 1].weight);
                 mode = 1;
                 grp.gated = true;

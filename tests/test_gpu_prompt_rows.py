@@ -234,3 +234,33 @@ def test_norms_of_the_widest_rows(pkg, oracle, width):
     model.decode(ids[-1:])
     assert np.abs(pkg.bf16_to_f32(model.logits()) - ref).max() <= 2e-2 * np.abs(ref).max()
     model.close(), store.close()
+
+
+def test_gate_values_that_are_partly_overwritten_and_read(pkg, oracle):
+    """Behind the activation something overwrites half of the gate's values and a product reads all of them: in a step of 20 sequences the
+    other half is what the gate's product left there."""
+    P, vocab, width, half, batch = pkg.plan, 256, 128, 64, 20
+    rng = np.random.default_rng(8)
+    store = pkg.WeightStore(0)
+    rows = {n: _bf(pkg, rng.normal(size=(vocab, w))) for n, w in (("x", width), ("narrow", half))}
+    for n, v in rows.items():
+        store.add_dense(n, v)
+    q4 = {n: pkg.synth_q4(width, width, seed=i, centered=True) for i, n in enumerate(("gate", "up"))}
+    q4["head"] = pkg.synth_q4(vocab, width, seed=5, centered=True)
+    for n, v in q4.items():
+        store.add_q4_mlx(n, *v)
+    steps = [P._step(P.STEP_EMBED, out_buf=P.BUF_S1, n=width, weight="x"), P._step(P.STEP_QGEMV, in_buf=P.BUF_S1, out_buf=P.BUF_S2, n=width, k=width, weight="gate"),
+             P._step(P.STEP_QGEMV, in_buf=P.BUF_S1, out_buf=P.BUF_S3, n=width, k=width, weight="up"),
+             P._step(P.STEP_SWIGLU, in_buf=P.BUF_S2, in2_buf=P.BUF_S3, out_buf=P.BUF_S0, n=width),
+             P._step(P.STEP_EMBED, out_buf=P.BUF_S2, n=half, weight="narrow"), P._step(P.STEP_EMBED, out_buf=P.BUF_S3, n=width, weight="x"),
+             P._step(P.STEP_QGEMV, in_buf=P.BUF_S2, out_buf=P.BUF_LOGITS, n=vocab, k=width, weight="head"),
+             P._step(P.STEP_EMBED, out_buf=P.BUF_S2, n=width, weight="x"), P._step(P.STEP_ARGMAX, in_buf=P.BUF_LOGITS, n=vocab)]
+    model = pkg.InferenceModel(store, steps, pkg.BuffersDesc(hidden=width, slot_dim=width, vocab=vocab, max_seq=64, max_batch=batch))
+    tokens = rng.integers(0, vocab, size=batch)
+    model.decode(tokens)
+    gate = oracle.qgemm(np.ascontiguousarray(rows["x"][tokens]), *q4["gate"])
+    ref = oracle.qgemm(np.concatenate([rows["narrow"][tokens], gate[:, half:]], axis=1), *q4["head"])
+    got, ref = pkg.bf16_to_f32(model.logits()).reshape(batch, vocab), pkg.bf16_to_f32(ref)
+    # gate values that round the other way (2^-8 of one) and one bf16 rounding on either side
+    assert np.abs(got - ref).max() <= 1.5e-2 * np.abs(ref).max()
+    model.close(), store.close()
