@@ -243,6 +243,19 @@ int step_writes(const swlm_step& s, int buf, int tp) {
     }
     return n;
 }
+// the same of a compiled launch
+int launch_reads(const Launch& L, int buf, int tp) {
+    if (L.kind != L_QGEMV) return step_reads(L.st, buf, tp);
+    if (L.norm.kind) return std::max(step_reads(L.norm, buf, tp), L.x_buf == buf ? L.norm.n : 0);
+    return L.st.in_buf == buf ? L.w->k : 0;
+}
+int launch_writes(const Launch& L, int buf, int tp) {
+    if (L.kind != L_QGEMV) return step_writes(L.st, buf, tp);
+    int n = L.norm.kind && buf == SWLM_BUF_RESIDUAL ? step_writes(L.norm, buf, tp) : 0;   // (the norm's own result stays inside)
+    for (int q = 0; q < L.n_seg; ++q)
+        if (L.seg_buf[q] == buf) n = std::max(n, L.seg_end[q] - (q ? L.seg_end[q - 1] : 0));
+    return n;
+}
 // Are the first n values of a buffer written anew by what runs at `first` and behind it, before any of them is read? `otherwise`: the
 // answer when nothing reads them and nothing writes them all.
 template <typename Reads, typename Writes>
@@ -468,17 +481,14 @@ int compile_plan(swlm_plan* plan) {
         Launch& A = plan->launches[i];
         Launch& B = plan->launches[i + 1];
         if (A.kind != L_QK_NORM || B.kind != L_ATTN || swlm_kv_bits(d.kv_scheme) || (B.st.head_dim != 64 && B.st.head_dim != 128)) continue;
-        if (A.st.in_buf != B.st.in_buf || A.st.in2_buf != B.st.in2_buf || A.st.in_buf == A.st.in2_buf || A.st.heads != B.st.heads || A.st.head_dim != B.st.head_dim) continue;
+        if (A.st.in_buf != B.st.in_buf || A.st.in2_buf != B.st.in2_buf || A.st.in_buf == A.st.in2_buf || A.st.heads != B.st.heads ||
+            A.st.kv_heads != B.st.kv_heads || A.st.head_dim != B.st.head_dim) continue;
         bool ok = B.st.in3_buf != A.st.in_buf && B.st.in3_buf != A.st.in2_buf;
         for (int buf : {A.st.in_buf, A.st.in2_buf}) {
-            bool written = B.st.out_buf == buf;
-            for (size_t j = i + 2; j < plan->launches.size() && ok && !written; ++j) {
-                const Launch& C = plan->launches[j];
-                if ((C.norm.kind ? C.x_buf : C.st.in_buf) == buf || C.st.in2_buf == buf || C.st.in3_buf == buf || (C.kind == L_SSM && C.st.in4_buf == buf)) ok = false;
-                written = C.kind != L_QGEMV && C.kind != L_QK_NORM && C.kind != L_ARGMAX && C.st.out_buf == buf;
-                for (int q = 0; q < C.n_seg && C.kind == L_QGEMV; ++q) written |= C.seg_buf[q] == buf;
-            }
-            ok &= written;
+            const int n = (buf == A.st.in_buf ? A.st.heads : A.st.kv_heads) * A.st.head_dim / ctx->tp_size;
+            ok = ok && (launch_writes(B, buf, ctx->tp_size) >= n ||
+                        replaced_unread(i + 2, plan->launches.size(), n, false, [&](size_t j) { return launch_reads(plan->launches[j], buf, ctx->tp_size); },
+                                        [&](size_t j) { return launch_writes(plan->launches[j], buf, ctx->tp_size); }));
         }
         if (!ok) continue;
         B.qk = A.st; B.d1 = A.d1; B.d2 = A.d2;

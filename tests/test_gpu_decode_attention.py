@@ -47,6 +47,37 @@ def test_norm_in_the_attention_launch_is_the_norm_of_its_own(pkg, heads, kv_head
     apart.close(), inside.close(), store.close()
 
 
+def test_normed_queries_that_are_partly_overwritten_and_read(pkg):
+    """Behind the attention something overwrites the first head of q and a product reads all of it: the second head is the normed one, as in
+    the row executor (more than 16 sequences), where the norm is a launch of its own."""
+    P, vocab, hd, heads = pkg.plan, 256, 64, 2
+    width, rng = heads * hd, np.random.default_rng(3)
+    store = pkg.WeightStore(0)
+    for name, n in (("q", width), ("k", width), ("v", width), ("one", hd)):
+        store.add_dense(name, _bf(pkg, rng.normal(size=(vocab, n))))
+    store.add_dense("qn", _bf(pkg, 3 + 0.2 * rng.normal(size=hd)))
+    store.add_dense("kn", _bf(pkg, 1 + 0.2 * rng.normal(size=hd)))
+    store.add_q4_mlx("head", *pkg.synth_q4(vocab, width, seed=5, centered=True))
+    steps = [P._step(P.STEP_EMBED, out_buf=b, n=width, weight=w) for b, w in ((P.BUF_S1, "q"), (P.BUF_S2, "k"), (P.BUF_S3, "v"))]
+    steps += [P._step(P.STEP_QK_NORM, in_buf=P.BUF_S1, in2_buf=P.BUF_S2, heads=heads, kv_heads=heads, head_dim=hd, eps=1e-5, weight="qn", weight2="kn"),
+              P._step(P.STEP_ATTN_DECODE, layer=0, in_buf=P.BUF_S1, in2_buf=P.BUF_S2, in3_buf=P.BUF_S3, out_buf=P.BUF_S0, heads=heads, kv_heads=heads,
+                      head_dim=hd, scale=hd ** -0.5),
+              P._step(P.STEP_EMBED, out_buf=P.BUF_S1, n=hd, weight="one"), P._step(P.STEP_EMBED, out_buf=P.BUF_S2, n=width, weight="k"),
+              P._step(P.STEP_QGEMV, in_buf=P.BUF_S1, out_buf=P.BUF_LOGITS, n=vocab, k=width, weight="head"),
+              P._step(P.STEP_EMBED, out_buf=P.BUF_S1, n=width, weight="q"), P._step(P.STEP_ARGMAX, in_buf=P.BUF_LOGITS, n=vocab)]
+    tokens = rng.integers(0, vocab, size=20)
+    got = []
+    for batch in (1, 3, 20):
+        model = pkg.InferenceModel(store, steps, pkg.BuffersDesc(hidden=width, slot_dim=width, vocab=vocab, max_seq=64, max_batch=batch, kv_layers=1,
+                                                                 kv_heads=heads, head_dim=hd))
+        model.decode(tokens[:batch])
+        got.append(pkg.bf16_to_f32(model.logits()).reshape(batch, vocab))
+        model.close()
+    for g in got[:2]:   # one bf16 rounding (2^-9 of the largest) on either side, sums in another order
+        assert np.abs(g - got[2][:len(g)]).max() <= 1e-2 * np.abs(got[2]).max()
+    store.close()
+
+
 @pytest.mark.parametrize("batch,kv_heads,hd,max_seq", [
     (19, 8, 64, 320), (37, 4, 128, 320), (38, 4, 64, 320), (64, 8, 128, 320),   # short caches: one or two splits
     (19, 8, 64, 1536), (25, 8, 64, 2000),                                       # 152 and 200 pairs in long caches: three splits
