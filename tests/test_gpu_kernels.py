@@ -99,8 +99,8 @@ def test_qgemm_group128_matches_oracle(pkg, store, oracle, n, k, m):
 
 
 @pytest.mark.parametrize("m", [17, 40, 63])
-def test_qgemm_17_to_63_rows_ride_in_one_tensor_core_tile(pkg, store, oracle, m):
-    """Between 17 and 63 token rows the product runs once over the weights, in a 64-token tensor-core tile whose
+def test_qgemm_17_to_63_rows_run_once_over_the_weights(pkg, store, oracle, m):
+    """Between 17 and 63 token rows the product runs once over the weights, in a tensor-core tile of 32 or 64 rows whose
     remaining rows are zero (the reference's gemm_q4_g64 re-reads the weights for every row,
     Generator/MetalSourceGenerator+Quantized.swift:88-156)."""
     n, k = 512, 1024

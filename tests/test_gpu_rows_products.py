@@ -52,8 +52,8 @@ def test_rows_of_very_different_size(pkg, oracle):
 @pytest.mark.parametrize("n,k", [(128, 64), (200, 192), (1000, 320), (4096, 4096), (264, 14336), (72, 16448)])
 @pytest.mark.parametrize("m", [17, 32, 33, 64, 65, 129, 300])
 def test_products_on_the_tensor_cores(pkg, oracle, n, k, m):
-    """Tiles of 32, 64, 128 and 256 rows with remainders; half steps of K and of the appended group sums; K over 1, 2, 4 and 8 CTAs;
-    rows longer than what the conversion keeps in registers."""
+    """Tiles of 32, 64 and 128 rows with remainders; half steps of K and of the appended group sums; K over one, two and four CTAs; rows longer
+    than what the conversion keeps in registers. (Pairs of SMs and two CTAs per SM: test_forms_of_the_tensor_core_products.)"""
     if n * k * m > 2 ** 31:
         m = min(m, 65)
     store = pkg.WeightStore(0)
@@ -68,7 +68,7 @@ def test_products_on_the_tensor_cores(pkg, oracle, n, k, m):
 
 
 def test_more_tiles_than_multiprocessors(pkg, oracle):
-    """The long form walks several tiles per CTA; its results are compared at rows of the first, a middle and the last tile."""
+    """Five tiles of 128 rows in 112 rows of tiles: nearly four rounds of the GPU. Results are compared at rows of the first, middle and last tiles."""
     n, k, m = 14336, 512, 600
     store = pkg.WeightStore(0)
     w, s, b = pkg.synth_q4(n, k, seed=9, centered=True)
