@@ -2499,8 +2499,7 @@ int swlm_op_qgemm_dev(swlm_ctx* ctx, const char* weight, int m, const void* x_de
         return launch_qgemm_tc(*w, m, static_cast<const __nv_bfloat16*>(x_dev), w->k, out, QGEMV_EPI_STORE, GATED_ACT_SILU, ctx->op_xh, ctx->tc_status, stream);
     }
     if (m <= 0) return SWLM_OK;
-    rc = op_scratch(ctx, *w, m);
-    if (rc) return rc;
+    if (!qgemv_rows_takes(*w, m) && (rc = op_scratch(ctx, *w, m))) return rc;   // (the kernel of few rows needs neither parts nor counters)
     QGemvLaunch a;
     a.w = w; a.m = m;
     a.x = static_cast<const __nv_bfloat16*>(x_dev); a.x_stride = w->k;
