@@ -55,17 +55,8 @@ __device__ __forceinline__ bool mbar_wait_cluster_warp(unsigned long long* bar, 
 
 // Shared-memory matrix descriptor: K-major operand, 128-byte swizzle, rows of 128 bytes, 8-row groups 1024
 // bytes apart (stride byte offset); leading byte offset unused for this layout; descriptor version 1.
-__device__ __forceinline__ unsigned long long umma_desc(unsigned smem_addr) {
-    unsigned long long d = 0;
-    d |= (unsigned long long)((smem_addr & 0x3FFFFu) >> 4);
-    d |= (unsigned long long)(1024u >> 4) << 32;
-    d |= 1ull << 46;
-    d |= 2ull << 61;
-    return d;
-}
-
-// The same descriptor as its low word (the rest is constant for this layout): places 32 bytes apart along K differ by 2, a tile
-// `bytes` further on by bytes / 16. Built where it is used, so that a loop over the MMAs of a step adds 32-bit numbers only.
+// Its low word holds the address, the high one is constant: places 32 bytes apart along K differ by 2, a tile `bytes` further on by
+// bytes / 16. Put together where it is used, so that a loop over the MMAs of a step adds 32-bit numbers only.
 __device__ __forceinline__ unsigned umma_desc_lo(unsigned smem_addr) { return (smem_addr & 0x3FFFFu) >> 4; }
 constexpr unsigned kUmmaDescHi = (1024u >> 4) | 1u << 14 | 2u << 29;
 
