@@ -375,31 +375,71 @@ __device__ __forceinline__ bool tc_dequant(const QGemmTcParams& p, TcBars<STAGES
     return ok;
 }
 
-// Results of one lane's 16 columns from c0 on: `row0 + lane` is its weight row.
-__device__ __forceinline__ void tc_store16(const QGemmTcParams& p, const unsigned (&v)[16], int row0, int token0) {
+// Where a lane's results go: its weight row of one output, or the row of a gate row and its up row together.
+struct TcDst { __nv_bfloat16* y; int stride; bool live; };
+__device__ __forceinline__ TcDst tc_dst(const QGemmTcParams& p, int row0) {
     const int lane = threadIdx.x & 31, row = row0 + lane;
-    if (!p.gated) {
-        if (row >= p.out.end[2]) return;
-        const int q = row < p.out.end[0] ? 0 : row < p.out.end[1] ? 1 : 2;
-        const int stride = q == 0 ? p.out.stride[0] : q == 1 ? p.out.stride[1] : p.out.stride[2];
-        __nv_bfloat16* dst = (q == 0 ? p.out.y[0] : q == 1 ? p.out.y[1] : p.out.y[2]) + (row - (q == 0 ? 0 : q == 1 ? p.out.end[0] : p.out.end[1])) + (size_t)token0 * stride;
+    if (p.gated) { const int r = (row >> 4) * 8 + (row & 7); return {p.out.y[0] + r, p.out.stride[0], r < p.out.end[0]}; }
+    const int q = row < p.out.end[0] ? 0 : row < p.out.end[1] ? 1 : 2;
+    return {(q == 0 ? p.out.y[0] : q == 1 ? p.out.y[1] : p.out.y[2]) + (row - (q == 0 ? 0 : q == 1 ? p.out.end[0] : p.out.end[1])),
+            q == 0 ? p.out.stride[0] : q == 1 ? p.out.stride[1] : p.out.stride[2], row < p.out.end[2]};
+}
+// silu(gate) * up; 1 / (1 + e) by the unit's reciprocal (one unit in the last place): a division's slow path is a branch, behind which
+// eight independent values would be worked out one after the other
+__device__ __forceinline__ float tc_swiglu(float gate, float up) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.0f + expf(-gate)));
+    return gate * r * up;
+}
+template <bool GELU>
+__device__ __forceinline__ void tc_emit_gated(const QGemmTcParams& p, const TcDst& d, const unsigned* v, float fac, int fac0, int token0) {
+    // gate rows sit in the lanes of the first eight of 16, up rows in the others: a gate lane finishes even columns, its up lane odd ones.
+    // Both are rounded to bf16 first because the reference stores them to bf16 scratch before `swiglu` reads them
+    // (Primitives/ElementwiseFragment.swift:49-54).
+    const int up_lane = (threadIdx.x >> 3) & 1;
+    __nv_bfloat16 res[8];
 #pragma unroll
-        for (int i = 0; i < 16; ++i)
-            if (token0 + i < p.m) dst[(size_t)i * stride] = __float2bfloat16_rn(__uint_as_float(v[i]) * tc_rscale(p, token0 + i));
+    for (int i = 0; i < 8; ++i) {
+        const unsigned own = up_lane ? v[2 * i + 1] : v[2 * i], other = __shfl_xor_sync(0xffffffffu, up_lane ? v[2 * i] : v[2 * i + 1], 8);
+        const float sc = __shfl_sync(0xffffffffu, fac, fac0 + 2 * i + up_lane);
+        const float gate = __bfloat162float(__float2bfloat16_rn(__uint_as_float(up_lane ? other : own) * sc));
+        const float up = __bfloat162float(__float2bfloat16_rn(__uint_as_float(up_lane ? own : other) * sc));
+        res[i] = __float2bfloat16_rn(GELU ? gated_activation(gate, up, GATED_ACT_GELU_TANH) : tc_swiglu(gate, up));
+    }
+    if (!d.live) return;
+    __nv_bfloat16* y = d.y + (size_t)(token0 + up_lane) * d.stride;
+    if (token0 + 16 <= p.m) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) y[(size_t)(2 * i) * d.stride] = res[i];
+    } else {
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+            if (token0 + 2 * i + up_lane < p.m) y[(size_t)(2 * i) * d.stride] = res[i];
+    }
+}
+// 16 columns of a warp's 32 rows, tokens token0 on; lane fac0 + i holds the factor of token0 + i. What bounds a tile's end is the chain
+// behind its accumulators, which the next tile's MMAs wait for: a load of the factor, a test, an activation and a store for each column
+// in turn took as long as 18 steps of 128 columns (gate and up of 16384 x 2048 over 2010 rows: 257 us, 37 per tile). Without a branch
+// between the columns and with the factors in registers beforehand they overlap. Prompt of 2011 tokens, 16 layers of width 2048:
+// 8298 -> 6335 us; 4096 tokens, 4 layers of width 4096: 10410 -> 9092 us; 14336 x 4096 at 512 rows 64.4 -> 60.6 us.
+__device__ __forceinline__ void tc_emit16(const QGemmTcParams& p, const TcDst& d, const unsigned* v, float fac, int fac0, int token0) {
+    if (p.gated) {
+        if (p.gated_act == GATED_ACT_GELU_TANH) tc_emit_gated<true>(p, d, v, fac, fac0, token0);
+        else tc_emit_gated<false>(p, d, v, fac, fac0, token0);
         return;
     }
-    // gate rows sit in the lanes of the first eight of 16, up rows in the others: a gate lane finishes even columns, its up lane odd ones
-    const bool up_lane = lane & 8;
-    const int out_row = (row >> 4) * 8 + (row & 7);
+    __nv_bfloat16 res[16];
 #pragma unroll
-    for (int i = 0; i < 16; i += 2) {
-        const float other = __uint_as_float(__shfl_xor_sync(0xffffffffu, up_lane ? v[i] : v[i + 1], 8));
-        const int token = token0 + i + (up_lane ? 1 : 0);
-        if (token < p.m) {
-            const float sc = tc_rscale(p, token);
-            if (up_lane) tc_store_gated(p, token, out_row, other * sc, __uint_as_float(v[i + 1]) * sc);
-            else tc_store_gated(p, token, out_row, __uint_as_float(v[i]) * sc, other * sc);
-        }
+    for (int i = 0; i < 16; ++i) res[i] = __float2bfloat16_rn(__uint_as_float(v[i]) * __shfl_sync(0xffffffffu, fac, fac0 + i));
+    if (!d.live) return;
+    __nv_bfloat16* y = d.y + (size_t)token0 * d.stride;
+    if (token0 + 16 <= p.m) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) y[(size_t)i * d.stride] = res[i];
+    } else {
+#pragma unroll
+        for (int i = 0; i < 16; ++i)
+            if (token0 + i < p.m) y[(size_t)i * d.stride] = res[i];
     }
 }
 
@@ -490,19 +530,28 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__((kTcDeqWarps + 2 + k
         unsigned par = 0;
         pdl_wait();   // (the rows' factors)
         for (int tile = first; tile < p.n_tiles; tile += pairs, par ^= 1u) {
+            const int tok0 = tile % p.tok_tiles * 256 + half * 128;
+            const TcDst dst = tc_dst(p, tile / p.tok_tiles * 256 + rank * kTcRows + (warp & 3) * 32);
+            float fac = tc_rscale(p, min(tok0 + lane, p.m - 1));   // of 32 tokens, one per lane, requested before they are needed
             if (!mbar_wait_warp(&bars.acc_full, par)) { tc_fail(p.status, &bars.failed, 4); break; }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const int row0 = tile / p.tok_tiles * 256 + rank * kTcRows + (warp & 3) * 32, tok0 = tile % p.tok_tiles * 256;
+            float next = 0.f;
 #pragma unroll 1
-            for (int c0 = half * 128; c0 < (half + 1) * 128; c0 += 16) {
-                if (tok0 + c0 >= p.m) break;  // uniform across the warp
+            for (int c = 0; c < 128; c += 16) {
+                const int token = tok0 + c;
                 unsigned v[16];
-                tmem_ld16(tmem_d + ((unsigned)((warp & 3) * 32) << 16) + (unsigned)c0, v);
-                tc_store16(p, v, row0, tok0 + c0);
+                if (!(c & 16)) next = tc_rscale(p, min(token + 32 + lane, p.m - 1));
+                if (token < p.m) tmem_ld16(tmem_d + ((unsigned)((warp & 3) * 32) << 16) + (unsigned)(half * 128 + c), v);
+                const bool last = c == 112 || token + 16 >= p.m;   // uniform across the warp
+                if (last) {   // the accumulators have been read
+                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                    __syncwarp();
+                    if (lane == 0) tc_arrive_tmem(acc_empty);
+                }
+                if (token < p.m) tc_emit16(p, dst, v, fac, c & 16, token);
+                if (last) break;
+                if (c & 16) fac = next;
             }
-            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-            __syncwarp();
-            if (lane == 0) tc_arrive_tmem(acc_empty);
         }
         __syncwarp();
     }
@@ -585,7 +634,7 @@ __global__ void __launch_bounds__((kTcDeqWarps + 2) * 32, PER_SM) qgemm_tc_short
             unsigned v[CW];
             tmem_ld16(tmem_d + ((unsigned)((warp & 3) * 32) << 16) + (unsigned)c0, v);
             if (p.splits == 1) {
-                tc_store16(p, v, row0 + (warp & 3) * 32, tok0 + c0);
+                tc_emit16(p, tc_dst(p, row0 + (warp & 3) * 32), v, tc_rscale(p, min(tok0 + c0 + (lane & 15), p.m - 1)), 0, tok0 + c0);
                 continue;
             }
 #pragma unroll
