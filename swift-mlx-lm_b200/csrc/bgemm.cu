@@ -4,16 +4,20 @@
 //                    rows per warp and K cut across the warps of a CTA; the norm in front of the product can run in the
 //                    prologue, gate and up in one launch with the gated activation in the epilogue. Activations bf16 or fp32
 //                    (with fp32 ones the product is a true fp32 product: a bf16 weight is exact in fp32).
-//   bgemm_tc_kernel  more rows, bf16 activations: tcgen05.mma with both operands staged by TMA (128-byte swizzle), two tiles
-//                    of 128 weight rows side by side in tensor memory, K cut across CTAs when there are few tiles. The two
-//                    tiles are 256 consecutive rows, or 128 rows of gate and the same rows of up. Grouped form: activation rows
-//                    sorted by expert, a device table names the expert and the rows of every tile.
+//   bgemm_tc_kernel  more rows, bf16 activations: tcgen05.mma with both operands staged by TMA (128-byte swizzle), one SM or a pair of
+//                    them per tile, gate and up side by side in tensor memory, K cut over the CTAs of a cluster when there are few
+//                    tiles. Grouped form: activation rows sorted by expert, a device table names the expert and the rows of every
+//                    tile.
 //   sgemm_kernel     more rows, fp32 activations: fp32 FMAs on 64 x 64 tiles.
 #include <algorithm>
 #include <cstdlib>
 
+#include <cooperative_groups.h>
+
 #include "swlm_internal.h"
 #include "tc_device.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace swlm {
 namespace {
@@ -318,8 +322,14 @@ __global__ void __launch_bounds__(kGemvThreads, 2) bgemv_kernel(const GemvParams
     }
 }
 
-// ---- many rows, bf16: tcgen05 -----------------------------------------------------------------------------------------
-constexpr int kTileRows = 128;       // weight rows of one accumulator = UMMA M
+// ---- many rows, bf16: tcgen05, K over the CTAs of a cluster ---------------------------------------------------------------
+// CTA groups of CG = 1 or 2 take a tile of 128 CG weight rows x BN activation rows over one K range; `ranges` groups side by side in a
+// cluster take the K ranges and meet through distributed shared memory (the ring's, which is free by then): each sums the ranges of
+// BN / ranges activation rows, in order, and stores them.
+// What bounds it: what an SM takes in from L2 (about 38 bytes per clock with all of them reading). A pair of SMs holds 256 x BN results
+// with half of the activations in either's shared memory: 512 rows through 2048 x 16384 (gate and up) move 201 MB instead of the 268 MB
+// of one SM per tile.
+constexpr int kTileRows = 128;       // weight rows of a CTA = its lanes of tensor memory
 constexpr int kTcK = 64;             // columns per stage = one 128-byte swizzle row
 constexpr int kTcEpilogueWarps = 8;
 constexpr int kTcWarps = 2 + kTcEpilogueWarps;   // TMA, MMA, epilogue
@@ -327,27 +337,48 @@ constexpr int kTcBlock = kTcWarps * 32;
 
 struct TcParams {
     int n, m, steps;                 // weight rows, activation rows, 64-column steps of K
+    int ranges;                      // K ranges = CTA groups of a cluster
     int split;                       // weight rows from here on (a multiple of 256) meet the activations of wmap2's place
-    int split_steps;                 // steps per K range (gridDim.z ranges); == steps when K is not cut
     GatedAct act;
-    const int4* tiles;               // grouped form: (expert, first row, rows, 0) of tile blockIdx.x; n = rows of one expert's matrix
+    const int4* tiles;               // grouped form: (expert, first row, rows, 0) of tile blockIdx.y; n = rows of one expert's matrix
     ProductOut out;
-    float* part;                     // [range][gated ? 2 : 1][m][n] when K is cut
     int* status;
 };
 
-// kind::f16: D fp32, A = B = bf16, both K-major, M = 128
-__host__ __device__ constexpr unsigned tc_idesc(int bn) {
-    return (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(bn >> 3) << 17) | ((unsigned)(kTileRows >> 4) << 24);
+__device__ __forceinline__ unsigned cluster_place(unsigned addr, int rank) {   // the same shared-memory place in another CTA of the cluster
+    unsigned r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void st_cluster_v4(unsigned addr, unsigned a, unsigned b, unsigned c, unsigned d) {
+    asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
+
+// kind::f16: D fp32, A = B = bf16, both K-major
+__host__ __device__ constexpr unsigned tc_idesc(int m, int bn) {
+    return (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(bn >> 3) << 17) | ((unsigned)(m >> 4) << 24);
 }
 // (descriptors by their low words)
+template <int CG>
 __device__ __forceinline__ void umma_bf16(unsigned d_tmem, unsigned a_lo, unsigned b_lo, unsigned idesc, unsigned accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t.reg .b64 a, b;\n\t"
-        "setp.ne.b32 p, %5, 0;\n\t"
-        "mov.b64 a, {%1, %3};\n\tmov.b64 b, {%2, %3};\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %4, p;\n\t}"
-        ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(kUmmaDescHi), "r"(idesc), "r"(accumulate) : "memory");
+    if (CG == 1)
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t.reg .b64 a, b;\n\t"
+            "setp.ne.b32 p, %5, 0;\n\t"
+            "mov.b64 a, {%1, %3};\n\tmov.b64 b, {%2, %3};\n\t"
+            "tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %4, p;\n\t}"
+            ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(kUmmaDescHi), "r"(idesc), "r"(accumulate) : "memory");
+    else
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t.reg .b64 a, b;\n\t"
+            "setp.ne.b32 p, %5, 0;\n\t"
+            "mov.b64 a, {%1, %3};\n\tmov.b64 b, {%2, %3};\n\t"
+            "tcgen05.mma.cta_group::2.kind::f16 [%0], a, b, %4, p;\n\t}"
+            ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(kUmmaDescHi), "r"(idesc), "r"(accumulate) : "memory");
+}
+// arrival at the same barrier of both CTAs of the pair when the MMAs issued so far are done; `pair`: the bits of their cluster ranks
+__device__ __forceinline__ void umma_commit_to(unsigned long long* bar, unsigned short pair) {
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_u32(bar)), "h"(pair) : "memory");
 }
 
 __device__ __forceinline__ void tmem_ld16(unsigned (&v)[16], unsigned at) {
@@ -358,169 +389,252 @@ __device__ __forceinline__ void tmem_ld16(unsigned (&v)[16], unsigned at) {
         : "r"(at) : "memory");
 }
 
-template <int BN, int STAGES, bool GATED>
+// `count` (at most 16) results of one weight row, activation rows `token` on. No branch between the values of a batch: their
+// exponentials and stores overlap.
+__device__ __forceinline__ void tc_emit(const TcParams& p, const ProductRow& dst, float (&val)[16], int token, int count) {
+    if (p.out.biased) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) val[i] += dst.bias;
+    }
+    if (p.out.softcap > 0.f) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) val[i] = p.out.softcap * tanhf(val[i] / p.out.softcap);
+    }
+    if (p.out.gelu) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) val[i] = gelu_erf(val[i]);
+    }
+    unsigned char* y = dst.y + (size_t)token * dst.stride;
+    if (dst.f32) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i)
+            if (i < count) *reinterpret_cast<float*>(y + i * dst.stride) = val[i];
+    } else {
+#pragma unroll
+        for (int i = 0; i < 16; ++i)
+            if (i < count) *reinterpret_cast<__nv_bfloat16*>(y + i * dst.stride) = __float2bfloat16_rn(val[i]);
+    }
+}
+// gated_activation without a branch between values: tanh-GELU as g / (1 + e^-2u), the same function; 1 / x by the unit's reciprocal
+// (one unit in the last place)
+__device__ __forceinline__ float tc_gated(float g, float up, const GatedAct& act) {
+    const bool clamped = act.kind == GATED_ACT_CLAMPED;
+    if (clamped) { g = fminf(g, act.limit); up = fminf(fmaxf(up, -act.limit), act.limit) + 1.0f; }
+    const float u = act.kind == GATED_ACT_GELU_TANH ? 1.5957691216f * (g + 0.044715f * g * g * g) : clamped ? act.alpha * g : g;
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.0f + expf(-u)));
+    return g * r * up;
+}
+
+template <int CG, int BN, int STAGES, bool GATED>
 __global__ void __launch_bounds__(kTcBlock) bgemm_tc_kernel(const TcParams p, const __grid_constant__ CUtensorMap xmap,
-                                                           const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUtensorMap wmap2) {
+                                                            const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUtensorMap wmap2) {
     extern __shared__ __align__(1024) unsigned char tc_raw[];
     unsigned char* smem = tc_raw + ((1024 - (smem_u32(tc_raw) & 1023)) & 1023);   // swizzle atoms
-    constexpr int A_BYTES = kTileRows * 128, B_BYTES = BN * 128;
-    constexpr unsigned kCols = 2 * BN < 32 ? 32 : 2 * BN;
+    constexpr int NACC = GATED ? 2 : 1;
+    constexpr int A_BYTES = kTileRows * 128, B_BYTES = BN / CG * 128, STAGE = NACC * A_BYTES + B_BYTES;
+    constexpr unsigned kCols = NACC * BN;
+    static_assert(kCols >= 32 && kCols <= 512, "tensor memory");
+    static_assert((GATED && BN == 256) || STAGES * STAGE >= NACC * (BN + 4 * 8 / CG) * kTileRows * 4, "the ring takes what the cluster sends");
     __shared__ __align__(8) unsigned long long full_bar[STAGES], empty_bar[STAGES], done_bar;
     __shared__ unsigned tmem_base;
-    __shared__ int failed;
+    __shared__ int failed_word;
+    volatile int* const failed = &failed_word;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    int tok0 = blockIdx.x * BN, tok_end = p.m, wrow0 = 0;     // wrow0: first row of the expert's matrix
+    const int crank = (int)blockIdx.x, rank = crank % CG, range = crank / CG;   // place in the cluster, in the group; K range
+    int tok0 = blockIdx.y * BN, tok_end = p.m, wrow0 = 0;      // wrow0: first row of the expert's matrix
     if (p.tiles) {
         pdl_wait();   // (the table is the preceding kernel's)
-        const int4 tile = p.tiles[blockIdx.x];
-        if (tile.z == 0) { pdl_launch_dependents(); return; }
+        const int4 tile = p.tiles[blockIdx.y];
+        if (tile.z == 0) { pdl_launch_dependents(); return; }   // (the same for all CTAs of a cluster)
         wrow0 = tile.x * p.n;
         tok0 = tile.y;
         tok_end = tile.y + tile.z;
     }
-    const int row0 = blockIdx.y * (GATED ? kTileRows : 2 * kTileRows);
-    const int nt = !GATED && row0 + kTileRows >= p.n ? 1 : 2;                       // accumulators in use
-    const int stage_bytes = nt * A_BYTES + B_BYTES;
-    constexpr int STAGE = 2 * A_BYTES + B_BYTES;
-    const int step0 = blockIdx.z * p.split_steps;
-    const int steps = min(p.split_steps, p.steps - step0);
+    const int row0 = (int)blockIdx.z * (kTileRows * CG) + rank * kTileRows;
+    const int step0 = p.steps * range / p.ranges, steps = p.steps * (range + 1) / p.ranges - step0;
     if (tid == 0) {
         for (int s = 0; s < STAGES; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
         mbar_init(&done_bar, 1);
-        failed = 0;
+        failed_word = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) {
         __syncwarp();
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base)), "r"(kCols) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        if (CG == 1) {
+            asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base)), "r"(kCols) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        } else {
+            asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base)), "r"(kCols) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+        }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
+    const cg::cluster_group cluster = cg::this_cluster();
+    if (CG == 2) cluster.sync();   // both CTAs' barriers are ready
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const unsigned tmem = tmem_base;
     pdl_launch_dependents();   // behind the allocation: a successor that wants tensor memory cannot get in between
 
     if (warp == 0) {
-        if (lane == 0) {
-            // the weights of the first stages do not depend on the preceding kernel; the activations do
-            const int ahead = min(STAGES, steps);
-            auto weights = [&](int kt, int s) {
-                const unsigned bar = smem_u32(&full_bar[s]), dst = smem_u32(smem + s * STAGE);
-                mbar_expect(bar, (unsigned)stage_bytes);
-                tma_load_2d(dst, &wmap, (step0 + kt) * kTcK, wrow0 + row0, bar);
-                if (nt == 2) tma_load_2d(dst + A_BYTES, GATED ? &wmap2 : &wmap, (step0 + kt) * kTcK, wrow0 + (GATED ? row0 : row0 + kTileRows), bar);
-            };
-            auto activations = [&](int kt, int s) {
-                tma_load_2d(smem_u32(smem + s * STAGE) + 2 * A_BYTES, !GATED && row0 >= p.split ? &wmap2 : &xmap, (step0 + kt) * kTcK, tok0, smem_u32(&full_bar[s]));
-            };
-            for (int kt = 0; kt < ahead; ++kt) weights(kt, kt);
-            pdl_wait();
-            for (int kt = 0; kt < ahead; ++kt) activations(kt, kt);
-            int issued = ahead;
-            for (int kt = ahead; kt < steps; ++kt) {
-                const int s = kt % STAGES;
-                if (!mbar_wait(&empty_bar[s], (unsigned)((kt / STAGES - 1) & 1))) { atomicExch(p.status, 31); failed = 1; break; }
-                weights(kt, s);
-                activations(kt, s);
-                issued = kt + 1;
-            }
-            if (failed)   // copies already requested still write shared memory
-                for (int kt = issued > STAGES ? issued - STAGES : 0; kt < issued; ++kt) mbar_wait(&full_bar[kt % STAGES], (unsigned)((kt / STAGES) & 1));
-        }
-        __syncwarp();
-    } else if (warp == 1) {
-        // the warp runs its loop as a whole, one lane issues (a lone lane's loop took longer over its eight MMAs than a step of 128
-        // activation rows takes to multiply)
-        constexpr unsigned idesc = tc_idesc(BN);
+        // The warp runs its loop as a whole, one lane issues. The weights of the first stages do not depend on the preceding kernel; the
+        // activations do. Of a pair both CTAs' copies count on the barrier of the CTA that issues the MMAs; the other's may get there
+        // before the bytes are announced: the phase ends with the announcement at the earliest.
         const bool el = elect_one();
-        int s = 0;
+        const CUtensorMap* const x = !GATED && row0 - rank * kTileRows >= p.split ? &wmap2 : &xmap;
+        const unsigned full0 = CG == 1 ? smem_u32(&full_bar[0]) : cluster_place(smem_u32(&full_bar[0]), crank - rank), ring = smem_u32(smem);
+        auto load = [&](unsigned dst, const CUtensorMap* map, int col, int row, int s) {
+            if (CG == 1) tma_load_2d(dst, map, col, row, full0 + 8u * s);
+            else tma_load_2d_pair(dst, map, col, row, full0 + 8u * s);
+        };
+        auto weights = [&](int kt, int s) {
+            if (rank == 0) mbar_expect(full0 + 8u * s, (unsigned)(CG * STAGE));
+            load(ring + s * STAGE, &wmap, (step0 + kt) * kTcK, wrow0 + row0, s);
+            if (GATED) load(ring + s * STAGE + A_BYTES, &wmap2, (step0 + kt) * kTcK, wrow0 + row0, s);
+        };
+        auto activations = [&](int kt, int s) { load(ring + s * STAGE + NACC * A_BYTES, x, (step0 + kt) * kTcK, tok0 + rank * (BN / CG), s); };
+        const int ahead = min(STAGES, steps);
+        if (el)
+            for (int kt = 0; kt < ahead; ++kt) weights(kt, kt);
+        __syncwarp();
+        pdl_wait();
+        if (el)
+            for (int kt = 0; kt < ahead; ++kt) activations(kt, kt);
+        __syncwarp();
+        int s = 0, kt = ahead;
         unsigned par = 0;
-        for (int kt = 0; kt < steps; ++kt) {
-            if (!mbar_wait_warp(&full_bar[s], par)) { if (el) { atomicExch(p.status, 32); failed = 1; } break; }
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            if (el) {
-                const unsigned a = umma_desc_lo(smem_u32(smem + s * STAGE)), b = a + 2 * A_BYTES / 16;
-#pragma unroll
-                for (int j = 0; j < kTcK / 16; ++j) {
-                    const unsigned acc = j > 0 ? 1u : kt > 0 ? 1u : 0u;
-                    umma_bf16(tmem, a + 2 * j, b + 2 * j, idesc, acc);
-                    if (nt == 2) umma_bf16(tmem + BN, a + A_BYTES / 16 + 2 * j, b + 2 * j, idesc, acc);
-                }
-                umma_commit(&empty_bar[s]);
-            }
+        bool ok = true;
+        for (; kt < steps; ++kt) {
+            if (!mbar_wait_warp(&empty_bar[s], par)) { ok = false; break; }
+            if (el) { weights(kt, s); activations(kt, s); }
             __syncwarp();
             if (++s == STAGES) { s = 0; par ^= 1u; }
         }
-        if (el) umma_commit(&done_bar);   // also behind whatever was issued before a failure
+        if (!ok) {   // copies already requested still write shared memory (in a pair's second CTA, whose barrier this is not, the limit of the wait is the time they get)
+            if (el) { atomicExch(p.status, 31); *failed = 1; }
+            for (int i = kt > STAGES ? kt - STAGES : 0; i < kt; ++i) mbar_wait_warp(&full_bar[i % STAGES], (unsigned)((i / STAGES) & 1));
+        }
         __syncwarp();
-    } else {
-        // ---- epilogue: a warp reads the 32 accumulator lanes of its quarter (warp & 3), lane = weight row; the two warps of a
-        // quarter take turns with the activation rows ----
-        pdl_wait();   // the outputs may still be read by the kernel before this one
-        const bool ok = mbar_wait(&done_bar, 0u);
-        if (!ok) { atomicExch(p.status, 33); }
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        if (ok && !failed) {
-            const int quarter = warp & 3;
-            const bool cut = gridDim.z > 1;
-#pragma unroll 1
-            for (int t = 0; t < (GATED && !cut ? 1 : nt); ++t) {
-                const int row = row0 + (GATED ? 0 : t * kTileRows) + quarter * 32 + lane;
-                const ProductRow dst = cut ? ProductRow{reinterpret_cast<unsigned char*>(p.part + ((size_t)blockIdx.z * (GATED ? 2 : 1) + (GATED ? t : 0)) * p.m * p.n + row), (size_t)p.n * 4, true, 0.f}
-                                           : product_row<true>(p.out, row);
-#pragma unroll 1
-                for (int c0 = 16 * ((warp - 2) >> 2); c0 < BN; c0 += 16 * (kTcEpilogueWarps / 4)) {
-                    if (tok0 + c0 >= tok_end) break;   // uniform across the warp
-                    unsigned v[16], u[16];
-                    const unsigned at = tmem + ((unsigned)(quarter * 32) << 16) + (unsigned)(t * BN + c0);
-                    tmem_ld16(v, at);
-                    if (GATED && !cut) tmem_ld16(u, at + BN);
-                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                    if (row < p.n) {
-                        const int count = tok_end - tok0 - c0;
-                        unsigned char* y = dst.y + (size_t)(tok0 + c0) * dst.stride;
+    } else if (warp == 1) {
+        if (rank == 0) {
+            // the warp runs its loop as a whole, one lane issues (a lone lane's loop took longer over its eight MMAs than a step of 128
+            // activation rows takes to multiply)
+            constexpr unsigned idesc = tc_idesc(kTileRows * CG, BN);
+            const unsigned short pair = (unsigned short)(3u << crank);
+            const bool el = elect_one();
+            int s = 0;
+            unsigned par = 0;
+            for (int kt = 0; kt < steps; ++kt) {
+                const bool ok = CG == 1 ? mbar_wait_warp(&full_bar[s], par) : mbar_wait_cluster_warp(&full_bar[s], par);
+                if (!ok) { if (el) { atomicExch(p.status, 32); *failed = 1; } break; }
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                if (el) {
+                    const unsigned a = umma_desc_lo(smem_u32(smem + s * STAGE)), b = a + NACC * A_BYTES / 16;
 #pragma unroll
-                        for (int i = 0; i < 16; ++i) {
-                            float val = __uint_as_float(v[i]);
-                            if (GATED && !cut) val = gated_activation(val, __uint_as_float(u[i]), p.act);
-                            val += dst.bias;
-                            if (p.out.softcap > 0.f && !cut) val = p.out.softcap * tanhf(val / p.out.softcap);
-                            if (p.out.gelu && !cut) val = gelu_erf(val);
-                            if (i < count) {
-                                if (dst.f32) *reinterpret_cast<float*>(y) = val;
-                                else *reinterpret_cast<__nv_bfloat16*>(y) = __float2bfloat16_rn(val);
-                            }
-                            y += dst.stride;
-                        }
+                    for (int j = 0; j < kTcK / 16; ++j) {
+                        const unsigned acc = j > 0 ? 1u : kt > 0 ? 1u : 0u;
+                        umma_bf16<CG>(tmem, a + 2 * j, b + 2 * j, idesc, acc);
+                        if (GATED) umma_bf16<CG>(tmem + BN, a + A_BYTES / 16 + 2 * j, b + 2 * j, idesc, acc);
+                    }
+                    if (CG == 1) umma_commit(&empty_bar[s]);
+                    else umma_commit_to(&empty_bar[s], pair);
+                }
+                __syncwarp();
+                if (++s == STAGES) { s = 0; par ^= 1u; }
+            }
+            if (el) {   // also behind whatever was issued before a failure
+                if (CG == 1) umma_commit(&done_bar);
+                else umma_commit_to(&done_bar, pair);
+            }
+        }
+        __syncwarp();
+    }
+    // ---- results: a warp reads the 32 accumulator lanes of its quarter (warp & 3), lane = weight row; the two warps of a quarter
+    // take turns with the activation rows ----
+    const int epi = warp - 2, quarter = warp & 3, row = row0 + quarter * 32 + lane;
+    const unsigned lanes = tmem + ((unsigned)(quarter * 32) << 16);
+    bool ok = true;
+    if (epi >= 0) {
+        pdl_wait();   // the outputs may still be read by the kernel before this one
+        ok = mbar_wait_warp(&done_bar, 0u);
+        if (!ok && lane == 0) { atomicExch(p.status, 33); *failed = 1; }
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    }
+    if (p.ranges == 1) {
+        if (epi >= 0 && ok && !*failed) {
+            const ProductRow dst = product_row<true>(p.out, row);
+#pragma unroll 1
+            for (int c0 = 16 * (epi >> 2); c0 < BN; c0 += 16 * (kTcEpilogueWarps / 4)) {
+                const int token = tok0 + c0;
+                if (token >= tok_end) break;   // uniform across the warp
+                unsigned v[16], u[16];
+                tmem_ld16(v, lanes + (unsigned)c0);
+                if (GATED) tmem_ld16(u, lanes + (unsigned)(BN + c0));
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                float val[16];
+#pragma unroll
+                for (int i = 0; i < 16; ++i) val[i] = GATED ? tc_gated(__uint_as_float(v[i]), __uint_as_float(u[i]), p.act) : __uint_as_float(v[i]);
+                if (row < p.n) tc_emit(p, dst, val, token, min(16, tok_end - token));
+                __syncwarp();
+            }
+        }
+    } else {
+        // part (accumulator a, range z, column c of the receiver's) at [((a ranges + z) 128 + weight row) pitch + c], four columns at a time
+        const int own = BN / p.ranges, pitch = own + 4;   // (a multiple of four; eight lanes' pieces meet no bank twice)
+        cluster.sync();   // every ring of the cluster is free
+        if (epi >= 0 && ok) {
+#pragma unroll 1
+            for (int c0 = 16 * (epi >> 2); c0 < BN; c0 += 16 * (kTcEpilogueWarps / 4)) {
+                if (tok0 + c0 >= tok_end) break;
+#pragma unroll
+                for (int a = 0; a < NACC; ++a) {
+                    unsigned v[16];
+                    tmem_ld16(v, lanes + (unsigned)(a * BN + c0));
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                    for (int i = 0; i < 16; i += 4) {
+                        const int owner = (c0 + i) / own, c = c0 + i - owner * own;
+                        st_cluster_v4(cluster_place(smem_u32(smem), owner * CG + rank) + (unsigned)(((a * p.ranges + range) * kTileRows + quarter * 32 + lane) * pitch + c) * 4u, v[i], v[i + 1], v[i + 2], v[i + 3]);
                     }
                 }
+            }
+        }
+        cluster.sync();
+        if (epi >= 0 && ok && !*failed) {
+            const float* got = reinterpret_cast<const float*>(smem) + (quarter * 32 + lane) * pitch;
+            const ProductRow dst = product_row<true>(p.out, row);
+#pragma unroll 1
+            for (int first = 8 * (epi >> 2); first < own; first += 8 * (kTcEpilogueWarps / 4)) {
+                const int token = tok0 + range * own + first, count = min(min(8, own - first), tok_end - token);
+                if (count <= 0) break;
+                float val[16] = {}, up[16] = {};
+#pragma unroll 1
+                for (int z = 0; z < p.ranges; ++z)
+#pragma unroll
+                    for (int i = 0; i < 8; i += 4)
+                        if (first + i < own) {
+                            const float4 g = *reinterpret_cast<const float4*>(got + z * (kTileRows * pitch) + first + i);
+                            val[i] += g.x; val[i + 1] += g.y; val[i + 2] += g.z; val[i + 3] += g.w;
+                            if (GATED) {
+                                const float4 u = *reinterpret_cast<const float4*>(got + (p.ranges + z) * (kTileRows * pitch) + first + i);
+                                up[i] += u.x; up[i + 1] += u.y; up[i + 2] += u.z; up[i + 3] += u.w;
+                            }
+                        }
+                if (GATED) {
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) val[i] = tc_gated(val[i], up[i], p.act);
+                }
+                if (row < p.n) tc_emit(p, dst, val, token, count);
             }
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
-    if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kCols) : "memory");
-}
-
-// Sum of the K ranges in order, then the store (GATED: activation(gate sum) * up sum).
-template <bool GATED>
-__global__ void __launch_bounds__(256) bgemm_sum_kernel(const float* part, int ranges, int m, int n, GatedAct act, const ProductOut out) {
-    pdl_launch_dependents();
-    pdl_wait();
-    const size_t total = (size_t)m * n;
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= n) return;
-    for (int t = blockIdx.y; t < m; t += gridDim.y) {
-        const size_t i = (size_t)t * n + r;
-        float a = 0.f, b = 0.f;
-#pragma unroll 4
-        for (int z = 0; z < ranges; ++z) {
-            const float* base = part + (size_t)z * (GATED ? 2 : 1) * total;
-            a += __ldcg(base + i);
-            if (GATED) b += __ldcg(base + total + i);
-        }
-        product_store<!GATED>(out, t, r, GATED ? gated_activation(a, b, act) : a);
+    if (CG == 2) cluster.sync();   // no MMA of the pair reads tensor memory or arrives at a barrier of a CTA that has left
+    if (warp == 1) {
+        if (CG == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kCols) : "memory");
+        else asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kCols) : "memory");
     }
 }
 
@@ -627,63 +741,90 @@ int bf16_map(const __nv_bfloat16* p, int ld, int rows, int k, int box_rows, CUte
     return SWLM_OK;
 }
 
-struct TcShape { int bn, ranges, split_steps, tiles_m, tiles_n; };
+struct TcShape { int cg, bn, per_sm, ranges, tiles_m, tiles_n; };
+constexpr int kTcSMs = 148;
+template <int BN, int PER_SM, bool GATED>
+constexpr int tc_stages() {
+    return BN == 32 ? (GATED ? 6 : 10) / PER_SM : BN == 64 ? (GATED ? 5 : 8 / PER_SM) : BN == 128 ? (GATED ? 5 : 8) : (GATED ? 4 : 7);
+}
+template <int CG, int BN, int PER_SM, bool GATED>
+constexpr size_t tc_smem() { return (size_t)tc_stages<BN, PER_SM, GATED>() * ((GATED ? 2 : 1) * kTileRows * 128 + BN / CG * 128) + 1024; }
+
+int g_tc_clusters[4] = {kTcSMs, kTcSMs / 2, 0, 0};   // clusters of 1, 2, 4, 8 CTAs that run at once, one CTA per SM
+
+// How a product runs: the form with the least time by what was measured for n = 2048 .. 32768, K = 512 .. 8192, 16 .. 1024 rows (us;
+// graphs of launches, weights from memory). A step of 64 columns takes 0.21 (the round trip of a stage over the ring's depth; 0.25 with
+// half the depth, two CTAs per SM; 0.3 with 256 rows, 0.7 with gate and up of 256), or what L2 gives all CTAs together (12 TB/s). A launch
+// starts and ends in 3, tanh-GELU of 256 rows takes 4 more. The exchange between K ranges costs 2 (32 rows) to 5 (128): 2048 x 8192 at
+// 512 rows 27.3 / 21.0 for 1 and 2 ranges, at 16 rows 28.3 / 16.7 / 11.2 / 10.7 for 1, 2, 4, 8. Clusters of eight do not fill the GPU at
+// one CTA per SM (128 CTAs in eights: 16.9 instead of 10.7). Against one SM per 256 x 128 tile with the ranges' sums in memory and added by a
+// second launch: 3664 x 2048 at 512 rows 28.9 -> 11.3, 2048 x 8192 31.3 -> 21.0, gate and up of 8192 x 2048 59.5 -> 31.5; at 16 rows
+// 8.7 -> 6.7, 12.6 -> 10.7, 21.3 -> 15.0.
 TcShape tc_shape(int n, int k, int m, bool gated) {
-    TcShape t;
-    t.bn = m > 128 ? 256 : m > 64 ? 128 : m > 32 ? 64 : 32;
-    // too few tiles to fill the GPU: half as many rows per tile before K is cut
-    const int rows_n = gated ? kTileRows : 2 * kTileRows;
-    if (t.bn == 256 && (m + 255) / 256 * ((n + rows_n - 1) / rows_n) < 100) t.bn = 128;
-    t.tiles_m = (m + t.bn - 1) / t.bn;
-    t.tiles_n = (n + (gated ? kTileRows : 2 * kTileRows) - 1) / (gated ? kTileRows : 2 * kTileRows);
-    const int steps = (k + kTcK - 1) / kTcK, tiles = t.tiles_m * t.tiles_n;
-    int ranges = tiles * 2 > 148 ? 1 : std::min(std::min(148 / tiles, std::max(1, steps / 4)), 16);
-    t.split_steps = (steps + ranges - 1) / ranges;
-    t.ranges = (steps + t.split_steps - 1) / t.split_steps;
-    return t;
+    TcShape best{};
+    const int steps = (k + kTcK - 1) / kTcK;
+    double least = 1e30;
+    for (int bn = 32; bn <= 256; bn *= 2)
+        for (int per_sm = 1; per_sm <= (bn == 32 || (bn == 64 && !gated) ? 2 : 1); ++per_sm) {
+            const int cg = bn <= 64 ? 1 : 2, tiles_m = (m + bn - 1) / bn, tiles_n = (n + kTileRows * cg - 1) / (kTileRows * cg);
+            const double bytes = (gated ? 2 : 1) * kTileRows * 128 + bn / cg * 128, ends = 3 + (gated ? bn / 64 : bn / 128);
+            const double alone = bn == 256 ? (gated ? 0.7 : 0.3) : per_sm == 2 ? 0.25 : 0.21;
+            for (int i = 0; i < 4; ++i) {
+                const int z = (1 << i) / cg;   // clusters of 1, 2, 4, 8 CTAs
+                if (z < 1 || z > steps || (gated && bn == 256 && z > 1)) continue;
+                const long long groups = (long long)tiles_m * tiles_n, slots = (long long)g_tc_clusters[i] * per_sm;
+                const double waves = (double)((groups + slots - 1) / slots);
+                const double step = std::max(alone, bytes * (double)(std::min(groups, slots) << i) / 12e6);
+                const double cost = waves * (step * ((steps + z - 1) / z) + ends) + (z > 1 ? 1.5 + bn / 40.0 + 0.2 * z : 0.0);
+                if (cost < least) { least = cost; best = {cg, bn, per_sm, z, tiles_m, tiles_n}; }
+            }
+        }
+    return best;
 }
 
-template <int BN, int STAGES>
-constexpr size_t tc_smem() { return (size_t)STAGES * (2 * kTileRows * 128 + BN * 128) + 1024; }
-template <int BN, int STAGES, bool GATED>
+template <int CG, int BN, int PER_SM, bool GATED>
 int tc_attr() {
-    SWLM_CUDA(cudaFuncSetAttribute(bgemm_tc_kernel<BN, STAGES, GATED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc_smem<BN, STAGES>()));
+    SWLM_CUDA(cudaFuncSetAttribute(bgemm_tc_kernel<CG, BN, tc_stages<BN, PER_SM, GATED>(), GATED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc_smem<CG, BN, PER_SM, GATED>()));
     return SWLM_OK;
 }
-template <int BN, int STAGES>
+template <int CG, int BN, int PER_SM, bool GATED>
 int tc_launch(const ProductLaunch& a, const TcShape& t, cudaStream_t s) {
-    const bool gated = a.w2 != nullptr;
     TcParams p{};
-    p.n = a.experts ? a.w->n / a.experts : a.w->n; p.tiles = a.tiles; p.m = a.m; p.steps = (a.w->k + kTcK - 1) / kTcK; p.split_steps = t.split_steps; p.act = a.act; p.out = a.out; p.part = a.part; p.status = a.status;
+    p.n = a.experts ? a.w->n / a.experts : a.w->n; p.tiles = a.tiles; p.m = a.m; p.steps = (a.w->k + kTcK - 1) / kTcK; p.ranges = t.ranges; p.act = a.act; p.out = a.out; p.status = a.status;
     CUtensorMap xmap, wmap, wmap2;
-    int rc = bf16_map(static_cast<const __nv_bfloat16*>(a.x), a.x_stride, a.m, a.w->k, BN, &xmap);
+    int rc = bf16_map(static_cast<const __nv_bfloat16*>(a.x), a.x_stride, a.m, a.w->k, BN / CG, &xmap);
     if (!rc) rc = bf16_map(a.w->data, a.w->ld, a.w->n, a.w->k, kTileRows, &wmap);
     wmap2 = wmap;
     p.split = a.x2 ? a.split : p.n;
-    if (!rc && a.x2) rc = bf16_map(static_cast<const __nv_bfloat16*>(a.x2), a.x2_stride, a.m, a.w->k, BN, &wmap2);
-    if (!rc && gated) rc = bf16_map(a.w2->data, a.w2->ld, a.w2->n, a.w2->k, kTileRows, &wmap2);
+    if (!rc && a.x2) rc = bf16_map(static_cast<const __nv_bfloat16*>(a.x2), a.x2_stride, a.m, a.w->k, BN / CG, &wmap2);
+    if (!rc && GATED) rc = bf16_map(a.w2->data, a.w2->ld, a.w2->n, a.w2->k, kTileRows, &wmap2);
     if (rc) return rc;
-    const dim3 grid((unsigned)t.tiles_m, (unsigned)t.tiles_n, (unsigned)t.ranges);
-    cudaError_t e = gated ? launch_k(bgemm_tc_kernel<BN, STAGES, true>, grid, dim3(kTcBlock), tc_smem<BN, STAGES>(), s, p, xmap, wmap, wmap2)
-                          : launch_k(bgemm_tc_kernel<BN, STAGES, false>, grid, dim3(kTcBlock), tc_smem<BN, STAGES>(), s, p, xmap, wmap, wmap2);
-    if (e != cudaSuccess) return cuda_fail(e, "bgemm launch");
-    if (t.ranges > 1) {
-        const dim3 g((unsigned)((p.n + 255) / 256), (unsigned)std::min(p.m, std::max(64, 8 * 148 * 256 / p.n)));
-        e = gated ? launch_k(bgemm_sum_kernel<true>, g, dim3(256), 0, s, (const float*)a.part, t.ranges, p.m, p.n, p.act, p.out)
-                  : launch_k(bgemm_sum_kernel<false>, g, dim3(256), 0, s, (const float*)a.part, t.ranges, p.m, p.n, p.act, p.out);
-        if (e != cudaSuccess) return cuda_fail(e, "bgemm sum launch");
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(CG * t.ranges), (unsigned)t.tiles_m, (unsigned)t.tiles_n); cfg.blockDim = dim3(kTcBlock); cfg.dynamicSmemBytes = tc_smem<CG, BN, PER_SM, GATED>(); cfg.stream = s;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)(CG * t.ranges); attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr; cfg.numAttrs = pdl_enabled() ? 2 : 1;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, bgemm_tc_kernel<CG, BN, tc_stages<BN, PER_SM, GATED>(), GATED>, p, xmap, wmap, wmap2);
+    return e == cudaSuccess ? SWLM_OK : cuda_fail(e, "bgemm launch");
+}
+template <bool GATED>
+int tc_pick(const ProductLaunch& a, const TcShape& t, cudaStream_t s) {
+    switch (t.bn) {
+    case 32: return t.per_sm == 2 ? tc_launch<1, 32, 2, GATED>(a, t, s) : tc_launch<1, 32, 1, GATED>(a, t, s);
+    case 64: return t.per_sm == 2 && !GATED ? tc_launch<1, 64, GATED ? 1 : 2, GATED>(a, t, s) : tc_launch<1, 64, 1, GATED>(a, t, s);
+    case 128: return tc_launch<2, 128, 1, GATED>(a, t, s);
+    default: return tc_launch<2, 256, 1, GATED>(a, t, s);
     }
-    return SWLM_OK;
 }
 
 TcShape grouped_shape(const ProductLaunch& a) {
     TcShape t;
-    const int n = a.w->n / a.experts, rows_n = a.w2 ? kTileRows : 2 * kTileRows;
-    t.bn = a.group_bn;
-    t.tiles_m = a.max_tiles;
-    t.tiles_n = (n + rows_n - 1) / rows_n;
-    t.ranges = 1;
-    t.split_steps = (a.w->k + kTcK - 1) / kTcK;
+    const int n = a.w->n / a.experts;
+    t.bn = a.group_bn; t.cg = t.bn <= 64 ? 1 : 2; t.per_sm = t.bn <= 64 ? 2 : 1; t.ranges = 1;
+    t.tiles_m = a.max_tiles; t.tiles_n = (n + kTileRows * t.cg - 1) / (kTileRows * t.cg);
     return t;
 }
 
@@ -696,8 +837,18 @@ bool gemv_fits(int m, int k, bool x_f32, bool norm) {
 
 int bgemm_init() {
     int rc;
-    if ((rc = tc_attr<32, 4, false>()) || (rc = tc_attr<32, 4, true>()) || (rc = tc_attr<64, 4, false>()) || (rc = tc_attr<64, 4, true>()) ||
-        (rc = tc_attr<128, 4, false>()) || (rc = tc_attr<128, 4, true>()) || (rc = tc_attr<256, 3, false>()) || (rc = tc_attr<256, 3, true>())) return rc;
+    if ((rc = tc_attr<1, 32, 1, false>()) || (rc = tc_attr<1, 32, 2, false>()) || (rc = tc_attr<1, 32, 1, true>()) || (rc = tc_attr<1, 32, 2, true>()) ||
+        (rc = tc_attr<1, 64, 1, false>()) || (rc = tc_attr<1, 64, 2, false>()) || (rc = tc_attr<1, 64, 1, true>()) || (rc = tc_attr<2, 128, 1, false>()) ||
+        (rc = tc_attr<2, 128, 1, true>()) || (rc = tc_attr<2, 256, 1, false>()) || (rc = tc_attr<2, 256, 1, true>())) return rc;
+    for (int i = 2; i < 4; ++i) {
+        cudaLaunchConfig_t cfg = {};
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = 1u << i; attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        cfg.gridDim = dim3(1u << i, 1, 64); cfg.blockDim = dim3(kTcBlock); cfg.dynamicSmemBytes = tc_smem<1, 32, 1, false>(); cfg.attrs = attr; cfg.numAttrs = 1;
+        SWLM_CUDA(cudaOccupancyMaxActiveClusters(&g_tc_clusters[i], bgemm_tc_kernel<1, 32, tc_stages<32, 1, false>(), false>, &cfg));
+        if (g_tc_clusters[i] < 1) { set_error("dense product: no cluster of %d CTAs fits this device", 1 << i); return SWLM_ERR_UNSUPPORTED; }
+    }
     return SWLM_OK;
 }
 
@@ -710,24 +861,12 @@ bool product_takes_two(int m, int k, int split, bool x_f32) {
     return !x_f32 && split % (2 * kTileRows) == 0;   // no tile has rows of both
 }
 
-size_t product_part_floats(int n, int k, int m, bool gated) {
-    if (gemv_fits(m, k, false, false)) return 0;
-    const TcShape t = tc_shape(n, k, m, gated);
-    return t.ranges > 1 ? (size_t)t.ranges * (gated ? 2 : 1) * m * n : 0;
-}
-
 // tiles about as tall as an expert has rows on average
 int grouped_bn(int rows, int experts) {
     const int avg = rows / std::max(1, experts);
     return avg > 160 ? 256 : avg > 64 ? 128 : avg > 24 ? 64 : 32;
 }
 int grouped_max_tiles(int rows, int experts) { return std::min(rows, experts) + rows / grouped_bn(rows, experts); }
-
-int product_launch_count(const ProductLaunch& a) {
-    if (a.experts) return 1;
-    if (gemv_fits(a.m, a.w->k, a.x_f32, a.norm.mode != 0) || a.x_f32) return 1;
-    return tc_shape(a.w->n, a.w->k, a.m, a.w2 != nullptr).ranges > 1 ? 2 : 1;
-}
 
 int launch_product(const ProductLaunch& a, cudaStream_t s) {
     if (a.m <= 0) return SWLM_OK;
@@ -753,13 +892,7 @@ int launch_product(const ProductLaunch& a, cudaStream_t s) {
     }
     if (((a.x_stride | a.x2_stride) & 7) || ((reinterpret_cast<uintptr_t>(a.x) | reinterpret_cast<uintptr_t>(a.x2)) & 15)) { set_error("dense product: activation rows must be 16-byte aligned"); return SWLM_ERR_INVALID; }
     const TcShape t = a.experts ? grouped_shape(a) : tc_shape(a.w->n, a.w->k, a.m, gated);
-    if (t.ranges > 1 && (!a.part || a.part_floats < (size_t)t.ranges * (gated ? 2 : 1) * a.m * a.w->n)) { set_error("dense product: scratch too small"); return SWLM_ERR_INVALID; }
-    switch (t.bn) {
-    case 32: return tc_launch<32, 4>(a, t, s);
-    case 64: return tc_launch<64, 4>(a, t, s);
-    case 128: return tc_launch<128, 4>(a, t, s);
-    default: return tc_launch<256, 3>(a, t, s);
-    }
+    return gated ? tc_pick<true>(a, t, s) : tc_pick<false>(a, t, s);
 }
 
 }  // namespace swlm

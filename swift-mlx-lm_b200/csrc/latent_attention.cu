@@ -931,10 +931,10 @@ int launch_long(const LatentLaunch& a, cudaStream_t s, int* launches) {
         x.out.end[0] = a.heads * a.dim; x.out.end[1] = x.out.end[2] = x.out.end[3] = a.ukv->n;
         x.out.y[0] = a.expand + l.k; x.out.stride[0] = a.heads * a.dim;
         x.out.y[1] = a.expand + l.v; x.out.stride[1] = a.heads * a.vdim;
-        x.part = a.part; x.part_floats = a.part_floats; x.status = a.status;
+        x.status = a.status;
         const int rc = launch_product(x, s);
         if (rc) return rc;
-        *launches += 2 + product_launch_count(x);
+        *launches += 3;
     }
     const dim3 grid(a.n_tiles, a.heads);
     switch (prefill_form(a.dim, a.row.rot, a.vdim)) {

@@ -520,18 +520,17 @@ int launch_routed(const RoutedLaunch& a, cudaStream_t s, int* launches) {
     if ((rc = launch_product(d, s))) return rc;
     if (shared) {
         ProductLaunch u;
-        u.w = a.shared_up; u.m = a.m; u.x = a.x; u.x_stride = a.x_stride; u.part = a.part; u.part_floats = a.part_floats; u.status = a.status;
+        u.w = a.shared_up; u.m = a.m; u.x = a.x; u.x_stride = a.x_stride; u.status = a.status;
         u.out.y[0] = p.shared_mid; u.out.stride[0] = p.shared_stride; u.out.gelu = 1;
         for (int& end : u.out.end) end = a.shape.shared_ff;
         if ((rc = launch_product(u, s))) return rc;
-        *launches += product_launch_count(u);
         ProductLaunch w = u;
         w.w = a.shared_down; w.x = p.shared_mid; w.x_stride = p.shared_stride;
         p.shared_y = reinterpret_cast<const float*>(a.scratch + l.shared_y); p.shared_y_stride = up8(a.shape.width);
         w.out.y[0] = a.scratch + l.shared_y; w.out.stride[0] = p.shared_y_stride; w.out.f32[0] = 1; w.out.gelu = 0;
         for (int& end : w.out.end) end = a.shape.width;
         if ((rc = launch_product(w, s))) return rc;
-        *launches += product_launch_count(w);
+        *launches += 2;
     }
     e = launch_k(routed_sum_kernel, dim3((a.shape.width + kRtThreads * 4 - 1) / (kRtThreads * 4), a.m), dim3(kRtThreads), 0, s, p);
     if (e != cudaSuccess) return cuda_fail(e, "routed sum launch");

@@ -681,29 +681,17 @@ int bufs_rows(swlm_state* s, StreamBufs* b, int rows, int wants) {
     return SWLM_OK;
 }
 
-size_t part_need(const swlm_plan* plan, int rows, int wants) {
-    size_t need = 0;
-    if (plan->all_f32()) return 0;
-    for (const Launch& L : plan->launches)
-        if (L.kind == L_PRODUCT && L.x2_buf >= 0) for (const Matrix* m : {L.m1, &L.part[0], &L.part[1]}) need = std::max(need, product_part_floats(m->n, m->k, rows, false));
-        else if (L.kind == L_PRODUCT) need = std::max(need, product_part_floats(L.m1->n, L.m1->k, L.seg_buf[0] == SWLM_BUF_LOGITS ? wants : rows, L.m2 != nullptr));
-        else if (L.kind == L_ROUTED && L.m4) need = std::max(need, std::max(product_part_floats(L.m4->n, L.m4->k, rows, false), product_part_floats(L.m5->n, L.m5->k, rows, false)));
-    return need;
-}
-
 // scratch of a batch; r.splits_pages bounds the splits
 int bufs_scratch(swlm_state* s, StreamBufs* b, const RowBatch& r) {
     const swlm_plan* plan = s->plan;
     int rc;
-    size_t part = part_need(plan, r.rows, r.wants), expand = 0;
+    size_t expand = 0;
     for (const Launch& L : plan->launches) {
         if (L.kind != L_LATENT || r.n_long == 0) continue;
         const LatentLayer& ll = plan->latent[L.st.layer];
         const int ctx = r.total_ctx[L.window_set];
         expand = std::max(expand, latent_expand_bytes(ll.row, L.st.heads, L.st.head_dim, L.st.value_dim, ctx));
-        part = std::max(part, product_part_floats(L.st.heads * (L.st.head_dim + L.st.value_dim), ll.rank, ctx, false));
     }
-    if ((rc = grow(&b->part, &b->part_cap, part, s->stream))) return rc;
     if ((rc = grow(&b->expand, &b->expand_cap, expand, s->stream))) return rc;
     size_t delta = 0, routed = 0;
     for (const Launch& L : plan->launches) {
@@ -726,7 +714,7 @@ int bufs_scratch(swlm_state* s, StreamBufs* b, const RowBatch& r) {
 
 void bufs_free(StreamBufs* b) {
     for (void* p : b->buf) cudaFree(p);
-    cudaFree(b->res2); cudaFree(b->results); cudaFree(b->meta); cudaFree(b->argmax_out); cudaFree(b->qcat); cudaFree(b->partial); cudaFree(b->part);
+    cudaFree(b->res2); cudaFree(b->results); cudaFree(b->meta); cudaFree(b->argmax_out); cudaFree(b->qcat); cudaFree(b->partial);
     cudaFree(b->expand); cudaFree(b->delta); cudaFree(b->routed); cudaFree(b->argmax_val); cudaFree(b->argmax_idx);
     *b = StreamBufs{};
 }
@@ -818,7 +806,7 @@ int enqueue_rows_stream(swlm_state* s, StreamBufs* b, const RowBatch& r, bool bo
             ProductLaunch a;
             a.w = L.m1; a.w2 = L.m2; a.act = L.act; a.m = m; a.x_f32 = f32;
             a.x = static_cast<unsigned char*>(b->buf[st.in_buf]) + (size_t)st.in_off * stored_bytes(plan, st.in_buf); a.x_stride = s->width[st.in_buf];
-            a.part = b->part; a.part_floats = b->part_cap; a.status = s->pf_status;
+            a.status = s->pf_status;
             if (head && idx && !L.norm.kind) { set_error("the output head must follow a norm that nothing else reads"); return SWLM_ERR_UNSUPPORTED; }
             if (L.norm.kind) {
                 const StreamNorm n = norm_of(s, b, r, L, L.norm, L.norm_w, L.res_in, L.res_out);
@@ -844,7 +832,7 @@ int enqueue_rows_stream(swlm_state* s, StreamBufs* b, const RowBatch& r, bool bo
                     const int buf = L.seg_buf[1 + h];
                     c.out.y[0] = b->buf[buf]; c.out.stride[0] = s->width[buf]; c.out.f32[0] = stored_f32(plan, buf) ? 1 : 0; c.out.end[0] = c.w->n;
                     rc = launch_product(c, stream);
-                    s->launches += product_launch_count(c);
+                    s->launches += 1;
                 }
                 if (!rc) rc = launch_stream_gated(m, L.m1->n, b->buf[L.seg_buf[1]], s->width[L.seg_buf[1]], b->buf[L.seg_buf[2]], s->width[L.seg_buf[2]],
                                                   b->buf[L.seg_buf[0]], s->width[L.seg_buf[0]], f32, L.act, stream);
@@ -869,13 +857,13 @@ int enqueue_rows_stream(swlm_state* s, StreamBufs* b, const RowBatch& r, bool bo
                             c.out.end[q] = a.out.end[from] - (h ? a.split : 0);
                         }
                         rc = launch_product(c, stream);
-                        s->launches += product_launch_count(c);
+                        s->launches += 1;
                     }
                     break;
                 }
             }
             rc = launch_product(a, stream);
-            s->launches += product_launch_count(a);
+            s->launches += 1;
             break;
         }
         case L_SWIGLU:
@@ -913,7 +901,7 @@ int enqueue_rows_stream(swlm_state* s, StreamBufs* b, const RowBatch& r, bool bo
             a.z = static_cast<const float*>(b->buf[st.in2_buf]); a.z_stride = s->width[st.in2_buf];
             a.gate = L.m1; a.up = L.m2; a.down = L.m3; a.shared_up = L.m4; a.shared_down = L.m5;
             a.softmax = st.score_act == SWLM_SCORE_SOFTMAX; a.group_best = st.group_best == 1 ? 1 : 2; a.raw_weights = st.raw_weights;
-            a.part = b->part; a.part_floats = b->part_cap; a.correction = L.dv[0] ? L.dv[0]->data : nullptr;
+            a.correction = L.dv[0] ? L.dv[0]->data : nullptr;
             a.out = static_cast<float*>(b->buf[st.out_buf]); a.out_stride = s->width[st.out_buf];
             a.scratch = b->routed; a.counts = s->routed_counts; a.status = s->pf_status;
             int n = 0;
@@ -977,7 +965,7 @@ int enqueue_rows_stream(swlm_state* s, StreamBufs* b, const RowBatch& r, bool bo
             a.qcat = b->qcat; a.partial = b->partial;
             a.n_long = r.n_long; a.long_rows = r.long_rows; a.n_spans = r.n_spans; a.n_tiles = r.n_tiles; a.tiles = r.tiles;
             if (r.n_spans) { a.spans = r.spans[L.window_set]; a.total_ctx = r.total_ctx[L.window_set]; }
-            a.expand = b->expand; a.part = b->part; a.part_floats = b->part_cap; a.status = s->pf_status;
+            a.expand = b->expand; a.status = s->pf_status;
             a.only_attention = latent_kernel;
             int n = 0;
             rc = launch_latent(a, stream, &n);
@@ -1136,22 +1124,15 @@ int stream_launches_per_step(const swlm_plan* plan) {
         const Launch& L = plan->launches[li];
         if (L.fused && token_input_fits(token_input(&L), m, plan->desc.hidden)) { n += 1; li += L.fused; continue; }
         if (L.kind == L_PRODUCT) {
-            ProductLaunch a;
-            a.w = L.m1; a.w2 = L.m2; a.m = m; a.x_f32 = plan->all_f32();
-            const bool fused = L.norm.kind && product_takes_norm(m, L.m1->k);
-            if (fused) a.norm.mode = L.norm.kind;
-            else if (L.norm.kind) n += 1;
-            if (L.m2 && !product_takes_gate(m, L.m1->k, a.x_f32)) { a.w2 = nullptr; n += 2 * product_launch_count(a) + 1; }
-            else if (L.x2_buf >= 0 && !product_takes_two(m, L.m1->k, L.part[0].n, plan->all_f32()))
-                for (const Matrix& part : L.part) { a.w = &part; n += product_launch_count(a); }
-            else n += product_launch_count(a);
+            if (L.norm.kind && !product_takes_norm(m, L.m1->k)) n += 1;
+            if (L.m2 && !product_takes_gate(m, L.m1->k, plan->all_f32())) n += 3;
+            else n += L.x2_buf >= 0 && !product_takes_two(m, L.m1->k, L.part[0].n, plan->all_f32()) ? 2 : 1;
         } else if (L.kind == L_DELTA) n += delta_step_fits(plan->delta[L.st.layer].shape) ? 1 : 3;
         else if (L.kind == L_RETENTION) n += retention_step_fits(L.st.key_dim, L.st.value_dim) ? 1 : 2;
         else if (L.kind == L_GROUPED) n += grouped_appends(plan->grouped[L.st.layer].row, plan->all_f32(), L.st.rope_dim) ? 1 : 2;
         else if (L.kind == L_ROUTED) {
             n += m <= 4 || plan->all_f32() ? 2 : 5;
-            if (L.m4 && m > 4 && !plan->all_f32())
-                for (const Matrix* w : {L.m4, L.m5}) { ProductLaunch a; a.w = w; a.m = m; n += product_launch_count(a); }
+            if (L.m4 && m > 4 && !plan->all_f32()) n += 2;
         }
         else n += L.kind == L_LATENT ? 3 : L.kind == L_ARGMAX ? 2 : 1;
     }

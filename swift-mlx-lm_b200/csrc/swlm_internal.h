@@ -415,7 +415,6 @@ struct ProductLaunch {
     const void* x2 = nullptr; int x2_stride = 0, split = 0;   // weight rows from `split` on meet these activations (only when product_takes_two)
     StreamNorm norm;                // x = this norm's result (only when product_takes_norm)
     ProductOut out;
-    float* part = nullptr; size_t part_floats = 0;   // split-K sums
     int* status = nullptr;          // device word set when a bounded wait expired
     // Grouped form (bf16, tensor cores): w holds the rows of `experts` matrices one after the other, activation rows are sorted
     // by expert, and tiles[i] = (expert, first row, rows, 0) names the rows of tile i (at most group_bn; 0 rows: nothing to do).
@@ -430,8 +429,6 @@ int grouped_max_tiles(int rows, int experts);
 bool product_takes_norm(int m, int k);
 bool product_takes_gate(int m, int k, bool x_f32);
 bool product_takes_two(int m, int k, int split, bool x_f32);
-int product_launch_count(const ProductLaunch& a);
-size_t product_part_floats(int n, int k, int m, bool gated);
 
 // Geometry of one cached latent row: rank latent entries padded to rp, then rot rotated entries padded to rotp; `pitch`
 // entries from row to row (in bf16 pools an odd multiple of 16 bytes, so that eight consecutive rows of a page copied
@@ -468,7 +465,6 @@ struct LatentLaunch {
     int n_long = 0; const int32_t* long_rows = nullptr;
     int n_spans = 0; const LatentSpan* spans = nullptr; int n_tiles = 0; const int2* tiles = nullptr; int total_ctx = 0;
     unsigned char* expand = nullptr;
-    float* part = nullptr; size_t part_floats = 0;
     int* status = nullptr;
     bool only_attention = false;   // timing hook: the attention kernel alone
 };
@@ -480,7 +476,7 @@ size_t latent_expand_bytes(const LatentRow& r, int heads, int dim, int vdim, int
 // can rows of this layer be attended in spans over expanded keys and values?
 bool latent_expands(const LatentRow& r, int dim, int vdim, bool f32);
 constexpr int kLatentQueryTile = 128;
-// launches (for the counters): short part 3, span part 4 or 5
+// launches (for the counters): short part 3, span part 4
 int launch_latent(const LatentLaunch& a, cudaStream_t s, int* launches);
 
 // ---- the residual stream between sublayers (stream_join.cu) ------------------------------------------------------------
@@ -646,7 +642,6 @@ struct RoutedLaunch {
     float* out = nullptr; int out_stride = 0;
     unsigned char* scratch = nullptr;
     unsigned* counts = nullptr;                            // [kMaxExperts], zero between launches
-    float* part = nullptr; size_t part_floats = 0;         // split-K sums of the shared products
     int* status = nullptr;
 };
 constexpr int kMaxExperts = 1024, kMaxTop = 64;

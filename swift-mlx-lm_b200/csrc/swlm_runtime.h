@@ -114,7 +114,6 @@ struct StreamBufs {
     int32_t* argmax_out = nullptr;
     float* qcat = nullptr; size_t qcat_cap = 0;          // latent attention: absorbed queries
     float* partial = nullptr; size_t partial_cap = 0;    // latent attention: partial results per split
-    float* part = nullptr; size_t part_cap = 0;          // products: sums of K ranges
     unsigned char* expand = nullptr; size_t expand_cap = 0;
     float* delta = nullptr; size_t delta_cap = 0;        // gated delta rule: records and read-outs of portions
     unsigned char* routed = nullptr; size_t routed_cap = 0;

@@ -129,6 +129,44 @@ def test_gate_and_up_in_one_launch(pkg, store, dtype, rows, act_name, n, k):
     m.close()
 
 
+@pytest.mark.parametrize("gated", [False, True])
+@pytest.mark.parametrize("rows, n, k", [
+    (17, 40, 3000), (30, 2056, 200),      # 32 rows per tile: K over eight CTAs, four columns each; one range, ragged weight rows
+    (60, 136, 4096), (33, 1100, 1032),    # 64 rows: K over a cluster, tails of rows and columns
+    (100, 264, 2048), (130, 520, 72),     # pairs of SMs, two steps of K
+    (257, 520, 1096), (700, 4104, 264),   # several tiles of rows, the last of one row; 256 rows per tile
+])
+def test_products_of_a_portion(pkg, store, gated, rows, n, k):
+    """Dense products of many rows on the tensor cores, alone or with gate and up together, against the plain ones: every form of tile,
+    K ranges that meet within a cluster, remainders on all sides."""
+    P, rng, vocab, scale = pkg.plan, np.random.default_rng(rows + n), 64, 1.0 / np.sqrt(k)
+    tag = f"{rows}.{n}.{k}"
+    w, u = (vc.to_bf16_bits(scale * rng.standard_normal((n, k))) for _ in range(2))
+    table = vc.to_bf16_bits(rng.standard_normal((vocab, k)))
+    store.add_matrix(f"p.w{tag}", w)
+    store.add_matrix(f"p.u{tag}", u)
+    store.add_dense(f"p.e{tag}", table)
+    store.add_dense(f"p.n{tag}", vc.to_bf16_bits(np.zeros(k)))
+    steps = [P._step(P.STEP_EMBED, out_buf=P.BUF_HIDDEN, n=k, weight=f"p.e{tag}"),
+             P._step(P.STEP_COPY_RMSNORM, in_buf=P.BUF_HIDDEN, out_buf=P.BUF_S0, n=k, eps=1e-5, weight_bias=1.0, weight=f"p.n{tag}"),
+             P._step(P.STEP_PRODUCT, in_buf=P.BUF_S0, out_buf=P.BUF_S1, n=n, k=k, weight=f"p.w{tag}")]
+    if gated:
+        steps += [P._step(P.STEP_PRODUCT, in_buf=P.BUF_S0, out_buf=P.BUF_S2, n=n, k=k, weight=f"p.u{tag}"),
+                  P._step(P.STEP_GEGLU, in_buf=P.BUF_S1, in2_buf=P.BUF_S2, out_buf=P.BUF_S1, n=n)]
+    m = model_of(pkg, store, steps, "bfloat16", k, vocab=vocab, batch=1, max_seq=1024)
+    tokens = rng.integers(0, vocab, size=rows)
+    m.run_batch([(0, tokens.tolist(), [])], logits=False)
+    x = m.read_buffer_f32(P.BUF_S0, rows, k).astype(np.float64)
+    close(x, plain.rms_norm(vc.from_bf16_bits(table)[tokens], np.zeros(k), 1e-5, 1.0), "bfloat16")
+    want = plain.linear(x, vc.from_bf16_bits(w))
+    if gated:
+        want = plain.gelu_tanh(want) * plain.linear(x, vc.from_bf16_bits(u))
+    got = m.read_buffer_f32(P.BUF_S1, rows, n)
+    # a result is rounded once to bf16: half of 2^-8 of itself at most, and never more than that of the largest in its row
+    assert (np.abs(got - want) <= 2.0 ** -8 * np.abs(want).max(axis=1, keepdims=True)).all()
+    m.close()
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 def test_argmax_takes_the_lowest_of_equal_logits(pkg, store, dtype):
     P, rng = pkg.plan, np.random.default_rng(4)
