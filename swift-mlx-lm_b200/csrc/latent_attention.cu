@@ -6,7 +6,7 @@
 //     query (q_plain . W_uk c = (W_uk^T q_plain) . c), rotates, and appends the row's own latent; an attention kernel works
 //     on the cached rows as one key / value head shared by all query heads, split over the context; latent_out_kernel merges
 //     the splits, applies the value projection and the output gate.
-//   * in spans (prompt portions): latent_append_kernel appends and rotates, latent_gather_kernel lines the cached rows of the
+//   * in spans (prompt portions): latent_append_kernel appends, rotates and lines the cached rows of the
 //     spans up, one tensor-core product expands them to keys and values per head, latent_prefill_kernel is a tiled causal
 //     attention over them with the gate in its epilogue.
 //
@@ -121,10 +121,10 @@ __device__ __forceinline__ float rotated(const LatentParams& p, const V& x, int 
     return e.first ? x(i) * c - x(e.partner) * s : x(i) * c + x(e.partner) * s;
 }
 
-// The row a warp appends: norm of the latent, rotation of the shared key part, zeros in the padding.
+// The row a warp appends: norm of the latent, rotation of the shared key part, zeros in the padding; the row's entries go to two places.
 constexpr int kAppendRegs = 16;   // latent entries per lane that are read once
 template <typename T>
-__device__ __forceinline__ void append_row(const LatentParams& p, int r, int lane) {
+__device__ __forceinline__ void append_row(const LatentParams& p, int r, int lane, T* latent, T* rotated_part) {
     const float* src = p.kv + (size_t)r * p.kv_stride;
     const int pos = p.row_pos[r], seq = p.row_seq[r];
     float v[kAppendRegs];
@@ -136,17 +136,22 @@ __device__ __forceinline__ void append_row(const LatentParams& p, int r, int lan
     for (int j = 0; j < kAppendRegs; ++j) ss = fmaf(v[j], v[j], ss);
     for (int i = lane + 32 * kAppendRegs; i < p.row.rank; i += 32) { const float x = src[i]; ss = fmaf(x, x, ss); }
     for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+    auto put = [&](int i, float x) { lat_put(dst + i, x); if (i < p.row.rank) lat_put(latent + i, x); };
     const float sc = 1.0f / sqrtf(ss / (float)p.row.rank + p.eps);
 #pragma unroll
     for (int j = 0; j < kAppendRegs; ++j) {
         const int i = lane + 32 * j;
-        if (i < p.row.rp) lat_put(dst + i, i < p.row.rank ? v[j] * sc * (__bfloat162float(p.norm_w[i]) + p.weight_bias) : 0.f);
+        if (i < p.row.rp) put(i, i < p.row.rank ? v[j] * sc * (__bfloat162float(p.norm_w[i]) + p.weight_bias) : 0.f);
     }
     for (int i = lane + 32 * kAppendRegs; i < p.row.rp; i += 32)
-        lat_put(dst + i, i < p.row.rank ? src[i] * sc * (__bfloat162float(p.norm_w[i]) + p.weight_bias) : 0.f);
+        put(i, i < p.row.rank ? src[i] * sc * (__bfloat162float(p.norm_w[i]) + p.weight_bias) : 0.f);
     const float* rot = src + p.row.rank;
     auto at = [&](int i) { return rot[i]; };
-    for (int i = lane; i < p.row.pitch - p.row.rp; i += 32) lat_put(dst + p.row.rp + i, i < p.row.rot ? rotated(p, at, pos, i) : 0.f);
+    for (int i = lane; i < p.row.pitch - p.row.rp; i += 32) {
+        const float x = i < p.row.rot ? rotated(p, at, pos, i) : 0.f;
+        lat_put(dst + p.row.rp + i, x);
+        if (i < p.row.rot) lat_put(rotated_part + i, x);
+    }
 }
 
 // The same by a CTA of 256 threads: everything that does not depend on something else is requested at once.
@@ -643,46 +648,69 @@ cudaError_t launch_out(const LatentLaunch& a, const LatentParams& p, cudaStream_
 }
 
 // ---- spans: append and rotate ------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(128) latent_append_kernel(const LatentParams p) {
+// One launch: CTAs below n_rows take a new row each (warp 0 appends its latent, to the cache and to its place among the spans' rows; the
+// others rotate its queries), the rest line up the spans' older rows (from position `lo` on), a warp each: latents [total_ctx][ctx_ld],
+// rotated parts [total_ctx][rot_ld]. A sequence is in a batch once, so that no older row is written by this launch.
+constexpr int kAppWarps = 8;
+__global__ void __launch_bounds__(kAppWarps * 32) latent_append_kernel(const LatentParams p) {
     pdl_launch_dependents();
     pdl_wait();
-    const int r = batch_row(p, blockIdx.x), lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (warp == 0) { append_row<__nv_bfloat16>(p, r, lane); return; }
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if ((int)blockIdx.x >= p.n_rows) {
+        const int row = ((int)blockIdx.x - p.n_rows) * kAppWarps + warp;
+        if (row >= p.total_ctx) return;
+        int sp = 0;
+        while (sp + 1 < p.n_spans && p.spans[sp + 1].ctx0 <= row) ++sp;
+        const LatentSpan span = p.spans[sp];
+        const int pos = span.lo + row - span.ctx0;
+        if (pos >= span.pos0) return;   // a new row
+        const __nv_bfloat16* src = cached_row<__nv_bfloat16>(p, span.seq, pos);
+        for (int i = lane; i < p.ctx_ld / 8; i += 32) reinterpret_cast<uint4*>(p.ctx_latent + (size_t)row * p.ctx_ld)[i] = reinterpret_cast<const uint4*>(src)[i];
+        for (int i = lane; i < p.rot_ld / 8; i += 32) reinterpret_cast<uint4*>(p.ctx_rot + (size_t)row * p.rot_ld)[i] = reinterpret_cast<const uint4*>(src + p.row.rp)[i];
+        return;
+    }
+    const int r = batch_row(p, blockIdx.x);
+    if (warp == 0) {
+        int sp = 0;
+        while (sp + 1 < p.n_spans && p.spans[sp + 1].row0 <= r) ++sp;
+        const LatentSpan span = p.spans[sp];
+        const size_t at = span.ctx0 + span.pos0 + r - span.row0 - span.lo;
+        append_row<__nv_bfloat16>(p, r, lane, p.ctx_latent + at * p.ctx_ld, p.ctx_rot + at * p.rot_ld);
+        return;
+    }
     const int half = p.rot_dims >> 1, per_head = p.dim + p.row.rot, pos = p.row_pos[r];
     __nv_bfloat16* q = static_cast<__nv_bfloat16*>(p.q) + (size_t)r * p.q_stride + p.dim;
     const int step = rotary_step(p.rot_dims, p.rot_neighbours);
+    constexpr int kAhead = 4;   // heads of a warp whose pairs are requested together
     for (int i = lane; i < half; i += 32) {
         float c, s;
         angle(p, pos, i, c, s);
-        for (int h = warp - 1; h < p.heads; h += 3) {
-            __nv_bfloat16* x = q + (size_t)h * per_head + rotary_first(i, p.rot_neighbours);
-            const float u = __bfloat162float(x[0]), v = __bfloat162float(x[step]);
-            x[0] = __float2bfloat16_rn(u * c - v * s);
-            x[step] = __float2bfloat16_rn(v * c + u * s);
+        for (int h0 = warp - 1; h0 < p.heads; h0 += kAhead * (kAppWarps - 1)) {
+            __nv_bfloat16* x = q + (size_t)h0 * per_head + rotary_first(i, p.rot_neighbours);
+            const size_t to_next = (size_t)(kAppWarps - 1) * per_head;
+            float u[kAhead], v[kAhead];
+#pragma unroll
+            for (int j = 0; j < kAhead; ++j)
+                if (h0 + j * (kAppWarps - 1) < p.heads) { u[j] = __bfloat162float(x[j * to_next]); v[j] = __bfloat162float(x[j * to_next + step]); }
+#pragma unroll
+            for (int j = 0; j < kAhead; ++j)
+                if (h0 + j * (kAppWarps - 1) < p.heads) {
+                    x[j * to_next] = __float2bfloat16_rn(u[j] * c - v[j] * s);
+                    x[j * to_next + step] = __float2bfloat16_rn(v[j] * c + u[j] * s);
+                }
         }
     }
 }
 
-// Cached rows of the spans (from position `lo` on), one after the other: latents [total_ctx][ctx_ld], rotated parts [total_ctx][rot_ld].
-__global__ void __launch_bounds__(128) latent_gather_kernel(const LatentParams p) {
-    pdl_launch_dependents();
-    pdl_wait();
-    const int row = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-    if (row >= p.total_ctx) return;
-    int sp = 0;
-    while (sp + 1 < p.n_spans && p.spans[sp + 1].ctx0 <= row) ++sp;
-    const LatentSpan span = p.spans[sp];
-    const __nv_bfloat16* src = cached_row<__nv_bfloat16>(p, span.seq, span.lo + row - span.ctx0);
-    for (int i = lane; i < p.ctx_ld / 8; i += 32) reinterpret_cast<uint4*>(p.ctx_latent + (size_t)row * p.ctx_ld)[i] = reinterpret_cast<const uint4*>(src)[i];
-    for (int i = lane; i < p.rot_ld / 8; i += 32) reinterpret_cast<uint4*>(p.ctx_rot + (size_t)row * p.rot_ld)[i] = reinterpret_cast<const uint4*>(src + p.row.rp)[i];
-}
-
 // ---- spans: tiled causal attention over expanded keys and values --------------------------------------------------------
-// CTA (tile of 128 query rows of a span, head), 8 warps of 16 query rows; key tiles of 64 through two shared-memory stages.
-constexpr int kPfThreads = 256, kPfKeys = 64;
+// CTA (half a tile of query rows of a span, head), 4 x 2 warps: 16 query rows and every other 32 keys, merged at the end; key tiles of
+// 64 through two shared-memory stages. What bounds it: the chain of products, softmax and products of one warp per key tile; a portion has
+// few tiles, so that SMs are there for halves of them. 497 rows x 16 heads (us under ncu): 47 with whole tiles on 64 CTAs, 46 with halves,
+// 30 with a chunk's addresses worked out once, 26 with the keys over two warps.
+constexpr int kPfRows = kLatentQueryTile / 2, kPfThreads = kPfRows * 4, kPfKeys = 64;
 template <int KQ, int NV>
 constexpr size_t latent_prefill_smem() {
-    return (size_t)2 * kPfKeys * ((KQ * 16 + 8) + (NV * 16 + 8)) * 2 + (size_t)kLatentQueryTile * (KQ * 16 + 8) * 2;
+    return (size_t)2 * kPfKeys * ((KQ * 16 + 8) + (NV * 16 + 8)) * 2 + (size_t)kPfRows * (KQ * 16 + 8) * 2;
 }
 template <int KQ, int NV>   // 16-column steps of query / key rows, 16-column steps of value rows
 __global__ void __launch_bounds__(kPfThreads, 1) latent_prefill_kernel(const LatentParams p) {
@@ -694,30 +722,35 @@ __global__ void __launch_bounds__(kPfThreads, 1) latent_prefill_kernel(const Lat
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3, h = blockIdx.y;
     const int dim_p = (p.dim + 15) & ~15;
     // zeros in the padding columns of both stages and of the query tile, written once
-    for (int i = tid; i < 2 * STAGE / 8; i += kPfThreads) reinterpret_cast<uint4*>(kv_sm)[i] = make_uint4(0, 0, 0, 0);
-    for (int i = tid; i < kLatentQueryTile * PK / 8; i += kPfThreads) reinterpret_cast<uint4*>(q_sm)[i] = make_uint4(0, 0, 0, 0);
+    if (p.dim != dim_p || dim_p + p.row.rot != KQ * 16 || p.vdim != NV * 16) {
+        for (int i = tid; i < 2 * STAGE / 8; i += kPfThreads) reinterpret_cast<uint4*>(kv_sm)[i] = make_uint4(0, 0, 0, 0);
+        for (int i = tid; i < kPfRows * PK / 8; i += kPfThreads) reinterpret_cast<uint4*>(q_sm)[i] = make_uint4(0, 0, 0, 0);
+    }
     pdl_launch_dependents();
     __syncthreads();
     pdl_wait();
-    const int2 tile = p.tiles[blockIdx.x];
+    const int2 tile = p.tiles[blockIdx.x >> 1];   // (the longest first: the second half of a tile before the first)
     const LatentSpan span = p.spans[tile.x];
-    const int q0 = tile.y * kLatentQueryTile, nq = min(kLatentQueryTile, span.count - q0);
+    const int q0 = tile.y * kLatentQueryTile + (blockIdx.x & 1 ? 0 : kPfRows), nq = min(kPfRows, span.count - q0);
+    if (nq <= 0) return;
     const int first_pos = span.pos0 + q0, last_pos = first_pos + nq - 1;
     const int kt0 = first_seen(p, first_pos) / kPfKeys, n_tiles = last_pos / kPfKeys + 1;   // key tiles the first row sees from, and all
     const int cd = p.dim >> 3, cr = p.row.rot >> 3, cv = p.vdim >> 3;
-    // 16-byte chunk tid, tid + 256, ... of a tile as (row, chunk of the row), without divisions in the loop
-    const int per_row = cd + cr + cv, r_first = tid / per_row, c_first = tid - r_first * per_row, r_step = kPfThreads / per_row, c_step = kPfThreads - r_step * per_row;
+    // a thread brings the same 16-byte chunk of every rows_at-th row: where it lies and where it goes is known once (worked out for every
+    // chunk, with a branch between keys, rotated parts and values, that took longer than the products)
+    const int per_row = cd + cr + cv, rows_at = kPfThreads / per_row, r_first = tid / per_row, c_own = tid - r_first * per_row;
+    const bool is_v = c_own >= cd + cr, is_k = c_own < cd;
+    const int c_part = is_k ? c_own : is_v ? c_own - cd - cr : c_own - cd;
+    const __nv_bfloat16* const src0 = (is_k ? p.ctx_k + (size_t)h * p.dim : is_v ? p.ctx_v + (size_t)h * p.vdim : p.ctx_rot) + 8 * c_part;
+    const int src_ld = is_k ? p.heads * p.dim : is_v ? p.heads * p.vdim : p.rot_ld;
+    const unsigned dst_ld = (is_v ? PV : PK) * 2, dst0 = smem_u32(kv_sm) + (is_v ? kPfKeys * PK + 8 * c_part : is_k ? 8 * c_part : dim_p + 8 * c_part) * 2 + r_first * dst_ld;
     auto load_tile = [&](int kt, int stage) {
-        __nv_bfloat16* ks = kv_sm + stage * STAGE;
-        __nv_bfloat16* vs = ks + kPfKeys * PK;
-        for (int r = r_first, c = c_first; r < kPfKeys; r += r_step + (c + c_step >= per_row), c += c_step - (c + c_step >= per_row ? per_row : 0)) {
-            const size_t row = span.ctx0 + min(kt * kPfKeys + r, last_pos) - span.lo;
-            const __nv_bfloat16* src;
-            __nv_bfloat16* dst;
-            if (c < cd) { src = p.ctx_k + row * ((size_t)p.heads * p.dim) + (size_t)h * p.dim + 8 * c; dst = ks + r * PK + 8 * c; }
-            else if (c < cd + cr) { src = p.ctx_rot + row * p.rot_ld + 8 * (c - cd); dst = ks + r * PK + dim_p + 8 * (c - cd); }
-            else { src = p.ctx_v + row * ((size_t)p.heads * p.vdim) + (size_t)h * p.vdim + 8 * (c - cd - cr); dst = vs + r * PV + 8 * (c - cd - cr); }
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+        if (r_first < rows_at) {
+            const int at = span.ctx0 - span.lo + kt * kPfKeys, limit = last_pos - kt * kPfKeys;   // (rows past the last repeat it)
+            unsigned dst = dst0 + stage * (STAGE * 2);
+#pragma unroll 4
+            for (int r = r_first; r < kPfKeys; r += rows_at, dst += rows_at * dst_ld)
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src0 + (size_t)(at + min(r, limit)) * src_ld) : "memory");
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
@@ -732,8 +765,9 @@ __global__ void __launch_bounds__(kPfThreads, 1) latent_prefill_kernel(const Lat
     }
     load_tile(kt0, kt0 & 1);   // one group with the query rows
     unsigned qa[KQ][4];
-    const int pos_a = first_pos + warp * 16 + g, pos_b = pos_a + 8;   // positions of this lane's two rows
-    const int warp_first = first_pos + warp * 16, warp_last = min(warp_first + 15, last_pos);
+    const int rows_of = (warp & 3) * 16, keys_of = (warp >> 2) * (kPfKeys / 2);
+    const int pos_a = first_pos + rows_of + g, pos_b = pos_a + 8;   // positions of this lane's two rows
+    const int warp_first = first_pos + rows_of, warp_last = min(warp_first + 15, last_pos);
     float m_a = -INFINITY, m_b = -INFINITY, l_a = 0.f, l_b = 0.f;
     float oacc[2 * NV][4];
 #pragma unroll
@@ -749,29 +783,39 @@ __global__ void __launch_bounds__(kPfThreads, 1) latent_prefill_kernel(const Lat
         __syncthreads();
         if (kt == kt0) {
 #pragma unroll
-            for (int k = 0; k < KQ; ++k) lat_ldsm(qa[k], smem_u32(q_sm) + (unsigned)((warp * 16 + (lane & 15)) * PK + 16 * k + 8 * (lane >> 4)) * 2u);
+            for (int k = 0; k < KQ; ++k) lat_ldsm(qa[k], smem_u32(q_sm) + (unsigned)((rows_of + (lane & 15)) * PK + 16 * k + 8 * (lane >> 4)) * 2u);
         }
-        if (warp_first <= last_pos && kt * kPfKeys <= warp_last && (kt + 1) * kPfKeys > warp_seen) {
-            const unsigned kb = smem_u32(kv_sm + (kt & 1) * STAGE), vb = kb + (unsigned)(kPfKeys * PK) * 2u;
-            float sacc[8][4];
+        const int key0 = kt * kPfKeys + keys_of, key_end = key0 + kPfKeys / 2;
+        if (warp_first <= last_pos && key0 <= warp_last && key_end > warp_seen) {
+            const unsigned kb = smem_u32(kv_sm + (kt & 1) * STAGE), vb = kb + (unsigned)(kPfKeys * PK) * 2u;   // of the tile
+            float sacc[4][4];
 #pragma unroll
-            for (int j = 0; j < 8; ++j) sacc[j][0] = sacc[j][1] = sacc[j][2] = sacc[j][3] = 0.f;
+            for (int j = 0; j < 4; ++j) sacc[j][0] = sacc[j][1] = sacc[j][2] = sacc[j][3] = 0.f;
+            {   // the next 16 columns' keys are on their way while these are multiplied
+                const unsigned krow = kb + (unsigned)((keys_of + (lane & 7) + 8 * (lane >> 4)) * PK + 8 * ((lane >> 3) & 1)) * 2u;
+                unsigned b[2][2][4];
 #pragma unroll
-            for (int k = 0; k < KQ; ++k)
+                for (int jp = 0; jp < 2; ++jp) lat_ldsm(b[0][jp], krow + (unsigned)(jp * 16 * PK) * 2u);
 #pragma unroll
-                for (int jp = 0; jp < 4; ++jp) {
-                    unsigned b[4];
-                    lat_ldsm(b, kb + (unsigned)((jp * 16 + (lane & 7) + 8 * (lane >> 4)) * PK + 16 * k + 8 * ((lane >> 3) & 1)) * 2u);
-                    lat_mma(sacc[2 * jp], qa[k], b[0], b[1]);
-                    lat_mma(sacc[2 * jp + 1], qa[k], b[2], b[3]);
+                for (int k = 0; k < KQ; ++k) {
+                    if (k + 1 < KQ) {
+#pragma unroll
+                        for (int jp = 0; jp < 2; ++jp) lat_ldsm(b[(k + 1) & 1][jp], krow + (unsigned)(jp * 16 * PK + 16 * (k + 1)) * 2u);
+                    }
+#pragma unroll
+                    for (int jp = 0; jp < 2; ++jp) {
+                        lat_mma(sacc[2 * jp], qa[k], b[k & 1][jp][0], b[k & 1][jp][1]);
+                        lat_mma(sacc[2 * jp + 1], qa[k], b[k & 1][jp][2], b[k & 1][jp][3]);
+                    }
                 }
-            const bool edge = (kt + 1) * kPfKeys - 1 > warp_first || kt * kPfKeys < full_from;   // some row does not see the whole tile
+            }
+            const bool edge = key_end - 1 > warp_first || key0 < full_from;   // some row does not see all of these keys
             float mx_a = -INFINITY, mx_b = -INFINITY;
 #pragma unroll
-            for (int j = 0; j < 8; ++j)
+            for (int j = 0; j < 4; ++j)
 #pragma unroll
                 for (int e = 0; e < 2; ++e) {
-                    const int key = kt * kPfKeys + 8 * j + 2 * t + e;
+                    const int key = key0 + 8 * j + 2 * t + e;
                     const float a = !edge || (key <= pos_a && key >= seen_a) ? sacc[j][e] * p.scale_log2 : -INFINITY;
                     const float b = !edge || (key <= pos_b && key >= seen_b) ? sacc[j][2 + e] * p.scale_log2 : -INFINITY;
                     sacc[j][e] = a; sacc[j][2 + e] = b;
@@ -787,7 +831,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) latent_prefill_kernel(const Lat
             m_a = mn_a; m_b = mn_b;
             float sa = 0.f, sb = 0.f;
 #pragma unroll
-            for (int j = 0; j < 8; ++j)
+            for (int j = 0; j < 4; ++j)
 #pragma unroll
                 for (int e = 0; e < 2; ++e) {
                     sacc[j][e] = exp2f(sacc[j][e] - ra); sa += sacc[j][e];
@@ -798,8 +842,15 @@ __global__ void __launch_bounds__(kPfThreads, 1) latent_prefill_kernel(const Lat
 #pragma unroll
                 for (int j = 0; j < 2 * NV; ++j) { oacc[j][0] *= ca; oacc[j][1] *= ca; oacc[j][2] *= cb; oacc[j][3] *= cb; }
             }
+            // (16 keys, 32 columns of values) per step, the next step's values on their way; the halves of a weight that share a result lie
+            // four products apart
+            constexpr int JW = NV % 2 ? 1 : 2, STEPS = NV / JW;
+            const unsigned vrow = vb + (unsigned)((keys_of + (lane & 7) + 8 * ((lane >> 3) & 1)) * PV + 8 * (lane >> 4)) * 2u;
+            unsigned bv[2][JW][4];
 #pragma unroll
-            for (int kk = 0; kk < 4; ++kk) {
+            for (int w = 0; w < JW; ++w) lat_ldsm_trans(bv[0][w], vrow + (unsigned)(16 * w) * 2u);
+#pragma unroll
+            for (int kk = 0; kk < 2; ++kk) {
                 unsigned ah[4], al[4];
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {   // (row g, keys 0-7), (row g + 8, keys 0-7), (row g, keys 8-15), (row g + 8, keys 8-15)
@@ -809,13 +860,19 @@ __global__ void __launch_bounds__(kPfThreads, 1) latent_prefill_kernel(const Lat
                     al[e] = lat_pack(x - xh, y - yh);
                 }
 #pragma unroll
-                for (int j = 0; j < NV; ++j) {
-                    unsigned b[4];
-                    lat_ldsm_trans(b, vb + (unsigned)((16 * kk + (lane & 7) + 8 * ((lane >> 3) & 1)) * PV + 16 * j + 8 * (lane >> 4)) * 2u);
-                    lat_mma(oacc[2 * j], ah, b[0], b[1]);
-                    lat_mma(oacc[2 * j], al, b[0], b[1]);
-                    lat_mma(oacc[2 * j + 1], ah, b[2], b[3]);
-                    lat_mma(oacc[2 * j + 1], al, b[2], b[3]);
+                for (int st = 0; st < STEPS; ++st) {
+                    const int at = kk * STEPS + st, next = at + 1;
+                    if (next < 2 * STEPS) {
+#pragma unroll
+                        for (int w = 0; w < JW; ++w) lat_ldsm_trans(bv[next & 1][w], vrow + (unsigned)(16 * (next / STEPS) * PV + 16 * (next % STEPS * JW + w)) * 2u);
+                    }
+#pragma unroll
+                    for (int half = 0; half < 2; ++half)
+#pragma unroll
+                        for (int w = 0; w < JW; ++w) {
+                            lat_mma(oacc[2 * (st * JW + w)], half ? al : ah, bv[at & 1][w][0], bv[at & 1][w][1]);
+                            lat_mma(oacc[2 * (st * JW + w) + 1], half ? al : ah, bv[at & 1][w][2], bv[at & 1][w][3]);
+                        }
                 }
             }
         }
@@ -824,10 +881,30 @@ __global__ void __launch_bounds__(kPfThreads, 1) latent_prefill_kernel(const Lat
     asm volatile("cp.async.wait_group 0;" ::: "memory");
 #pragma unroll
     for (int o = 1; o < 4; o <<= 1) { l_a += __shfl_xor_sync(0xffffffffu, l_a, o); l_b += __shfl_xor_sync(0xffffffffu, l_b, o); }
+    {   // the two warps of a row: the second one's sums through shared memory (the loop ends with a barrier)
+        float* const other = reinterpret_cast<float*>(pf_raw) + (size_t)((warp & 3) * 32 + lane);
+        if (warp >= 4) {
+            other[0] = m_a; other[128] = m_b; other[256] = l_a; other[384] = l_b;
+#pragma unroll
+            for (int j = 0; j < 2 * NV; ++j)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) other[(4 + 4 * j + e) * 128] = oacc[j][e];
+        }
+        __syncthreads();
+        if (warp >= 4) return;
+        const float o_a = other[0], o_b = other[128], t_a = fmaxf(m_a, o_a), t_b = fmaxf(m_b, o_b);   // (every row sees its own key: the larger one is finite)
+        const float fa = exp2f(m_a - t_a), fb = exp2f(m_b - t_b), ga = exp2f(o_a - t_a), gb = exp2f(o_b - t_b);
+        m_a = t_a; m_b = t_b;
+        l_a = l_a * fa + other[256] * ga; l_b = l_b * fb + other[384] * gb;
+#pragma unroll
+        for (int j = 0; j < 2 * NV; ++j)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) oacc[j][e] = oacc[j][e] * (e < 2 ? fa : fb) + other[(4 + 4 * j + e) * 128] * (e < 2 ? ga : gb);
+    }
     const float sink = sink_log2(p, h);
 #pragma unroll
     for (int half = 0; half < 2; ++half) {
-        const int rr = warp * 16 + g + 8 * half;
+        const int rr = rows_of + g + 8 * half;
         if (rr >= nq) continue;
         const int row = span.row0 + q0 + rr;
         const float gate = p.gate ? 1.0f / (1.0f + expf(-p.gate[(size_t)row * p.gate_stride + h])) : 1.0f;
@@ -921,10 +998,8 @@ int launch_long(const LatentLaunch& a, cudaStream_t s, int* launches) {
     p.ctx_v = reinterpret_cast<__nv_bfloat16*>(a.expand + l.v);
     cudaError_t e;
     if (!a.only_attention) {
-        e = launch_k(latent_append_kernel, dim3(a.n_long), dim3(128), 0, s, p);
+        e = launch_k(latent_append_kernel, dim3(a.n_long + (a.total_ctx > a.n_long ? (a.total_ctx + kAppWarps - 1) / kAppWarps : 0)), dim3(kAppWarps * 32), 0, s, p);
         if (e != cudaSuccess) return cuda_fail(e, "latent append launch");
-        e = launch_k(latent_gather_kernel, dim3((a.total_ctx + 3) / 4), dim3(128), 0, s, p);
-        if (e != cudaSuccess) return cuda_fail(e, "latent gather launch");
         ProductLaunch x;
         x.w = a.ukv; x.m = a.total_ctx; x.x = p.ctx_latent; x.x_stride = l.ctx_ld;
         x.out.count = 2;
@@ -934,9 +1009,9 @@ int launch_long(const LatentLaunch& a, cudaStream_t s, int* launches) {
         x.status = a.status;
         const int rc = launch_product(x, s);
         if (rc) return rc;
-        *launches += 3;
+        *launches += 2;
     }
-    const dim3 grid(a.n_tiles, a.heads);
+    const dim3 grid(2 * a.n_tiles, a.heads);
     switch (prefill_form(a.dim, a.row.rot, a.vdim)) {
     case PF_SMALL: e = launch_k(latent_prefill_kernel<4, 5>, grid, dim3(kPfThreads), latent_prefill_smem<4, 5>(), s, p); break;
     case PF_MEDIUM: e = launch_k(latent_prefill_kernel<8, 8>, grid, dim3(kPfThreads), latent_prefill_smem<8, 8>(), s, p); break;

@@ -476,7 +476,7 @@ size_t latent_expand_bytes(const LatentRow& r, int heads, int dim, int vdim, int
 // can rows of this layer be attended in spans over expanded keys and values?
 bool latent_expands(const LatentRow& r, int dim, int vdim, bool f32);
 constexpr int kLatentQueryTile = 128;
-// launches (for the counters): short part 3, span part 4
+// launches (for the counters): short part 3, span part 3
 int launch_latent(const LatentLaunch& a, cudaStream_t s, int* launches);
 
 // ---- the residual stream between sublayers (stream_join.cu) ------------------------------------------------------------
