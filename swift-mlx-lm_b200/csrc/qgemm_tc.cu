@@ -28,7 +28,8 @@
 // 509 us, 10.7 TB/s), 512 arrivals per group, eight MMAs issued by a lone lane (470 to 850 clocks), and two waves of CTAs, the second
 // half empty. What bounds it now: the MMAs of the long form (about 0.65 of their rate under the power cap), dequantising in the short one.
 // Measured: 14336 x 4096 at 512 rows 88 -> 63 us (950 TFLOP/s); 28672 x 4096 at 2048 rows 705 us under ncu -> 442 us (1090 TFLOP/s);
-// 28672 x 4096 at 41 rows 68 us under ncu -> 38 us; 14336 -> 4096 at 41 rows 50.7 + 8.8 (a second launch) -> 30 us.
+// 28672 x 4096 at 41 rows 68 us under ncu -> 38 us (28 with the form of few rows); 14336 -> 4096 at 41 rows 50.7 + 8.8 (a second
+// launch) -> 30 us (23.5).
 //
 // Every mbarrier wait is bounded: on expiry an error word is set, the CTA stops issuing, waits (bounded) for the copies and MMAs
 // it has in flight, frees its TMEM and returns.
@@ -60,12 +61,12 @@ struct QGemmTcParams {
     const uint4* tiles;       // [row tile][k-tile][32 lanes], see Q4Tiled
     const unsigned* sb;       // [row tile][k-tile / 4][16 rows][4] pairs
     int row_tiles, kt;        // row tiles, k-tiles (groups of 64, a multiple of four)
-    int g_pad;                // columns of one plane of appended group sums
     const float* rscale;      // [m]: the inverse of each row's power of two
     int m;
     int real_steps, steps;    // steps over the weights; those over the appended columns follow
     int tok_tiles, n_tiles;   // long form: tiles of 256 rows, all tiles
     int splits;               // short form: CTAs of a cluster along K
+    int whole, left;          // few rows: passes of eight row tiles per CTA; row tiles of the last one
     int gated, gated_act;     // rows 0-7 of a row tile are gate rows, rows 8-15 the up rows that belong to them
     TcSegments out;           // weight rows [end[q-1], end[q]) go to out.y[q][token][row - end[q-1]]
     int* status;              // set non-zero when a bounded wait expired
@@ -144,6 +145,7 @@ struct RingPos {
     int s = 0; unsigned par = 0;
     __device__ __forceinline__ void next() { if (++s == N) { s = 0; par ^= 1u; } }
     __device__ __forceinline__ void skip2() { s += 2; if (s >= N) { s -= N; par ^= 1u; } }
+    __device__ __forceinline__ void skip3() { s += 3; if (s >= N) { s -= N; par ^= 1u; } }
 };
 
 template <int STAGES>
@@ -238,25 +240,27 @@ __device__ __forceinline__ void tc_unpack(const uint4& wq, __half2 lo, __half2 h
             a[4 * j + r] = *reinterpret_cast<const unsigned*>(&h);
         }
 }
-// The A operand of 64 appended columns from col0 on (counted from the first of them): c = 64 (zero + 8 scale) as an fp16 pair
-// (hi, lo); plane 0 carries c_hi (against sum_hi), plane 1 c_lo (against sum_hi), plane 2 c_hi (against sum_lo). The activation
-// side holds sum / 64 so that neither factor leaves fp16's range.
+// The A operand of 64 appended columns, block `blk` of them: c = 64 (zero + 8 scale) of 64 groups as an fp16 pair (hi, lo). Of three
+// blocks one after the other the first carries c_hi (against sum_hi), the second c_lo (against sum_hi), the third c_hi (against sum_lo).
+// The activation side holds sum / 64 so that neither factor leaves fp16's range.
 template <bool F16SB>
-__device__ __forceinline__ void tc_appended(const QGemmTcParams& p, int rt, int col0, unsigned (&a)[16]) {
+__device__ __forceinline__ float tc_const(unsigned pair) { return 64.0f * fmaf(8.0f, tc_scale<F16SB>(pair), tc_zero<F16SB>(pair)); }
+template <bool F16SB>
+__device__ __forceinline__ void tc_appended(const QGemmTcParams& p, int rt, int blk, unsigned (&a)[16]) {
     const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-    const int plane = col0 / p.g_pad, st0 = (col0 - plane * p.g_pad) >> 2;   // four groups per 16-byte entry
+    const int plane = blk % 3, st0 = blk / 3 * 16;   // four groups per 16-byte entry
 #pragma unroll
     for (int j = 0; j < 4; ++j)
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             const int st = st0 + 4 * j + t;
             uint4 v = make_uint4(0, 0, 0, 0);
-            if (rt < p.row_tiles && plane < 3 && st < p.kt / 4) v = __ldg(reinterpret_cast<const uint4*>(p.sb) + ((size_t)rt * (p.kt / 4) + st) * 16 + g + 8 * h);
+            if (rt < p.row_tiles && st < p.kt / 4) v = __ldg(reinterpret_cast<const uint4*>(p.sb) + ((size_t)rt * (p.kt / 4) + st) * 16 + g + 8 * h);
             const unsigned u[4] = {v.x, v.y, v.z, v.w};
             float c[4];
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
-                const float cf = 64.0f * fmaf(8.0f, tc_scale<F16SB>(u[i]), tc_zero<F16SB>(u[i])), hi = __half2float(__float2half_rn(cf));
+                const float cf = tc_const<F16SB>(u[i]), hi = __half2float(__float2half_rn(cf));
                 c[i] = plane == 1 ? cf - hi : hi;
             }
 #pragma unroll
@@ -265,6 +269,30 @@ __device__ __forceinline__ void tc_appended(const QGemmTcParams& p, int rt, int 
                 a[4 * j + 2 * h + i] = *reinterpret_cast<const unsigned*>(&pr);
             }
         }
+}
+// c_hi and c_lo of 64 groups of a row tile at once
+template <bool F16SB>
+__device__ __forceinline__ void tc_appended_pair(const QGemmTcParams& p, int rt, int block, unsigned (&hi)[16], unsigned (&lo)[16]) {
+    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    uint4 v[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int st = block * 16 + 4 * (i >> 1) + t;
+        v[i] = st < p.kt / 4 ? __ldg(reinterpret_cast<const uint4*>(p.sb) + ((size_t)rt * (p.kt / 4) + st) * 16 + g + 8 * (i & 1)) : make_uint4(0, 0, 0, 0);
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const unsigned u[4] = {v[i].x, v[i].y, v[i].z, v[i].w};
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const float c0 = tc_const<F16SB>(u[2 * e]), c1 = tc_const<F16SB>(u[2 * e + 1]);
+            const __half2 h = __floats2half2_rn(c0, c1);
+            const float2 f = __half22float2(h);
+            const __half2 l = __floats2half2_rn(c0 - f.x, c1 - f.y);
+            hi[2 * i + e] = *reinterpret_cast<const unsigned*>(&h);
+            lo[2 * i + e] = *reinterpret_cast<const unsigned*>(&l);
+        }
+    }
 }
 
 // Everything a dequantising warp does: the steps [lo, hi) of tiles `tile`, `tile` + stride, ... below `end`, of all of which it takes
@@ -365,7 +393,7 @@ __device__ __forceinline__ bool tc_dequant(const QGemmTcParams& p, TcBars<STAGES
 #pragma unroll 1
             for (int half = 0; half < 2; ++half) {
                 unsigned a[16];
-                tc_appended<F16SB>(p, rt_of(tile) + own_rt, (kt - p.real_steps) * kTcStep + half * 64, a);
+                tc_appended<F16SB>(p, rt_of(tile) + own_rt, (kt - p.real_steps) * (kTcStep / 64) + half, a);
                 tmem_st_frag(a_dst + (unsigned)a_slot * 64u + half * 32u, a);
             }
             if (!finish()) ok = false;
@@ -377,8 +405,7 @@ __device__ __forceinline__ bool tc_dequant(const QGemmTcParams& p, TcBars<STAGES
 
 // Where a lane's results go: its weight row of one output, or the row of a gate row and its up row together.
 struct TcDst { __nv_bfloat16* y; int stride; bool live; };
-__device__ __forceinline__ TcDst tc_dst(const QGemmTcParams& p, int row0) {
-    const int lane = threadIdx.x & 31, row = row0 + lane;
+__device__ __forceinline__ TcDst tc_dst(const QGemmTcParams& p, int row) {
     if (p.gated) { const int r = (row >> 4) * 8 + (row & 7); return {p.out.y[0] + r, p.out.stride[0], r < p.out.end[0]}; }
     const int q = row < p.out.end[0] ? 0 : row < p.out.end[1] ? 1 : 2;
     return {(q == 0 ? p.out.y[0] : q == 1 ? p.out.y[1] : p.out.y[2]) + (row - (q == 0 ? 0 : q == 1 ? p.out.end[0] : p.out.end[1])),
@@ -531,7 +558,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__((kTcDeqWarps + 2 + k
         pdl_wait();   // (the rows' factors)
         for (int tile = first; tile < p.n_tiles; tile += pairs, par ^= 1u) {
             const int tok0 = tile % p.tok_tiles * 256 + half * 128;
-            const TcDst dst = tc_dst(p, tile / p.tok_tiles * 256 + rank * kTcRows + (warp & 3) * 32);
+            const TcDst dst = tc_dst(p, tile / p.tok_tiles * 256 + rank * kTcRows + (warp & 3) * 32 + lane);
             float fac = tc_rscale(p, min(tok0 + lane, p.m - 1));   // of 32 tokens, one per lane, requested before they are needed
             if (!mbar_wait_warp(&bars.acc_full, par)) { tc_fail(p.status, &bars.failed, 4); break; }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -561,12 +588,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__((kTcDeqWarps + 2 + k
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_d), "r"(kTmemCols) : "memory");
 }
 
-// ---- short kernel: few activation rows, or few tiles. K is cut over the CTAs of a cluster; each sends its part of a tile's results
+// ---- short form: 65 to 128 activation rows, or few tiles. K is cut over the CTAs of a cluster; each sends its part of a tile's results
 // to the CTA that finishes a row, through distributed shared memory (the ring's, which is free by then). ---------------------------
-template <int BN, int STAGES, int PER_SM, bool F16SB>
-__global__ void __launch_bounds__((kTcDeqWarps + 2) * 32, PER_SM) qgemm_tc_short_kernel(const QGemmTcParams p, const __grid_constant__ CUtensorMap xmap) {
-    constexpr unsigned kTmemCols = PER_SM == 1 ? 512 : 256;
-    constexpr int SA = (int)(kTmemCols - BN) / 64 > kTcMaxA ? kTcMaxA : (int)(kTmemCols - BN) / 64;   // what two CTAs of an SM have room for
+template <int BN, int STAGES, bool F16SB>
+__global__ void __launch_bounds__((kTcDeqWarps + 2) * 32, 1) qgemm_tc_short_kernel(const QGemmTcParams p, const __grid_constant__ CUtensorMap xmap) {
+    constexpr unsigned kTmemCols = 512;                      // accumulator, four weight tiles
+    constexpr int SA = kTcMaxA;
+    static_assert(BN + SA * 64 <= 512, "tensor memory");
     constexpr unsigned STAGE_BYTES = BN * 256;
     static_assert((size_t)STAGES * STAGE_BYTES >= (size_t)BN * kTcRows * 4, "the ring takes what the cluster sends");
     extern __shared__ __align__(1024) unsigned char smem_raw[];
@@ -623,7 +651,7 @@ __global__ void __launch_bounds__((kTcDeqWarps + 2) * 32, PER_SM) qgemm_tc_short
     if (!done && lane == 0) tc_fail(p.status, &bars.failed, 5);
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const int r = (warp & 3) * 32 + lane;
-    constexpr int CW = 16;                          // columns per read; with 32 columns two of a quarter's four warps read
+    constexpr int CW = 16;                          // columns per read
     const cg::cluster_group cluster = cg::this_cluster();
     if (p.splits > 1) cluster.sync();               // every ring of the cluster is free
     const int own = BN / p.splits;                  // columns that a CTA of the cluster finishes
@@ -634,7 +662,7 @@ __global__ void __launch_bounds__((kTcDeqWarps + 2) * 32, PER_SM) qgemm_tc_short
             unsigned v[CW];
             tmem_ld16(tmem_d + ((unsigned)((warp & 3) * 32) << 16) + (unsigned)c0, v);
             if (p.splits == 1) {
-                tc_emit16(p, tc_dst(p, row0 + (warp & 3) * 32), v, tc_rscale(p, min(tok0 + c0 + (lane & 15), p.m - 1)), 0, tok0 + c0);
+                tc_emit16(p, tc_dst(p, row0 + r), v, tc_rscale(p, min(tok0 + c0 + (lane & 15), p.m - 1)), 0, tok0 + c0);
                 continue;
             }
 #pragma unroll
@@ -668,14 +696,337 @@ __global__ void __launch_bounds__((kTcDeqWarps + 2) * 32, PER_SM) qgemm_tc_short
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_d), "r"(kTmemCols) : "memory");
 }
 
+// ---- few activation rows (up to 64): a persistent CTA per SM, or a cluster of two along K ------------------------------------------
+// What bounds it: the dequantising warps (about 330 instructions per 4096 weights; without the subtractions and multiplications a pass of
+// eight row tiles would take 0.45 us per step instead of 0.6), before that what surrounds them: in steps of 128 x 128 with a wait, a
+// fetch and an arrival for each, appended columns worked out three times, two CTAs on some SMs and one on others, 28672 x 4096 at 41 rows
+// took 34 us, 128256 x 4096 139, 4096 x 14336 25, 6144 x 4096 17.7. Now 28, 87, 23.5 and 12. Hence
+//   * a unit of work is 16 weight rows x 256 columns, the streaming layout's contiguous 2304 bytes: addresses by addition, one wait, one
+//     arrival and one set of scales for 16 words of nibbles per lane. A warp reads a unit into registers and requests the next but one in
+//     its place;
+//   * row tiles (16 rows) are dealt to the SMs one by one: passes of eight per SM over one contiguous window of the matrix, what is left
+//     evenly. Row tile j of a pass takes lanes 32 (j & 3) + 16 (j >> 2) of tensor memory, so that four already occupy all four schedulers
+//     (a warp reaches the lanes of its quarter only); six warps per quarter, three steps of two row tiles;
+//   * two accumulators: four warps of their own store a pass while the next one is multiplied;
+//   * the wait for a step's activations is made by a dequantising warp, so that the MMA warp has one wait per step (16 MMAs at 30 clocks,
+//     about 200 for a wait). CTAs that start at different places of K, so as not to ask for the same activations at the same time, took
+//     longer (12 -> 19 us for 4096 x 4096).
+// K over a cluster (few row tiles, long K): one pass, the parts meet in distributed shared memory.
+constexpr int kSlCols = 256;                    // columns of K per step
+constexpr int kSlWarps = 24;                    // dequantising: six of a quarter, three steps of two row tiles
+constexpr int kSlAhead = 2;                     // units of a warp in its ring, behind the one in its registers
+constexpr int kSlUnitBytes = 4 * 512 + 256;     // four 16 x 64 tiles and 16 rows' four scale / zero pairs
+constexpr int kSlRingBytes = kSlWarps * kSlAhead * kSlUnitBytes;
+constexpr int kSlSlots = 3;                     // dequantised 128 x 256 tiles in tensor memory, 128 columns each
+constexpr int kSlEpiWarps = 4;
+constexpr int kSlThreads = (kSlWarps + 2 + kSlEpiWarps) * 32;
+
+template <int STAGES>
+struct SlBars {
+    unsigned long long full[STAGES], empty[STAGES];        // activations of a step
+    unsigned long long ready[kSlSlots], free[kSlSlots];    // a weight tile is in tensor memory (eight arrivals); its MMAs are done
+    unsigned long long acc_full[2], acc_empty[2];
+    unsigned tmem;
+    int failed;
+};
+// row tiles of this CTA (group of them along K) in pass `pass`: the first and how many
+struct SlPass { int first, count; };
+__device__ __forceinline__ SlPass sl_pass(const QGemmTcParams& p, int pass, int cta, int ctas) {
+    if (pass < p.whole) return {(pass * ctas + cta) * 8, 8};
+    const int lo = (int)((unsigned)(p.left * cta) / (unsigned)ctas);   // (left < 8 ctas)
+    return {p.whole * ctas * 8 + lo, (int)((unsigned)(p.left * (cta + 1)) / (unsigned)ctas) - lo};
+}
+
+template <int BN, int STAGES, bool F16SB>
+__global__ void __launch_bounds__(kSlThreads, 1) qgemm_slab_kernel(const QGemmTcParams p, const __grid_constant__ CUtensorMap xmap) {
+    constexpr unsigned kTmemCols = 512;                    // accumulators 2 BN, weight tiles 3 x 128
+    static_assert(2 * BN + kSlSlots * 128 <= 512, "tensor memory");
+    constexpr unsigned STAGE_BYTES = BN * kSlCols * 2, HALF = BN * 128;   // (boxes of 64 columns)
+    static_assert((size_t)STAGES * STAGE_BYTES >= (size_t)BN * kTcRows * 4, "the ring takes what the cluster sends");
+    extern __shared__ __align__(1024) unsigned char smem_raw[];
+    unsigned char* const ring_ptr = smem_raw + ((1024 - (smem_u32(smem_raw) & 1023)) & 1023);
+    const unsigned ring = smem_u32(ring_ptr);
+    __shared__ __align__(8) SlBars<STAGES> bars;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int rank = (int)blockIdx.x % p.splits, cta = (int)blockIdx.x / p.splits, ctas = (int)gridDim.x / p.splits;
+    const int lo = p.steps * rank / p.splits, hi = p.steps * (rank + 1) / p.splits, steps = hi - lo;
+    const int passes = p.n_tiles;
+    const int real = max(0, min(hi, p.real_steps) - lo);   // steps over weights; those over appended columns, 192 of them each, follow
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < STAGES; ++s) { mbar_init(&bars.full[s], 1); mbar_init(&bars.empty[s], 1); }
+        for (int s = 0; s < kSlSlots; ++s) { mbar_init(&bars.ready[s], 8); mbar_init(&bars.free[s], 1); }
+        for (int s = 0; s < 2; ++s) { mbar_init(&bars.acc_full[s], 1); mbar_init(&bars.acc_empty[s], kSlEpiWarps); }
+        bars.failed = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 0) {
+        __syncwarp();
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&bars.tmem)), "r"(kTmemCols) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const unsigned tmem_d = bars.tmem, tmem_a = tmem_d + 2 * BN;
+    pdl_launch_dependents();   // (behind the allocation: a CTA of the next kernel cannot take tensor memory that this one still waits for)
+    volatile int* const failed = &bars.failed;
+
+    if (warp == kSlWarps) {   // ---- MMAs
+        const bool el = elect_one();
+        RingPos<STAGES> at;
+        RingPos<kSlSlots> a;
+        bool ok = true;
+        for (int pass = 0; pass < passes && ok; ++pass) {
+            const int d = pass & 1;
+            if (pass >= 2 && !mbar_wait_warp(&bars.acc_empty[d], (unsigned)((pass >> 1) - 1) & 1u)) { ok = false; break; }   // (stored two passes ago)
+            for (int k = 0; k < steps; ++k) {
+                if (!mbar_wait_warp(&bars.ready[a.s], a.par)) { ok = false; break; }   // (whoever made it ready has waited for the activations)
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                if (el) {
+                    const unsigned b = umma_desc_lo(ring + at.s * STAGE_BYTES);
+#pragma unroll
+                    for (int j = 0; j < kSlCols / 16; ++j)
+                        if (j < 12 || k < real)
+                            umma_f16_ta<1>(tmem_d + d * BN, tmem_a + a.s * 128u + 8u * j, b + (j >> 2) * (HALF / 16) + 2 * (j & 3), umma_idesc(kTcRows, BN), j > 0 || k > 0 ? 1u : 0u);
+                    umma_commit(&bars.empty[at.s]);
+                    umma_commit(&bars.free[a.s]);
+                }
+                __syncwarp();
+                at.next();
+                a.next();
+            }
+            if (ok && el) umma_commit(&bars.acc_full[d]);
+            __syncwarp();
+        }
+        if (!ok) {   // the MMAs issued so far end before tensor memory is freed: an arrival of their own, which nothing else makes
+            if (el) { tc_fail(p.status, &bars.failed, 2); umma_commit(&bars.free[a.s]); }
+            mbar_wait_warp(&bars.free[a.s], a.par);
+        }
+        __syncwarp();
+    } else if (warp == kSlWarps + 1) {   // ---- activations
+        const bool el = elect_one();
+        pdl_wait();                         // they come from the kernel just before this one
+        RingPos<STAGES> at;
+        int issued = 0;
+        const int total = passes * steps;
+        bool ok = true;
+        for (int j = 0; issued < total; ++issued) {
+            const bool whole = j < real;
+            const int x = whole ? (lo + j) * kSlCols : p.real_steps * kSlCols + (lo + j - p.real_steps) * 192;
+            if (issued >= STAGES && !mbar_wait_warp(&bars.empty[at.s], at.par ^ 1u)) { ok = false; break; }
+            if (*failed) { ok = false; break; }
+            if (el) {
+                const unsigned bar = smem_u32(&bars.full[at.s]), stage = ring + at.s * STAGE_BYTES;
+                mbar_expect(bar, whole ? STAGE_BYTES : 3 * HALF);
+#pragma unroll
+                for (int q = 0; q < 4; ++q)
+                    if (q < 3 || whole) tma_load_2d(stage + q * HALF, &xmap, x + q * 64, 0, bar);
+            }
+            __syncwarp();
+            at.next();
+            if (++j == steps) j = 0;
+        }
+        if (!ok && el) tc_fail(p.status, &bars.failed, 3);
+        // every copy has landed before the ring is given to the cluster, or the CTA leaves
+        for (int i = issued > STAGES ? issued - STAGES : 0; i < issued; ++i) mbar_wait_warp(&bars.full[i % STAGES], (unsigned)((i / STAGES) & 1));
+        __syncwarp();
+    } else if (warp < kSlWarps) {   // ---- dequantising warps: quarter warp & 3 of the lanes, number warp >> 2 of the quarter's four
+        const int quarter = warp & 3, number = warp >> 2;
+        const int tile_of = number / 3, first = number - 3 * tile_of;
+        const unsigned ready0 = smem_u32(&bars.ready[0]), free0 = smem_u32(&bars.free[0]), full0 = smem_u32(&bars.full[0]);
+        const unsigned my_ring = ring + STAGES * STAGE_BYTES + warp * (kSlAhead * kSlUnitBytes);
+        const int kt4 = p.kt / 4;
+        const bool lands = warp == 0 || warp == 4 || warp == 8;   // quarter 0's first tile, present in every pass: waits for the step's activations
+        // A warp takes every third step of all passes, and so always the same slot: when it waits for the MMAs of the step three before its
+        // own, it has waited for those of the step six before, the slot's phase before, itself. (A wait by parity cannot tell a phase from
+        // the one two before.) Where the quarter has one row tile or none, in the last pass, its first three warps make the arrivals of
+        // the others.
+        // request side: this warp's units over real weights, in order
+        int f_pass = 0, f_j = first, f_left = 0;   // f_left: units of the tile still to request
+        const uint4* f_w = nullptr;
+        const uint4* f_s = nullptr;
+        auto f_seek = [&]() {   // on to a pass with a tile and units over real weights
+            for (; f_pass < passes; ++f_pass) {
+                const SlPass t = sl_pass(p, f_pass, cta, ctas);
+                const int at_j = f_j;
+                f_j += (steps - f_j + 2) / 3 * 3 - steps;   // its first place in the next pass
+                f_left = at_j < real ? (real - at_j + 2) / 3 : 0;
+                if (quarter + 4 * tile_of < t.count && f_left > 0) {
+                    const size_t at = (size_t)(t.first + quarter + 4 * tile_of) * kt4 + lo + at_j;
+                    f_w = p.tiles + at * 128 + lane;
+                    f_s = reinterpret_cast<const uint4*>(p.sb) + at * 16 + lane;
+                    ++f_pass;
+                    return;
+                }
+            }
+            f_left = 0;
+        };
+        f_seek();
+        auto fetch = [&](unsigned dst) {
+            if (f_left > 0) {
+                asm volatile(
+                    "cp.async.cg.shared.global [%0], [%1], 16;\n"
+                    "cp.async.cg.shared.global [%0+512], [%1+512], 16;\n"
+                    "cp.async.cg.shared.global [%0+1024], [%1+1024], 16;\n"
+                    "cp.async.cg.shared.global [%0+1536], [%1+1536], 16;\n" ::"r"(dst), "l"(f_w) : "memory");
+                if (lane < 16) asm volatile("cp.async.cg.shared.global [%0+2048], [%1], 16;" ::"r"(dst), "l"(f_s) : "memory");
+                f_w += 3 * 128;
+                f_s += 3 * 16;
+                if (--f_left == 0) f_seek();
+            }
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        };
+        unsigned src = my_ring;
+        fetch(my_ring + lane * 16);
+        fetch(my_ring + kSlUnitBytes + lane * 16);
+        RingPos<STAGES> stage;
+        stage.s = first;
+        const unsigned ready_bar = ready0 + 8u * first, free_bar = free0 + 8u * first;
+        unsigned free_par = 1u;        // (of the slot's phase before the first one: over from the start)
+        int j = first;
+        bool ok = true;
+        auto begin = [&]() {   // the MMAs that read this slot are done
+            const bool done = mbar_wait_warp(free_bar, free_par);
+            free_par ^= 1u;
+            return done;
+        };
+        for (int pass = 0; pass < passes && ok; ++pass, j -= steps) {
+            const SlPass t = sl_pass(p, pass, cta, ctas);
+            const bool there = quarter + 4 * tile_of < t.count, alone = quarter + 4 >= t.count;
+            if (alone && tile_of) break;   // (the last pass)
+            const unsigned dst = tmem_a + ((unsigned)(quarter * 32 + tile_of * 16) << 16) + first * 128u;
+            auto finish = [&]() {
+                asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");   // the stores are ordered before the MMAs of the warp that waits
+                if (lands && !mbar_wait_warp(full0 + 8u * stage.s, stage.par)) return false;
+                __syncwarp();
+                if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0], %1;" ::"r"(ready_bar), "r"(alone ? 2 : 1) : "memory");
+                stage.skip3();
+                return true;
+            };
+            if (!there) {
+                for (; j < steps && ok; j += 3) ok = begin() && finish();
+                continue;
+            }
+            for (; j < real && ok; j += 3) {
+                asm volatile("cp.async.wait_group %0;" ::"n"(kSlAhead - 1) : "memory");
+                __syncwarp();
+                uint4 w[4], s_lo, s_hi;
+#pragma unroll
+                for (int q = 0; q < 4; ++q)
+                    asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(w[q].x), "=r"(w[q].y), "=r"(w[q].z), "=r"(w[q].w)   : "r"(src + lane * 16 + q * 512) : "memory");
+                asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(s_lo.x), "=r"(s_lo.y), "=r"(s_lo.z), "=r"(s_lo.w)   : "r"(src + 2048 + (lane >> 2) * 16) : "memory");
+                asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(s_hi.x), "=r"(s_hi.y), "=r"(s_hi.z), "=r"(s_hi.w)   : "r"(src + 2176 + (lane >> 2) * 16) : "memory");
+                __syncwarp();
+                fetch(src + lane * 16);   // (read by all lanes)
+                src = my_ring + (my_ring + kSlUnitBytes - src);
+                if (!begin()) { ok = false; break; }
+                const unsigned sl[4] = {s_lo.x, s_lo.y, s_lo.z, s_lo.w}, sh[4] = {s_hi.x, s_hi.y, s_hi.z, s_hi.w};
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    unsigned a[16];
+                    tc_unpack(w[q], tc_scale2<F16SB>(sl[q]), tc_scale2<F16SB>(sh[q]), a);
+                    tmem_st_frag(dst + 32u * q, a);
+                }
+                ok = finish();
+            }
+            for (; j < steps && ok; j += 3) {
+                unsigned a[16], a_lo[16];
+                tc_appended_pair<F16SB>(p, t.first + quarter + 4 * tile_of, lo + j - p.real_steps, a, a_lo);
+                if (!begin()) { ok = false; break; }
+                tmem_st_frag(dst, a);
+                tmem_st_frag(dst + 32u, a_lo);
+                tmem_st_frag(dst + 64u, a);
+                ok = finish();
+            }
+        }
+        if (!ok && lane == 0) tc_fail(p.status, &bars.failed, 1);
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncwarp();
+    } else if (p.splits == 1) {   // ---- results of a pass: a warp has its quarter's lanes, two row tiles of 16
+        const int quarter = warp & 3;
+        pdl_wait();   // (the rows' factors)
+        float fac[BN > 32 ? 2 : 1];
+#pragma unroll
+        for (int i = 0; i < (BN > 32 ? 2 : 1); ++i) fac[i] = tc_rscale(p, min(32 * i + lane, p.m - 1));
+        for (int pass = 0; pass < passes; ++pass) {
+            const SlPass t = sl_pass(p, pass, cta, ctas);
+            const int d = pass & 1, j = quarter + 4 * (lane >> 4);
+            TcDst dst = tc_dst(p, (t.first + j) * 16 + (lane & 15));
+            dst.live = dst.live && j < t.count;
+            if (!mbar_wait_warp(&bars.acc_full[d], (unsigned)(pass >> 1) & 1u)) { if (lane == 0) tc_fail(p.status, &bars.failed, 4); break; }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+            for (int c0 = 0; c0 < BN; c0 += 16) {
+                if (c0 >= p.m) break;
+                unsigned v[16];
+                tmem_ld16(tmem_d + ((unsigned)(quarter * 32) << 16) + (unsigned)(d * BN + c0), v);
+                tc_emit16(p, dst, v, fac[c0 / 32], c0 & 16, c0);
+                __syncwarp();
+            }
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) tc_arrive(smem_u32(&bars.acc_empty[d]));
+        }
+        __syncwarp();
+    }
+    if (p.splits > 1) {
+        // one pass; each CTA of the cluster sends its part of the columns that another one finishes
+        pdl_wait();   // (the rows' factors)
+        const bool done = mbar_wait_warp(&bars.acc_full[0], 0u);
+        if (!done && lane == 0) tc_fail(p.status, &bars.failed, 5);
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const cg::cluster_group cluster = cg::this_cluster();
+        cluster.sync();                                 // every ring of the cluster is free
+        const int own = BN / p.splits;                  // columns that a CTA of the cluster finishes
+        const SlPass t = sl_pass(p, 0, cta, ctas);
+        if (done && warp < kTcDeqWarps) {
+            const int r = (warp & 3) * 32 + lane;
+#pragma unroll 1
+            for (int c0 = (warp >> 2) * 16; c0 < BN; c0 += 64) {
+                if (c0 >= p.m) break;
+                unsigned v[16];
+                tmem_ld16(tmem_d + ((unsigned)((warp & 3) * 32) << 16) + (unsigned)c0, v);
+#pragma unroll
+                for (int i = 0; i < 16; ++i) {
+                    const int c = c0 + i, owner = c / own;
+                    if (c < p.m) reinterpret_cast<float*>(cluster.map_shared_rank(ring_ptr, owner))[(rank * own + (c - owner * own)) * kTcRows + r] = __uint_as_float(v[i]);
+                }
+            }
+        }
+        cluster.sync();
+        const float* got = reinterpret_cast<const float*>(ring_ptr);
+        const int rows = p.gated ? kTcRows / 2 : kTcRows;
+        for (int o = threadIdx.x; o < own * rows; o += blockDim.x) {
+            const int cl = o / rows, i = o % rows, token = rank * own + cl;
+            if (token >= p.m) continue;
+            // row tile j of the pass and its row; where its lane is (gated: a gate row, its up row eight further on)
+            const int j = p.gated ? i >> 3 : i >> 4, in = p.gated ? i & 7 : i & 15, ra = 32 * (j & 3) + 16 * (j >> 2) + in;
+            if (j >= t.count) continue;
+            const float* src = got + cl * kTcRows + ra;
+            float va = 0.f, vb = 0.f;
+            for (int z = 0; z < p.splits; ++z) {   // ranges in order
+                va += src[z * own * kTcRows];
+                if (p.gated) vb += src[z * own * kTcRows + 8];
+            }
+            const float sc = tc_rscale(p, token);
+            if (p.gated) tc_store_gated(p, token, (t.first + j) * 8 + in, va * sc, vb * sc);
+            else tc_store(p.out, token, (t.first + j) * 16 + in, va * sc);
+        }
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_d), "r"(kTmemCols) : "memory");
+}
+
 // Activations bf16 -> fp16, one CTA per row: the row's largest magnitude goes to [2^14, 2^15), so that nothing overflows fp16 and
 // every element within 2^-28 of the largest converts exactly (bf16 carries 8 significant bits, fp16 11). rscale[row] = the inverse
 // factor. Within a group of 64 column 16 t + 4 j + i goes to place 16 j + 4 t + i, the order of the weights' fragments. Behind the k
-// values (and zeros up to the weights' padding) the row gets three planes of g_pad columns: sum / 64 of every group of 64 converted values as an fp16
-// pair, laid out (hi, hi, lo) to meet the (c_hi, c_lo, c_hi) planes of the weight side; the rest is zeros.
+// values (and zeros up to the weights' padding) the row gets, for every 64 groups, three blocks of 64 columns: sum / 64 of every group of 64 converted values as an fp16
+// pair, laid out (hi, hi, lo) to meet the (c_hi, c_lo, c_hi) blocks of the weight side; the rest is zeros.
 // HOLD: a row of up to 16384 values stays in registers between the two passes (reading 4 bytes per lane twice took 24 us for
 // 2048 x 4096 under ncu, this takes 15).
-struct F16Rows { int k, k_pad, g_pad; __half* xh; int stride; float* rscale; };   // columns, padded, of a plane; the copy and its pitch
+struct F16Rows { int k, k_pad; __half* xh; int stride; float* rscale; };   // columns, padded; the copy and its pitch
 // bf16 magnitudes order like their bit patterns: two 16-bit maxima at a time
 __device__ __forceinline__ unsigned f16_top(unsigned mx, const uint4& v) {
     mx = __vmaxu2(mx, v.x & 0x7FFF7FFFu); mx = __vmaxu2(mx, v.y & 0x7FFF7FFFu);
@@ -715,16 +1066,17 @@ __device__ __forceinline__ void f16_put(const F16Rows& f, __half* out, int i, co
     if ((lane & 7) == 0) {
         const float sc = sum * 0.015625f;
         const __half hi = __float2half_rn(sc), lo = __float2half_rn(sc - __half2float(hi));
-        __half* ext = out + f.k_pad + (i >> 3);
-        ext[0] = hi; ext[f.g_pad] = hi; ext[2 * f.g_pad] = lo;
+        const int group = i >> 3;
+        __half* ext = out + f.k_pad + (group >> 6) * 192 + (group & 63);
+        ext[0] = hi; ext[64] = hi; ext[128] = lo;
     }
 }
-// what lies behind the values and behind the planes' groups
+// what lies behind the values and behind the last group
 __device__ __forceinline__ void f16_pad(const F16Rows& f, __half* out, int row, int sh) {
     for (int i = f.k + threadIdx.x; i < f.k_pad; i += 256) out[i] = __ushort_as_half(0);
     const int groups = f.k / 64;
     for (int i = threadIdx.x; i < f.stride - f.k_pad; i += 256)
-        if (i >= 3 * f.g_pad || i % f.g_pad >= groups) out[f.k_pad + i] = __ushort_as_half(0);
+        if (i / 192 * 64 + (i & 63) >= groups) out[f.k_pad + i] = __ushort_as_half(0);
     if (threadIdx.x == 0) f.rscale[row] = __uint_as_float((unsigned)(127 - sh) << 23);
 }
 
@@ -841,17 +1193,20 @@ int make_x_map(const __half* x, int x_stride, int m, int bn, CUtensorMap* map) {
     if (r != CUDA_SUCCESS) { set_error("qgemm (tcgen05): cuTensorMapEncodeTiled failed (%d)", (int)r); return SWLM_ERR_CUDA; }
     return SWLM_OK;
 }
-// forms: short with 32 or 64 activation rows per tile and two CTAs or one per SM, with 128 and one, long with 256; their stages
-constexpr int kTcStages32x2 = 6, kTcStages32 = 8, kTcStages64x2 = 3, kTcStages64 = 6, kTcStages128 = 4, kTcStagesPair = 5;
+// stages of the form with 128 activation rows per tile and of the pair's
+constexpr int kTcStages128 = 4, kTcStagesPair = 5;
 constexpr int kTcSMs = 148;
 
+int ext_blocks(int kt) { return (kt + 63) / 64; }   // blocks of 64 groups
+constexpr int sl_stages(int bn) { return bn == 32 ? 6 : bn == 48 ? 4 : 3; }
+constexpr size_t sl_smem_bytes(int bn) { return (size_t)sl_stages(bn) * bn * kSlCols * 2 + kSlRingBytes + 1024; }
 template <typename K>
 int tc_init_one(K kernel, size_t smem) {
     SWLM_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     return SWLM_OK;
 }
-template <int BN, int STAGES, int PER_SM>
 int tc_launch_short(QGemmTcParams& p, bool f16, const __half* xh, int xh_stride, int splits, cudaStream_t s) {
+    constexpr int BN = 128, STAGES = kTcStages128;
     CUtensorMap xmap;
     const int rc = make_x_map(xh, xh_stride, p.m, BN, &xmap);
     if (rc) return rc;
@@ -865,9 +1220,31 @@ int tc_launch_short(QGemmTcParams& p, bool f16, const __half* xh, int xh_stride,
     attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr; cfg.numAttrs = pdl_enabled() ? 2 : 1;
-    const cudaError_t e = f16 ? cudaLaunchKernelEx(&cfg, qgemm_tc_short_kernel<BN, STAGES, PER_SM, true>, p, xmap)
-                              : cudaLaunchKernelEx(&cfg, qgemm_tc_short_kernel<BN, STAGES, PER_SM, false>, p, xmap);
+    const cudaError_t e = f16 ? cudaLaunchKernelEx(&cfg, qgemm_tc_short_kernel<BN, STAGES, true>, p, xmap)
+                              : cudaLaunchKernelEx(&cfg, qgemm_tc_short_kernel<BN, STAGES, false>, p, xmap);
     return e == cudaSuccess ? SWLM_OK : cuda_fail(e, "qgemm_tc short launch");
+}
+template <int BN>
+int sl_launch(QGemmTcParams& p, bool f16, const __half* xh, int xh_stride, int splits, cudaStream_t s) {
+    CUtensorMap xmap;
+    const int rc = make_x_map(xh, xh_stride, p.m, BN, &xmap);
+    if (rc) return rc;
+    p.real_steps = p.kt * 64 / kSlCols; p.steps = p.real_steps + ext_blocks(p.kt); p.splits = splits;
+    const int ctas = std::min(kTcSMs / splits, p.row_tiles);
+    p.whole = p.row_tiles / (8 * ctas); p.left = p.row_tiles - p.whole * 8 * ctas;
+    p.n_tiles = p.whole + (p.left > 0);
+    if (splits > 1 && p.n_tiles > 1) { set_error("qgemm (tcgen05): passes"); return SWLM_ERR_INVALID; }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(ctas * splits)); cfg.blockDim = dim3(kSlThreads); cfg.dynamicSmemBytes = sl_smem_bytes(BN); cfg.stream = s;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)splits; attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr; cfg.numAttrs = pdl_enabled() ? 2 : 1;
+    const cudaError_t e = f16 ? cudaLaunchKernelEx(&cfg, qgemm_slab_kernel<BN, sl_stages(BN), true>, p, xmap)
+                              : cudaLaunchKernelEx(&cfg, qgemm_slab_kernel<BN, sl_stages(BN), false>, p, xmap);
+    return e == cudaSuccess ? SWLM_OK : cuda_fail(e, "qgemm_tc slab launch");
 }
 int tc_launch_long(QGemmTcParams& p, bool f16, const __half* xh, int xh_stride, cudaStream_t s) {
     CUtensorMap xmap;
@@ -883,47 +1260,52 @@ int tc_launch_long(QGemmTcParams& p, bool f16, const __half* xh, int xh_stride, 
     return e == cudaSuccess ? SWLM_OK : cuda_fail(e, "qgemm_tc launch");
 }
 
-// columns of one plane of appended group sums (whole 64s) and of all of them in whole steps, for `kt` groups
-int ext_plane_cols(int kt) { return (kt + 63) / 64 * 64; }
-int ext_cols(int kt) { return (3 * ext_plane_cols(kt) + kTcStep - 1) / kTcStep * kTcStep; }
+// appended columns for `kt` groups, in whole steps
+int ext_cols(int kt) { return (192 * ext_blocks(kt) + kTcStep - 1) / kTcStep * kTcStep; }
 int kt_padded(int k) { return (k / 64 + 3) / 4 * 4; }
 
-// How a product of m rows over `tiles16` row tiles runs: the form with the least time by what was measured over K = 2048 .. 14336,
-// n = 2048 .. 128256 and m = 20 .. 512 (us; graphs of launches, weights from memory). A CTA alone on its SM takes 0.45 us per step
-// (0.5 with 128 rows), two of them 0.9; a pair of the long form 0.87. A launch starts and ends in about 6. Cutting K over a cluster
-// costs the exchange: 5 over four CTAs, 7 to 9 over two (4096 x 4096 at 41 rows: 20.7 / 19.1 / 14.7 for 1, 2, 4; 14336 -> 4096: 62 / 43 / 30),
-// and over eight more than it saves (2048 x 2048: 11.6 for 4, 18.6 for 8). One CTA per SM with its deeper rings is the better
-// form while all tiles fit the GPU (16384 x 2048 at 41 rows 14.6 against 19.9), two per SM beyond (28672 x 4096: 37.6 against 42.5).
-struct TcChoice { int bn, per_sm, splits; };
+// How a product of m > 64 rows over `tiles16` row tiles runs: the form with the least time by what was measured over K = 2048 .. 14336,
+// n = 2048 .. 128256 and m = 65 .. 512 (us; graphs of launches, weights from memory). A CTA with 128 activation rows takes 0.5 us per
+// step, a pair of the long form 0.87. A launch starts and ends in about 6. Cutting K over a cluster costs the exchange: 5 over four CTAs,
+// 9 over two.
+struct TcChoice { int bn, splits; };
 TcChoice tc_choose(int m, int tiles16, int steps) {
-    const int row_tiles = (tiles16 + 7) / 8, bn = m <= 32 ? 32 : m <= 64 ? 64 : 128;
-    const long long tiles = (long long)row_tiles * ((m + bn - 1) / bn);
-    TcChoice best{bn, 1, 1};
+    const long long tiles = (long long)((tiles16 + 7) / 8) * ((m + 127) / 128);
+    TcChoice best{128, 1};
     double least = 1e30;
     auto offer = [&](double cost, const TcChoice& c) { if (cost < least) { least = cost; best = c; } };
-    for (int z = 1; z <= 4 && z <= steps; z *= 2) {
-        const double exchange = z == 1 ? 0 : z == 4 ? 5 : bn == 128 ? 9 : 7;
-        offer((double)((tiles * z + kTcSMs - 1) / kTcSMs) * ((bn == 128 ? 0.5 : 0.45) * ((steps + z - 1) / z) + 2) + 4 + exchange, {bn, 1, z});
-    }
-    if (bn <= 64 && tiles > kTcSMs) offer((double)((tiles + 2 * kTcSMs - 1) / (2 * kTcSMs)) * (0.9 * steps + 2) + 4, {bn, 2, 1});
+    for (int z = 1; z <= 4 && z <= steps; z *= 2)
+        offer((double)((tiles * z + kTcSMs - 1) / kTcSMs) * (0.5 * ((steps + z - 1) / z) + 2) + 4 + (z == 1 ? 0 : z == 4 ? 5 : 9), {128, z});
     if (m > 128) {
         const long long pairs = (long long)((tiles16 + 15) / 16) * ((m + 255) / 256);
-        offer((double)((pairs + kTcSMs / 2 - 1) / (kTcSMs / 2)) * (0.87 * steps + 1.5) + 5, {256, 1, 1});
+        offer((double)((pairs + kTcSMs / 2 - 1) / (kTcSMs / 2)) * (0.87 * steps + 1.5) + 5, {256, 1});
     }
     return best;
+}
+// CTAs along K of a product of up to 64 rows: two where row tiles are few and K is long. A step of 256 columns takes 0.42 us with up to
+// four row tiles per CTA and 0.62 with more, meeting in a cluster 6 (4096 x 14336 at 41 rows 29.4 us alone, 23.5 in pairs, 34.5 in fours;
+// 4096 x 4096 12.2 and 14.2).
+int sl_splits(int row_tiles, int kt) {
+    const int steps = kt / 4 + ext_blocks(kt);
+    auto time = [&](int z) {
+        const int ctas = std::min(kTcSMs / z, row_tiles), whole = row_tiles / (8 * ctas), most = (row_tiles - whole * 8 * ctas + ctas - 1) / ctas;
+        return ((whole * 0.62) + (most > 4 ? 0.62 : most > 0 ? 0.42 : 0.0)) * ((steps + z - 1) / z) + (z > 1 ? 6.0 : 0.0);
+    };
+    return steps >= 2 && row_tiles <= 8 * (kTcSMs / 2) && time(2) < time(1) ? 2 : 1;
 }
 
 }  // namespace
 
-template <int BN, int STAGES, int PER_SM>
-static int tc_init_short() {
-    const int rc = tc_init_one(qgemm_tc_short_kernel<BN, STAGES, PER_SM, false>, tc_smem_bytes(BN, STAGES));
-    return rc ? rc : tc_init_one(qgemm_tc_short_kernel<BN, STAGES, PER_SM, true>, tc_smem_bytes(BN, STAGES));
+template <int BN>
+static int sl_init() {
+    const int rc = tc_init_one(qgemm_slab_kernel<BN, sl_stages(BN), false>, sl_smem_bytes(BN));
+    return rc ? rc : tc_init_one(qgemm_slab_kernel<BN, sl_stages(BN), true>, sl_smem_bytes(BN));
 }
 int qgemm_tc_init() {
     int rc;
-    if ((rc = tc_init_short<32, kTcStages32x2, 2>()) || (rc = tc_init_short<32, kTcStages32, 1>()) || (rc = tc_init_short<64, kTcStages64x2, 2>()) ||
-        (rc = tc_init_short<64, kTcStages64, 1>()) || (rc = tc_init_short<128, kTcStages128, 1>()) ||
+    if ((rc = sl_init<32>()) || (rc = sl_init<48>()) || (rc = sl_init<64>()) ||
+        (rc = tc_init_one(qgemm_tc_short_kernel<128, kTcStages128, false>, tc_smem_bytes(128, kTcStages128))) ||
+        (rc = tc_init_one(qgemm_tc_short_kernel<128, kTcStages128, true>, tc_smem_bytes(128, kTcStages128))) ||
         (rc = tc_init_one(qgemm_tc_kernel<kTcStagesPair, false>, tc_smem_bytes(kTcPairRows, kTcStagesPair))) ||
         (rc = tc_init_one(qgemm_tc_kernel<kTcStagesPair, true>, tc_smem_bytes(kTcPairRows, kTcStagesPair))) ||
         (rc = tc_init_one(norm_to_f16_kernel<0>, (size_t)kNormMaxDim * 4)) || (rc = tc_init_one(norm_to_f16_kernel<1>, (size_t)kNormMaxDim * 4)) ||
@@ -939,7 +1321,7 @@ int qgemm_tc_launch_count(bool reuse_x) { return (reuse_x ? 0 : 1) + 1; }
 
 static F16Rows f16_rows(int m, int k, void* scratch) {
     F16Rows f{};
-    f.k = k; f.k_pad = kt_padded(k) * 64; f.g_pad = ext_plane_cols(kt_padded(k)); f.xh = static_cast<__half*>(scratch); f.stride = xh_cols(k);
+    f.k = k; f.k_pad = kt_padded(k) * 64; f.xh = static_cast<__half*>(scratch); f.stride = xh_cols(k);
     f.rscale = reinterpret_cast<float*>(static_cast<unsigned char*>(scratch) + ((size_t)m * f.stride * 2 + 255) / 256 * 256);
     return f;
 }
@@ -968,7 +1350,7 @@ int launch_qgemm_tc(const Q4Tiled& w, int m, const __nv_bfloat16* x, int x_strid
         return SWLM_ERR_INVALID;
     }
     QGemmTcParams p{};
-    p.tiles = w.tiles; p.sb = reinterpret_cast<const unsigned*>(w.sb); p.row_tiles = w.row_tiles; p.kt = w.kt_pad; p.g_pad = f.g_pad;
+    p.tiles = w.tiles; p.sb = reinterpret_cast<const unsigned*>(w.sb); p.row_tiles = w.row_tiles; p.kt = w.kt_pad;
     p.rscale = f.rscale;
     p.m = m; p.status = status;
     p.real_steps = w.kt_pad * 64 / kTcStep; p.steps = xh_stride / kTcStep;
@@ -982,10 +1364,14 @@ int launch_qgemm_tc(const Q4Tiled& w, int m, const __nv_bfloat16* x, int x_strid
                                            : launch_k(x_to_f16_kernel<false>, dim3((unsigned)m), dim3(256), 0, s, x, x_stride, f);
         if (e != cudaSuccess) return cuda_fail(e, "x_to_f16 launch");
     }
+    if (m <= 64) {
+        const int z = sl_splits(w.row_tiles, p.kt);
+        if (m <= 32) return sl_launch<32>(p, w.sb_f16, xh, xh_stride, z, s);
+        if (m <= 48) return sl_launch<48>(p, w.sb_f16, xh, xh_stride, z, s);
+        return sl_launch<64>(p, w.sb_f16, xh, xh_stride, z, s);
+    }
     const TcChoice c = tc_choose(m, w.row_tiles, p.steps);
-    if (c.bn == 32) return c.per_sm == 2 ? tc_launch_short<32, kTcStages32x2, 2>(p, w.sb_f16, xh, xh_stride, c.splits, s) : tc_launch_short<32, kTcStages32, 1>(p, w.sb_f16, xh, xh_stride, c.splits, s);
-    if (c.bn == 64) return c.per_sm == 2 ? tc_launch_short<64, kTcStages64x2, 2>(p, w.sb_f16, xh, xh_stride, c.splits, s) : tc_launch_short<64, kTcStages64, 1>(p, w.sb_f16, xh, xh_stride, c.splits, s);
-    if (c.bn == 128) return tc_launch_short<128, kTcStages128, 1>(p, w.sb_f16, xh, xh_stride, c.splits, s);
+    if (c.bn == 128) return tc_launch_short(p, w.sb_f16, xh, xh_stride, c.splits, s);
     return tc_launch_long(p, w.sb_f16, xh, xh_stride, s);
 }
 

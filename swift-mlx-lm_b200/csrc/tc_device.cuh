@@ -24,6 +24,8 @@ __device__ __forceinline__ void mbar_init(unsigned long long* bar, unsigned coun
         ".reg .pred p, q;\n\t"                                                         \
         ".reg .u32 n;\n\t"                                                             \
         "mov.u32 n, 0;\n\t"                                                            \
+        "mbarrier.test_wait.parity" SEM ".shared::cta.b64 p, [%1], %2;\n\t"            \
+        "@p bra SWLM_DONE;\n\t"                                                        \
         "SWLM_TRY:\n\t"                                                                \
         "mbarrier.try_wait.parity" SEM ".shared::cta.b64 p, [%1], %2;\n\t"             \
         "@p bra SWLM_DONE;\n\t"                                                        \

@@ -82,7 +82,8 @@ def test_more_tiles_than_multiprocessors(pkg, oracle):
 
 def _form(m, rows, k, gated=False):
     """Which form `tc_choose` takes for m activation rows, by its estimates of the time: (rows per tile, CTAs per SM, CTAs along K) and the
-    number of steps. The tests below name the form they are about; they have to follow when the rule moves."""
+    number of steps. The tests below name the form they are about; they have to follow when the rule moves. (Up to 64 rows `qgemm_slab_kernel`
+    has taken the place of these forms: test_products_of_17_to_64_rows.)"""
     kt = (k // 64 + 3) // 4 * 4
     steps = (kt * 64 + -(-3 * (-(-kt // 64) * 64) // 128) * 128) // 128
     tiles16 = -(-rows // 8) if gated else -(-rows // 16)
@@ -125,6 +126,47 @@ def test_forms_of_the_tensor_core_products(pkg, oracle, m, n, k, form, steps):
     store.add_q4_staf("staf", pkg.formats.repack_mlx_to_staf(w, s, b), n, k)
     assert rel_err(pkg.bf16_to_f32(store.qgemm("staf", x, n))[rows], ref).max() <= RTOL
     store.close()
+
+
+@pytest.mark.parametrize("m", [17, 32, 33, 48, 49, 64])
+@pytest.mark.parametrize("n,k", [
+    (16, 64), (130, 704),               # one row tile; nine on nine CTAs, three steps with padding
+    (18944, 256), (19010, 320),         # eight row tiles for every SM and nothing, or five tiles, left
+    (9600, 2304), (136, 9216),          # four or five row tiles per SM; K over two CTAs
+    (600, 16448),                       # K over two CTAs, five steps of appended columns, all of them in the second one
+])
+def test_products_of_17_to_64_rows(pkg, oracle, n, k, m):
+    """Passes of the SMs over row tiles of 16, whole and not; 32, 48 and 64 rows with remainders; bf16 and fp16 scales."""
+    store = pkg.WeightStore(0)
+    w, s, b = pkg.synth_q4(n, k, seed=n + k, centered=True)
+    x = pkg.f32_to_bf16(np.random.default_rng(m).normal(size=(m, k)).astype(np.float32))
+    store.add_q4_mlx("mlx", w, s, b)
+    ref = pkg.bf16_to_f32(oracle.qgemm(x, w, s, b))
+    assert rel_err(pkg.bf16_to_f32(store.qgemm("mlx", x, n)), ref).max() <= RTOL
+    store.add_q4_staf("staf", pkg.formats.repack_mlx_to_staf(w, s, b), n, k)
+    assert rel_err(pkg.bf16_to_f32(store.qgemm("staf", x, n)), ref).max() <= RTOL
+    store.close()
+
+
+@pytest.mark.parametrize("m,ff,k", [(24, 512, 9216), (40, 19008, 320), (64, 64, 576)])
+def test_gated_products_of_17_to_64_rows(pkg, oracle, m, ff, k):
+    """The same with gate and up together: two CTAs along K, more than one pass, fewer row tiles than SMs."""
+    P, vocab = pkg.plan, 256
+    rng = np.random.default_rng(m + k)
+    store, q4, table = _gated_store(pkg, rng, vocab, k, ff, False)
+    desc = pkg.BuffersDesc(hidden=k, slot_dim=max(ff, k), vocab=vocab, max_seq=16, max_batch=m)
+    steps = [P._step(P.STEP_EMBED, out_buf=P.BUF_S3, n=k, weight="rows")] + _gated_steps(P, k, ff) + [
+        P._step(P.STEP_QGEMV, in_buf=P.BUF_S0, out_buf=P.BUF_LOGITS, n=vocab, k=ff, weight="down"),
+        P._step(P.STEP_EMBED, out_buf=P.BUF_S1, n=k, weight="rows"), P._step(P.STEP_EMBED, out_buf=P.BUF_S2, n=k, weight="rows"),
+        P._step(P.STEP_ARGMAX, in_buf=P.BUF_LOGITS, n=vocab)]
+    model = pkg.InferenceModel(store, steps, desc)
+    tokens = rng.integers(0, vocab, size=m)
+    model.decode(tokens)
+    got = pkg.bf16_to_f32(model.read_buffer(P.BUF_S0, ff))
+    ref = _gated_ref(pkg, oracle, table[tokens], q4)
+    for i in range(m):
+        assert rel_err(got[i], ref[i]).max() <= 2 * RTOL   # two products' errors
+    model.close(), store.close()
 
 
 @pytest.mark.parametrize("staf", [False, True])
