@@ -20,6 +20,7 @@
 //     the split's later blocks are asked into L2 as soon as it has; q, k and v of the new token are requested
 //     before any of that, and each RoPE pair is rotated once in shared memory.
 // Prompt chunks take the tensor-core kernel of attn_prompt.cu.
+#include <algorithm>
 #include <atomic>
 #include <cstdlib>
 #include <cmath>
@@ -108,11 +109,15 @@ __device__ __forceinline__ float rope_elem(const float* v, int d, int rope_dim, 
 // MODE 3: the same behind a per-head RMS norm of q and the new k (a form of its own: plans without that norm keep their code).
 // MODE 2: prompt ingestion: "sequence" b is prompt token b of ONE sequence at position pos_base + b; all of the
 //         chunk's k/v rows are already in the cache (rope_append_kernel), token b attends rows 0..pos_base+b.
+// MODE 4: as MODE 0 over a grid of CTAs that fill the GPU once: all blocks of 64 cached rows of all (sequence, KV head) pairs lie one after
+//         the other and every CTA takes the same number of them, of one pair or several. What a CTA has of a pair goes to one of its two
+//         places for partial results (pairs that began in an earlier CTA to the first), and the last CTA of a pair to arrive merges them.
 template <int HD, int MODE>
 __global__ void __launch_bounds__(kSplitThreads) attn_split_kernel(const typename AttnArgs<MODE>::type p) {
     constexpr bool DECODE = MODE == 1 || MODE == 3;
     constexpr bool QK_NORM = MODE == 3;
     constexpr bool PREFILL = MODE == 2;
+    constexpr bool STREAM = MODE == 4;
     const int cta_linear = (blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
     if (p.trace && threadIdx.x == 0) p.trace[cta_linear * 4] = attn_timer_ns();
     pdl_launch_dependents();
@@ -123,7 +128,6 @@ __global__ void __launch_bounds__(kSplitThreads) attn_split_kernel(const typenam
     constexpr int VH = HD / 64;   // 64-dimension halves of V
     constexpr int VPR = HD / 8;   // 16-byte vectors per head row
     constexpr int PITCH = HD + 2; // row pitch of q in shared memory: the 8-byte fragment reads below hit 16 different bank pairs
-    const int split = blockIdx.x, kvh = blockIdx.y, b = blockIdx.z;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
     const int G = p.heads / p.kv_heads;
     const bool rotate = (DECODE || PREFILL) && p.rope_dim > 0;
@@ -136,12 +140,44 @@ __global__ void __launch_bounds__(kSplitThreads) attn_split_kernel(const typenam
     pdl_wait();
     if (p.trace && threadIdx.x == 0) p.trace[cta_linear * 4 + 1] = attn_timer_ns();
 
+    constexpr int kBlock = kSplitWarps * 16;
+    // blocks of a pair and of all, this CTA's share
+    const int nb = STREAM ? (p.ctx_len + kBlock - 1) / kBlock : 0;
+    const unsigned total = STREAM ? (unsigned)(p.splits * nb) : 1u;
+    unsigned unit = 0, unit_end = 1;
+    if constexpr (STREAM) {
+        unit = (unsigned)((unsigned long long)blockIdx.x * total / gridDim.x);
+        unit_end = (unsigned)((unsigned long long)(blockIdx.x + 1) * total / gridDim.x);
+    }
+
     __shared__ __align__(16) float qk[kMaxGroup + 1][PITCH];  // rows 0..G-1: q of the group, row G: the new k
     __shared__ float vraw[HD];                                // new v
     __shared__ float self_score[kMaxGroup];                   // q . k of the new token, log2 domain
     __shared__ float osm[kSplitWarps][kMaxGroup][HD + 4];
     __shared__ float msm[kSplitWarps][kMaxGroup], lsm[kSplitWarps][kMaxGroup];
 
+    do {
+    int split = blockIdx.x, kvh = blockIdx.y, b = blockIdx.z;   // STREAM: split 0 has the pair's first blocks
+    int nsplit = p.splits, blk0 = 0, blk1 = 0, cta_first = 0;   // blk0, blk1: this CTA's blocks of the pair; the CTA that has its first one
+    if constexpr (STREAM) {
+        const unsigned pair = unit / (unsigned)nb, first = pair * nb;
+        b = (int)(pair / (unsigned)p.kv_heads);
+        kvh = (int)pair - b * p.kv_heads;
+        blk0 = (int)(unit - first);
+        blk1 = min(nb, blk0 + (int)(unit_end - unit));
+        // the CTA of block x of all: the last one that starts at or before it
+        auto cta_of = [&](unsigned x) { return (int)((((unsigned long long)x + 1) * gridDim.x - 1) / total); };
+        cta_first = cta_of(first);
+        nsplit = cta_of(first + nb - 1) - cta_first + 1;
+        split = blk0 == 0 ? 0 : 1;
+        unit += (unsigned)(blk1 - blk0);
+    }
+    // a partial result's place: split `z` of the pair, head r of the group
+    auto slot_of = [&](int z, int r) {
+        if (STREAM) return (size_t)(2 * (cta_first + z) + (z == 0 ? 1 : 0)) * G + r;
+        return ((size_t)b * p.heads + (size_t)kvh * G + r) * p.splits + z;
+    };
+    auto hop = [&](int z) { return STREAM ? (slot_of(z, 0) - slot_of(0, 0)) * HD : (size_t)z * HD; };   // from split 0's result to z's
     // ---- q and the new k and v are requested first: they do not depend on the position --------------------
     uint4 qv = make_uint4(0, 0, 0, 0), kv = qv, vv = qv;
     const bool has_q = tid < G * VPR;
@@ -161,10 +197,9 @@ __global__ void __launch_bounds__(kSplitThreads) attn_split_kernel(const typenam
     // ---- tokens of this split: blocks of 64 tokens, block j belongs to split j % splits. A split's first block
     // does not depend on the context length, so in a decode step it is requested before the position has arrived
     // (rows are clamped to the cache's last row there; what lies beyond the context is masked below).
-    constexpr int kBlock = kSplitWarps * 16;
-    const int t_begin = split * kBlock;
-    const int t_end = n_ctx;
-    const int t_stride = p.splits * kBlock;
+    const int t_begin = STREAM ? blk0 * kBlock : split * kBlock;
+    const int t_end = STREAM ? min(n_ctx, blk1 * kBlock) : n_ctx;
+    const int t_stride = STREAM ? kBlock : p.splits * kBlock;
 
     // K and V of 16 tokens per warp live in registers; the first batch is requested before the rest of the
     // prologue so that its trip to HBM overlaps it
@@ -196,7 +231,7 @@ __global__ void __launch_bounds__(kSplitThreads) attn_split_kernel(const typenam
     // sliding window (Generator/MetalSourceGenerator+Attention.swift:851-853): cached rows below t_lo are left out.
     // A split whose first blocks lie wholly below the window starts at its first block that reaches into it.
     const int t_lo = p.window > 0 ? max(0, n_ctx + (DECODE ? 1 : 0) - p.window) : 0;
-    if (t_lo / kBlock > split) {
+    if (!STREAM && t_lo / kBlock > split) {
         const int skip = (t_lo / kBlock - split + p.splits - 1) / p.splits;
         tok0 = (split + skip * p.splits) * kBlock + warp * 16;
         if (!p.q_first && tok0 < t_end) { load_k(tok0, t_end - 1); load_v(tok0, t_end - 1); }
@@ -421,7 +456,7 @@ __global__ void __launch_bounds__(kSplitThreads) attn_split_kernel(const typenam
             o = fmaf(wgt, osm[w][r][d], o);
             l = fmaf(wgt, lsm[w][r], l);
         }
-        const size_t slot = ((size_t)b * p.heads + (size_t)kvh * G + r) * p.splits + split;
+        const size_t slot = STREAM ? (size_t)(2 * blockIdx.x + (blk0 == 0 ? 1 : 0)) * G + r : slot_of(split, r);
         __stcg(p.part_o + slot * HD + d, o);
         if (d == 0) { __stcg(p.part_ml + slot * 2, mx); __stcg(p.part_ml + slot * 2 + 1, l); }
     }
@@ -435,16 +470,16 @@ __global__ void __launch_bounds__(kSplitThreads) attn_split_kernel(const typenam
         unsigned* ctr = p.counters + (size_t)b * p.kv_heads + kvh;
         unsigned prev;
         asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(prev) : "l"(ctr) : "memory");
-        is_last = prev == (unsigned)p.splits - 1u;
+        is_last = prev == (unsigned)nsplit - 1u;
         if (is_last) *ctr = 0u;  // ready for the next launch
     }
     __syncthreads();
     if (p.trace && threadIdx.x == 0) p.trace[cta_linear * 4 + 3] = attn_timer_ns();
-    if (!is_last) return;
+    if (is_last) {
 
     // Everything that does not depend on the split weights is requested first: the (max, sum) pairs and the
     // first 16 partial outputs of this thread's four dimensions travel together.
-    constexpr int kPre = 32;
+    constexpr int kPre = STREAM && HD == 128 ? 16 : 32;
     const int n_out4 = G * HD / 4;  // float4 outputs of the group
     float* wsm = &osm[1][0][0];     // [G][splits] weights (splits <= 64: fits the reused buffer)
     float* msm2 = &osm[2][0][0];    // [G][splits] split maxima
@@ -453,9 +488,9 @@ __global__ void __launch_bounds__(kSplitThreads) attn_split_kernel(const typenam
 #pragma unroll
     for (int j = 0; j < 2; ++j) {
         const int idx = tid + j * kSplitThreads;
-        if (idx < G * p.splits) {
-            const int r = idx / p.splits, sidx = idx - r * p.splits;
-            const size_t slot = ((size_t)b * p.heads + (size_t)kvh * G + r) * p.splits + sidx;
+        if (idx < G * nsplit) {
+            const int r = idx / nsplit, sidx = idx - r * nsplit;
+            const size_t slot = slot_of(sidx, r);
             ml[j] = __ldcg(reinterpret_cast<const float2*>(p.part_ml + slot * 2));
         }
     }
@@ -463,18 +498,18 @@ __global__ void __launch_bounds__(kSplitThreads) attn_split_kernel(const typenam
     const float* po0 = nullptr;
     if (tid < n_out4) {
         const int r = tid / (HD / 4), d4 = tid - r * (HD / 4);
-        po0 = p.part_o + (((size_t)b * p.heads + (size_t)kvh * G + r) * p.splits) * HD + d4 * 4;
+        po0 = p.part_o + slot_of(0, r) * HD + d4 * 4;
 #pragma unroll
         for (int sidx = 0; sidx < kPre; ++sidx)
-            if (sidx < p.splits) pre[sidx] = __ldcg(reinterpret_cast<const float4*>(po0 + (size_t)sidx * HD));
+            if (sidx < nsplit) pre[sidx] = __ldcg(reinterpret_cast<const float4*>(po0 + hop(sidx)));
     }
     for (int j = 0; j < 2; ++j) {
         const int idx = tid + j * kSplitThreads;
-        if (idx < G * p.splits) { msm2[idx] = ml[j].x; lsm2[idx] = ml[j].y; }
+        if (idx < G * nsplit) { msm2[idx] = ml[j].x; lsm2[idx] = ml[j].y; }
     }
-    for (int idx = tid + 2 * kSplitThreads; idx < G * p.splits; idx += kSplitThreads) {
-        const int r = idx / p.splits, sidx = idx - r * p.splits;
-        const size_t slot = ((size_t)b * p.heads + (size_t)kvh * G + r) * p.splits + sidx;
+    for (int idx = tid + 2 * kSplitThreads; idx < G * nsplit; idx += kSplitThreads) {
+        const int r = idx / nsplit, sidx = idx - r * nsplit;
+        const size_t slot = slot_of(sidx, r);
         msm2[idx] = __ldcg(p.part_ml + slot * 2);
         lsm2[idx] = __ldcg(p.part_ml + slot * 2 + 1);
     }
@@ -486,14 +521,14 @@ __global__ void __launch_bounds__(kSplitThreads) attn_split_kernel(const typenam
     for (int r = warp; r < G; r += kSplitWarps) {
         const float m_self = DECODE ? self_score[r] : -INFINITY;
         float mx = m_self;
-        for (int sidx = lane; sidx < p.splits; sidx += 32) mx = fmaxf(mx, msm2[r * p.splits + sidx]);
+        for (int sidx = lane; sidx < nsplit; sidx += 32) mx = fmaxf(mx, msm2[r * nsplit + sidx]);
         for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
         float den = 0.f;
-        for (int sidx = lane; sidx < p.splits; sidx += 32) {
-            const float ms = msm2[r * p.splits + sidx];
+        for (int sidx = lane; sidx < nsplit; sidx += 32) {
+            const float ms = msm2[r * nsplit + sidx];
             const float w = ms == -INFINITY ? 0.f : exp2f(ms - mx);
-            wsm[r * p.splits + sidx] = w;
-            den = fmaf(w, lsm2[r * p.splits + sidx], den);
+            wsm[r * nsplit + sidx] = w;
+            den = fmaf(w, lsm2[r * nsplit + sidx], den);
         }
         for (int o = 16; o > 0; o >>= 1) den += __shfl_xor_sync(0xffffffffu, den, o);
         const float ws = DECODE ? exp2f(m_self - mx) : 0.f;
@@ -503,8 +538,8 @@ __global__ void __launch_bounds__(kSplitThreads) attn_split_kernel(const typenam
     __syncthreads();
     for (int idx = tid; idx < n_out4; idx += kSplitThreads) {
         const int r = idx / (HD / 4), d4 = idx - r * (HD / 4);
-        const float* po = p.part_o + (((size_t)b * p.heads + (size_t)kvh * G + r) * p.splits) * HD + d4 * 4;
-        const float* wr = wsm + r * p.splits;
+        const float* po = p.part_o + slot_of(0, r) * HD + d4 * 4;
+        const float* wr = wsm + r * nsplit;
         float4 num = make_float4(0.f, 0.f, 0.f, 0.f);
         if (DECODE) {
             const float ws = w_self[r];
@@ -514,16 +549,16 @@ __global__ void __launch_bounds__(kSplitThreads) attn_split_kernel(const typenam
         if (idx == tid) {  // this thread's first output: its first partials are already in registers
 #pragma unroll
             for (int sidx = 0; sidx < kPre; ++sidx)
-                if (sidx < p.splits) {
+                if (sidx < nsplit) {
                     const float w = wr[sidx];
                     num.x = fmaf(w, pre[sidx].x, num.x); num.y = fmaf(w, pre[sidx].y, num.y);
                     num.z = fmaf(w, pre[sidx].z, num.z); num.w = fmaf(w, pre[sidx].w, num.w);
                 }
-            s0 = min(kPre, p.splits);
+            s0 = min(kPre, nsplit);
         }
 #pragma unroll 16
-        for (int sidx = s0; sidx < p.splits; ++sidx) {
-            const float4 v4 = __ldcg(reinterpret_cast<const float4*>(po + (size_t)sidx * HD));
+        for (int sidx = s0; sidx < nsplit; ++sidx) {
+            const float4 v4 = __ldcg(reinterpret_cast<const float4*>(po + hop(sidx)));
             const float w = wr[sidx];
             num.x = fmaf(w, v4.x, num.x); num.y = fmaf(w, v4.y, num.y);
             num.z = fmaf(w, v4.z, num.z); num.w = fmaf(w, v4.w, num.w);
@@ -538,6 +573,9 @@ __global__ void __launch_bounds__(kSplitThreads) attn_split_kernel(const typenam
         __syncthreads();
         if (threadIdx.x == 0) p.trace[(gridDim.x * gridDim.y * gridDim.z + (blockIdx.z * gridDim.y + blockIdx.y)) * 4] = attn_timer_ns();  // merged
     }
+    }   // is_last
+    if (STREAM) __syncthreads();   // (shared memory is written again for the next pair)
+    } while (STREAM && unit < unit_end);
 }
 
 // Prompt ingestion: rotate the chunk's k rows (token b at position pos_base + b) and append them and the v rows to
@@ -997,13 +1035,24 @@ __global__ void __launch_bounds__(kQ8Threads, ROTOR && G <= 4 ? 2 : 0) attn_q8_s
     }
 }
 
+// MODE 4's CTAs: two per SM; no more than 63 per KV head and sequence, so that a pair has 64 partial results at most (what the merge has
+// room for)
+constexpr int kStreamCtas = 296;
+int stream_ctas(int pairs) { return std::min(kStreamCtas, 63 * pairs); }
+// Flash-decode over sequences of equal length: MODE 4 where the splits of all pairs leave more than a fifth of their rounds of the GPU (two
+// CTAs per SM) empty. us with splits / so, 8 KV heads of 128: 13 x 5000 rows (0.70 full) 57 / 50, 24 x 2048 (0.65) 46 / 40,
+// 41 x 2557 (0.55) 108 / 76; 16 x 4096 and 64 x 1024 (0.86) 47.5 / 50 and 55 / 54. Short caches lose what a CTA pays for each pair
+// (64 x 300 23 / 26). Decode steps, where each pair's start is longer, lost in every batch (41 ragged sequences, 4 layers: 1053 / 1100 a step).
+bool attn_streams(int m, int kv_heads, int ctx_len) {
+    const long long pairs = (long long)m * kv_heads, ctas = pairs * attn_pick_splits(m, kv_heads, ctx_len), rounds = (ctas + kStreamCtas - 1) / kStreamCtas;
+    return pairs >= 100 && ctx_len >= 512 && ctas * 5 < rounds * kStreamCtas * 4 && pairs * ((ctx_len + 63) / 64) < (1ll << 31);
+}
 template <int MODE>
-int launch_both(const typename AttnArgs<MODE>::type& p, int m, int hd, cudaStream_t s) {
-    const dim3 grid(p.splits, p.kv_heads, m);
+int launch_both(const typename AttnArgs<MODE>::type& p, const dim3& grid, int hd, cudaStream_t s) {
     if (hd == 128) {
-        launch_k(attn_split_kernel<128, MODE>, dim3(grid), dim3(kSplitThreads), 0, s, p);
+        launch_k(attn_split_kernel<128, MODE>, grid, dim3(kSplitThreads), 0, s, p);
     } else if (hd == 64) {
-        launch_k(attn_split_kernel<64, MODE>, dim3(grid), dim3(kSplitThreads), 0, s, p);
+        launch_k(attn_split_kernel<64, MODE>, grid, dim3(kSplitThreads), 0, s, p);
     } else {
         set_error("attention: head_dim %d not supported (64 or 128)", hd);
         return SWLM_ERR_UNSUPPORTED;
@@ -1045,6 +1094,10 @@ int attn_pick_splits(int m, int kv_heads, int max_ctx, bool ragged) {
 
 size_t attn_scratch_floats(int m, int heads, int head_dim, int splits) {
     return (size_t)m * heads * splits * (head_dim + 2);
+}
+size_t flash_scratch_floats(int m, int heads, int kv_heads, int hd, int ctx_len) {
+    const size_t apart = attn_scratch_floats(m, heads, hd, attn_pick_splits(m, kv_heads, ctx_len));
+    return attn_streams(m, kv_heads, ctx_len) ? std::max(apart, (size_t)2 * stream_ctas(m * kv_heads) * (heads / kv_heads) * (hd + 2)) : apart;
 }
 
 static int check_group(int heads, int kv_heads) {
@@ -1118,13 +1171,13 @@ int launch_attn_decode(const AttnLaunch& a, cudaStream_t s) {
         if (e != cudaSuccess) return cuda_fail(e, "rope_append launch");
         // tensor cores when the query heads of a KV head fill the 128 rows of a tile evenly; else a token at a time
         if (attn_prompt_takes(a)) return launch_attn_prompt(a, s);
-        return launch_both<2>(p, a.m, a.head_dim, s);
+        return launch_both<2>(p, dim3(p.splits, p.kv_heads, a.m), a.head_dim, s);
     }
-    if (!a.q_norm) return launch_both<1>(p, a.m, a.head_dim, s);
+    if (!a.q_norm) return launch_both<1>(p, dim3(p.splits, p.kv_heads, a.m), a.head_dim, s);
     AttnNormParams n{};
     static_cast<AttnParams&>(n) = p;
     n.q_norm = a.q_norm; n.k_norm = a.k_norm; n.qk_eps = a.qk_eps; n.qk_bias = a.qk_bias;
-    return launch_both<3>(n, a.m, a.head_dim, s);
+    return launch_both<3>(n, dim3(n.splits, n.kv_heads, a.m), a.head_dim, s);
 }
 
 int launch_flash_decode_plain(int m, int heads, int kv_heads, int hd, int ctx_len, int ctx_stride, float scale,
@@ -1143,9 +1196,11 @@ int launch_flash_decode_plain(int m, int heads, int kv_heads, int hd, int ctx_le
     p.position = nullptr; p.ctx_len = ctx_len;
     p.out = out; p.out_stride = heads * hd;
     p.part_o = scratch;
-    p.part_ml = scratch + (size_t)m * heads * splits * hd;
+    const bool stream = attn_streams(m, kv_heads, ctx_len);
+    if (stream) p.splits = m * kv_heads;   // (MODE 4: pairs)
+    p.part_ml = scratch + (stream ? (size_t)2 * stream_ctas(m * kv_heads) * (heads / kv_heads) : (size_t)m * heads * splits) * hd;
     p.counters = counters;
-    return launch_both<0>(p, m, hd, s);
+    return stream ? launch_both<4>(p, dim3((unsigned)stream_ctas(m * kv_heads)), hd, s) : launch_both<0>(p, dim3(splits, kv_heads, m), hd, s);
 }
 
 // ---- allocation-free flash-decode ---------------------------------------------------------------------
@@ -1181,7 +1236,7 @@ int launch_flash_decode_static(int device, int m, int heads, int kv_heads, int h
     }
     const int splits = attn_pick_splits(m, kv_heads, ctx_len);
     const size_t counter_bytes = (((size_t)m * kv_heads * sizeof(unsigned)) + 255) / 256 * 256;
-    const size_t need = counter_bytes + attn_scratch_floats(m, heads, hd, splits) * sizeof(float);
+    const size_t need = counter_bytes + flash_scratch_floats(m, heads, kv_heads, hd, ctx_len) * sizeof(float);
     if (need > kStaticScratchBytes) {
         set_error("flash-decode (static scratch): batch %d x %d heads x %d splits needs %zu bytes, the built-in scratch holds %zu",
                   m, heads, splits, need, kStaticScratchBytes);

@@ -2582,7 +2582,7 @@ static int flash_args_ok(int b, int heads, int kv_heads, int hd, int ctx_len, in
 
 size_t swlm_op_flash_decode_scratch_bytes(int b, int heads, int kv_heads, int hd, int ctx_len) {
     if (b <= 0 || heads <= 0 || kv_heads <= 0 || hd <= 0 || ctx_len <= 0) return 0;
-    return attn_scratch_floats(b, heads, hd, flash_splits(b, kv_heads, ctx_len)) * sizeof(float);
+    return flash_scratch_floats(b, heads, kv_heads, hd, ctx_len) * sizeof(float);
 }
 
 int swlm_op_flash_decode_dev(swlm_ctx* ctx, int b, int heads, int kv_heads, int hd, int ctx_len, int ctx_stride,

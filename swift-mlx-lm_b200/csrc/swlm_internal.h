@@ -314,6 +314,7 @@ int launch_attn_prompt(const AttnLaunch& a, cudaStream_t s);
 // ragged: the sequences may be of unequal length
 int attn_pick_splits(int m, int kv_heads, int max_ctx, bool ragged = false);
 size_t attn_scratch_floats(int m, int heads, int head_dim, int splits);
+size_t flash_scratch_floats(int m, int heads, int kv_heads, int hd, int ctx_len);   // of launch_flash_decode_plain
 // decode: q rows are unrotated; RoPE, KV append and the current token's unrounded term are handled inside.
 int launch_attn_decode(const AttnLaunch& a, cudaStream_t s);
 // generic flash-decode over an existing cache (q already rotated), ctx_len fixed on the host.

@@ -460,6 +460,28 @@ def test_flash_decode_op_long_context(pkg, store, B, ctx):
 
 # ---- recurrent (gated delta rule) step ---------------------------------------------------------------------
 
+@pytest.mark.parametrize("B,H,KV,D,ctx", [(13, 32, 8, 128, 1000), (41, 32, 8, 128, 519), (100, 8, 1, 64, 700), (25, 24, 8, 64, 2049), (19, 8, 8, 128, 512), (600, 4, 1, 128, 512)])
+def test_flash_decode_op_of_batches_that_fill_no_whole_round(pkg, store, B, H, KV, D, ctx):
+    """Blocks of all (sequence, KV head) pairs dealt evenly to the CTAs: pairs in one, two and three parts, several pairs per CTA, last
+    blocks of one row; against a PyTorch fp32 reference. Twice: the counters are zero again."""
+    import torch
+    lib, g = pkg.load_library(), torch.Generator(device="cuda").manual_seed(B + ctx)
+    q = torch.randn((B, H, D), device="cuda", generator=g).bfloat16()
+    k, v = (torch.randn((B, KV, ctx + 3, D), device="cuda", generator=g).bfloat16() for _ in range(2))
+    k[:, :, ctx:], v[:, :, ctx:] = float("nan"), float("nan")
+    scratch = torch.empty(lib.swlm_op_flash_decode_scratch_bytes(B, H, KV, D, ctx), device="cuda", dtype=torch.uint8)
+    qf, kf, vf = q.float().reshape(B, KV, H // KV, D), k[:, :, :ctx].float(), v[:, :, :ctx].float()
+    want = (torch.softmax(qf @ kf.transpose(2, 3) / D ** 0.5, dim=-1) @ vf).reshape(B, H, D)
+    for _ in range(2):
+        out = torch.full((B, H, D), float("nan"), device="cuda", dtype=torch.bfloat16)
+        torch.cuda.synchronize()
+        lib.check(lib.swlm_op_flash_decode_dev(store.handle, B, H, KV, D, ctx, ctx + 3, 1.0 / D ** 0.5, q.data_ptr(), k.data_ptr(), v.data_ptr(),
+                                               out.data_ptr(), scratch.data_ptr(), torch.cuda.current_stream().cuda_stream))
+        torch.cuda.synchronize()
+        # one rounding of the result to bf16 (2^-9 of itself), keys and weights as bf16 pairs (2^-16)
+        assert ((out.float() - want).abs() <= 2.0 ** -8 * want.abs() + 2.0 ** -12 * vf.abs().max()).all()
+
+
 @pytest.mark.parametrize("heads,groups,dk,dv,K,batch", [(4, 2, 16, 16, 4, 1), (32, 16, 128, 128, 4, 1), (8, 8, 64, 128, 3, 2),
                                                         (6, 2, 32, 64, 4, 3)])
 def test_ssm_recurrence_matches_oracle_over_steps(pkg, store, oracle, heads, groups, dk, dv, K, batch):
