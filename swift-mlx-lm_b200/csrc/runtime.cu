@@ -2036,6 +2036,15 @@ int swlm_state_set_prefill_chunk(swlm_state* s, int tokens) {
     return SWLM_OK;
 }
 
+int swlm_host_alloc(size_t bytes, void** out) {
+    if (!out || bytes == 0) { set_error("null argument"); return SWLM_ERR_INVALID; }
+    *out = nullptr;
+    const cudaError_t e = cudaHostAlloc(out, bytes, cudaHostAllocPortable);
+    if (e != cudaSuccess) { cudaGetLastError(); return cuda_fail(e, "cudaHostAlloc"); }
+    return SWLM_OK;
+}
+void swlm_host_free(void* p) { if (p) cudaFreeHost(p); }
+
 int swlm_read_buffer(swlm_state* s, int buf, uint16_t* dst, int count_per_row) {
     if (s && s->plan->stream()) { set_error("this plan keeps fp32 buffers: use the _f32 form"); return SWLM_ERR_UNSUPPORTED; }
     if (!s || !dst || !buf_ok(buf) || count_per_row > s->width[buf]) { set_error("bad buffer read"); return SWLM_ERR_INVALID; }

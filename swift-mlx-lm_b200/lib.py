@@ -162,6 +162,8 @@ SIGNATURES = {
     "swlm_read_tokens": (_I, [_P, _I, _P]),
     "swlm_sync": (_I, [_P]),
     "swlm_read_logits": (_I, [_P, _P, C.c_size_t]),
+    "swlm_host_alloc": (_I, [C.c_size_t, C.POINTER(_P)]),
+    "swlm_host_free": (None, [_P]),
     "swlm_read_buffer": (_I, [_P, _I, _P, _I]),
     "swlm_write_buffer": (_I, [_P, _I, _P, _I]),
     "swlm_read_kv": (_I, [_P, _I, _I, _I, _I, _I, _P]),

@@ -9,6 +9,9 @@ failed decode returns token -1 as `MetalDecodeExecutor` does (Execution/MetalDec
 from __future__ import annotations
 
 import ctypes as C
+import math
+import threading
+import weakref
 from typing import Optional, Sequence
 
 import numpy as np
@@ -93,6 +96,45 @@ class WeightStore:
         return out
 
 
+class ResultBlocks:
+    """Page-locked memory for large results that go to the caller as arrays. The copy from the GPU then runs at the bus's rate instead of
+    through the driver's staging (2 MB of logits: 57 us instead of 147). Two blocks, made with the model; a block is given out again when
+    nothing refers to its array, or to a view of it, any more. Results that do not fit, that are small, or that come while both blocks are
+    in use, lie in ordinary memory."""
+
+    COUNT, SMALLEST = 2, 1 << 20
+
+    def __init__(self, lib: Library, size: int):
+        self.lib, self.size, self.idle, self.lock, self.closed = lib, size, [], threading.Lock(), False
+        for _ in range(self.COUNT if size >= self.SMALLEST else 0):
+            block = C.c_void_p()
+            if lib.swlm_host_alloc(size, C.byref(block)) == 0:
+                self.idle.append(block.value)
+
+    def empty(self, shape, dtype) -> np.ndarray:
+        size = math.prod(shape) * np.dtype(dtype).itemsize
+        with self.lock:
+            at = self.idle.pop() if self.idle and self.SMALLEST <= size <= self.size else None
+        if at is None:
+            return np.empty(shape, dtype=dtype)
+        memory = (C.c_char * size).from_address(at)
+        weakref.finalize(memory, self._back, at).atexit = False
+        return np.frombuffer(memory, dtype=dtype).reshape(shape)
+
+    def _back(self, at: int) -> None:
+        with self.lock:
+            if not self.closed:
+                self.idle.append(at)
+                return
+        self.lib.swlm_host_free(at)
+
+    def close(self) -> None:
+        with self.lock:
+            self.closed, idle, self.idle = True, self.idle, []
+        for at in idle:
+            self.lib.swlm_host_free(at)
+
+
 class InferenceModel:
     """Compiled plan + one isolated runtime state."""
 
@@ -106,8 +148,11 @@ class InferenceModel:
         self.lib.check(self.lib.swlm_plan_build(store.handle, arr, len(steps), C.byref(desc), C.byref(self.plan)))
         self.state = C.c_void_p()
         self.lib.check(self.lib.swlm_state_create(self.plan, C.byref(self.state)))
+        self.results = ResultBlocks(self.lib, self.batch * int(desc.vocab) * (4 if desc.stream_dtype else 2))
 
     def close(self) -> None:
+        if getattr(self, "results", None):
+            self.results.close()
         if getattr(self, "state", None):
             self.lib.swlm_state_destroy(self.state)
             self.state = C.c_void_p()
@@ -184,10 +229,10 @@ class InferenceModel:
     def logits(self) -> np.ndarray:
         """[batch][vocab] of the last decode step: bf16 bit patterns, or fp32 for an fp32-stream plan."""
         if self.desc.stream_dtype:
-            out = np.empty((self.batch, int(self.desc.vocab)), dtype=np.float32)
+            out = self.results.empty((self.batch, int(self.desc.vocab)), np.float32)
             self.lib.check(self.lib.swlm_read_logits_f32(self.state, _ptr(out), out.size))
             return out
-        out = np.empty((self.batch, int(self.desc.vocab)), dtype=np.uint16)
+        out = self.results.empty((self.batch, int(self.desc.vocab)), np.uint16)
         self.lib.check(self.lib.swlm_read_logits(self.state, _ptr(out), out.size))
         return out
 
@@ -271,7 +316,7 @@ class InferenceModel:
         want_counts = np.array([len(e[2]) for e in entries], dtype=np.int32)
         wants = np.array([p for e in entries for p in e[2]] or [0], dtype=np.int32)
         n = int(want_counts.sum())
-        out = np.empty((n, int(self.desc.vocab)), dtype=np.float32) if logits else None
+        out = self.results.empty((n, int(self.desc.vocab)), np.float32) if logits else None
         greedy = np.empty(max(n, 1), dtype=np.int32)
         self.lib.check(self.lib.swlm_run_batch(self.state, len(entries), _ptr(seqs), _ptr(counts), _ptr(tokens), _ptr(want_counts), _ptr(wants),
                                                _ptr(out) if n and logits else None, _ptr(greedy) if n else None))

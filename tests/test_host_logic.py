@@ -340,3 +340,45 @@ def test_transformer_recipe_with_qk_norm(pkg, oracle):
         out.append(pkg.bf16_to_f32(m.read_buffer(P.BUF_LOGITS, base["vocab"]))[0].copy())
         assert 0 <= int(tok[0]) < base["vocab"]
     assert np.max(np.abs(out[0] - out[1])) > 1e-3
+
+
+def test_result_blocks_are_given_out_again_when_nothing_refers_to_them(pkg):
+    """Arrays over page-locked blocks (a stand-in for the library here): never two at a time on one block, views keep it, ordinary memory
+    when none is idle or the result does not fit, every block freed once whatever the order of close and the last array's end."""
+    import ctypes as C
+
+    import numpy as np
+
+    class Library:
+        def __init__(self):
+            self.live = {}
+
+        def swlm_host_alloc(self, size, out):
+            memory = C.create_string_buffer(size)
+            out._obj.value = C.addressof(memory)
+            self.live[C.addressof(memory)] = memory
+            return 0
+
+        def swlm_host_free(self, at):
+            del self.live[at]
+
+    lib = Library()
+    blocks = pkg.model.ResultBlocks(lib, 2 << 20)
+    a, b = blocks.empty((2, 1 << 19), np.uint16), blocks.empty((1 << 18,), np.float32)
+    where = {x.ctypes.data for x in (a, b)}
+    assert where == set(lib.live)
+    c = blocks.empty((1 << 20,), np.uint16)
+    assert c.ctypes.data not in where and blocks.empty((4,), np.uint16).ctypes.data not in where
+    view = a[1:].view(np.int16)
+    del a
+    assert blocks.empty((1 << 20,), np.uint16).ctypes.data not in where
+    del view
+    assert blocks.empty((1 << 22,), np.uint16).ctypes.data not in where   # larger than a block
+    d = blocks.empty((1 << 20,), np.uint16)
+    assert d.ctypes.data in where and d.ctypes.data != b.ctypes.data
+    del b
+    blocks.close()
+    assert set(lib.live) == {d.ctypes.data}
+    d[:] = 7
+    del d
+    assert not lib.live
