@@ -291,6 +291,30 @@ def test_qk_norm_swiglu_embed_argmax(pkg, store, oracle):
     gm.close()
 
 
+@pytest.mark.parametrize("batch,heads,kvh,hd", [(63, 3, 1, 64), (64, 1, 1, 64), (64, 31, 3, 64), (64, 24, 8, 128), (64, 5, 2, 128), (64, 4, 2, 32)])
+def test_qk_norm_of_many_rows(pkg, store, oracle, batch, heads, kvh, hd):
+    """From 64 rows on a CTA takes a whole row, four heads of a warp at a time: head counts on both sides of a round of 32, the last row count of
+    the few-row form and a head dimension that only it has."""
+    P = pkg.plan
+    gm, om = _mini(pkg, store, oracle, batch=batch, slot=4096, head_dim=hd, kv_heads=kvh)
+    rng = np.random.default_rng(hd + heads)
+    wq, wk = _bf(pkg, 1 + rng.normal(0, 0.1, size=hd)), _bf(pkg, 1 + rng.normal(0, 0.1, size=hd))
+    name = f"rows{batch}.{heads}.{hd}."
+    for mdl in (store, om):
+        mdl.add_dense(name + "q", wq)
+        mdl.add_dense(name + "k", wk)
+    q, k = _bf(pkg, rng.normal(size=(batch, heads * hd))), _bf(pkg, rng.normal(size=(batch, kvh * hd)))
+    step = P._step(P.STEP_QK_NORM, in_buf=P.BUF_S1, in2_buf=P.BUF_S2, heads=heads, kv_heads=kvh, head_dim=hd, eps=1e-5, weight_bias=0.5,
+                   weight=name + "q", weight2=name + "k")
+    for mdl in (gm, om):
+        mdl.write_buffer(P.BUF_S1, q)
+        mdl.write_buffer(P.BUF_S2, k)
+        mdl.run_step(step)
+    for buf, cnt in ((P.BUF_S1, heads * hd), (P.BUF_S2, kvh * hd)):
+        assert rel_err(pkg.bf16_to_f32(gm.read_buffer(buf, cnt)), pkg.bf16_to_f32(om.read_buffer(buf, cnt))).max() <= RTOL
+    gm.close()
+
+
 def test_argmax_full_vocab(pkg, store, oracle):
     P = pkg.plan
     vocab = 128256
