@@ -249,6 +249,11 @@ template <bool F16SB>
 __device__ __forceinline__ void tc_appended(const QGemmTcParams& p, int rt, int blk, unsigned (&a)[16]) {
     const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     const int plane = blk % 3, st0 = blk / 3 * 16;   // four groups per 16-byte entry
+    if (st0 >= p.kt / 4) {   // (padding to whole steps)
+#pragma unroll
+        for (int i = 0; i < 16; ++i) a[i] = 0u;
+        return;
+    }
 #pragma unroll
     for (int j = 0; j < 4; ++j)
 #pragma unroll
@@ -390,10 +395,19 @@ __device__ __forceinline__ bool tc_dequant(const QGemmTcParams& p, TcBars<STAGES
         }
         for (; kt < hi && ok; kt += 2) {
             if (!begin()) { ok = false; break; }
+            const int blk = (kt - p.real_steps) * (kTcStep / 64), rt = rt_of(tile) + own_rt;
+            if (blk % 3 == 0 && rt < p.row_tiles) {   // hi and lo of the same groups
+                unsigned a[16], a_lo[16];
+                tc_appended_pair<F16SB>(p, rt, blk / 3, a, a_lo);
+                tmem_st_frag(a_dst + (unsigned)a_slot * 64u, a);
+                tmem_st_frag(a_dst + (unsigned)a_slot * 64u + 32u, a_lo);
+                if (!finish()) ok = false;
+                continue;
+            }
 #pragma unroll 1
             for (int half = 0; half < 2; ++half) {
                 unsigned a[16];
-                tc_appended<F16SB>(p, rt_of(tile) + own_rt, (kt - p.real_steps) * (kTcStep / 64) + half, a);
+                tc_appended<F16SB>(p, rt, blk + half, a);
                 tmem_st_frag(a_dst + (unsigned)a_slot * 64u + half * 32u, a);
             }
             if (!finish()) ok = false;
