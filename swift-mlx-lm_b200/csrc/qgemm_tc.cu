@@ -1038,8 +1038,9 @@ __global__ void __launch_bounds__(kSlThreads, 1) qgemm_slab_kernel(const QGemmTc
 // factor. Within a group of 64 column 16 t + 4 j + i goes to place 16 j + 4 t + i, the order of the weights' fragments. Behind the k
 // values (and zeros up to the weights' padding) the row gets, for every 64 groups, three blocks of 64 columns: sum / 64 of every group of 64 converted values as an fp16
 // pair, laid out (hi, hi, lo) to meet the (c_hi, c_lo, c_hi) blocks of the weight side; the rest is zeros.
-// HOLD: a row of up to 16384 values stays in registers between the two passes (reading 4 bytes per lane twice took 24 us for
-// 2048 x 4096 under ncu, this takes 15).
+// CH: eights of a row per thread, held in registers between the two passes (reading 4 bytes per lane twice took 24 us for 2048 x 4096 under
+// ncu); 0: a row of more than 16384 values is read twice. Few rows want short chains: two eights and up to 1024 threads; many rows want
+// all of them resident at once and no warp without work: four eights. 2010 rows of 2048: 6.4 us under ncu, of 256 threads 9.4.
 struct F16Rows { int k, k_pad; __half* xh; int stride; float* rscale; };   // columns, padded; the copy and its pitch
 // bf16 magnitudes order like their bit patterns: two 16-bit maxima at a time
 __device__ __forceinline__ unsigned f16_top(unsigned mx, const uint4& v) {
@@ -1052,8 +1053,7 @@ __device__ __forceinline__ int f16_shift(unsigned mx, unsigned* red) {
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = mx;
     __syncthreads();
     mx = 0;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) mx = max(mx, red[i]);
+    for (int i = 0; i < (int)(blockDim.x >> 5); ++i) mx = max(mx, red[i]);
     const int e = (int)(mx >> 7);                                   // biased exponent of the largest magnitude
     return (e == 0 || e == 255) ? 0 : max(-100, min(100, 141 - e));
 }
@@ -1087,106 +1087,117 @@ __device__ __forceinline__ void f16_put(const F16Rows& f, __half* out, int i, co
 }
 // what lies behind the values and behind the last group
 __device__ __forceinline__ void f16_pad(const F16Rows& f, __half* out, int row, int sh) {
-    for (int i = f.k + threadIdx.x; i < f.k_pad; i += 256) out[i] = __ushort_as_half(0);
+    for (int i = f.k + threadIdx.x; i < f.k_pad; i += blockDim.x) out[i] = __ushort_as_half(0);
     const int groups = f.k / 64;
-    for (int i = threadIdx.x; i < f.stride - f.k_pad; i += 256)
+    for (int i = threadIdx.x; i < f.stride - f.k_pad; i += blockDim.x)
         if (i / 192 * 64 + (i & 63) >= groups) out[f.k_pad + i] = __ushort_as_half(0);
     if (threadIdx.x == 0) f.rscale[row] = __uint_as_float((unsigned)(127 - sh) << 23);
 }
 
-template <bool HOLD>
-__global__ void __launch_bounds__(256) x_to_f16_kernel(const __nv_bfloat16* x, int x_stride, const F16Rows f) {
+constexpr int f16_max_threads(int ch) { return ch == 4 ? 512 : ch == 2 ? 1024 : 256; }
+constexpr int kF16FewRows = 296;   // two per SM
+int f16_threads(int k, int ch) { return ch ? (k / 8 + 32 * ch - 1) / (32 * ch) * 32 : 256; }
+
+template <int CH>
+__global__ void __launch_bounds__(f16_max_threads(CH)) x_to_f16_kernel(const __nv_bfloat16* x, int x_stride, const F16Rows f) {
     pdl_launch_dependents();
     pdl_wait();
-    constexpr int CH = HOLD ? 8 : 1;
-    __shared__ unsigned red[8];
-    const int row = blockIdx.x, tid = threadIdx.x, n8 = f.k / 8;
+    __shared__ unsigned red[32];
+    const int row = blockIdx.x, tid = threadIdx.x, n8 = f.k / 8, nt = blockDim.x;
     const uint4* src = reinterpret_cast<const uint4*>(x + (size_t)row * x_stride);
-    uint4 held[CH];
+    uint4 held[CH ? CH : 1];
     unsigned mx = 0;
-    if (HOLD) {
+    if (CH) {
 #pragma unroll
         for (int c = 0; c < CH; ++c) {
             held[c] = make_uint4(0, 0, 0, 0);
-            if (tid + c * 256 < n8) held[c] = src[tid + c * 256];
+            if (tid + c * nt < n8) held[c] = src[tid + c * nt];
         }
 #pragma unroll
         for (int c = 0; c < CH; ++c) mx = f16_top(mx, held[c]);
     } else {
-        for (int i = tid; i < n8; i += 256) mx = f16_top(mx, src[i]);
+        for (int i = tid; i < n8; i += nt) mx = f16_top(mx, src[i]);
     }
     const int sh = f16_shift(mx, red);
     const float mul = __uint_as_float((unsigned)(127 + sh) << 23);  // 2^sh
     __half* out = f.xh + (size_t)row * f.stride;
-    if (HOLD) {
+    if (CH) {
 #pragma unroll
         for (int c = 0; c < CH; ++c)
-            if (tid + c * 256 < n8) f16_put(f, out, tid + c * 256, held[c], mul);
+            if (tid + c * nt < n8) f16_put(f, out, tid + c * nt, held[c], mul);
     } else {
-        for (int i = tid; i < n8; i += 256) f16_put(f, out, i, src[i], mul);
+        for (int i = tid; i < n8; i += nt) f16_put(f, out, i, src[i], mul);
     }
     f16_pad(f, out, row, sh);
 }
 
 // A norm step (see rmsnorm_kernel) whose result goes to its buffer and, converted, to the product behind it: one pass instead of two
-// launches. MODE: 0 copy, 1 residual add and copy, 2 residual add.
-template <int MODE>
-__global__ void __launch_bounds__(256) norm_to_f16_kernel(const __nv_bfloat16* in, int in_stride, __nv_bfloat16* residual, int res_stride, const __nv_bfloat16* weight,
-                                                          float eps, float weight_bias, __nv_bfloat16* y, int y_stride, const F16Rows f) {
+// launches. MODE: 0 copy, 1 residual add and copy, 2 residual add. A row stays in registers, its weights come before the wait for the
+// kernel in front; CH as above. 2010 rows of 2048: 9.9 us under ncu; with 256 threads, the row in shared memory and the weights behind the
+// first sum 11.3. A decode step of 41 sequences of the 8B transformer is 5 % faster for both, a prompt 1 to 2 %.
+template <int MODE, int CH>
+__global__ void __launch_bounds__(f16_max_threads(CH)) norm_to_f16_kernel(const __nv_bfloat16* in, int in_stride, __nv_bfloat16* residual, int res_stride,
+                                                                          const __nv_bfloat16* weight, float eps, float weight_bias, __nv_bfloat16* y, int y_stride,
+                                                                          const F16Rows f) {
     pdl_launch_dependents();
+    __shared__ unsigned red[32];
+    __shared__ float sums[32];
+    const int row = blockIdx.x, tid = threadIdx.x, n8 = f.k / 8, nt = blockDim.x;
+    auto pack = [](float a, float b) { const __nv_bfloat162 v = __floats2bfloat162_rn(a, b); return *reinterpret_cast<const unsigned*>(&v); };
+    uint4 w[CH], v[CH], r[CH];
+#pragma unroll
+    for (int c = 0; c < CH; ++c) {
+        w[c] = make_uint4(0, 0, 0, 0);
+        if (tid + c * nt < n8) w[c] = reinterpret_cast<const uint4*>(weight)[tid + c * nt];
+    }
     pdl_wait();
-    extern __shared__ __align__(16) float norm_h[];   // the unrounded row, then the rounded one in its place (a thread's own eights)
-    __shared__ unsigned red[8];
-    __shared__ float sums[8];
-    const int row = blockIdx.x, tid = threadIdx.x, n8 = f.k / 8;
     const uint4* in4 = reinterpret_cast<const uint4*>(in + (size_t)row * in_stride);
     uint4* res4 = reinterpret_cast<uint4*>(residual + (size_t)row * res_stride);
-    auto pack = [](float a, float b) { const __nv_bfloat162 v = __floats2bfloat162_rn(a, b); return *reinterpret_cast<const unsigned*>(&v); };
-    float ss = 0.f;
-    for (int i = tid; i < n8; i += 256) {
-        const uint4 v = in4[i];
-        const unsigned u[4] = {v.x, v.y, v.z, v.w};
-        float h[8];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) { h[2 * j] = __uint_as_float(u[j] << 16); h[2 * j + 1] = __uint_as_float(u[j] & 0xFFFF0000u); }
-        if (MODE != 0) {
-            const uint4 r = res4[i];
-            const unsigned q[4] = {r.x, r.y, r.z, r.w};
+    for (int c = 0; c < CH; ++c) {
+        v[c] = r[c] = make_uint4(0, 0, 0, 0);
+        if (tid + c * nt < n8) { v[c] = in4[tid + c * nt]; if (MODE != 0) r[c] = res4[tid + c * nt]; }
+    }
+    float h[CH][8], ss = 0.f;
 #pragma unroll
-            for (int j = 0; j < 4; ++j) { h[2 * j] += __uint_as_float(q[j] << 16); h[2 * j + 1] += __uint_as_float(q[j] & 0xFFFF0000u); }
+    for (int c = 0; c < CH; ++c) {
+        const unsigned u[4] = {v[c].x, v[c].y, v[c].z, v[c].w}, q[4] = {r[c].x, r[c].y, r[c].z, r[c].w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            h[c][2 * j] = __uint_as_float(u[j] << 16); h[c][2 * j + 1] = __uint_as_float(u[j] & 0xFFFF0000u);
+            if (MODE != 0) { h[c][2 * j] += __uint_as_float(q[j] << 16); h[c][2 * j + 1] += __uint_as_float(q[j] & 0xFFFF0000u); }
         }
-        if (MODE != 2) res4[i] = make_uint4(pack(h[0], h[1]), pack(h[2], h[3]), pack(h[4], h[5]), pack(h[6], h[7]));
+        if (MODE != 2 && tid + c * nt < n8)
+            res4[tid + c * nt] = make_uint4(pack(h[c][0], h[c][1]), pack(h[c][2], h[c][3]), pack(h[c][4], h[c][5]), pack(h[c][6], h[c][7]));
 #pragma unroll
-        for (int e = 0; e < 8; ++e) ss = fmaf(h[e], h[e], ss);
-        reinterpret_cast<float4*>(norm_h)[2 * i] = make_float4(h[0], h[1], h[2], h[3]);
-        reinterpret_cast<float4*>(norm_h)[2 * i + 1] = make_float4(h[4], h[5], h[6], h[7]);
+        for (int e = 0; e < 8; ++e) ss = fmaf(h[c][e], h[c][e], ss);
     }
     for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
     if ((tid & 31) == 0) sums[tid >> 5] = ss;
     __syncthreads();
     float total = 0.f;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) total += sums[i];
+    for (int i = 0; i < (nt >> 5); ++i) total += sums[i];
     const float rs = rsqrtf(total / (float)f.k + eps);
     unsigned mx = 0;
-    for (int i = tid; i < n8; i += 256) {
-        const uint4 w = reinterpret_cast<const uint4*>(weight)[i];
-        const unsigned u[4] = {w.x, w.y, w.z, w.w};
-        const float4 a = reinterpret_cast<const float4*>(norm_h)[2 * i], b = reinterpret_cast<const float4*>(norm_h)[2 * i + 1];
-        const float h[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+#pragma unroll
+    for (int c = 0; c < CH; ++c) {
+        const unsigned u[4] = {w[c].x, w[c].y, w[c].z, w[c].w};
         unsigned o[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j)
-            o[j] = pack(h[2 * j] * rs * (__uint_as_float(u[j] << 16) + weight_bias), h[2 * j + 1] * rs * (__uint_as_float(u[j] & 0xFFFF0000u) + weight_bias));
-        const uint4 v = make_uint4(o[0], o[1], o[2], o[3]);
-        reinterpret_cast<uint4*>(y + (size_t)row * y_stride)[i] = v;
-        reinterpret_cast<uint4*>(norm_h)[2 * i] = v;
-        mx = f16_top(mx, v);
+            o[j] = pack(h[c][2 * j] * rs * (__uint_as_float(u[j] << 16) + weight_bias), h[c][2 * j + 1] * rs * (__uint_as_float(u[j] & 0xFFFF0000u) + weight_bias));
+        v[c] = make_uint4(o[0], o[1], o[2], o[3]);
+        if (tid + c * nt < n8) {
+            reinterpret_cast<uint4*>(y + (size_t)row * y_stride)[tid + c * nt] = v[c];
+            mx = f16_top(mx, v[c]);
+        }
     }
     const int sh = f16_shift(mx, red);
     const float mul = __uint_as_float((unsigned)(127 + sh) << 23);
     __half* out = f.xh + (size_t)row * f.stride;
-    for (int i = tid; i < n8; i += 256) f16_put(f, out, i, reinterpret_cast<const uint4*>(norm_h)[2 * i], mul);
+#pragma unroll
+    for (int c = 0; c < CH; ++c)
+        if (tid + c * nt < n8) f16_put(f, out, tid + c * nt, v[c], mul);
     f16_pad(f, out, row, sh);
 }
 
@@ -1321,9 +1332,7 @@ int qgemm_tc_init() {
         (rc = tc_init_one(qgemm_tc_short_kernel<128, kTcStages128, false>, tc_smem_bytes(128, kTcStages128))) ||
         (rc = tc_init_one(qgemm_tc_short_kernel<128, kTcStages128, true>, tc_smem_bytes(128, kTcStages128))) ||
         (rc = tc_init_one(qgemm_tc_kernel<kTcStagesPair, false>, tc_smem_bytes(kTcPairRows, kTcStagesPair))) ||
-        (rc = tc_init_one(qgemm_tc_kernel<kTcStagesPair, true>, tc_smem_bytes(kTcPairRows, kTcStagesPair))) ||
-        (rc = tc_init_one(norm_to_f16_kernel<0>, (size_t)kNormMaxDim * 4)) || (rc = tc_init_one(norm_to_f16_kernel<1>, (size_t)kNormMaxDim * 4)) ||
-        (rc = tc_init_one(norm_to_f16_kernel<2>, (size_t)kNormMaxDim * 4))) return rc;
+        (rc = tc_init_one(qgemm_tc_kernel<kTcStagesPair, true>, tc_smem_bytes(kTcPairRows, kTcStagesPair)))) return rc;
     return SWLM_OK;
 }
 
@@ -1344,11 +1353,14 @@ int launch_norm_to_f16(int mode, int m, int dim, const __nv_bfloat16* in, int in
                        float eps, float weight_bias, __nv_bfloat16* out, int out_stride, void* scratch, cudaStream_t s) {
     if (dim % 64 || in_stride % 8 || res_stride % 8 || out_stride % 8 || dim > kNormMaxDim) { set_error("rmsnorm: dim=%d", dim); return SWLM_ERR_INVALID; }
     const F16Rows f = f16_rows(m, dim, scratch);
-    const size_t smem = (size_t)dim * 4;
+    const int ch = m <= kF16FewRows ? 2 : 4;
+    auto go = [&](auto kernel) {
+        return launch_k(kernel, dim3((unsigned)m), dim3((unsigned)f16_threads(dim, ch)), 0, s, in, in_stride, residual, res_stride, weight, eps, weight_bias, out, out_stride, f);
+    };
     cudaError_t e;
-    if (mode == SWLM_STEP_COPY_RMSNORM) e = launch_k(norm_to_f16_kernel<0>, dim3((unsigned)m), dim3(256), smem, s, in, in_stride, residual, res_stride, weight, eps, weight_bias, out, out_stride, f);
-    else if (mode == SWLM_STEP_RESADD_COPY_RMSNORM) e = launch_k(norm_to_f16_kernel<1>, dim3((unsigned)m), dim3(256), smem, s, in, in_stride, residual, res_stride, weight, eps, weight_bias, out, out_stride, f);
-    else e = launch_k(norm_to_f16_kernel<2>, dim3((unsigned)m), dim3(256), smem, s, in, in_stride, residual, res_stride, weight, eps, weight_bias, out, out_stride, f);
+    if (mode == SWLM_STEP_COPY_RMSNORM) e = ch == 2 ? go(norm_to_f16_kernel<0, 2>) : go(norm_to_f16_kernel<0, 4>);
+    else if (mode == SWLM_STEP_RESADD_COPY_RMSNORM) e = ch == 2 ? go(norm_to_f16_kernel<1, 2>) : go(norm_to_f16_kernel<1, 4>);
+    else e = ch == 2 ? go(norm_to_f16_kernel<2, 2>) : go(norm_to_f16_kernel<2, 4>);
     return e == cudaSuccess ? SWLM_OK : cuda_fail(e, "norm_to_f16 launch");
 }
 
@@ -1374,8 +1386,9 @@ int launch_qgemm_tc(const Q4Tiled& w, int m, const __nv_bfloat16* x, int x_strid
     for (int q = out.count; q < 3; ++q) p.out.end[q] = p.out.end[out.count - 1];   // never stored to
     // (reuse_x: the scratch still holds the copy of these very rows, made for the product before this one or by their norm)
     if (!reuse_x) {
-        const cudaError_t e = w.k <= 16384 ? launch_k(x_to_f16_kernel<true>, dim3((unsigned)m), dim3(256), 0, s, x, x_stride, f)
-                                           : launch_k(x_to_f16_kernel<false>, dim3((unsigned)m), dim3(256), 0, s, x, x_stride, f);
+        const int ch = w.k > 16384 ? 0 : m <= kF16FewRows ? 2 : 4;
+        auto go = [&](auto kernel) { return launch_k(kernel, dim3((unsigned)m), dim3((unsigned)f16_threads(w.k, ch)), 0, s, x, x_stride, f); };
+        const cudaError_t e = ch == 0 ? go(x_to_f16_kernel<0>) : ch == 2 ? go(x_to_f16_kernel<2>) : go(x_to_f16_kernel<4>);
         if (e != cudaSuccess) return cuda_fail(e, "x_to_f16 launch");
     }
     if (m <= 64) {

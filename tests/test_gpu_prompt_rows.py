@@ -236,6 +236,45 @@ def test_norms_of_the_widest_rows(pkg, oracle, width):
     model.close(), store.close()
 
 
+@pytest.mark.parametrize("tokens", [296, 297])
+@pytest.mark.parametrize("width", [64, 2368])
+def test_norms_of_a_portion(pkg, oracle, width, tokens):
+    """Norms that write a product's fp16 rows, with and without a residual: two and four eights of a row per thread on both sides of the
+    line between them, a row of one warp and one whose last eights fill a warp in part. Their rows are read as a layer's cached values."""
+    P, vocab, hd = pkg.plan, 304, 64
+    rng = np.random.default_rng(width)
+    desc = pkg.BuffersDesc(hidden=width, slot_dim=width, vocab=vocab, max_seq=tokens + 8, max_batch=1, kv_layers=1, kv_heads=1, head_dim=hd)
+    store = pkg.WeightStore(0)
+    table, weight = _bf(pkg, rng.normal(size=(vocab, width))), _bf(pkg, 1 + 0.1 * rng.normal(size=width))
+    store.add_dense("rows", table), store.add_dense("norm", weight)
+    q4 = {n: pkg.synth_q4(r, c, seed=i, centered=True) for i, (n, r, c) in enumerate((("mix", width, width), ("q", hd, width), ("k", hd, width), ("v", hd, width), ("head", vocab, hd)))}
+    for n, v in q4.items():
+        store.add_q4_mlx(n, *v)
+    norm_step = dict(in_buf=P.BUF_HIDDEN, out_buf=P.BUF_S0, n=width, eps=1e-5, weight="norm")
+    steps = [P._step(P.STEP_EMBED, out_buf=P.BUF_HIDDEN, n=width, weight="rows"),
+             P._step(P.STEP_COPY_RMSNORM, **norm_step),
+             P._step(P.STEP_QGEMV, in_buf=P.BUF_S0, out_buf=P.BUF_HIDDEN, n=width, k=width, weight="mix"),
+             P._step(P.STEP_RESADD_COPY_RMSNORM, **norm_step)]
+    steps += [P._step(P.STEP_QGEMV, in_buf=P.BUF_S0, out_buf=buf, n=hd, k=width, weight=n) for n, buf in (("q", P.BUF_S1), ("k", P.BUF_S2), ("v", P.BUF_S3))]
+    steps += [P._step(P.STEP_ATTN_DECODE, layer=0, in_buf=P.BUF_S1, in2_buf=P.BUF_S2, in3_buf=P.BUF_S3, out_buf=P.BUF_S0, heads=1, kv_heads=1, head_dim=hd, scale=hd ** -0.5),
+              P._step(P.STEP_QGEMV, in_buf=P.BUF_S0, out_buf=P.BUF_LOGITS, n=vocab, k=hd, weight="head"),
+              P._step(P.STEP_ARGMAX, in_buf=P.BUF_LOGITS, n=vocab)]
+
+    def norm(h):
+        return pkg.f32_to_bf16((h / np.sqrt((h * h).mean(1, keepdims=True) + 1e-5) * pkg.bf16_to_f32(weight)).astype(np.float32))
+
+    ids = rng.integers(0, vocab, size=tokens + 1)   # (the last token takes the single step)
+    x = pkg.bf16_to_f32(table[ids[:-1]])
+    mixed = pkg.bf16_to_f32(oracle.qgemm(norm(x), *q4["mix"]))
+    ref = pkg.bf16_to_f32(oracle.qgemm(norm(x + mixed), *q4["v"]))
+    model = pkg.InferenceModel(store, steps, desc)
+    model.set_prefill_chunk(tokens)
+    model.prefill_sequence(0, ids)
+    got = pkg.bf16_to_f32(model.read_kv(1, 0, 0, 0, tokens))
+    assert np.abs(got - ref).max() <= 2e-2 * np.abs(ref).max()   # four bf16 roundings of 2^-9 in front of the sums
+    model.close(), store.close()
+
+
 def test_gate_values_that_are_partly_overwritten_and_read(pkg, oracle):
     """Behind the activation something overwrites half of the gate's values and a product reads all of them: in a step of 20 sequences the
     other half is what the gate's product left there."""

@@ -148,6 +148,20 @@ def test_products_of_17_to_64_rows(pkg, oracle, n, k, m):
     store.close()
 
 
+@pytest.mark.parametrize("m", [296, 297])
+@pytest.mark.parametrize("k", [64, 2368, 16384, 16448])
+def test_rows_of_a_product_as_fp16(pkg, oracle, k, m):
+    """Rows on their way to fp16: two and four eights of a row per thread on both sides of the line between them, a row of one warp, one whose
+    last eights fill a warp in part, the longest that stays in registers and one that is read twice."""
+    n = 48
+    store = pkg.WeightStore(0)
+    w, s, b = pkg.synth_q4(n, k, seed=n + k, centered=True)
+    x = pkg.f32_to_bf16(np.random.default_rng(m).normal(size=(m, k)).astype(np.float32))
+    store.add_q4_mlx("mlx", w, s, b)
+    assert rel_err(pkg.bf16_to_f32(store.qgemm("mlx", x, n)), pkg.bf16_to_f32(oracle.qgemm(x, w, s, b))).max() <= RTOL
+    store.close()
+
+
 @pytest.mark.parametrize("m,ff,k", [(24, 512, 9216), (40, 19008, 320), (64, 64, 576)])
 def test_gated_products_of_17_to_64_rows(pkg, oracle, m, ff, k):
     """The same with gate and up together: two CTAs along K, more than one pass, fewer row tiles than SMs."""
