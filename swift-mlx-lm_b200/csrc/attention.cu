@@ -1100,9 +1100,10 @@ int attn_pick_splits(int m, int kv_heads, int max_ctx, bool ragged) {
 size_t attn_scratch_floats(int m, int heads, int head_dim, int splits) {
     return (size_t)m * heads * splits * (head_dim + 2);
 }
+// What either form needs from 100 pairs on: scratch taken for a longer context or for more sequences serves what it served without MODE 4.
 size_t flash_scratch_floats(int m, int heads, int kv_heads, int hd, int ctx_len) {
     const size_t apart = attn_scratch_floats(m, heads, hd, attn_pick_splits(m, kv_heads, ctx_len));
-    return attn_streams(m, kv_heads, ctx_len) ? std::max(apart, (size_t)2 * stream_ctas(m * kv_heads) * (heads / kv_heads) * (hd + 2)) : apart;
+    return (long long)m * kv_heads >= 100 ? std::max(apart, (size_t)2 * kStreamCtas * (heads / kv_heads) * (hd + 2)) : apart;
 }
 
 static int check_group(int heads, int kv_heads) {

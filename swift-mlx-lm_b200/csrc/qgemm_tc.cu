@@ -26,10 +26,10 @@
 // What bounded the kernel this one replaced (one group per step, weights by TMA as 128 rows of 32 bytes, one tile per CTA): the L2
 // traffic of 256 activation rows per 128 weight rows (with seven of eight MMAs left out 2048 x 28672 x 4096 still took 411 of
 // 509 us, 10.7 TB/s), 512 arrivals per group, eight MMAs issued by a lone lane (470 to 850 clocks), and two waves of CTAs, the second
-// half empty. What bounds it now: the MMAs of the long form (about 0.65 of their rate under the power cap), dequantising in the short one.
-// Measured: 14336 x 4096 at 512 rows 88 -> 63 us (950 TFLOP/s); 28672 x 4096 at 2048 rows 705 us under ncu -> 442 us (1090 TFLOP/s);
-// 28672 x 4096 at 41 rows 68 us under ncu -> 38 us (28 with the form of few rows); 14336 -> 4096 at 41 rows 50.7 + 8.8 (a second
-// launch) -> 30 us (23.5).
+// half empty. What bounds it now: the MMAs of the long form (about 0.7 of their rate under the power cap, one and a half waves of tiles at
+// 512 rows), dequantising in the short one. 17 to 64 rows have a kernel of their own (qgemm_slab_kernel).
+// Measured: 14336 x 4096 at 512 rows 88 -> 65 us, with results stored by rows, appended columns in blocks and a test in front of every
+// wait 57 (1050 TFLOP/s); 28672 x 4096 at 2048 rows 705 us under ncu -> 442 us with pairs of SMs.
 //
 // Every mbarrier wait is bounded: on expiry an error word is set, the CTA stops issuing, waits (bounded) for the copies and MMAs
 // it has in flight, frees its TMEM and returns.
