@@ -8,9 +8,9 @@ failed decode returns token -1 as `MetalDecodeExecutor` does (Execution/MetalDec
 """
 from __future__ import annotations
 
+import collections
 import ctypes as C
 import math
-import threading
 import weakref
 from typing import Optional, Sequence
 
@@ -105,7 +105,9 @@ class ResultBlocks:
     COUNT, SMALLEST = 2, 1 << 20
 
     def __init__(self, lib: Library, size: int):
-        self.lib, self.size, self.idle, self.lock, self.closed = lib, size, [], threading.Lock(), False
+        # No lock: a collection that ends an array may start anywhere in these functions, in the same thread. A block is in one place at a
+        # time, and a deque's `append` and `pop` are single steps for other threads and for collections alike.
+        self.lib, self.size, self.idle, self.closed = lib, size, collections.deque(), False
         for _ in range(self.COUNT if size >= self.SMALLEST else 0):
             block = C.c_void_p()
             if lib.swlm_host_alloc(size, C.byref(block)) == 0:
@@ -113,26 +115,31 @@ class ResultBlocks:
 
     def empty(self, shape, dtype) -> np.ndarray:
         size = math.prod(shape) * np.dtype(dtype).itemsize
-        with self.lock:
-            at = self.idle.pop() if self.idle and self.SMALLEST <= size <= self.size else None
+        at = self._take() if self.SMALLEST <= size <= self.size else None
         if at is None:
             return np.empty(shape, dtype=dtype)
         memory = (C.c_char * size).from_address(at)
         weakref.finalize(memory, self._back, at).atexit = False
         return np.frombuffer(memory, dtype=dtype).reshape(shape)
 
+    def _take(self) -> Optional[int]:
+        try:
+            return self.idle.pop()
+        except IndexError:
+            return None
+
     def _back(self, at: int) -> None:
-        with self.lock:
-            if not self.closed:
-                self.idle.append(at)
-                return
-        self.lib.swlm_host_free(at)
+        self.idle.append(at)
+        if self.closed:   # (closed only now: whoever takes the block first frees it)
+            self._free()
+
+    def _free(self) -> None:
+        while (at := self._take()) is not None:
+            self.lib.swlm_host_free(at)
 
     def close(self) -> None:
-        with self.lock:
-            self.closed, idle, self.idle = True, self.idle, []
-        for at in idle:
-            self.lib.swlm_host_free(at)
+        self.closed = True
+        self._free()
 
 
 class InferenceModel:

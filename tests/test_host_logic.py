@@ -342,27 +342,30 @@ def test_transformer_recipe_with_qk_norm(pkg, oracle):
     assert np.max(np.abs(out[0] - out[1])) > 1e-3
 
 
+class HostMemory:
+    """The library's page-locked blocks out of ordinary memory."""
+
+    def __init__(self):
+        self.live = {}
+
+    def swlm_host_alloc(self, size, out):
+        import ctypes as C
+
+        memory = C.create_string_buffer(size)
+        out._obj.value = C.addressof(memory)
+        self.live[C.addressof(memory)] = memory
+        return 0
+
+    def swlm_host_free(self, at):
+        del self.live[at]
+
+
 def test_result_blocks_are_given_out_again_when_nothing_refers_to_them(pkg):
     """Arrays over page-locked blocks (a stand-in for the library here): never two at a time on one block, views keep it, ordinary memory
     when none is idle or the result does not fit, every block freed once whatever the order of close and the last array's end."""
-    import ctypes as C
-
     import numpy as np
 
-    class Library:
-        def __init__(self):
-            self.live = {}
-
-        def swlm_host_alloc(self, size, out):
-            memory = C.create_string_buffer(size)
-            out._obj.value = C.addressof(memory)
-            self.live[C.addressof(memory)] = memory
-            return 0
-
-        def swlm_host_free(self, at):
-            del self.live[at]
-
-    lib = Library()
+    lib = HostMemory()
     blocks = pkg.model.ResultBlocks(lib, 2 << 20)
     a, b = blocks.empty((2, 1 << 19), np.uint16), blocks.empty((1 << 18,), np.float32)
     where = {x.ctypes.data for x in (a, b)}
@@ -381,4 +384,41 @@ def test_result_blocks_are_given_out_again_when_nothing_refers_to_them(pkg):
     assert set(lib.live) == {d.ctypes.data}
     d[:] = 7
     del d
+    assert not lib.live
+
+
+def test_result_blocks_when_a_collection_ends_an_array(pkg):
+    """Arrays left in reference cycles end wherever a collection starts, in the middle of giving out the next one or of closing too: no call
+    waits for itself, and every block is freed once."""
+    import gc
+    import threading
+
+    import numpy as np
+
+    lib, done = HostMemory(), []
+
+    def work():
+        for start in range(20):
+            blocks = pkg.model.ResultBlocks(lib, 1 << 20)
+            for i in range(400):
+                if i % 5 == 0:
+                    cycle = [blocks.empty((1 << 20,), np.uint8)]
+                    cycle.append(cycle)
+                    del cycle
+                    gc.set_threshold(1 + (start + i // 5) % 40)   # (the collection that ends it starts at another place each time)
+                blocks.empty((1 << 20,), np.uint8)
+            blocks.close()
+            done.append(None)
+
+    thresholds = gc.get_threshold()
+    gc.freeze()
+    try:
+        worker = threading.Thread(target=work, daemon=True)
+        worker.start()
+        worker.join(30)
+    finally:
+        gc.set_threshold(*thresholds)
+        gc.unfreeze()
+    assert len(done) == 20
+    gc.collect()
     assert not lib.live
