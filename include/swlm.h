@@ -150,7 +150,7 @@ int swlm_sync(swlm_state* state);
  * (Sources/SwiftLM/LanguageModelContext.swift:2197-2209): bf16 [max_batch][vocab]. */
 int swlm_read_logits(swlm_state* state, uint16_t* dst, size_t count);
 /* Page-locked host memory for results (any of the calls that copy to the host take it as `dst`): copies run at the bus's
- * rate, and belong to no state. */
+ * rate, and belong to no state. Leaves the calling thread on the device of the context made last. */
 int swlm_host_alloc(size_t bytes, void** out);
 void swlm_host_free(void* p);
 /* Copy a logical buffer (SWLM_BUF_*) to the host: [max_batch][count_per_row] bf16.

@@ -8,6 +8,7 @@
 // Where the reference encodes and commits a command buffer per token and blocks on it, this runtime
 // captures the whole step into one CUDA graph and keeps position, input token and output token on
 // the device, so consecutive greedy steps need no host round trip.
+#include <atomic>
 #include <cstdarg>
 #include <cstdio>
 #include <cstdlib>
@@ -1362,6 +1363,10 @@ int swlm_device_count(void) {
     return n;
 }
 
+// The device of the context made last: one that is set up. Page-locked memory is good for all devices, but a thread that has not chosen one
+// would set the first one up for it.
+static std::atomic<int> g_used_device{-1};
+
 int swlm_ctx_create(int device_id, int tp_rank, int tp_size, swlm_ctx** out) {
     if (!out) { set_error("null out"); return SWLM_ERR_INVALID; }
     *out = nullptr;
@@ -1377,6 +1382,7 @@ int swlm_ctx_create(int device_id, int tp_rank, int tp_size, swlm_ctx** out) {
     ctx->device = device_id; ctx->tp_rank = tp_rank; ctx->tp_size = tp_size;
     cudaError_t e = cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking);
     if (e != cudaSuccess) { delete ctx; return cuda_fail(e, "cudaStreamCreate"); }
+    g_used_device.store(device_id, std::memory_order_relaxed);
     int rc = qgemv_init();
     if (!rc) rc = qgemv_rows_init();
     if (!rc) rc = norm_init();
@@ -2039,6 +2045,8 @@ int swlm_state_set_prefill_chunk(swlm_state* s, int tokens) {
 int swlm_host_alloc(size_t bytes, void** out) {
     if (!out || bytes == 0) { set_error("null argument"); return SWLM_ERR_INVALID; }
     *out = nullptr;
+    const int device = g_used_device.load(std::memory_order_relaxed);
+    if (device >= 0) SWLM_CUDA(cudaSetDevice(device));
     const cudaError_t e = cudaHostAlloc(out, bytes, cudaHostAllocPortable);
     if (e != cudaSuccess) { cudaGetLastError(); return cuda_fail(e, "cudaHostAlloc"); }
     return SWLM_OK;

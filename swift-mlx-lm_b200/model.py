@@ -98,9 +98,10 @@ class WeightStore:
 
 class ResultBlocks:
     """Page-locked memory for large results that go to the caller as arrays. The copy from the GPU then runs at the bus's rate instead of
-    through the driver's staging (2 MB of logits: 57 us instead of 147). Two blocks, made with the model; a block is given out again when
-    nothing refers to its array, or to a view of it, any more. Results that do not fit, that are small, or that come while both blocks are
-    in use, lie in ordinary memory."""
+    through the driver's staging (2 MB of logits: 57 us instead of 147). At most two blocks, each made when a large result first finds none
+    idle: that call pays for it, and a model whose results nobody reads holds none. A block is given out again when nothing refers to its
+    array, or to a view of it, any more. Results that do not fit, that are small, or that come while both blocks are in use, lie in ordinary
+    memory."""
 
     COUNT, SMALLEST = 2, 1 << 20
 
@@ -108,14 +109,11 @@ class ResultBlocks:
         # No lock: a collection that ends an array may start anywhere in these functions, in the same thread. A block is in one place at a
         # time, and a deque's `append` and `pop` are single steps for other threads and for collections alike.
         self.lib, self.size, self.idle, self.closed = lib, size, collections.deque(), False
-        for _ in range(self.COUNT if size >= self.SMALLEST else 0):
-            block = C.c_void_p()
-            if lib.swlm_host_alloc(size, C.byref(block)) == 0:
-                self.idle.append(block.value)
+        self.unmade = collections.deque(range(self.COUNT))
 
     def empty(self, shape, dtype) -> np.ndarray:
         size = math.prod(shape) * np.dtype(dtype).itemsize
-        at = self._take() if self.SMALLEST <= size <= self.size else None
+        at = self._take() or self._make() if self.SMALLEST <= size <= self.size and not self.closed else None
         if at is None:
             return np.empty(shape, dtype=dtype)
         memory = (C.c_char * size).from_address(at)
@@ -127,6 +125,14 @@ class ResultBlocks:
             return self.idle.pop()
         except IndexError:
             return None
+
+    def _make(self) -> Optional[int]:
+        try:
+            self.unmade.pop()   # (a block that cannot be had is not asked for again)
+        except IndexError:
+            return None
+        block = C.c_void_p()
+        return block.value if self.lib.swlm_host_alloc(self.size, C.byref(block)) == 0 else None
 
     def _back(self, at: int) -> None:
         self.idle.append(at)

@@ -422,3 +422,37 @@ def test_result_blocks_when_a_collection_ends_an_array(pkg):
     assert len(done) == 20
     gc.collect()
     assert not lib.live
+
+
+def test_result_blocks_are_made_when_a_large_result_comes(pkg):
+    """None with the model, none for small results or for ones that do not fit, the second when the first is in use, none behind one that could
+    not be had, none of a closed model."""
+    import numpy as np
+
+    lib = HostMemory()
+    blocks = pkg.model.ResultBlocks(lib, 2 << 20)
+    assert not lib.live
+    blocks.empty((1 << 10,), np.uint16), blocks.empty((1 << 21,), np.uint16)
+    assert not lib.live
+    for _ in range(3):
+        blocks.empty((1 << 20,), np.uint16)
+        assert len(lib.live) == 1
+    a, b, c = (blocks.empty((1 << 20,), np.uint16) for _ in range(3))
+    assert {x.ctypes.data for x in (a, b)} == set(lib.live) and c.ctypes.data not in lib.live
+    del a, b
+    blocks.close()
+    assert not lib.live and blocks.empty((1 << 20,), np.uint16).size == 1 << 20 and not lib.live
+
+    class Full(HostMemory):
+        asked = 0
+
+        def swlm_host_alloc(self, size, out):
+            self.asked += 1
+            return -2
+
+    lib = Full()
+    blocks = pkg.model.ResultBlocks(lib, 2 << 20)
+    for _ in range(5):
+        assert blocks.empty((1 << 20,), np.uint16).size == 1 << 20
+    assert lib.asked == 2
+    blocks.close()
