@@ -415,15 +415,12 @@ __device__ __forceinline__ void tc_emit(const TcParams& p, const ProductRow& dst
             if (i < count) *reinterpret_cast<__nv_bfloat16*>(y + i * dst.stride) = __float2bfloat16_rn(val[i]);
     }
 }
-// gated_activation without a branch between values: tanh-GELU as g / (1 + e^-2u), the same function; 1 / x by the unit's reciprocal
-// (one unit in the last place)
+// gated_activation without a branch between values: tanh-GELU as g / (1 + e^-2u), the same function
 __device__ __forceinline__ float tc_gated(float g, float up, const GatedAct& act) {
     const bool clamped = act.kind == GATED_ACT_CLAMPED;
     if (clamped) { g = fminf(g, act.limit); up = fminf(fmaxf(up, -act.limit), act.limit) + 1.0f; }
     const float u = act.kind == GATED_ACT_GELU_TANH ? 1.5957691216f * (g + 0.044715f * g * g * g) : clamped ? act.alpha * g : g;
-    float r;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.0f + expf(-u)));
-    return g * r * up;
+    return 0.25f * g * four_over(1.0f + expf(-u)) * up;
 }
 
 template <int CG, int BN, int STAGES, bool GATED>

@@ -425,13 +425,8 @@ __device__ __forceinline__ TcDst tc_dst(const QGemmTcParams& p, int row) {
     return {(q == 0 ? p.out.y[0] : q == 1 ? p.out.y[1] : p.out.y[2]) + (row - (q == 0 ? 0 : q == 1 ? p.out.end[0] : p.out.end[1])),
             q == 0 ? p.out.stride[0] : q == 1 ? p.out.stride[1] : p.out.stride[2], row < p.out.end[2]};
 }
-// silu(gate) * up; 1 / (1 + e) by the unit's reciprocal (one unit in the last place): a division's slow path is a branch, behind which
-// eight independent values would be worked out one after the other
-__device__ __forceinline__ float tc_swiglu(float gate, float up) {
-    float r;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.0f + expf(-gate)));
-    return gate * r * up;
-}
+// silu(gate) * up
+__device__ __forceinline__ float tc_swiglu(float gate, float up) { return 0.25f * gate * four_over(1.0f + expf(-gate)) * up; }
 template <bool GELU>
 __device__ __forceinline__ void tc_emit_gated(const QGemmTcParams& p, const TcDst& d, const unsigned* v, float fac, int fac0, int token0) {
     // gate rows sit in the lanes of the first eight of 16, up rows in the others: a gate lane finishes even columns, its up lane odd ones.

@@ -107,4 +107,15 @@ inline TensorMapEncodeFn tensor_map_encode_fn() {
     return fn;
 }
 
+// 4 / x of x >= 1, infinity included: the unit's reciprocal (one unit in the last place) and one step of Newton's iteration, without a
+// branch (a division's slow path is one, behind which a lane's independent values would be worked out one after the other: 6 % of a
+// prompt). Times four, because the reciprocal of a large x is subnormal, which the unit takes for zero.
+__device__ __forceinline__ float four_over(float x) {
+    const float q = 0.25f * x;
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(q));
+    const float refined = fmaf(r, fmaf(-q, r, 1.0f), r);
+    return q < INFINITY ? refined : 0.0f;
+}
+
 }  // namespace swlm

@@ -236,6 +236,33 @@ def test_gated_products_of_a_prompt(pkg, oracle, staf, m, ff, k, steps):
     model.close(), store.close()
 
 
+@pytest.mark.parametrize("m", [20, 64])
+def test_gates_far_below_zero(pkg, m):
+    """Gates down to where 1 + e^-gate is about to overflow, times the gate again as up: products that bf16 still holds come out to its
+    precision."""
+    P, vocab, k, ff = pkg.plan, 512, 64, 64
+    store = pkg.WeightStore(0)
+    values = pkg.f32_to_bf16(np.linspace(-88.5, 88.5, vocab).astype(np.float32))
+    table = np.zeros((vocab, k), dtype=np.uint16)
+    table[:, 0] = values
+    store.add_dense("rows", table)
+    ones = (np.full((ff, k // 8), 0x11111111, dtype=np.uint32), pkg.f32_to_bf16(np.ones((ff, k // 64), dtype=np.float32)), np.zeros((ff, k // 64), dtype=np.uint16))
+    store.add_q4_mlx("gate", *ones), store.add_q4_mlx("up", *ones), store.add_q4_mlx("down", *pkg.synth_q4(vocab, ff, seed=1, centered=True))
+    desc = pkg.BuffersDesc(hidden=k, slot_dim=k, vocab=vocab, max_seq=16, max_batch=m)
+    steps = [P._step(P.STEP_EMBED, out_buf=P.BUF_S3, n=k, weight="rows")] + _gated_steps(P, k, ff) + [
+        P._step(P.STEP_QGEMV, in_buf=P.BUF_S0, out_buf=P.BUF_LOGITS, n=vocab, k=ff, weight="down"),
+        P._step(P.STEP_EMBED, out_buf=P.BUF_S1, n=k, weight="rows"), P._step(P.STEP_EMBED, out_buf=P.BUF_S2, n=k, weight="rows"),
+        P._step(P.STEP_ARGMAX, in_buf=P.BUF_LOGITS, n=vocab)]
+    model = pkg.InferenceModel(store, steps, desc)
+    tokens = np.arange(m) * (vocab - 1) // (m - 1)
+    model.decode(tokens)
+    v = pkg.bf16_to_f32(values).astype(np.float64)[tokens][:, None]
+    want = v * v / (1.0 + np.exp(-v))
+    # one rounding to bf16 (2^-9), an exponential of an argument near 88 in 32 bits and three products (2^-21)
+    assert (np.abs(pkg.bf16_to_f32(model.read_buffer(P.BUF_S0, ff)) - want) <= 2.0 ** -8 * np.abs(want)).all()
+    model.close(), store.close()
+
+
 def _gated_store(pkg, rng, vocab, k, ff, staf, down=None):
     table = pkg.f32_to_bf16(rng.normal(size=(vocab, k)).astype(np.float32))
     q4 = {name: pkg.synth_q4(n, kk, seed=i, centered=True) for i, (name, n, kk) in enumerate((("gate", ff, k), ("up", ff, k), ("down", down or vocab, ff)))}

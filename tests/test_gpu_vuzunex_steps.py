@@ -129,6 +129,34 @@ def test_gate_and_up_in_one_launch(pkg, store, dtype, rows, act_name, n, k):
     m.close()
 
 
+@pytest.mark.parametrize("rows", [17, 300])
+def test_gates_of_a_portion_far_below_zero(pkg, store, rows):
+    """Gates down to where 1 + e^-gate is about to overflow, times the gate again as up: products that bf16 still holds come out to its
+    precision."""
+    P, k, n = pkg.plan, 64, 1000
+    weight = np.zeros((n, k), dtype=np.uint16)
+    weight[:, 0] = vc.to_bf16_bits(np.linspace(-88.5, 88.5, n) / 8)
+    table = np.zeros((8, k), dtype=np.uint16)
+    table[:, 0] = vc.to_bf16_bits(np.ones(8))
+    for name in ("far.g", "far.u"):
+        store.add_matrix(f"{name}{rows}", weight)
+    store.add_dense(f"far.e{rows}", table)
+    store.add_dense(f"far.n{rows}", np.zeros(k, dtype=np.uint16))
+    steps = [P._step(P.STEP_EMBED, out_buf=P.BUF_HIDDEN, n=k, weight=f"far.e{rows}"),
+             P._step(P.STEP_COPY_RMSNORM, in_buf=P.BUF_HIDDEN, out_buf=P.BUF_S0, n=k, eps=0.0, weight_bias=1.0, weight=f"far.n{rows}"),
+             P._step(P.STEP_PRODUCT, in_buf=P.BUF_S0, out_buf=P.BUF_S1, n=n, k=k, weight=f"far.g{rows}"),
+             P._step(P.STEP_PRODUCT, in_buf=P.BUF_S0, out_buf=P.BUF_S2, n=n, k=k, weight=f"far.u{rows}"),
+             P._step(P.STEP_SWIGLU, in_buf=P.BUF_S1, in2_buf=P.BUF_S2, out_buf=P.BUF_S1, n=n)]
+    m = model_of(pkg, store, steps, "bfloat16", k, batch=1, max_seq=512)
+    m.run_batch([(0, [1] * rows, [])], logits=False)
+    assert (m.read_buffer_f32(P.BUF_S0, rows, k)[:, 0] == 8.0).all()
+    v = 8.0 * vc.from_bf16_bits(weight[:, 0]).astype(np.float64)
+    want = v * v / (1.0 + np.exp(-v))
+    # one rounding to bf16 (2^-9), an exponential of an argument near 88 in 32 bits and three products (2^-21)
+    assert (np.abs(m.read_buffer_f32(P.BUF_S1, rows, n) - want) <= 2.0 ** -8 * np.abs(want)).all()
+    m.close()
+
+
 @pytest.mark.parametrize("gated", [False, True])
 @pytest.mark.parametrize("rows, n, k", [
     (17, 40, 3000), (30, 2056, 200),      # 32 rows per tile: K over eight CTAs, four columns each; one range, ragged weight rows
