@@ -262,6 +262,10 @@ int swlm_op_qgemm_dev(swlm_ctx* ctx, const char* weight, int m, const void* x_de
 /* generateUnifiedDequantToBFloat (Generator/MetalSourceGenerator+Quantized.swift:361-416):
  * the stored tensor unpacked to bf16 [n][k] on the host, from the device layout. */
 int swlm_op_dequant_bf16(swlm_ctx* ctx, const char* weight, uint16_t* out_bf16);
+/* The form that a tensor-core product of m activation rows takes (gated: gate and up of n rows each, together), for tests that mean a
+ * certain one. Dense: form = {CTAs of a tile, activation rows of a tile, CTAs per SM, K ranges of a cluster}; clusters = how many clusters
+ * of 1, 2, 4, 8 CTAs the device runs at once, NULL: the current device. */
+int swlm_op_dense_form(int m, int n, int k, int gated, const int* clusters, int* form);
 /* Flash-decode over caller-provided device tensors: q [b][heads][hd] (RoPE already applied),
  * k,v [b][kv_heads][ctx_stride][hd] bf16, attends over [0, ctx_len); out [b][heads][hd] bf16.
  * scratch_dev needs swlm_op_flash_decode_scratch_bytes(). */

@@ -11,6 +11,7 @@
 //   sgemm_kernel     more rows, fp32 activations: fp32 FMAs on 64 x 64 tiles.
 #include <algorithm>
 #include <cstdlib>
+#include <mutex>
 
 #include <cooperative_groups.h>
 
@@ -747,7 +748,16 @@ constexpr int tc_stages() {
 template <int CG, int BN, int PER_SM, bool GATED>
 constexpr size_t tc_smem() { return (size_t)tc_stages<BN, PER_SM, GATED>() * ((GATED ? 2 : 1) * kTileRows * 128 + BN / CG * 128) + 1024; }
 
-int g_tc_clusters[4] = {kTcSMs, kTcSMs / 2, 0, 0};   // clusters of 1, 2, 4, 8 CTAs that run at once, one CTA per SM
+// Clusters of 1, 2, 4, 8 CTAs that run at once on a device, one CTA per SM; 0: it takes none of that size, and products do without. Filled
+// when the device's first context is made, before any launch on it.
+struct TcClusters { std::once_flag once; int at[4] = {kTcSMs, kTcSMs / 2, 0, 0}; };
+constexpr int kTcDevices = 64;
+TcClusters g_tc_clusters[kTcDevices + 1];   // (the last one: devices beyond, without clusters of 4 and 8)
+TcClusters& tc_clusters() {
+    int device = 0;
+    if (cudaGetDevice(&device) != cudaSuccess) { cudaGetLastError(); return g_tc_clusters[kTcDevices]; }
+    return g_tc_clusters[std::min(device, kTcDevices)];
+}
 
 // How a product runs: the form with the least time by what was measured for n = 2048 .. 32768, K = 512 .. 8192, 16 .. 1024 rows (us;
 // graphs of launches, weights from memory). A step of 64 columns takes 0.21 (the round trip of a stage over the ring's depth; 0.25 with
@@ -757,7 +767,7 @@ int g_tc_clusters[4] = {kTcSMs, kTcSMs / 2, 0, 0};   // clusters of 1, 2, 4, 8 C
 // one CTA per SM (128 CTAs in eights: 16.9 instead of 10.7). Against one SM per 256 x 128 tile with the ranges' sums in memory and added by a
 // second launch: 3664 x 2048 at 512 rows 28.9 -> 11.3, 2048 x 8192 31.3 -> 21.0, gate and up of 8192 x 2048 59.5 -> 31.5; at 16 rows
 // 8.7 -> 6.7, 12.6 -> 10.7, 21.3 -> 15.0.
-TcShape tc_shape(int n, int k, int m, bool gated) {
+TcShape tc_shape(int n, int k, int m, bool gated, const int* clusters) {
     TcShape best{};
     const int steps = (k + kTcK - 1) / kTcK;
     double least = 1e30;
@@ -768,8 +778,8 @@ TcShape tc_shape(int n, int k, int m, bool gated) {
             const double alone = bn == 256 ? (gated ? 0.7 : 0.3) : per_sm == 2 ? 0.25 : 0.21;
             for (int i = 0; i < 4; ++i) {
                 const int z = (1 << i) / cg;   // clusters of 1, 2, 4, 8 CTAs
-                if (z < 1 || z > steps || (gated && bn == 256 && z > 1)) continue;
-                const long long groups = (long long)tiles_m * tiles_n, slots = (long long)g_tc_clusters[i] * per_sm;
+                if (z < 1 || z > steps || clusters[i] < 1 || (gated && bn == 256 && z > 1)) continue;
+                const long long groups = (long long)tiles_m * tiles_n, slots = (long long)clusters[i] * per_sm;
                 const double waves = (double)((groups + slots - 1) / slots);
                 const double step = std::max(alone, bytes * (double)(std::min(groups, slots) << i) / 12e6);
                 const double cost = waves * (step * ((steps + z - 1) / z) + ends) + (z > 1 ? 1.5 + bn / 40.0 + 0.2 * z : 0.0);
@@ -837,15 +847,20 @@ int bgemm_init() {
     if ((rc = tc_attr<1, 32, 1, false>()) || (rc = tc_attr<1, 32, 2, false>()) || (rc = tc_attr<1, 32, 1, true>()) || (rc = tc_attr<1, 32, 2, true>()) ||
         (rc = tc_attr<1, 64, 1, false>()) || (rc = tc_attr<1, 64, 2, false>()) || (rc = tc_attr<1, 64, 1, true>()) || (rc = tc_attr<2, 128, 1, false>()) ||
         (rc = tc_attr<2, 128, 1, true>()) || (rc = tc_attr<2, 256, 1, false>()) || (rc = tc_attr<2, 256, 1, true>())) return rc;
-    for (int i = 2; i < 4; ++i) {
-        cudaLaunchConfig_t cfg = {};
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = 1u << i; attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-        cfg.gridDim = dim3(1u << i, 1, 64); cfg.blockDim = dim3(kTcBlock); cfg.dynamicSmemBytes = tc_smem<1, 32, 1, false>(); cfg.attrs = attr; cfg.numAttrs = 1;
-        SWLM_CUDA(cudaOccupancyMaxActiveClusters(&g_tc_clusters[i], bgemm_tc_kernel<1, 32, tc_stages<32, 1, false>(), false>, &cfg));
-        if (g_tc_clusters[i] < 1) { set_error("dense product: no cluster of %d CTAs fits this device", 1 << i); return SWLM_ERR_UNSUPPORTED; }
-    }
+    TcClusters& of = tc_clusters();
+    if (&of == &g_tc_clusters[kTcDevices]) return SWLM_OK;
+    std::call_once(of.once, [&] {
+        for (int i = 2; i < 4; ++i) {
+            cudaLaunchConfig_t cfg = {};
+            cudaLaunchAttribute attr[1];
+            attr[0].id = cudaLaunchAttributeClusterDimension;
+            attr[0].val.clusterDim.x = 1u << i; attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+            cfg.gridDim = dim3(1u << i, 1, 64); cfg.blockDim = dim3(kTcBlock); cfg.dynamicSmemBytes = tc_smem<1, 32, 1, false>(); cfg.attrs = attr; cfg.numAttrs = 1;
+            int fit = 0;
+            if (cudaOccupancyMaxActiveClusters(&fit, bgemm_tc_kernel<1, 32, tc_stages<32, 1, false>(), false>, &cfg) != cudaSuccess) { cudaGetLastError(); fit = 0; }
+            of.at[i] = fit;
+        }
+    });
     return SWLM_OK;
 }
 
@@ -888,8 +903,16 @@ int launch_product(const ProductLaunch& a, cudaStream_t s) {
         return e == cudaSuccess ? SWLM_OK : cuda_fail(e, "sgemm launch");
     }
     if (((a.x_stride | a.x2_stride) & 7) || ((reinterpret_cast<uintptr_t>(a.x) | reinterpret_cast<uintptr_t>(a.x2)) & 15)) { set_error("dense product: activation rows must be 16-byte aligned"); return SWLM_ERR_INVALID; }
-    const TcShape t = a.experts ? grouped_shape(a) : tc_shape(a.w->n, a.w->k, a.m, gated);
+    const TcShape t = a.experts ? grouped_shape(a) : tc_shape(a.w->n, a.w->k, a.m, gated, tc_clusters().at);
     return gated ? tc_pick<true>(a, t, s) : tc_pick<false>(a, t, s);
 }
 
 }  // namespace swlm
+
+extern "C" int swlm_op_dense_form(int m, int n, int k, int gated, const int* clusters, int* form) {
+    using namespace swlm;
+    if (m <= 0 || n <= 0 || k <= 0 || !form || (clusters && (clusters[0] < 1 || clusters[1] < 1))) { set_error("bad argument"); return SWLM_ERR_INVALID; }
+    const TcShape t = tc_shape(n, k, m, gated != 0, clusters ? clusters : tc_clusters().at);
+    form[0] = t.cg; form[1] = t.bn; form[2] = t.per_sm; form[3] = t.ranges;
+    return SWLM_OK;
+}

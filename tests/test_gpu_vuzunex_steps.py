@@ -195,6 +195,25 @@ def test_products_of_a_portion(pkg, store, gated, rows, n, k):
     m.close()
 
 
+@pytest.mark.parametrize("gated, rows, n, k, form", [   # (CTAs of a tile, rows of a tile, CTAs per SM, K ranges)
+    (False, 34, 3464, 1624, (1, 32, 1, 2)), (False, 69, 1544, 1488, (1, 32, 2, 4)), (False, 601, 40, 2952, (1, 32, 2, 8)),
+    (False, 35, 6040, 2232, (1, 64, 1, 2)), (False, 35, 3224, 1784, (1, 64, 1, 4)), (False, 700, 40, 4296, (1, 64, 1, 8)),
+    (False, 199, 5448, 72, (1, 64, 2, 1)), (False, 35, 5016, 2504, (1, 64, 2, 4)),
+    (False, 361, 4264, 280, (2, 128, 1, 1)), (False, 73, 4616, 3784, (2, 128, 1, 2)), (False, 71, 2968, 3864, (2, 128, 1, 4)),
+    (False, 893, 2728, 72, (2, 256, 1, 1)), (False, 517, 7608, 4208, (2, 256, 1, 2)),
+    (True, 1001, 56, 1752, (1, 32, 1, 2)), (True, 69, 7416, 72, (1, 32, 2, 1)),
+    (True, 35, 8312, 344, (1, 64, 1, 1)), (True, 37, 3848, 2776, (1, 64, 1, 2)), (True, 917, 40, 4168, (1, 64, 1, 4)), (True, 35, 1432, 4936, (1, 64, 1, 8)),
+    (True, 133, 7976, 72, (2, 128, 1, 1)), (True, 67, 3864, 3824, (2, 128, 1, 2)), (True, 65, 2024, 3880, (2, 128, 1, 4)),
+    (True, 341, 6360, 72, (2, 256, 1, 1)),
+])
+def test_products_of_a_portion_by_form(pkg, store, gated, rows, n, k, form):
+    """Every form that the library chooses among, with remainders of rows, weight rows and columns."""
+    taken = np.zeros(4, dtype=np.int32)
+    store.lib.check(store.lib.swlm_op_dense_form(rows, n, k, int(gated), None, taken.ctypes.data))
+    assert tuple(taken.tolist()) == form
+    test_products_of_a_portion(pkg, store, gated, rows, n, k)
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 def test_argmax_takes_the_lowest_of_equal_logits(pkg, store, dtype):
     P, rng = pkg.plan, np.random.default_rng(4)

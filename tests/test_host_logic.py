@@ -456,3 +456,22 @@ def test_result_blocks_are_made_when_a_large_result_comes(pkg):
         assert blocks.empty((1 << 20,), np.uint16).size == 1 << 20
     assert lib.asked == 2
     blocks.close()
+
+
+def _dense_form(lib, m, n, k, gated, clusters):
+    form, of = np.zeros(4, dtype=np.int32), None if clusters is None else np.asarray(clusters, dtype=np.int32)
+    lib.check(lib.swlm_op_dense_form(m, n, k, gated, None if of is None else of.ctypes.data, form.ctypes.data))
+    return form.tolist()
+
+
+@pytest.mark.parametrize("clusters", [(148, 74, 0, 0), (148, 74, 34, 0), (7, 3, 1, 0), (1, 1, 0, 0), None])
+def test_dense_products_where_large_clusters_do_not_fit(pkg, clusters):
+    """A device that runs no cluster of four or eight CTAs takes the products without them (without a device: nothing is known of any)."""
+    lib, some = pkg.load_library(), clusters or (1, 1, 0, 0)
+    for gated in (0, 1):
+        for m in (17, 100, 300, 2048):
+            for n, k in ((40, 8192), (2048, 2048), (8192, 72)):
+                cg, bn, per_sm, ranges = _dense_form(lib, m, n, k, gated, clusters)
+                assert cg in (1, 2) and bn in (32, 64, 128, 256) and per_sm in (1, 2) and 1 <= ranges <= (k + 63) // 64
+                assert some[(cg * ranges).bit_length() - 1] > 0
+    assert _dense_form(lib, 17, 40, 8192, 0, (148, 74, 34, 15))[3] > 2   # (with them it takes more ranges)
