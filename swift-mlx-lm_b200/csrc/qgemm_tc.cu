@@ -598,9 +598,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__((kTcDeqWarps + 2 + k
 }
 
 // ---- short form: 65 to 128 activation rows, or few tiles. K is cut over the CTAs of a cluster; each sends its part of a tile's results
-// to the CTA that finishes a row, through distributed shared memory (the ring's, which is free by then). ---------------------------
+// to the CTA that finishes a row, through distributed shared memory (the ring's, which is free by then). 72 registers: what is left of an
+// SM's takes the CTAs that turn the next product's rows into fp16 (with 96 of them 2048 x 2048 at 256 rows took 18.3 us, with 72 14.7; 16.6 before
+// the end of a tile was worked out for 16 columns at once). ---------------------------------------------------------------------------
 template <int BN, int STAGES, bool F16SB>
-__global__ void __launch_bounds__((kTcDeqWarps + 2) * 32, 1) qgemm_tc_short_kernel(const QGemmTcParams p, const __grid_constant__ CUtensorMap xmap) {
+__global__ void __maxnreg__(72) qgemm_tc_short_kernel(const QGemmTcParams p, const __grid_constant__ CUtensorMap xmap) {
     constexpr unsigned kTmemCols = 512;                      // accumulator, four weight tiles
     constexpr int SA = kTcMaxA;
     static_assert(BN + SA * 64 <= 512, "tensor memory");
@@ -662,26 +664,34 @@ __global__ void __launch_bounds__((kTcDeqWarps + 2) * 32, 1) qgemm_tc_short_kern
     const int r = (warp & 3) * 32 + lane;
     constexpr int CW = 16;                          // columns per read
     const cg::cluster_group cluster = cg::this_cluster();
-    if (p.splits > 1) cluster.sync();               // every ring of the cluster is free
-    const int own = BN / p.splits;                  // columns that a CTA of the cluster finishes
-    if (done && warp < kTcDeqWarps) {
+    const int own = BN / p.splits;                  // columns that a CTA of the cluster finishes: whole reads
+    const unsigned lanes = tmem_d + ((unsigned)((warp & 3) * 32) << 16);
+    if (p.splits == 1) {
+        if (done && warp < kTcDeqWarps) {
+            const TcDst dst = tc_dst(p, row0 + r);
 #pragma unroll 1
-        for (int c0 = (warp >> 2) * CW; c0 < BN; c0 += 4 * CW) {
-            if (tok0 + c0 >= p.m) break;
-            unsigned v[CW];
-            tmem_ld16(tmem_d + ((unsigned)((warp & 3) * 32) << 16) + (unsigned)c0, v);
-            if (p.splits == 1) {
-                tc_emit16(p, tc_dst(p, row0 + r), v, tc_rscale(p, min(tok0 + c0 + (lane & 15), p.m - 1)), 0, tok0 + c0);
-                continue;
-            }
-#pragma unroll
-            for (int i = 0; i < CW; ++i) {
-                const int c = c0 + i, owner = c / own;
-                if (tok0 + c < p.m) reinterpret_cast<float*>(cluster.map_shared_rank(ring_ptr, owner))[(rank * own + (c - owner * own)) * kTcRows + r] = __uint_as_float(v[i]);
+            for (int c0 = (warp >> 2) * CW; c0 < BN; c0 += 4 * CW) {
+                if (tok0 + c0 >= p.m) break;
+                unsigned v[CW];
+                tmem_ld16(lanes + (unsigned)c0, v);
+                tc_emit16(p, dst, v, tc_rscale(p, min(tok0 + c0 + (lane & 15), p.m - 1)), 0, tok0 + c0);
             }
         }
-    }
-    if (p.splits > 1) {
+    } else {
+        cluster.sync();                             // every ring of the cluster is free
+        if (done && warp < kTcDeqWarps) {
+#pragma unroll 1
+            for (int c0 = (warp >> 2) * CW; c0 < BN; c0 += 4 * CW) {
+                if (tok0 + c0 >= p.m) break;
+                unsigned v[CW];
+                tmem_ld16(lanes + (unsigned)c0, v);
+                const int owner = c0 / own;
+                float* to = reinterpret_cast<float*>(cluster.map_shared_rank(ring_ptr, owner)) + (rank * own + (c0 - owner * own)) * kTcRows + r;
+#pragma unroll
+                for (int i = 0; i < CW; ++i)
+                    if (tok0 + c0 + i < p.m) to[i * kTcRows] = __uint_as_float(v[i]);
+            }
+        }
         cluster.sync();
         const float* got = reinterpret_cast<const float*>(ring_ptr);
         const int rows = p.gated ? kTcRows / 2 : kTcRows;
