@@ -266,6 +266,9 @@ int swlm_op_dequant_bf16(swlm_ctx* ctx, const char* weight, uint16_t* out_bf16);
  * certain one. Dense: form = {CTAs of a tile, activation rows of a tile, CTAs per SM, K ranges of a cluster}; clusters = how many clusters
  * of 1, 2, 4, 8 CTAs the device runs at once, NULL: the current device. */
 int swlm_op_dense_form(int m, int n, int k, int gated, const int* clusters, int* form);
+/* Quantized, 17 rows and more: form = {activation rows of a tile, CTAs of a cluster along K}; 32, 48 and 64 rows: all of them at once over
+ * persistent CTAs, 128: a CTA per tile, 256: pairs of SMs. */
+int swlm_op_qgemm_form(int m, int n, int k, int gated, int* form);
 /* Flash-decode over caller-provided device tensors: q [b][heads][hd] (RoPE already applied),
  * k,v [b][kv_heads][ctx_stride][hd] bf16, attends over [0, ctx_len); out [b][heads][hd] bf16.
  * scratch_dev needs swlm_op_flash_decode_scratch_bytes(). */

@@ -1228,6 +1228,30 @@ constexpr int kTcStages128 = 4, kTcStagesPair = 5;
 constexpr int kTcSMs = 148;
 
 int ext_blocks(int kt) { return (kt + 63) / 64; }   // blocks of 64 groups
+// CTAs (groups of `splits` along K) that share the row tiles. In a single pass as few as keep the largest share: with fewer SMs taken the next
+// launch's CTAs start beside them (8192 x 2048 at 41 rows 13.5 us with 148, 10.2 with 128; 4096 x 4096 16.6 and 13.8). Fours: 32 of the 34 to
+// 36 clusters that the GPU runs at once.
+int sl_ctas(int row_tiles, int splits) {
+    const int most = std::min(splits == 4 ? 32 : kTcSMs / splits, row_tiles), share = (row_tiles + most - 1) / most;
+    return share <= 8 ? (row_tiles + share - 1) / share : most;
+}
+// CTAs along K of a product of up to 64 rows: two or four where row tiles are few and K is long. A step of 256 columns takes 0.36 us and 0.05
+// for each row tile of the CTA up to four, 0.64 with more; meeting in a cluster 5 to 6. One, two and four, us at 41 rows: 2048 x 8192
+// 23.5 / 21.1 / 16.8, 4096 x 14336 36.6 / 29.4 / 24.1, 1000 x 16448 38.6 / 32.5 / 24.4; 4096 x 4096 14.4 / 15.8 / 13.8, 1024 x 4096
+// 13.1 / 15.7 / 12.9, 2048 x 2048 9.8 / 13.2 / 11.6.
+int sl_splits(int row_tiles, int kt) {
+    const int steps = kt / 4 + ext_blocks(kt);
+    auto time = [&](int z) {
+        const int ctas = sl_ctas(row_tiles, z), whole = row_tiles / (8 * ctas), share = (row_tiles - whole * 8 * ctas + ctas - 1) / ctas;
+        const double step = 0.64 * whole + (share > 4 ? 0.64 : share > 0 ? 0.36 + 0.05 * share : 0.0);
+        return step * ((steps + z - 1) / z) + (z > 1 ? 6.0 : 0.0);
+    };
+    int best = 1;
+    for (int z = 2; z <= 4; z *= 2)
+        if (steps >= z && row_tiles <= 8 * sl_ctas(row_tiles, z) && time(z) < time(best)) best = z;
+    return best;
+}
+
 constexpr int sl_stages(int bn) { return bn == 32 ? 6 : bn == 48 ? 4 : 3; }
 constexpr size_t sl_smem_bytes(int bn) { return (size_t)sl_stages(bn) * bn * kSlCols * 2 + kSlRingBytes + 1024; }
 template <typename K>
@@ -1260,7 +1284,7 @@ int sl_launch(QGemmTcParams& p, bool f16, const __half* xh, int xh_stride, int s
     const int rc = make_x_map(xh, xh_stride, p.m, BN, &xmap);
     if (rc) return rc;
     p.real_steps = p.kt * 64 / kSlCols; p.steps = p.real_steps + ext_blocks(p.kt); p.splits = splits;
-    const int ctas = std::min(kTcSMs / splits, p.row_tiles);
+    const int ctas = sl_ctas(p.row_tiles, splits);
     p.whole = p.row_tiles / (8 * ctas); p.left = p.row_tiles - p.whole * 8 * ctas;
     p.n_tiles = p.whole + (p.left > 0);
     if (splits > 1 && p.n_tiles > 1) { set_error("qgemm (tcgen05): passes"); return SWLM_ERR_INVALID; }
@@ -1294,12 +1318,14 @@ int tc_launch_long(QGemmTcParams& p, bool f16, const __half* xh, int xh_stride, 
 int ext_cols(int kt) { return (192 * ext_blocks(kt) + kTcStep - 1) / kTcStep * kTcStep; }
 int kt_padded(int k) { return (k / 64 + 3) / 4 * 4; }
 
-// How a product of m > 64 rows over `tiles16` row tiles runs: the form with the least time by what was measured over K = 2048 .. 14336,
-// n = 2048 .. 128256 and m = 65 .. 512 (us; graphs of launches, weights from memory). A CTA with 128 activation rows takes 0.5 us per
-// step, a pair of the long form 0.87. A launch starts and ends in about 6. Cutting K over a cluster costs the exchange: 5 over four CTAs,
-// 9 over two.
+// How a product of m rows over `tiles16` row tiles of `kt` groups runs: up to 64 rows the slab form with 32, 48 or 64; with more the form with
+// the least time by what was measured over K = 2048 .. 14336, n = 2048 .. 128256 and m = 65 .. 512 (us; graphs of launches, weights from
+// memory). A CTA with 128 activation rows takes 0.5 us per step, a pair of the long form 0.87. A launch starts and ends in about 6. Cutting K
+// over a cluster costs the exchange: 5 over four CTAs, 9 over two.
 struct TcChoice { int bn, splits; };
-TcChoice tc_choose(int m, int tiles16, int steps) {
+TcChoice tc_choose(int m, int tiles16, int kt) {
+    if (m <= 64) return {m <= 32 ? 32 : m <= 48 ? 48 : 64, sl_splits(tiles16, kt)};
+    const int steps = (kt * 64 + ext_cols(kt)) / kTcStep;
     const long long tiles = (long long)((tiles16 + 7) / 8) * ((m + 127) / 128);
     TcChoice best{128, 1};
     double least = 1e30;
@@ -1312,18 +1338,6 @@ TcChoice tc_choose(int m, int tiles16, int steps) {
     }
     return best;
 }
-// CTAs along K of a product of up to 64 rows: two where row tiles are few and K is long. A step of 256 columns takes 0.42 us with up to
-// four row tiles per CTA and 0.62 with more, meeting in a cluster 6 (4096 x 14336 at 41 rows 29.4 us alone, 23.5 in pairs, 34.5 in fours;
-// 4096 x 4096 12.2 and 14.2).
-int sl_splits(int row_tiles, int kt) {
-    const int steps = kt / 4 + ext_blocks(kt);
-    auto time = [&](int z) {
-        const int ctas = std::min(kTcSMs / z, row_tiles), whole = row_tiles / (8 * ctas), most = (row_tiles - whole * 8 * ctas + ctas - 1) / ctas;
-        return ((whole * 0.62) + (most > 4 ? 0.62 : most > 0 ? 0.42 : 0.0)) * ((steps + z - 1) / z) + (z > 1 ? 6.0 : 0.0);
-    };
-    return steps >= 2 && row_tiles <= 8 * (kTcSMs / 2) && time(2) < time(1) ? 2 : 1;
-}
-
 }  // namespace
 
 template <int BN>
@@ -1396,15 +1410,22 @@ int launch_qgemm_tc(const Q4Tiled& w, int m, const __nv_bfloat16* x, int x_strid
         const cudaError_t e = ch == 0 ? go(x_to_f16_kernel<0>) : ch == 2 ? go(x_to_f16_kernel<2>) : go(x_to_f16_kernel<4>);
         if (e != cudaSuccess) return cuda_fail(e, "x_to_f16 launch");
     }
-    if (m <= 64) {
-        const int z = sl_splits(w.row_tiles, p.kt);
-        if (m <= 32) return sl_launch<32>(p, w.sb_f16, xh, xh_stride, z, s);
-        if (m <= 48) return sl_launch<48>(p, w.sb_f16, xh, xh_stride, z, s);
-        return sl_launch<64>(p, w.sb_f16, xh, xh_stride, z, s);
+    const TcChoice c = tc_choose(m, w.row_tiles, p.kt);
+    switch (c.bn) {
+    case 32: return sl_launch<32>(p, w.sb_f16, xh, xh_stride, c.splits, s);
+    case 48: return sl_launch<48>(p, w.sb_f16, xh, xh_stride, c.splits, s);
+    case 64: return sl_launch<64>(p, w.sb_f16, xh, xh_stride, c.splits, s);
+    case 128: return tc_launch_short(p, w.sb_f16, xh, xh_stride, c.splits, s);
+    default: return tc_launch_long(p, w.sb_f16, xh, xh_stride, s);
     }
-    const TcChoice c = tc_choose(m, w.row_tiles, p.steps);
-    if (c.bn == 128) return tc_launch_short(p, w.sb_f16, xh, xh_stride, c.splits, s);
-    return tc_launch_long(p, w.sb_f16, xh, xh_stride, s);
 }
 
 }  // namespace swlm
+
+extern "C" int swlm_op_qgemm_form(int m, int n, int k, int gated, int* form) {
+    using namespace swlm;
+    if (m < kQGemmTcMinRows || n <= 0 || k <= 0 || k % 64 || !form) { set_error("bad argument"); return SWLM_ERR_INVALID; }
+    const TcChoice c = tc_choose(m, gated ? (n + 7) / 8 : (n + 15) / 16, kt_padded(k));
+    form[0] = c.bn; form[1] = c.splits;
+    return SWLM_OK;
+}

@@ -192,6 +192,7 @@ SIGNATURES = {
     "swlm_op_qgemm_dev": (_I, [_P, C.c_char_p, _I, _P, _P, _P]),
     "swlm_op_dequant_bf16": (_I, [_P, C.c_char_p, _P]),
     "swlm_op_dense_form": (_I, [_I, _I, _I, _I, _P, _P]),
+    "swlm_op_qgemm_form": (_I, [_I, _I, _I, _I, _P]),
     "swlm_op_flash_decode_scratch_bytes": (C.c_size_t, [_I, _I, _I, _I, _I]),
     "swlm_op_flash_decode_dev": (_I, [_P, _I, _I, _I, _I, _I, _I, C.c_float, _P, _P, _P, _P, _P, _P]),
     "swlm_op_flash_decode_noalloc_capacity": (C.c_size_t, []),

@@ -263,6 +263,61 @@ def test_gates_far_below_zero(pkg, m):
     model.close(), store.close()
 
 
+def _taken(pkg, m, n, k, gated=False):
+    """The form that the library takes: (activation rows of a tile, CTAs of a cluster along K)."""
+    lib, form = pkg.load_library(), np.zeros(2, dtype=np.int32)
+    lib.check(lib.swlm_op_qgemm_form(m, n, k, int(gated), form.ctypes.data))
+    return tuple(form.tolist())
+
+
+@pytest.mark.parametrize("m,n,k,form", [
+    (20, 600, 5184, (32, 4)), (41, 72, 5184, (48, 4)), (64, 2056, 8256, (64, 4)),      # eight, twelve and sixteen columns per CTA
+    (17, 4248, 8256, (32, 2)), (33, 4248, 8256, (48, 2)), (64, 4248, 8256, (64, 2)),
+    (20, 4104, 2048, (32, 1)), (50, 9480, 576, (64, 1)),      # 257 row tiles by twos and a single one, 593 by fives and fewer
+])
+def test_products_of_17_to_64_rows_by_form(pkg, oracle, m, n, k, form):
+    """K over one, two and four CTAs of a cluster, as few CTAs as keep the largest share of row tiles."""
+    assert _taken(pkg, m, n, k) == form
+    test_products_of_17_to_64_rows(pkg, oracle, n, k, m)
+
+
+@pytest.mark.parametrize("m,n,k,splits,steps", [(70, 2000, 4160, 4, 37), (100, 2048, 2112, 4, 20), (128, 136, 2112, 4, 20), (200, 1000, 2112, 4, 20), (65, 4800, 2304, 1, 20)])
+def test_products_of_65_to_256_rows_by_form(pkg, oracle, m, n, k, splits, steps):
+    """Tiles of 128 rows, whole and not, K over a cluster of four and by itself."""
+    assert _taken(pkg, m, n, k) == (128, splits)
+    test_forms_of_the_tensor_core_products(pkg, oracle, m, n, k, (128, 1, splits), steps)
+
+
+@pytest.mark.parametrize("m,ff,k,form", [(24, 512, 9216, (32, 4)), (41, 2240, 8256, (48, 2)), (64, 192, 5184, (64, 4)), (41, 64, 5184, (48, 4))])
+def test_gated_products_of_17_to_64_rows_by_form(pkg, oracle, m, ff, k, form):
+    assert _taken(pkg, m, ff, k, gated=True) == form
+    test_gated_products_of_17_to_64_rows(pkg, oracle, m, ff, k)
+
+
+@pytest.mark.parametrize("m,ff,k,splits", [(100, 1024, 2112, 4), (70, 2048, 4160, 4), (128, 64, 2112, 4), (80, 2432, 2304, 1)])
+def test_gated_products_of_65_to_128_rows_by_form(pkg, oracle, m, ff, k, splits):
+    """Gate and up together in tiles of 128 rows, as test_gated_products_of_a_prompt reads them."""
+    assert _taken(pkg, m, ff, k, gated=True) == (128, splits)
+    P, vocab, hd = pkg.plan, 128, 64
+    rng = np.random.default_rng(m + k)
+    store, q4, table = _gated_store(pkg, rng, vocab, k, ff, False, down=hd)
+    width = max(ff, k)
+    desc = pkg.BuffersDesc(hidden=k, slot_dim=width, vocab=vocab, max_seq=m + 8, max_batch=1, kv_layers=1, kv_heads=1, head_dim=hd)
+    steps = [P._step(P.STEP_EMBED, out_buf=P.BUF_S3, n=k, weight="rows")] + _gated_steps(P, k, ff) + [
+        P._step(P.STEP_QGEMV, in_buf=P.BUF_S0, out_buf=P.BUF_S2, n=hd, k=ff, weight="down"),
+        P._step(P.STEP_ATTN_DECODE, layer=0, in_buf=P.BUF_S3, in2_buf=P.BUF_S3, in3_buf=P.BUF_S2, out_buf=P.BUF_S1, heads=1, kv_heads=1, head_dim=hd, scale=0.125),
+        P._step(P.STEP_QGEMV, in_buf=P.BUF_S1, out_buf=P.BUF_LOGITS, n=vocab, k=hd, weight="head"), P._step(P.STEP_ARGMAX, in_buf=P.BUF_LOGITS, n=vocab)]
+    store.add_q4_mlx("head", *pkg.synth_q4(vocab, hd, seed=5, centered=True))
+    model = pkg.InferenceModel(store, steps, desc)
+    tokens = rng.integers(0, vocab, size=m)
+    model.prefill_sequence(0, tokens)
+    got = pkg.bf16_to_f32(model.read_kv(1, 0, 0, 0, m))
+    ref = pkg.bf16_to_f32(oracle.qgemm(pkg.f32_to_bf16(_gated_ref(pkg, oracle, table, q4)), *q4["down"]))[tokens]
+    for i in range(m):   # (the bound of that test)
+        assert np.abs(got[i] - ref[i]).max() <= 2.4e-2 * np.sqrt((ref[i] ** 2).mean()), i
+    model.close(), store.close()
+
+
 def _gated_store(pkg, rng, vocab, k, ff, staf, down=None):
     table = pkg.f32_to_bf16(rng.normal(size=(vocab, k)).astype(np.float32))
     q4 = {name: pkg.synth_q4(n, kk, seed=i, centered=True) for i, (name, n, kk) in enumerate((("gate", ff, k), ("up", ff, k), ("down", down or vocab, ff)))}
