@@ -470,7 +470,7 @@ __global__ void __launch_bounds__(kSplitThreads) attn_split_kernel(const typenam
 
     // Everything that does not depend on the split weights is requested first: the (max, sum) pairs and the
     // first 16 partial outputs of this thread's four dimensions travel together.
-    constexpr int kPre = STREAM && HD == 128 ? 16 : 32;
+    constexpr int kPre = STREAM ? 8 : 32;
     const int n_out4 = G * HD / 4;  // float4 outputs of the group
     float* wsm = &osm[1][0][0];     // [G][splits] weights (splits <= 64: fits the reused buffer)
     float* msm2 = &osm[2][0][0];    // [G][splits] split maxima
@@ -1040,17 +1040,26 @@ __global__ void __launch_bounds__(kQ8Threads, ROTOR && G <= 4 ? 2 : 0) attn_q8_s
     }
 }
 
-// MODE 4's CTAs: two per SM; no more than 63 per KV head and sequence, so that a pair has 64 partial results at most (what the merge has
-// room for)
-constexpr int kStreamCtas = 296;
-int stream_ctas(int pairs) { return std::min(kStreamCtas, 63 * pairs); }
-// Flash-decode over sequences of equal length: MODE 4 where the splits of all pairs leave more than a fifth of their rounds of the GPU (two
-// CTAs per SM) empty. us with splits / so, 8 KV heads of 128: 13 x 5000 rows (0.70 full) 57 / 50, 24 x 2048 (0.65) 46 / 40,
-// 41 x 2557 (0.55) 108 / 76; 16 x 4096 and 64 x 1024 (0.86) 47.5 / 50 and 55 / 54. Short caches lose what a CTA pays for each pair
-// (64 x 300 23 / 26). Decode steps, where each pair's start is longer, lost in every batch (41 ragged sequences, 4 layers: 1053 / 1100 a step).
-bool attn_streams(int m, int kv_heads, int ctx_len) {
-    const long long pairs = (long long)m * kv_heads, ctas = pairs * attn_pick_splits(m, kv_heads, ctx_len), rounds = (ctas + kStreamCtas - 1) / kStreamCtas;
-    return pairs >= 100 && ctx_len >= 512 && ctas * 5 < rounds * kStreamCtas * 4 && pairs * ((ctx_len + 63) / 64) < (1ll << 31);
+// MODE 4's CTAs: what the GPU holds at once, three per SM with heads of 64 and two with heads of 128. Every one of them needs a block (they do
+// not look whether they have one), and the merge has room for 64 partial results of a pair. 100 pairs of 8 blocks and more give both: with
+// 444 CTAs each takes a fifth of a pair's blocks at least, rounded down to one, so that a pair has eight partial results at most.
+constexpr int stream_ctas(int hd) { return hd == 64 ? 444 : 296; }
+constexpr int kStreamPairs = 100, kStreamRows = 512;
+static_assert(kStreamPairs * (kStreamRows / 64) >= stream_ctas(64) && 5 * kStreamPairs >= stream_ctas(64), "a block, a fifth of a pair");
+// Flash-decode over sequences of equal length: MODE 4 where the splits of all pairs leave a fifth of their rounds of the GPU empty (a quarter
+// with heads of 64) and that is worth more than what a CTA pays for the pairs it meets: five blocks of 64 rows per CTA, ten of heads of 64.
+// Over 13 .. 200 sequences of 512 .. 5000 rows and 1 .. 32 KV heads that is never slower than splits by more than the runs differ. us with
+// splits / so; heads of 128: 13 sequences x 5000 rows x 8 KV heads (rounds 0.70 full) 58.6 / 52.4, 24 x 2048 (0.65) 47.5 / 40.9, 41 x 3000
+// (0.55) 125 / 90, 41 x 512 29.2 / 23.8; not worth it: 13 x 512 11.8 / 14.4, 24 x 600 18.2 / 18.6; too full: 32 x 5000 (0.86) 106 / 123.
+// Heads of 64: 20 x 1024 (0.36) 17.7 / 15.4, 20 x 5000 69 / 41, 41 x 5000 (0.74) 75.4 / 71.9; not worth it: 32 x 512 12.8 / 15.2, 41 x 1024
+// 20.7 / 22.0; too full: 13 x 512 x 32 KV heads (0.94) 13.5 / 16.8, 56 x 600 x 32 (0.81) 65.5 / 71.2. Decode steps, where each pair's start
+// is longer, lost in every batch (41 ragged sequences, 4 layers: 1053 / 1100 a step).
+bool attn_streams(int m, int kv_heads, int hd, int ctx_len) {
+    const long long pairs = (long long)m * kv_heads, blocks = pairs * ((ctx_len + 63) / 64), ctas = pairs * attn_pick_splits(m, kv_heads, ctx_len);
+    if (pairs < kStreamPairs || ctx_len < kStreamRows || blocks >= (1ll << 31)) return false;
+    const int slots = stream_ctas(hd);
+    const double full = (double)ctas / (double)((ctas + slots - 1) / slots * slots), saved = (double)blocks / slots * (1.0 / full - 1.0);
+    return hd == 64 ? full < 0.75 && saved >= 10.0 : full < 0.8 && saved >= 5.0;
 }
 template <int MODE>
 int launch_both(const typename AttnArgs<MODE>::type& p, const dim3& grid, int hd, cudaStream_t s) {
@@ -1103,7 +1112,7 @@ size_t attn_scratch_floats(int m, int heads, int head_dim, int splits) {
 // What either form needs from 100 pairs on: scratch taken for a longer context or for more sequences serves what it served without MODE 4.
 size_t flash_scratch_floats(int m, int heads, int kv_heads, int hd, int ctx_len) {
     const size_t apart = attn_scratch_floats(m, heads, hd, attn_pick_splits(m, kv_heads, ctx_len));
-    return (long long)m * kv_heads >= 100 ? std::max(apart, (size_t)2 * kStreamCtas * (heads / kv_heads) * (hd + 2)) : apart;
+    return (long long)m * kv_heads >= kStreamPairs ? std::max(apart, (size_t)2 * stream_ctas(hd) * (heads / kv_heads) * (hd + 2)) : apart;
 }
 
 static int check_group(int heads, int kv_heads) {
@@ -1202,11 +1211,11 @@ int launch_flash_decode_plain(int m, int heads, int kv_heads, int hd, int ctx_le
     p.position = nullptr; p.ctx_len = ctx_len;
     p.out = out; p.out_stride = heads * hd;
     p.part_o = scratch;
-    const bool stream = attn_streams(m, kv_heads, ctx_len);
+    const bool stream = attn_streams(m, kv_heads, hd, ctx_len);
     if (stream) p.splits = m * kv_heads;   // (MODE 4: pairs)
-    p.part_ml = scratch + (stream ? (size_t)2 * stream_ctas(m * kv_heads) * (heads / kv_heads) : (size_t)m * heads * splits) * hd;
+    p.part_ml = scratch + (stream ? (size_t)2 * stream_ctas(hd) * (heads / kv_heads) : (size_t)m * heads * splits) * hd;
     p.counters = counters;
-    return stream ? launch_both<4>(p, dim3((unsigned)stream_ctas(m * kv_heads)), hd, s) : launch_both<0>(p, dim3(splits, kv_heads, m), hd, s);
+    return stream ? launch_both<4>(p, dim3((unsigned)stream_ctas(hd)), hd, s) : launch_both<0>(p, dim3(splits, kv_heads, m), hd, s);
 }
 
 // ---- allocation-free flash-decode ---------------------------------------------------------------------

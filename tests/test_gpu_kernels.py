@@ -506,6 +506,12 @@ def test_flash_decode_op_of_batches_that_fill_no_whole_round(pkg, store, B, H, K
         assert ((out.float() - want).abs() <= 2.0 ** -8 * want.abs() + 2.0 ** -12 * vf.abs().max()).all()
 
 
+@pytest.mark.parametrize("B,H,KV,D,ctx", [(19, 8, 8, 64, 1990), (13, 8, 8, 64, 6081), (100, 8, 1, 64, 6001), (13, 32, 8, 128, 2497), (20, 32, 8, 64, 1025), (20, 32, 8, 64, 960)])
+def test_flash_decode_op_of_pairs_in_many_parts(pkg, store, B, H, KV, D, ctx):
+    """Heads of 64 over three CTAs per SM, pairs in up to six parts; a length on either side of the line to splits."""
+    test_flash_decode_op_of_batches_that_fill_no_whole_round(pkg, store, B, H, KV, D, ctx)
+
+
 @pytest.mark.parametrize("heads,groups,dk,dv,K,batch", [(4, 2, 16, 16, 4, 1), (32, 16, 128, 128, 4, 1), (8, 8, 64, 128, 3, 2),
                                                         (6, 2, 32, 64, 4, 3)])
 def test_ssm_recurrence_matches_oracle_over_steps(pkg, store, oracle, heads, groups, dk, dv, K, batch):
