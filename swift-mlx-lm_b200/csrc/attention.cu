@@ -571,40 +571,67 @@ __global__ void __launch_bounds__(kSplitThreads) attn_split_kernel(const typenam
 
 // Prompt ingestion: rotate the chunk's k rows (token b at position pos_base + b) and append them and the v rows to
 // the cache of sequence 0, rounded to bf16 (Generator/MetalSourceGenerator+Attention.swift:761-805 does the same
-// per decode step). One warp per token: its angles are worked out once for all KV heads, whose loads are independent of one
-// another (a CTA per token and head, each with angles of its own: 20 us for 2048 tokens x 8 heads of 128 under ncu, now 14).
-constexpr int kRopeWarps = 4;
-__global__ void __launch_bounds__(kRopeWarps * 32) rope_append_kernel(const AttnParams p, int hd) {
+// per decode step). A warp takes one to four KV heads of a token at a time: their angles are worked out once, and their keys and values are
+// requested before any is stored (the cache may overlap its inputs for all the compiler knows: with each head's stores in front of the next
+// one's loads 40 tokens x 8 heads of 128 took 14.8 us under ncu, 2048 14.7). 40 tokens 4.5 us, 512 4.8, 1024 5.8, 2048 7.5; with a CTA per
+// token and head, each with angles of its own, 4.1, 7.2, 11.2 and 19.9.
+constexpr int kRopeWarps = 4, kRopeAhead = 4;
+__global__ void __launch_bounds__(kRopeWarps * 32) rope_append_kernel(const AttnParams p, int hd, int heads_each) {
     pdl_launch_dependents();
     pdl_wait();
     const int b = blockIdx.x * kRopeWarps + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-    const int pos = p.pos_base + b, pairs = p.rope_dim >> 1;
+    const int pos = p.pos_base + b, pairs = p.rope_dim >> 1, h_end = min(p.kv_heads, ((int)blockIdx.y + 1) * heads_each);
     if (b >= p.chunk_tokens || pos >= p.max_seq) return;
     const bool wide = ((hd | p.v_stride) & 7) == 0 && ((reinterpret_cast<uintptr_t>(p.v) | reinterpret_cast<uintptr_t>(p.vcache)) & 15) == 0 && (p.cache_head_stride & 7) == 0;
-    float cs[2], sn[2];   // (at most 64 pairs)
+    const __nv_bfloat16* const k_row = p.k + (size_t)b * p.k_stride;
+    const __nv_bfloat16* const v_row = p.v + (size_t)b * p.v_stride;
+    const size_t to_pos = (size_t)pos * hd;
+    const int vecs = hd >> 3;   // (at most 16)
+    float cs[2], sn[2];         // (at most 64 pairs)
 #pragma unroll
     for (int j = 0; j < 2; ++j)
         if (lane + 32 * j < pairs) sincosf((float)pos * p.inv_freq[lane + 32 * j], &sn[j], &cs[j]);
-#pragma unroll 4
-    for (int kvh = 0; kvh < p.kv_heads; ++kvh) {
-        const __nv_bfloat16* k = p.k + (size_t)b * p.k_stride + kvh * hd;
-        const size_t row = (size_t)kvh * p.cache_head_stride + (size_t)pos * hd;
-        const __nv_bfloat16* v = p.v + (size_t)b * p.v_stride + kvh * hd;
+    for (int h0 = (int)blockIdx.y * heads_each; h0 < h_end; h0 += kRopeAhead) {
+        const int heads = min(kRopeAhead, h_end - h0);
+        __nv_bfloat16 lo[kRopeAhead][2], hi[kRopeAhead][2];
+        uint4 v[kRopeAhead / 2];
 #pragma unroll
-        for (int j = 0; j < 2; ++j) {
-            const int i = lane + 32 * j;
-            if (i < pairs) {
-                const float lo = __bfloat162float(k[i]), hi = __bfloat162float(k[i + pairs]);
-                p.kcache[row + i] = __float2bfloat16_rn(lo * cs[j] - hi * sn[j]);
-                p.kcache[row + i + pairs] = __float2bfloat16_rn(lo * sn[j] + hi * cs[j]);
-            }
+        for (int u = 0; u < kRopeAhead; ++u)
+#pragma unroll
+            for (int j = 0; j < 2; ++j)
+                if (u < heads && lane + 32 * j < pairs) {
+                    const __nv_bfloat16* k = k_row + (h0 + u) * hd + lane + 32 * j;
+                    lo[u][j] = k[0]; hi[u][j] = k[pairs];
+                }
+        if (wide) {
+#pragma unroll
+            for (int j = 0; j < kRopeAhead / 2; ++j)
+                if (lane + 32 * j < heads * vecs) v[j] = *reinterpret_cast<const uint4*>(v_row + h0 * hd + 8 * (lane + 32 * j));
         }
-        for (int d = p.rope_dim + lane; d < hd; d += 32) p.kcache[row + d] = k[d];
-        if (wide)
-            for (int i = lane; i < hd / 8; i += 32)
-                reinterpret_cast<uint4*>(p.vcache + row)[i] = *reinterpret_cast<const uint4*>(v + 8 * i);
-        else
-            for (int d = lane; d < hd; d += 32) p.vcache[row + d] = v[d];
+#pragma unroll
+        for (int u = 0; u < kRopeAhead; ++u)
+#pragma unroll
+            for (int j = 0; j < 2; ++j)
+                if (u < heads && lane + 32 * j < pairs) {
+                    __nv_bfloat16* at = p.kcache + (size_t)(h0 + u) * p.cache_head_stride + to_pos + lane + 32 * j;
+                    const float x = __bfloat162float(lo[u][j]), y = __bfloat162float(hi[u][j]);
+                    at[0] = __float2bfloat16_rn(x * cs[j] - y * sn[j]);
+                    at[pairs] = __float2bfloat16_rn(x * sn[j] + y * cs[j]);
+                }
+        if (wide) {
+#pragma unroll
+            for (int j = 0; j < kRopeAhead / 2; ++j)
+                if (lane + 32 * j < heads * vecs) {
+                    const int u = (lane + 32 * j) / vecs, i = lane + 32 * j - u * vecs;
+                    reinterpret_cast<uint4*>(p.vcache + (size_t)(h0 + u) * p.cache_head_stride + to_pos)[i] = v[j];
+                }
+        }
+        for (int u = 0; u < heads; ++u) {
+            const size_t row = (size_t)(h0 + u) * p.cache_head_stride + to_pos;
+            for (int d = p.rope_dim + lane; d < hd; d += 32) p.kcache[row + d] = k_row[(h0 + u) * hd + d];
+            if (!wide)
+                for (int d = lane; d < hd; d += 32) p.vcache[row + d] = v_row[(h0 + u) * hd + d];
+        }
     }
 }
 
@@ -1182,7 +1209,12 @@ int launch_attn_decode(const AttnLaunch& a, cudaStream_t s) {
         if (a.head_dim > 128) { set_error("attention: head_dim %d not supported", a.head_dim); return SWLM_ERR_UNSUPPORTED; }
         p.pos_base = a.pos_base;
         p.chunk_tokens = a.m;
-        cudaError_t e = launch_k(rope_append_kernel, dim3((a.m + kRopeWarps - 1) / kRopeWarps), dim3(kRopeWarps * 32), 0, s, p, a.head_dim);
+        // (warps that take one KV head, two or four, us under ncu: 512 tokens of eight heads of 128 5.2 / 5.1 / 5.4, 1024 7.2 / 5.8 / 5.9, 2048
+        // 10.8 / 8.1 / 7.4)
+        const long long each = (long long)a.m * a.kv_heads;
+        const int heads_each = each <= 4096 ? 1 : each <= 8192 ? 2 : 4;
+        const dim3 grid((a.m + kRopeWarps - 1) / kRopeWarps, (a.kv_heads + heads_each - 1) / heads_each);
+        cudaError_t e = launch_k(rope_append_kernel, grid, dim3(kRopeWarps * 32), 0, s, p, a.head_dim, heads_each);
         if (e != cudaSuccess) return cuda_fail(e, "rope_append launch");
         // tensor cores when the query heads of a KV head fill the 128 rows of a tile evenly; else a token at a time
         if (attn_prompt_takes(a)) return launch_attn_prompt(a, s);

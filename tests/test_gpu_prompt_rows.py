@@ -109,6 +109,44 @@ def test_prompt_attention_is_the_repeated_single_step(pkg, heads, kv_heads, hd, 
     chunked.close(), single.close(), store.close()
 
 
+@pytest.mark.parametrize("kv_heads,hd,rope_dim", [(1, 64, 64), (5, 128, 128), (8, 64, 0), (9, 128, 40), (16, 64, 24)])
+@pytest.mark.parametrize("tokens", [33, 601, 1100])
+def test_rows_that_a_prompt_appends(pkg, kv_heads, hd, rope_dim, tokens):
+    """Every key and value row behind a prompt, KV heads by ones, twos and fours with remainders: values are copied, keys rotated in 32 bits
+    and rounded once. Tokens of odd length, so that a warp group is partly empty."""
+    P, vocab, heads = pkg.plan, 256, kv_heads
+    rng = np.random.default_rng(kv_heads + tokens)
+    width = heads * hd
+    desc = pkg.BuffersDesc(hidden=width, slot_dim=width, vocab=vocab, max_seq=tokens + 8, max_batch=1, kv_layers=1, kv_heads=kv_heads, head_dim=hd)
+    store = pkg.WeightStore(0)
+    k, v = (rng.normal(size=(vocab, width)).astype(np.float32) for _ in range(2))
+    for name, rows in (("q", k), ("k", k), ("v", v)):
+        store.add_dense(name, _bf(pkg, rows))
+    store.add_q4_mlx("head", *pkg.synth_q4(vocab, width, seed=5, centered=True))
+    model = pkg.InferenceModel(store, [
+        P._step(P.STEP_EMBED, out_buf=P.BUF_S1, n=width, weight="q"), P._step(P.STEP_EMBED, out_buf=P.BUF_S2, n=width, weight="k"),
+        P._step(P.STEP_EMBED, out_buf=P.BUF_S3, n=width, weight="v"),
+        P._step(P.STEP_ATTN_DECODE, layer=0, in_buf=P.BUF_S1, in2_buf=P.BUF_S2, in3_buf=P.BUF_S3, out_buf=P.BUF_S0, heads=heads, kv_heads=kv_heads,
+                head_dim=hd, rope_dim=rope_dim, rope_base=10000.0, scale=hd ** -0.5),
+        P._step(P.STEP_QGEMV, in_buf=P.BUF_S0, out_buf=P.BUF_LOGITS, n=vocab, k=width, weight="head"), P._step(P.STEP_ARGMAX, in_buf=P.BUF_LOGITS, n=vocab)], desc)
+    chosen = rng.integers(0, vocab, size=tokens)
+    model.prefill_sequence(0, chosen)
+    half = rope_dim // 2
+    angle = np.arange(tokens)[:, None] * 10000.0 ** (-2.0 * np.arange(half) / max(rope_dim, 1))
+    c, s = np.cos(angle), np.sin(angle)
+    for h in range(kv_heads):
+        at = slice(h * hd, (h + 1) * hd)
+        assert np.array_equal(model.read_kv(1, 0, 0, h, tokens), _bf(pkg, v)[chosen, at])
+        row = pkg.bf16_to_f32(_bf(pkg, k))[chosen, at].astype(np.float64)
+        x, y = row[:, :half].copy(), row[:, half:rope_dim].copy()
+        row[:, :half], row[:, half:rope_dim] = x * c - y * s, x * s + y * c
+        got = pkg.bf16_to_f32(model.read_kv(0, 0, 0, h, tokens))
+        # one rounding to bf16 (2^-9 of the value), an angle of up to 1100 whose frequency is a 32-bit number (2^-24 of it, 2^-13 of a pair of up
+        # to 4 x 2^0.5)
+        assert (np.abs(got - row) <= 2.0 ** -8 * np.abs(row) + 2.0 ** -10).all()
+    model.close(), store.close()
+
+
 @pytest.mark.parametrize("heads,kv_heads,hd,tokens", [(32, 32, 64, 512), (32, 8, 128, 512), (32, 4, 128, 256), (32, 4, 64, 448), (16, 16, 128, 480)])
 def test_prompt_attention_repeats_itself(pkg, heads, kv_heads, hd, tokens):
     """Every token's attended values, a few hundred times over: the same bits each time, and those of the single steps up to rounding.
