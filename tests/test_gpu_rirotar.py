@@ -184,6 +184,23 @@ def test_keys_just_inside_and_just_outside_the_window(load, dtype, heads, dim, v
     assert (rc.row_errors(plain.forward(m.cfg, without, tokens)[0], want) > 2.5 * limit).mean() > 0.2
 
 
+@pytest.mark.parametrize("heads, dim, vdim, rank, window", [(4, 32, 24, 48, 40), (3, 24, 40, 72, 64), (2, 32, 32, 64, 100)])
+def test_portions_of_several_sequences_behind_older_rows(load, heads, dim, vdim, rank, window):
+    """Portions of three sequences in one batch, beside a decoding row: their older rows begin to be seen at unequal places (behind the
+    start, on it, inside a page) and lie among the new ones that the same launch appends."""
+    m = edge_model(load, "bfloat16", heads, dim, vdim, rank, window)
+    older, new = (150, 30, 97, 61), (70, 64, 33, 1)
+    tokens = [m.tokens(older[i] + new[i], seed=20 + i) for i in range(4)]
+    for i in range(4):
+        m.model.run_batch([(i, tokens[i][:older[i]], [])], logits=False)
+    order = (2, 0, 3, 1)
+    logits, _ = m.model.run_batch([(i, tokens[i][older[i]:], list(range(new[i]))) for i in order])
+    at = 0
+    for i in order:
+        assert rc.row_errors(logits[at:at + new[i]], m.plain(tokens[i])[older[i]:]).max() <= 3e-2, i
+        at += new[i]
+
+
 def far_write_weights(weights, eps):
     """Token 299 alone writes to the state, token 298 asks for what it wrote, and nothing is forgotten: q of 298 is k of 299
     (opposite embeddings, opposite projections), and a component that all embeddings share keeps everyone else's step size at
