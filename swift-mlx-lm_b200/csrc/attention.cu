@@ -470,7 +470,9 @@ __global__ void __launch_bounds__(kSplitThreads) attn_split_kernel(const typenam
 
     // Everything that does not depend on the split weights is requested first: the (max, sum) pairs and the
     // first 16 partial outputs of this thread's four dimensions travel together.
-    constexpr int kPre = STREAM ? 8 : 32;
+    // (a pair of MODE 4 has eight parts at most. With heads of 64 room for more costs the third CTA per SM; with heads of 128 room for eight
+    // only gives a loop that is 5 to 13 % slower in long caches: 41 x 5000 rows 160 us, with sixteen 143)
+    constexpr int kPre = !STREAM ? 32 : HD == 128 ? 16 : 8;
     const int n_out4 = G * HD / 4;  // float4 outputs of the group
     float* wsm = &osm[1][0][0];     // [G][splits] weights (splits <= 64: fits the reused buffer)
     float* msm2 = &osm[2][0][0];    // [G][splits] split maxima
@@ -1074,19 +1076,19 @@ constexpr int stream_ctas(int hd) { return hd == 64 ? 444 : 296; }
 constexpr int kStreamPairs = 100, kStreamRows = 512;
 static_assert(kStreamPairs * (kStreamRows / 64) >= stream_ctas(64) && 5 * kStreamPairs >= stream_ctas(64), "a block, a fifth of a pair");
 // Flash-decode over sequences of equal length: MODE 4 where the splits of all pairs leave a fifth of their rounds of the GPU empty (a quarter
-// with heads of 64) and that is worth more than what a CTA pays for the pairs it meets: five blocks of 64 rows per CTA, ten of heads of 64.
+// with heads of 64) and that is worth more than what a CTA pays for the pairs it meets: 5.5 blocks of 64 rows per CTA, ten of heads of 64.
 // Over 13 .. 200 sequences of 512 .. 5000 rows and 1 .. 32 KV heads that is never slower than splits by more than the runs differ. us with
-// splits / so; heads of 128: 13 sequences x 5000 rows x 8 KV heads (rounds 0.70 full) 58.6 / 52.4, 24 x 2048 (0.65) 47.5 / 40.9, 41 x 3000
-// (0.55) 125 / 90, 41 x 512 29.2 / 23.8; not worth it: 13 x 512 11.8 / 14.4, 24 x 600 18.2 / 18.6; too full: 32 x 5000 (0.86) 106 / 123.
-// Heads of 64: 20 x 1024 (0.36) 17.7 / 15.4, 20 x 5000 69 / 41, 41 x 5000 (0.74) 75.4 / 71.9; not worth it: 32 x 512 12.8 / 15.2, 41 x 1024
-// 20.7 / 22.0; too full: 13 x 512 x 32 KV heads (0.94) 13.5 / 16.8, 56 x 600 x 32 (0.81) 65.5 / 71.2. Decode steps, where each pair's start
+// splits / so; heads of 128: 13 sequences x 5000 rows x 8 KV heads (rounds 0.70 full) 58.6 / 53.4, 24 x 2048 (0.65) 47.4 / 42.6, 41 x 3000
+// (0.55) 125 / 89, 41 x 512 28.8 / 25.0; not worth it: 13 x 512 12.0 / 14.8, 24 x 600 18.2 / 19.2; too full: 32 x 5000 (0.86) 106 / 108.
+// Heads of 64: 20 x 1024 (0.36) 17.7 / 15.4, 20 x 5000 69 / 41, 41 x 5000 (0.74) 75 / 72; not worth it: 32 x 512 12.8 / 15.2, 41 x 1024
+// 20.6 / 21.9; too full: 13 x 512 x 32 KV heads (0.94) 12.8 / 17.1, 56 x 600 x 32 (0.81) 67.0 / 67.8. Decode steps, where each pair's start
 // is longer, lost in every batch (41 ragged sequences, 4 layers: 1053 / 1100 a step).
 bool attn_streams(int m, int kv_heads, int hd, int ctx_len) {
     const long long pairs = (long long)m * kv_heads, blocks = pairs * ((ctx_len + 63) / 64), ctas = pairs * attn_pick_splits(m, kv_heads, ctx_len);
     if (pairs < kStreamPairs || ctx_len < kStreamRows || blocks >= (1ll << 31)) return false;
     const int slots = stream_ctas(hd);
     const double full = (double)ctas / (double)((ctas + slots - 1) / slots * slots), saved = (double)blocks / slots * (1.0 / full - 1.0);
-    return hd == 64 ? full < 0.75 && saved >= 10.0 : full < 0.8 && saved >= 5.0;
+    return hd == 64 ? full < 0.75 && saved >= 10.0 : full < 0.8 && saved >= 5.5;
 }
 template <int MODE>
 int launch_both(const typename AttnArgs<MODE>::type& p, const dim3& grid, int hd, cudaStream_t s) {
