@@ -482,6 +482,33 @@ def test_flash_decode_op_long_context(pkg, store, B, ctx):
     assert err.max() <= RTOL
 
 
+@pytest.mark.parametrize("size", [1, 4097, 1 << 20, (5 << 20) + 3])
+def test_page_locked_memory_for_results(pkg, store, size):
+    """Blocks of any size: copies from the GPU reach every byte, also behind a fork whose child has seen the block and whose parent has
+    written to it since."""
+    import os
+    import torch
+    lib, block = store.lib, C.c_void_p()
+    lib.check(lib.swlm_host_alloc(size, C.byref(block)))
+    host = torch.frombuffer((C.c_char * size).from_address(block.value), dtype=torch.uint8)
+    torch.cuda.init()   # (torch knows of no page-locked memory before)
+    assert host.is_pinned()
+    for turn in range(3):
+        data = torch.randint(0, 256, (size,), device="cuda", dtype=torch.uint8)
+        host.copy_(data)
+        want = data.cpu()
+        assert torch.equal(host, want)
+        seen = want.numpy().tobytes()
+        child = os.fork()
+        if child == 0:
+            os._exit(0 if C.string_at(block.value, size) == seen else 1)
+        assert os.waitpid(child, 0)[1] == 0
+        C.memset(block.value, turn, size)
+    del host
+    lib.swlm_host_free(block)
+    assert lib.swlm_host_alloc(0, C.byref(block)) != 0
+
+
 # ---- recurrent (gated delta rule) step ---------------------------------------------------------------------
 
 @pytest.mark.parametrize("B,H,KV,D,ctx", [(13, 32, 8, 128, 1000), (41, 32, 8, 128, 519), (100, 8, 1, 64, 700), (25, 24, 8, 64, 2049), (19, 8, 8, 128, 512), (600, 4, 1, 128, 512)])
