@@ -28,8 +28,8 @@
 // 509 us, 10.7 TB/s), 512 arrivals per group, eight MMAs issued by a lone lane (470 to 850 clocks), and two waves of CTAs, the second
 // half empty. What bounds it now: the MMAs of the long form (about 0.7 of their rate under the power cap, one and a half waves of tiles at
 // 512 rows), dequantising in the short one. 17 to 64 rows have a kernel of their own (qgemm_slab_kernel).
-// Measured: 14336 x 4096 at 512 rows 88 -> 65 us, with results stored by rows, appended columns in blocks and a test in front of every
-// wait 57 (1050 TFLOP/s); 28672 x 4096 at 2048 rows 705 us under ncu -> 442 us with pairs of SMs.
+// Measured: 14336 x 4096 at 512 rows 88 -> 65 us, with results stored by rows and appended columns in blocks 57 (1050 TFLOP/s; a test in front
+// of every wait makes no difference to the forms here); 28672 x 4096 at 2048 rows 705 us under ncu -> 442 us with pairs of SMs.
 //
 // Every mbarrier wait is bounded: on expiry an error word is set, the CTA stops issuing, waits (bounded) for the copies and MMAs
 // it has in flight, frees its TMEM and returns.
@@ -715,16 +715,18 @@ __global__ void __maxnreg__(72) qgemm_tc_short_kernel(const QGemmTcParams p, con
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_d), "r"(kTmemCols) : "memory");
 }
 
-// ---- few activation rows (up to 64): a persistent CTA per SM, or a cluster of two along K ------------------------------------------
+// ---- few activation rows (up to 64): persistent CTAs, one on an SM, or clusters of two or four along K ------------------------------
 // What bounds it: the dequantising warps (about 330 instructions per 4096 weights; without the subtractions and multiplications a pass of
 // eight row tiles would take 0.45 us per step instead of 0.6), before that what surrounds them: in steps of 128 x 128 with a wait, a
 // fetch and an arrival for each, appended columns worked out three times, two CTAs on some SMs and one on others, 28672 x 4096 at 41 rows
-// took 34 us, 128256 x 4096 139, 4096 x 14336 25, 6144 x 4096 17.7. Now 28, 87, 23.5 and 12. Hence
+// took 34 us, 128256 x 4096 139; now 28 and 87. With their rows on the way to fp16, one call after the other: 14336 x 4096 23.9 -> 18.5,
+// 4096 x 14336 32 -> 24, 6144 x 4096 21.0 -> 14.7, 2048 x 2048 13.2 -> 9.8. (What the compiler spills lies outside the loop over units: 0.6 % of
+// the instructions.) Hence
 //   * a unit of work is 16 weight rows x 256 columns, the streaming layout's contiguous 2304 bytes: addresses by addition, one wait, one
 //     arrival and one set of scales for 16 words of nibbles per lane. A warp reads a unit into registers and requests the next but one in
 //     its place;
-//   * row tiles (16 rows) are dealt to the SMs one by one: passes of eight per SM over one contiguous window of the matrix, what is left
-//     evenly. Row tile j of a pass takes lanes 32 (j & 3) + 16 (j >> 2) of tensor memory, so that four already occupy all four schedulers
+//   * row tiles (16 rows) are dealt to the CTAs one by one: passes of eight each over one contiguous window of the matrix, what is left
+//     evenly (sl_ctas: as few CTAs as that takes). Row tile j of a pass takes lanes 32 (j & 3) + 16 (j >> 2) of tensor memory, so that four already occupy all four schedulers
 //     (a warp reaches the lanes of its quarter only); six warps per quarter, three steps of two row tiles;
 //   * two accumulators: four warps of their own store a pass while the next one is multiplied;
 //   * the wait for a step's activations is made by a dequantising warp, so that the MMA warp has one wait per step (16 MMAs at 30 clocks,
@@ -849,7 +851,7 @@ __global__ void __launch_bounds__(kSlThreads, 1) qgemm_slab_kernel(const QGemmTc
         // every copy has landed before the ring is given to the cluster, or the CTA leaves
         for (int i = issued > STAGES ? issued - STAGES : 0; i < issued; ++i) mbar_wait_warp(&bars.full[i % STAGES], (unsigned)((i / STAGES) & 1));
         __syncwarp();
-    } else if (warp < kSlWarps) {   // ---- dequantising warps: quarter warp & 3 of the lanes, number warp >> 2 of the quarter's four
+    } else if (warp < kSlWarps) {   // ---- dequantising warps: quarter warp & 3 of the lanes, number warp >> 2 of the quarter's six
         const int quarter = warp & 3, number = warp >> 2;
         const int tile_of = number / 3, first = number - 3 * tile_of;
         const unsigned ready0 = smem_u32(&bars.ready[0]), free0 = smem_u32(&bars.free[0]), full0 = smem_u32(&bars.full[0]);
